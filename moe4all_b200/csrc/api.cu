@@ -340,6 +340,7 @@ int32_t infr_cuda_set_codebook(infr_cuda_ctx* ctx, int32_t dtype, const void* ta
   if (e == cudaSuccess) e = publish_codebooks_dense(dev);
   if (e == cudaSuccess) e = publish_codebooks_anyfmt(dev);
   if (e == cudaSuccess) e = publish_codebooks_grouped(dev);
+  if (e == cudaSuccess) e = publish_codebooks_tmem(dev);
   if (e == cudaSuccess) ctx->codebook[slot] = dev[slot];
   return check_cuda(ctx, e, "set_codebook");
 }

@@ -103,60 +103,63 @@ __device__ __forceinline__ void block_scan2(int& a, int& b, int& ta, int& tb, in
   tb = s_ws[65];
 }
 
+// Rows per tile of a segment of cnt rows: as few tiles of at most `tn` rows as hold them, all about as large (multiples
+// of 16), so that no tile's weights are unpacked for a handful of left-over rows.
+__device__ __forceinline__ int tile_height(int cnt, int tn) {
+  if (cnt <= tn) return tn;
+  const int n = (cnt + tn - 1) / tn;
+  return ((cnt + n - 1) / n + 15) & ~15;
+}
+
 // Exclusive scan of the per-expert counts (thread e holds the count of segment e), the tile table
-// (one entry per `tn` rows of a segment, the shared expert's rows appended as segment n_expert) and
-// the segment offsets, by the 1024 threads of one CTA.  Offsets stay in s_off for the caller.
-// Tiles are listed heaviest first - the full tiles of all segments, then the segments' last, partial
-// tiles by falling row count - so that the GEMM kernels' last wave of CTAs is made of the light ones
-// (a tile's index only names its slot in the token and activation arrays).  tn is a power of two.
+// (the shared expert's rows appended as segment n_expert) and the segment offsets, by the 1024 threads
+// of one CTA.  Offsets stay in s_off for the caller.  Segments are listed by falling tile height, so
+// that the GEMM kernels' last round of jobs is made of the light ones.
 __device__ __forceinline__ void segment_tables(int cnt, int n_expert, int shared_rows, int tn, int* __restrict__ seg_off,
                                                int* __restrict__ tile_expert, int* __restrict__ tile_row0,
                                                int* __restrict__ tile_rows, int* __restrict__ n_tiles, int* s_cnt, int* s_off,
                                                int* s_toff, int* s_ws) {
   const int tid = threadIdx.x;
   const int n_seg = n_expert + (shared_rows > 0 ? 1 : 0);
-  int off = cnt, foff = cnt / tn, total = 0, total_f = 0;  // rows and full tiles ahead of this segment
-  block_scan2(off, foff, total, total_f, s_ws);
+  auto tiles_of = [&](int c) { const int h = tile_height(c, tn); return (c + h - 1) / h; };
+  int off = cnt, nt = tiles_of(cnt), total = 0, total_t = 0;  // rows ahead of this segment
+  block_scan2(off, nt, total, total_t, s_ws);
   if (tid < n_seg) {
     s_cnt[tid] = cnt;
     s_off[tid] = off;
-    s_toff[tid] = foff;
   }
-  // partial tiles: the count over the CTA; segment 1024 (only with 1024 experts and a shared segment) is added below
-  int n_part = __syncthreads_count(tid < n_seg && (cnt & (tn - 1)) != 0);
-  if (n_seg > 1024) {
+  if (n_seg > 1024) {  // segment 1024: only with 1024 experts and a shared segment
     if (tid == 0) {
       s_cnt[1024] = shared_rows;
       s_off[1024] = total;
-      s_toff[1024] = total_f;
     }
     total += shared_rows;
-    total_f += shared_rows / tn;
-    n_part += (shared_rows & (tn - 1)) != 0;
+    total_t += tiles_of(shared_rows);
   }
   if (tid == 0) {
     s_off[n_seg] = total;
-    *n_tiles = total_f + n_part;
+    *n_tiles = total_t;
     seg_off[n_expert + 1] = total;  // total grouped rows, with or without a shared segment
   }
   __syncthreads();
+  for (int e = tid; e < n_seg; e += 1024)  // (height, tiles) of every segment
+    s_toff[e] = (min(s_cnt[e], tile_height(s_cnt[e], tn)) << 20) | tiles_of(s_cnt[e]);
+  __syncthreads();
   for (int e = tid; e <= n_seg; e += 1024) seg_off[e] = s_off[e];
   for (int e = tid; e < n_seg; e += 1024) {
-    const int nf = s_cnt[e] / tn, part = s_cnt[e] & (tn - 1);
-    for (int t = 0; t < nf; ++t) {
-      tile_expert[s_toff[e] + t] = e;
-      tile_row0[s_toff[e] + t] = s_off[e] + t * tn;
-      tile_rows[s_toff[e] + t] = tn;
+    const int c = s_cnt[e], mine = s_toff[e] >> 20;
+    if (!c) continue;
+    int t = 0;  // tiles of the segments with higher tiles, or as high in an earlier segment
+#pragma unroll 8
+    for (int o = 0; o < n_seg; ++o) {
+      const int v = s_toff[o], h = v >> 20;
+      t += (h > mine || (h == mine && o < e)) ? (v & 0xFFFFF) : 0;
     }
-    if (part) {
-      int rank = 0;  // partial tiles with more rows, or as many in an earlier segment
-      for (int o = 0; o < n_seg; ++o) {
-        const int po = s_cnt[o] & (tn - 1);
-        rank += (po > part) || (po == part && o < e);
-      }
-      tile_expert[total_f + rank] = e;
-      tile_row0[total_f + rank] = s_off[e] + nf * tn;
-      tile_rows[total_f + rank] = part;
+    const int h = tile_height(c, tn);
+    for (int r = 0; r < c; r += h, ++t) {
+      tile_expert[t] = e;
+      tile_row0[t] = s_off[e] + r;
+      tile_rows[t] = min(h, c - r);
     }
   }
 }
@@ -279,44 +282,13 @@ __global__ void __launch_bounds__(256) k_gather_rows(const float* __restrict__ x
   }
 }
 
-// The same rows as operand tiles for the tcgen05 kernels: [tile][K step of 64][256 rows][128 B],
-// every 128-byte line already in the 128-byte-swizzled order of its shared-memory image (16-byte
-// chunk c of row n at chunk position c ^ (n & 7)), so that a CTA fetches a step's whole token
-// operand with one bulk copy.  One warp per row of a tile.
-__global__ void __launch_bounds__(256) k_gather_tiles(const float* __restrict__ x, const int* __restrict__ pair_of_pos,
-                                                      const float* __restrict__ row_w, const int* __restrict__ seg_off,
-                                                      int n_seg_routed, int n_used,
-                                                      const int* __restrict__ tile_row0, const int* __restrict__ tile_rows,
-                                                      const int* __restrict__ n_tiles, int tn, int ne,
-                                                      unsigned char* __restrict__ xt) {
-  const int tile = blockIdx.y;
-  if (tile >= *n_tiles) return;
-  const int n = blockIdx.x * 8 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (n >= tile_rows[tile]) return;
-  const int row = tile_row0[tile] + n;
-  const int n_sorted = seg_off[n_seg_routed];
-  int tok;
-  float w = 1.0f;  // weight_before: the pair's routing weight on the expert's input row
-  if (row < n_sorted) {
-    tok = pair_of_pos ? pair_of_pos[row] / n_used : row;
-    if (row_w != nullptr && pair_of_pos != nullptr) w = row_w[pair_of_pos[row]];
-  } else {
-    tok = row - n_sorted;  // shared-expert segment: token order
-  }
-  const float4* src = reinterpret_cast<const float4*>(x + (size_t)tok * ne);
-  const size_t step_bytes = (size_t)tn * 128;
-  unsigned char* line0 = xt + (size_t)tile * (ne / 64) * step_bytes + (size_t)n * 128;
-  for (int i = lane; i < ne / 4; i += 32) {
-    float4 v = __ldg(src + i);
-    v.x *= w; v.y *= w; v.z *= w; v.w *= w;
-    const __half2 h02 = __floats2half2_rn(v.x, v.z), h13 = __floats2half2_rn(v.y, v.w);  // K order 0,2,1,3
-    uint2 o;
-    o.x = *reinterpret_cast<const uint32_t*>(&h02);
-    o.y = *reinterpret_cast<const uint32_t*>(&h13);
-    const int step = i >> 4, chunk = (i & 15) >> 1;
-    *reinterpret_cast<uint2*>(line0 + (size_t)step * step_bytes + ((chunk ^ (n & 7)) << 4) + (i & 1) * 8) = o;
-  }
+// Token rows -> f16 where they are (the tcgen05 kernels gather rows themselves), eight elements per thread.
+__global__ void __launch_bounds__(256) k_rows_f16(const float* __restrict__ x, size_t n8, __half* __restrict__ xh) {
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n8) return;
+  const float4 a = __ldg(reinterpret_cast<const float4*>(x) + 2 * i), b = __ldg(reinterpret_cast<const float4*>(x) + 2 * i + 1);
+  const __half2 h[4] = {__floats2half2_rn(a.x, a.z), __floats2half2_rn(a.y, a.w), __floats2half2_rn(b.x, b.z), __floats2half2_rn(b.y, b.w)};
+  reinterpret_cast<uint4*>(xh)[i] = *reinterpret_cast<const uint4*>(h);
 }
 
 // ---- tensor-core tile helpers ----------------------------------------------------------------------
@@ -688,49 +660,71 @@ __global__ void __launch_bounds__(256) k_unpermute_combine(const float* __restri
   }
 }
 
-// The shared segment starts right after the routed rows: its address is only known on the device.
-template <bool Y16>
-__global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __restrict__ y, const float* __restrict__ y_scale,
-                                                               const int* __restrict__ pos_of_pair,
+// Four outputs packed by the tcgen05 down kernel, times 2^8 / (1 - 2^-13) of what they stand for (see YP_POSTSCALE).
+__device__ __forceinline__ float4 unpack_y4(uint2 v) {
+  const uint32_t e = v.y >> 24;
+  const uint32_t q[4] = {v.x, v.x >> 14, __funnelshift_r(v.x, v.y, 28), v.y >> 10};
+  if (e == 255u)  // an infinite or NaN output among them: the top bits of each
+    return make_float4(__uint_as_float(q[0] << 18), __uint_as_float(q[1] << 18), __uint_as_float(q[2] << 18), __uint_as_float(q[3] << 18));
+  const float sc = __uint_as_float((e - 12u) << 23);
+  float f[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[i] = (__uint_as_float(((q[i] & 0x3FFFu) ^ 0x2000u) | 0x4B000000u) - 8396800.0f) * sc;
+  return make_float4(f[0], f[1], f[2], f[3]);
+}
+constexpr float YP_POSTSCALE = W_POSTSCALE * (8192.0f / 8191.0f);
+
+// The shared segment starts right after the routed rows: its address is only known on the device.  A thread makes four
+// outputs of a token: four consecutive ones from f32 rows, four of every eighth (of 32) from packed rows.
+template <bool PACKED>
+__global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __restrict__ y, const int* __restrict__ pos_of_pair,
                                                                const float* __restrict__ wts, const float* __restrict__ sh_logit,
                                                                const int* __restrict__ seg_off, int n_seg_routed, int has_shared,
                                                                int rows, int n_used, int ne, const float* residual,
                                                                const int32_t* __restrict__ ids, const float* __restrict__ down_scale,
                                                                int weight_before, float* dst) {
-  const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
-  if (c >= ne) return;
-  // four outputs of row `pos` of y (f32 rows; or the tcgen05 down kernel's f16 rows with one scale per 32)
+  const int item = blockIdx.x * 256 + threadIdx.x;
+  if (item * 4 >= ne) return;
+  const int c = PACKED ? (item >> 3) * 32 + (item & 7) : item * 4;
   auto y4 = [&](size_t pos) {
-    if (!Y16) return *reinterpret_cast<const float4*>(y + pos * ne + c);
-    const uint2 h = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(y) + pos * ne + c);
-    const float sc = y_scale[pos * (ne / 32) + (c >> 5)];
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&h.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&h.y));
-    return make_float4(a.x * sc, a.y * sc, b.x * sc, b.y * sc);
+    if (!PACKED) return *reinterpret_cast<const float4*>(y + pos * ne + c);
+    return unpack_y4(__ldg(reinterpret_cast<const uint2*>(y) + pos * (ne / 4) + item));
   };
   for (int t = blockIdx.y; t < rows; t += gridDim.y) {  // the grid's y extent stops at 65535
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
     for (int s = 0; s < n_used; ++s) {
       const int pos = pos_of_pair[(size_t)t * n_used + s];
       if (pos < 0) continue;
-      const float w = weight_before ? 1.0f : wts[(size_t)t * n_used + s];
-      float4 v = y4((size_t)pos);
-      if (down_scale != nullptr) {  // y = raw * scale[e], then the weighted sum (Op::MoeFfn::down_scale)
-        // ids may be the caller's: same clamp as the bucketing, which also reported the bad id
-        const float sc = down_scale[min(max(ids[(size_t)t * n_used + s], 0), n_seg_routed - 1)];
-        v.x *= sc; v.y *= sc; v.z *= sc; v.w *= sc;
-      }
+      float w = weight_before ? 1.0f : wts[(size_t)t * n_used + s];
+      if (PACKED) w *= YP_POSTSCALE;
+      // y = raw * scale[e], then the weighted sum (Op::MoeFfn::down_scale); ids may be the caller's: same clamp as the
+      // bucketing, which also reported the bad id
+      if (down_scale != nullptr) w *= down_scale[min(max(ids[(size_t)t * n_used + s], 0), n_seg_routed - 1)];
+      const float4 v = y4((size_t)pos);
       o.x += w * v.x; o.y += w * v.y; o.z += w * v.z; o.w += w * v.w;
     }
     if (has_shared) {
-      const float gsh = sh_logit ? 1.0f / (1.0f + __expf(-sh_logit[t])) : 1.0f;
+      float gsh = sh_logit ? 1.0f / (1.0f + __expf(-sh_logit[t])) : 1.0f;
+      if (PACKED) gsh *= YP_POSTSCALE;
       const float4 v = y4((size_t)(seg_off[n_seg_routed] + t));
       o.x += gsh * v.x; o.y += gsh * v.y; o.z += gsh * v.z; o.w += gsh * v.w;
     }
-    if (residual != nullptr) {  // MoeFfn -> Add; may alias dst: each element is read, then written, by this thread
-      const float4 h = *reinterpret_cast<const float4*>(residual + (size_t)t * ne + c);
-      o.x += h.x; o.y += h.y; o.z += h.z; o.w += h.w;
+    // MoeFfn -> Add; may alias dst: each element is read, then written, by this thread
+    if (PACKED) {
+      float* d = dst + (size_t)t * ne + c;
+      if (residual != nullptr) {
+        const float* h = residual + (size_t)t * ne + c;
+        o.x += h[0]; o.y += h[8]; o.z += h[16]; o.w += h[24];
+      }
+      d[0] = o.x; d[8] = o.y; d[16] = o.z; d[24] = o.w;
+    } else {
+      if (residual != nullptr) {
+        const float4 h = *reinterpret_cast<const float4*>(residual + (size_t)t * ne + c);
+        o.x += h.x; o.y += h.y; o.z += h.z; o.w += h.w;
+      }
+      *reinterpret_cast<float4*>(dst + (size_t)t * ne + c) = o;
     }
-    *reinterpret_cast<float4*>(dst + (size_t)t * ne + c) = o;
   }
 }
 
@@ -746,18 +740,18 @@ __global__ void __launch_bounds__(1024) k_tiles_from_offsets(const int* __restri
     int toff = 0;
     for (int e = 0; e < n_seg; ++e) {
       s_toff[e] = toff;
-      toff += (s_so[e + 1] - s_so[e] + tn - 1) / tn;
+      const int cnt = s_so[e + 1] - s_so[e], h = tile_height(cnt, tn);
+      toff += (cnt + h - 1) / h;
     }
     *n_tiles = toff;
   }
   __syncthreads();
   for (int e = tid; e < n_seg; e += 1024) {
-    const int cnt = seg_off[e + 1] - seg_off[e];
-    const int nt = (cnt + tn - 1) / tn;
-    for (int t = 0; t < nt; ++t) {
+    const int cnt = s_so[e + 1] - s_so[e], h = tile_height(cnt, tn);
+    for (int t = 0; t * h < cnt; ++t) {
       tile_expert[s_toff[e] + t] = e;
-      tile_row0[s_toff[e] + t] = seg_off[e] + t * tn;
-      tile_rows[s_toff[e] + t] = min(tn, cnt - t * tn);
+      tile_row0[s_toff[e] + t] = s_so[e] + t * h;
+      tile_rows[s_toff[e] + t] = min(h, cnt - t * h);
     }
   }
 }
@@ -770,11 +764,8 @@ size_t grouped_scratch_bytes(int rows_total, int n_pairs, int n_seg, int ne, int
   b += align_up((size_t)(n_seg + 2) * 4, 256) * 3;                 // counts, seg_off, fill
   b += align_up((size_t)(rows_total / TN + n_seg + 2) * 4, 256) * 3 + 256;  // tile table + n_tiles
   b += align_up((size_t)(n_pairs + 1) * 4, 256) * 2;               // pos_of_pair, pair_of_pos
-  // token arrays: rows grouped by expert (legacy tiles) or padded to whole 256-row tiles (tcgen05)
-  const size_t tile_rows_pad = ((size_t)rows_total / 256 + n_seg + 1) * 256;
-  const size_t tok_rows = tile_rows_pad > rows_pad ? tile_rows_pad : rows_pad;
-  b += align_up(tok_rows * ne * 2, 256);                           // xg
-  b += align_up(tok_rows * nff * 2, 256);                          // act
+  b += align_up(rows_pad * ne * 2, 256);                           // xg
+  b += align_up(rows_pad * nff * 2, 256);                          // act
   b += align_up(rows_pad * ne * 4, 256);                           // y
   return b;
 }
@@ -792,10 +783,10 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
   const int n_seg = c.n_expert + (c.shared_rows > 0 ? 1 : 0);
   const int rows_total = c.rows_bound;  // upper bound on sorted rows + shared rows
   const bool tuned = BankTypes{c.gate_dt, c.up_dt, c.down_dt}.tuned();
-  const bool use_umma = tuned && !c.legacy && umma_grouped_supported(c.ne, c.nff);
-  if (tuned && c.down_q4k && !use_umma)
+  const bool use_wt = !c.legacy && c.ne % 256 == 0 && c.nff % 256 == 0;
+  if (tuned && c.down_q4k && !use_wt)
     return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "grouped GEMM: Q4_K down banks need the tcgen05 tiles (ne, n_ff_exp multiples of 256, not path 3)");
-  const int tn = use_umma ? umma_tile_rows() : TN;
+  const int tn = use_wt ? wt_tile_rows() : TN;
   const int max_tiles = rows_total / tn + n_seg + 1;
   const int max_tiles_alloc = rows_total / TN + n_seg + 1;
   int* counts = reinterpret_cast<int*>(take((size_t)(n_seg + 2) * 4));
@@ -807,8 +798,7 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
   int* n_tiles = reinterpret_cast<int*>(take(256));
   int* pos_of_pair = reinterpret_cast<int*>(take((size_t)(c.n_pairs + 1) * 4));
   int* pair_of_pos = reinterpret_cast<int*>(take((size_t)(c.n_pairs + 1) * 4));
-  const size_t tile_rows_pad = ((size_t)rows_total / 256 + n_seg + 1) * 256;
-  const size_t tok_rows = std::max(tile_rows_pad, (size_t)rows_total + 256);
+  const size_t tok_rows = (size_t)rows_total + 256;
   __half* xg = reinterpret_cast<__half*>(take(tok_rows * c.ne * 2));
   __half* act = reinterpret_cast<__half*>(take(tok_rows * c.nff * 2));
   float* y = c.y_out ? c.y_out : reinterpret_cast<float*>(take(((size_t)rows_total + 256) * c.ne * 4));
@@ -830,9 +820,8 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
                                                                pos_of_pair, pair_of_pos);
       ctx->launches += 3;
     }
-    if (use_umma)
-      k_gather_tiles<<<dim3(tn / 8, max_tiles), 256, 0, st>>>(c.x, pair_of_pos, row_w, seg_off, n_seg_routed, c.n_used, tile_row0, tile_rows,
-                                                             n_tiles, tn, c.ne, reinterpret_cast<unsigned char*>(xg));
+    if (use_wt && !row_w)
+      k_rows_f16<<<(unsigned)(((size_t)c.rows * c.ne / 8 + 255) / 256), 256, 0, st>>>(c.x, (size_t)c.rows * c.ne / 8, xg);
     else
       k_gather_rows<<<(rows_total + 7) / 8, 256, 0, st>>>(c.x, pair_of_pos, row_w, seg_off, n_seg_routed, c.n_used, rows_total, c.ne, xg);
     ctx->launches += 1;
@@ -844,11 +833,7 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
     cudaError_t e = cudaMemcpyAsync(seg_off, c.seg_off_in + c.n_expert, 4, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(seg_off + 1, c.seg_off_in + c.n_expert, 4, cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) return check_cuda(ctx, e, "grouped: offsets copy");
-    if (use_umma)
-      k_gather_tiles<<<dim3(tn / 8, max_tiles), 256, 0, st>>>(c.x, nullptr, nullptr, seg_off, 0, 1, tile_row0, tile_rows, n_tiles, tn, c.ne,
-                                                             reinterpret_cast<unsigned char*>(xg));
-    else
-      k_gather_rows<<<(rows_total + 7) / 8, 256, 0, st>>>(c.x, nullptr, nullptr, seg_off, 0, 1, rows_total, c.ne, xg);
+    k_gather_rows<<<(rows_total + 7) / 8, 256, 0, st>>>(c.x, nullptr, nullptr, seg_off, 0, 1, rows_total, c.ne, xg);
     ctx->launches += 2;
   }
 
@@ -872,22 +857,23 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
   p.ne = c.ne;
   p.nff = c.nff;
   p.n_expert = c.n_expert;
-  p.down_q4k = c.down_q4k;
-  // tcgen05 tiles with the combine behind them: the raw rows cross memory as f16 (half the bytes out of the
-  // down kernel and into the combine); rows handed to the caller stay f32
-  p.y_f16 = (use_umma && c.dst != nullptr && c.y_out == nullptr && c.ne % 32 == 0 && !ctx->cfg.raw_rows_f32) ? 1 : 0;
-  p.y_scale = reinterpret_cast<float*>(reinterpret_cast<char*>(y) + ((size_t)rows_total + 256) * c.ne * 2);  // behind the f16 rows
+  // tcgen05 tiles with the combine behind them: the raw rows cross memory packed (half the bytes out of the down kernel
+  // and into the combine) for the Q4_K / Q6_K banks; rows handed to the caller stay f32
+  p.y_packed = (use_wt && tuned && c.dst != nullptr && c.y_out == nullptr && !ctx->cfg.raw_rows_f32) ? 1 : 0;
   p.gate_dt = c.gate_dt;
   p.up_dt = c.up_dt;
   p.down_dt = c.down_dt;
   p.act_kind = c.act_kind;
-  p.gu_rows = (int)(c.gate_stride / ((size_t)c.ne / 256 * Q4K_BLOCK_BYTES));
+  p.gu_rows = (int)(c.gate_stride / row_bytes(c.gate_dt, c.ne));
   p.clamp = c.clamp;
   p.status = ctx->status;
-  p.trace = ctx->trace;
-  p.trace_tile = (int)ctx->cfg.trace_tile;
-  if (use_umma) {
-    const int32_t rc = launch_umma_grouped(ctx, p, max_tiles);
+  if (use_wt) {
+    WtTokens t = {};
+    t.pair_of_pos = (c.ids && !row_w) ? pair_of_pos : nullptr;
+    t.seg_off = seg_off;
+    t.n_seg_routed = c.ids ? n_seg_routed : 0;
+    t.n_used = c.n_used;
+    const int32_t rc = launch_wt_grouped(ctx, p, t, max_tiles);
     if (rc) return rc;
   } else if (!tuned) {
     // banks in another format mix: the same tiles, weights unpacked through the generic code view
@@ -901,8 +887,8 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
     ctx->launches += 2;
   }
   if (c.dst) {
-    auto comb = p.y_f16 ? k_unpermute_combine_seg<true> : k_unpermute_combine_seg<false>;
-    comb<<<dim3((c.ne / 4 + 255) / 256, std::min(c.rows, 65535)), 256, 0, st>>>(y, p.y_scale, pos_of_pair, c.wts, c.sh_logit, seg_off, n_seg_routed,
+    auto comb = p.y_packed ? k_unpermute_combine_seg<true> : k_unpermute_combine_seg<false>;
+    comb<<<dim3((c.ne / 4 + 255) / 256, std::min(c.rows, 65535)), 256, 0, st>>>(y, pos_of_pair, c.wts, c.sh_logit, seg_off, n_seg_routed,
                                                                                  c.shared_rows > 0 ? 1 : 0, c.rows, c.n_used, c.ne, c.residual, c.ids, c.down_scale,
                                                                                  c.weight_before, c.dst);
     ctx->launches += 1;

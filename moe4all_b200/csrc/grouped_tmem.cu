@@ -1,0 +1,832 @@
+// Grouped expert GEMMs on the 5th-generation tensor cores with the unpacked weights in tensor memory.
+//
+// Same contract as the mma.sync kernels of grouped_ffn.cu (reference: CPU stages B-D
+// crates/infr-cpu/src/lib.rs:4051-4266; Vulkan native_gemm_mmq_q4k/q6k.comp): per expert segment
+//   act = silu(Wg x) * (Wu x)      (MODE 0, k_wt_gemm<0, ...>)
+//   y   = Wd act                   (MODE 1, k_wt_gemm<1, ...>)
+//
+// What bounds such a GEMM is the unpacking: every tile has to turn its blocks into f16 operands, whatever the number
+// of tokens behind them, and the operand then crosses shared memory twice (written by the producers, read by the
+// MMAs).  So the weights are the A operand and A lives in tensor memory: a producer thread owns one weight row, unpacks
+// 64 of its weights into 32 registers and stores them with one tcgen05.st into its lane - no swizzle, no shared-memory
+// traffic, no proxy fence.  The tokens are the B operand (N = the tile's tokens rounded up to 16, at most 160), so the
+// tensor-core time of a tile is proportional to its tokens.  Tensor memory: two accumulators of 160 columns (gate and
+// up rows, or the two halves of 256 output features) and three A stages of 64 columns (64 K elements of 256 rows).
+//
+// One persistent CTA per SM walks the jobs (tile, 256 weight rows), tiles listed heaviest first and dealt out in a
+// snake.  Warp roles (24 warps):
+//   0-15   producers, two groups of eight on alternate K steps; afterwards they drain the accumulators
+//   16     issues the MMAs (one elected lane)
+//   then   token loaders: gate/up - four warps bring rows of the f16 token matrix straight from where the tokens are
+//          (cp.async), two of them per K step; down - one warp, one bulk copy per K step of the tile's activations
+//   last   raw-block loaders: 256 weights of 256 rows at a time, into a ring: Q4_K, Q5_K and Q8_0 by tiled copies, formats
+//          whose rows of 256 weights are not whole 16-byte pieces word by word with cp.async (rows on an odd word pitch,
+//          free of bank conflicts)
+// All rings run on across jobs; every wait is bounded.
+#include <cuda.h>
+
+#include <algorithm>
+
+#include "formats.cuh"
+#include "kernels.cuh"
+#include "umma.cuh"
+#include "tma.cuh"
+
+namespace infr {
+namespace {
+
+constexpr int WN = 160;              // most tokens of a tile
+constexpr int WR = 256;              // weight rows of a job
+constexpr int W_PRODUCERS = 512;
+constexpr int W_THREADS = 768;
+constexpr int W_MMA_WARP = 16, W_TOK_WARP = 17;
+__host__ __device__ constexpr int wt_tok_warps(int mode) { return mode == 0 ? 4 : 1; }
+__host__ __device__ constexpr int wt_raw_warp(int mode) { return W_TOK_WARP + wt_tok_warps(mode); }
+__host__ __device__ constexpr int wt_raw_warps(int mode) { return mode == 0 ? 3 : 4; }
+constexpr uint32_t W_B_STAGE = WN * 128;       // 64 K elements of the tile's tokens
+constexpr uint32_t W_PATCH = 1280;             // per warp: 16 rows x 80 B (f16) or 8 rows x 144 B (f32)
+constexpr int W_MAX_RING = 4;
+constexpr int W_A_STAGES = 3;
+constexpr uint32_t W_A_COL = 2 * WN;           // first A column of tensor memory
+constexpr float W_PRESCALE = 256.0f;           // keeps block scales out of the f16 subnormals
+constexpr float W_POSTSCALE = 1.0f / 256.0f;
+
+__device__ __forceinline__ uint32_t h2_as_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
+__device__ __forceinline__ __half2 u32_as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
+__device__ __forceinline__ __half2 h2_const(uint32_t bits) { return u32_as_h2(bits | (bits << 16)); }
+
+// ---- tensor-memory and copy forms only this file uses ------------------------------------------------
+
+// 32 registers of every lane -> 32 consecutive columns of the lane's row (warp w: lanes 32 (w % 4) ..).
+__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n\t"
+      "tcgen05.wait::st.sync.aligned;"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
+        "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
+        "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+
+// 16 accumulator rows (lanes) x 16 columns at each of four addresses as 8x8 fragments: thread T holds of row T / 4 (v[0],
+// v[1]) and row T / 4 + 8 (v[2], v[3]) the columns 2 (T % 4), + 1; v[4..7] the same of the columns 8 further on.
+__device__ __forceinline__ void tmem_ld_16x16_quad(uint32_t ta, uint32_t tb, uint32_t tc, uint32_t td, float (&a)[8], float (&b)[8], float (&c)[8],
+                                                   float (&d)[8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%33];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%34];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%24,%25,%26,%27,%28,%29,%30,%31}, [%35];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]), "=f"(a[7]), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]),
+        "=f"(b[3]), "=f"(b[4]), "=f"(b[5]), "=f"(b[6]), "=f"(b[7]), "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]), "=f"(c[4]), "=f"(c[5]),
+        "=f"(c[6]), "=f"(c[7]), "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]), "=f"(d[4]), "=f"(d[5]), "=f"(d[6]), "=f"(d[7])
+      : "r"(ta), "r"(tb), "r"(tc), "r"(td)
+      : "memory");
+}
+
+// D[tmem] (+)= A[tmem] * B[smem]^T for one K = 16 slice; A: lane = row, a 32-bit column = two K elements.
+__device__ __forceinline__ void mma_f16_ta(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(acc)
+      : "memory");
+}
+
+// One lane of a converged warp.  Branching on this (and not on a lane number), in a branch the compiler knows to be
+// warp-uniform, keeps the MMA operands in uniform registers: 9 cycles per tcgen05.mma against 55 from `if (lane == 0)`.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+// One arrival on `bar` once all copies this thread has issued so far are there.
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// Bounded wait of these kernels: a look, then waits that the hardware suspends (spinning warps took a third of the issue
+// slots from the producers).  The limit is a few seconds.
+__device__ __forceinline__ bool wt_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  if (ok) return true;
+  for (uint32_t i = 0; i < (1u << 21); ++i) {
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(1000u) : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+// ---- unpacking: 64 weights of a row -> 32 columns, K order 0,2,1,3 inside every four ---------------------
+//
+// Codes become f16 by setting the exponent bits of 1024 (or 64 for codes that sit four bits up) above them, the
+// offset comes off exactly, and scale and min are applied by one multiply-add.
+
+// Scales of two groups, given as bytes 0 and 1 of `pair` (at most 63): d * code, both rounded once.
+__device__ __forceinline__ __half2 scale_pair(uint32_t pair, __half2 d) {
+  return __hmul2(__hsub2(u32_as_h2(__byte_perm(pair, 0x64u, 0x4140)), h2_const(0x6400u)), d);
+}
+
+// Step j of a Q4_K block; the row starts on a 16-byte boundary.
+__device__ __forceinline__ void unpack_q4k(const unsigned char* row, int j, uint32_t (&o)[32]) {
+  const uint4 hd = *reinterpret_cast<const uint4*>(row);
+  const uint4 qa = *reinterpret_cast<const uint4*>(row + 16 + 32 * j), qb = *reinterpret_cast<const uint4*>(row + 32 + 32 * j);
+  uint32_t scp, mp;
+  q4k_scale_min_pair(hd.y, hd.z, hd.w, j, scp, mp);
+  const __half2 dd = __hmul2(u32_as_h2(hd.x ^ 0x80000000u), h2_const(0x5C00u));  // 256 (d, -dmin)
+  const __half2 s2 = scale_pair(scp, __low2half2(dd)), m2 = scale_pair(mp, __high2half2(dd));
+  const __half2 sl = __low2half2(s2), sh = __high2half2(s2), ml = __low2half2(m2), mh = __high2half2(m2);
+  const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t v = w[i] >> 8;
+    const __half2 l02 = __hsub2(u32_as_h2((w[i] & 0x000F000Fu) | 0x64006400u), h2_const(0x6400u));
+    const __half2 l13 = __hsub2(u32_as_h2((v & 0x000F000Fu) | 0x64006400u), h2_const(0x6400u));
+    const __half2 h02 = __hsub2(u32_as_h2((w[i] & 0x00F000F0u) | 0x54005400u), h2_const(0x5400u));
+    const __half2 h13 = __hsub2(u32_as_h2((v & 0x00F000F0u) | 0x54005400u), h2_const(0x5400u));
+    o[2 * i] = h2_as_u32(__hfma2(l02, sl, ml));
+    o[2 * i + 1] = h2_as_u32(__hfma2(l13, sl, ml));
+    o[16 + 2 * i] = h2_as_u32(__hfma2(h02, sh, mh));
+    o[16 + 2 * i + 1] = h2_as_u32(__hfma2(h13, sh, mh));
+  }
+}
+
+// Four codes (bytes) with one scale: code - off exactly, times s.
+template <uint32_t OFF>  // f16 bits of 1024 + off
+__device__ __forceinline__ void codes4_mul(uint32_t c, __half2 s, uint32_t& o02, uint32_t& o13) {
+  o02 = h2_as_u32(__hmul2(__hsub2(u32_as_h2((c & 0x00FF00FFu) | 0x64006400u), h2_const(OFF)), s));
+  o13 = h2_as_u32(__hmul2(__hsub2(u32_as_h2(((c >> 8) & 0x00FF00FFu) | 0x64006400u), h2_const(OFF)), s));
+}
+
+// Two int8 scales (bytes of `w` picked by the selector) times d: exact integers in f16, one rounding.
+__device__ __forceinline__ __half2 i8_scale_pair(uint32_t w, uint32_t sel, __half2 d) {
+  return __hmul2(__hsub2(u32_as_h2(__byte_perm(w ^ 0x80808080u, 0x64u, sel)), h2_const(0x6480u)), d);
+}
+
+// Step 2 h + g of a Q6_K block; the block starts `mis` (0 or 16) bits into the first word of `row`.
+__device__ __forceinline__ void unpack_q6k(const uint32_t* row, int mis, int h, int g, uint32_t (&o)[32]) {
+  auto word = [&](int i) { return __funnelshift_r(row[i], row[i + 1], mis); };
+  const uint32_t sc = word(48 + 2 * h + g);  // scales of the step's four groups of 16
+  const __half2 d = __hmul2(u32_as_h2(__byte_perm(row[52] >> mis, 0u, 0x1010)), h2_const(0x5C00u));  // f16 d: bytes 208, 209
+  const __half2 s01 = i8_scale_pair(sc, 0x4140, d), s23 = i8_scale_pair(sc, 0x4342, d);
+  uint32_t hq[8];
+  {
+    uint32_t a = row[32 + 8 * h];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t b = row[33 + 8 * h + i];
+      hq[i] = __funnelshift_r(a, b, mis);
+      a = b;
+    }
+  }
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    const int rot = (4 - 4 * g - 2 * part) & 31;  // brings bits 2 qd, 2 qd + 1 of a byte to its bits 4, 5
+    const __half2 s_a = __low2half2(part ? s23 : s01), s_b = __high2half2(part ? s23 : s01);
+    uint32_t a = row[16 * h + 8 * part];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t b = row[16 * h + 8 * part + 1 + i];
+      const uint32_t L = __funnelshift_r(a, b, mis + 4 * g), H = __funnelshift_l(hq[i], hq[i], rot);
+      a = b;
+      const uint32_t c = (H & 0x30303030u) | (L & 0x0F0F0F0Fu);
+      const uint32_t c02 = __byte_perm(c, 0x64u, 0x4240), c13 = __byte_perm(c, 0x64u, 0x4341);
+      const __half2 s = i < 4 ? s_a : s_b;
+      o[16 * part + 2 * i] = h2_as_u32(__hmul2(__hsub2(u32_as_h2(c02), h2_const(0x6420u)), s));
+      o[16 * part + 2 * i + 1] = h2_as_u32(__hmul2(__hsub2(u32_as_h2(c13), h2_const(0x6420u)), s));
+    }
+  }
+}
+
+// A step of eight Q8_0 blocks: 68 bytes = two blocks, the first on a word boundary, the second two bytes past one.
+// w(i): word i of the step.
+template <typename Word>
+__device__ __forceinline__ void unpack_q80(Word w, uint32_t (&o)[32]) {
+  const uint32_t mid = w(8);
+  const __half2 d = __hmul2(u32_as_h2(__byte_perm(w(0), mid, 0x7610)), h2_const(0x5C00u));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) codes4_mul<0x6480u>(__funnelshift_r(w(i), w(i + 1), 16) ^ 0x80808080u, __low2half2(d), o[2 * i], o[2 * i + 1]);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) codes4_mul<0x6480u>(w(9 + i) ^ 0x80808080u, __high2half2(d), o[16 + 2 * i], o[16 + 2 * i + 1]);
+}
+// The row on a 16-byte boundary: the words of step J are words J .. J + 16 of five 16-byte pieces.
+template <int J>
+__device__ __forceinline__ void unpack_q80_row(const unsigned char* row, uint32_t (&o)[32]) {
+  uint32_t v[20];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const uint4 x = *reinterpret_cast<const uint4*>(row + 64 * J + 16 * i);
+    v[4 * i] = x.x, v[4 * i + 1] = x.y, v[4 * i + 2] = x.z, v[4 * i + 3] = x.w;
+  }
+  unpack_q80([&](int i) { return v[J + i]; }, o);
+}
+
+// Step j of a Q5_K (FIVE) or Q4_K block.  hd, qh: the block's first 16 bytes and its high bits; qs(i): code word i of the step.
+template <bool FIVE, typename Word>
+__device__ __forceinline__ void unpack_k45(const uint4& hd, const uint32_t (&qh)[8], Word qs, int j, uint32_t (&o)[32]) {
+  uint32_t scp, mp;
+  q4k_scale_min_pair(hd.y, hd.z, hd.w, j, scp, mp);
+  const __half2 dd = __hmul2(u32_as_h2(hd.x ^ 0x80000000u), h2_const(0x5C00u));
+  const __half2 s2 = scale_pair(scp, __low2half2(dd)), m2 = scale_pair(mp, __high2half2(dd));
+  const __half2 sl = __low2half2(s2), sh = __high2half2(s2), ml = __low2half2(m2), mh = __high2half2(m2);
+  const int rl = (4 - 2 * j) & 31, rh = (3 - 2 * j) & 31;  // brings bit 2 j (2 j + 1) of a byte to its bit 4
+  constexpr uint32_t B4 = FIVE ? 0x00100010u : 0u;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t w = qs(i), q = FIVE ? qh[i] : 0u;
+    const uint32_t bl = __funnelshift_l(q, q, rl), bh = __funnelshift_l(q, q, rh), wh = w >> 4;
+    const uint32_t l02 = (bl & B4) | ((w & 0x000F000Fu) | 0x64006400u), l13 = ((bl >> 8) & B4) | (((w >> 8) & 0x000F000Fu) | 0x64006400u);
+    const uint32_t h02 = (bh & B4) | ((wh & 0x000F000Fu) | 0x64006400u), h13 = ((bh >> 8) & B4) | (((wh >> 8) & 0x000F000Fu) | 0x64006400u);
+    o[2 * i] = h2_as_u32(__hfma2(__hsub2(u32_as_h2(l02), h2_const(0x6400u)), sl, ml));
+    o[2 * i + 1] = h2_as_u32(__hfma2(__hsub2(u32_as_h2(l13), h2_const(0x6400u)), sl, ml));
+    o[16 + 2 * i] = h2_as_u32(__hfma2(__hsub2(u32_as_h2(h02), h2_const(0x6400u)), sh, mh));
+    o[16 + 2 * i + 1] = h2_as_u32(__hfma2(__hsub2(u32_as_h2(h13), h2_const(0x6400u)), sh, mh));
+  }
+}
+// Word by word (any word boundary), and in 16-byte pieces.
+template <bool FIVE>
+__device__ __forceinline__ void unpack_k45_words(const uint32_t* row, int j, uint32_t (&o)[32]) {
+  uint32_t qh[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) qh[i] = FIVE ? row[4 + i] : 0u;
+  unpack_k45<FIVE>(make_uint4(row[0], row[1], row[2], row[3]), qh, [&](int i) { return row[(FIVE ? 12 : 4) + 8 * j + i]; }, j, o);
+}
+__device__ __forceinline__ void unpack_q5k_row(const unsigned char* row, int j, uint32_t (&o)[32]) {
+  const uint4 ha = *reinterpret_cast<const uint4*>(row + 16), hb = *reinterpret_cast<const uint4*>(row + 32);
+  const uint4 qa = *reinterpret_cast<const uint4*>(row + 48 + 32 * j), qb = *reinterpret_cast<const uint4*>(row + 64 + 32 * j);
+  const uint32_t qh[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w}, q[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+  unpack_k45<true>(*reinterpret_cast<const uint4*>(row), qh, [&](int i) { return q[i]; }, j, o);
+}
+
+// Step j of 256 weights in any format, through the code view (`row`: a copy in shared memory, words aligned as in the bank).
+__device__ __forceinline__ void unpack_codes(int dt, const unsigned char* row, int j, uint32_t (&o)[32]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t c[4];
+    float A, B;
+    int off;
+    fmt_codes16<false>(dt, row, 4 * j + q, c, A, B, off);
+    const __half2 a2 = __float2half2_rn(A * W_PRESCALE), b2 = __float2half2_rn(B * W_PRESCALE), o2 = __float2half2_rn((float)(1024 + off));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __half2 v02 = __hsub2(u32_as_h2((c[i] & 0x00FF00FFu) | 0x64006400u), o2), v13 = __hsub2(u32_as_h2(((c[i] >> 8) & 0x00FF00FFu) | 0x64006400u), o2);
+      o[8 * q + 2 * i] = h2_as_u32(__hfma2(v02, a2, b2));
+      o[8 * q + 2 * i + 1] = h2_as_u32(__hfma2(v13, a2, b2));
+    }
+  }
+}
+
+// ---- results ------------------------------------------------------------------------------------------
+
+// Two f32 as f16, saturated to the largest finite value.
+__device__ __forceinline__ uint32_t f16x2_sat(float a, float b) {
+  uint32_t r;
+  asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
+
+__device__ __forceinline__ float exp2_approx(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Out of line: the activations other than SiLU, and the clamp.
+__device__ __noinline__ float gated_act_general(int act, float clamp, float g, float u) { return gated_act<true>(act, clamp, g, u); }
+
+// Four outputs of the down kernel as 64 bits: a shared exponent (bits 56-63) and four 14-bit two's-complement
+// mantissas, the largest magnitude in [2^12, 2^13) (half a unit is at most 2^-13 of it, f16 would be at most 2^-12 of
+// each).  Exponent 255 - an infinite or NaN output among the four - takes the top 14 bits of each f32 instead.
+__device__ __forceinline__ uint2 pack_y4(float a, float b, float c, float d) {
+  float m;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(m), "f"(d), "f"(d));
+  const uint32_t e = max(__float_as_uint(m) & 0x7F800000u, 13u << 23);
+  uint32_t q[4];
+  if (e < (255u << 23)) {
+    // 2^(12 - exponent), a hair less so that the largest mantissa is 8191; adding 1.5 * 2^23 leaves the integer in the low bits
+    const float inv = __uint_as_float((266u << 23) - e - 2048u);
+    q[0] = __float_as_uint(fmaf(a, inv, 12582912.0f)), q[1] = __float_as_uint(fmaf(b, inv, 12582912.0f));
+    q[2] = __float_as_uint(fmaf(c, inv, 12582912.0f)), q[3] = __float_as_uint(fmaf(d, inv, 12582912.0f));
+  } else {
+    q[0] = __float_as_uint(a) >> 18, q[1] = __float_as_uint(b) >> 18, q[2] = __float_as_uint(c) >> 18, q[3] = __float_as_uint(d) >> 18;
+  }
+  return make_uint2((q[0] & 0x3FFFu) | ((q[1] & 0x3FFFu) << 14) | (q[2] << 28), ((q[2] >> 4) & 0x3FFu) | ((q[3] & 0x3FFFu) << 10) | (e << 1));
+}
+
+// ---- the kernel ---------------------------------------------------------------------------------------
+
+// Q4_K, Q5_K, Q8_0 (both roles): tiled copies, rows of whole 16-byte pieces; Q6_K, any: words, on an odd word pitch.
+enum WtFormat { WT_Q4K, WT_Q5K, WT_Q80, WT_Q6K, WT_ANY };
+__host__ __device__ constexpr bool wt_tiled(int fmt) { return fmt <= WT_Q80; }
+
+struct WtBars {
+  uint64_t full_a[W_A_STAGES], empty_a[W_A_STAGES];      // A stages in tensor memory
+  uint64_t full_b[W_MAX_RING], empty_b[W_MAX_RING];      // token stages
+  uint64_t full_raw[W_MAX_RING], empty_raw[W_MAX_RING];  // raw-block stages
+  uint64_t done, drained;                                // accumulators complete / read
+};
+
+// Position in a ring of n stages, running on across jobs.
+struct RingPos {
+  int s = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next(int n) {
+    if (++s == n) {
+      s = 0;
+      phase ^= 1;
+    }
+  }
+};
+
+struct WtParams {
+  GroupedParams g;
+  int n_blk;        // jobs per tile
+  int k_blocks;     // 256-element blocks along K
+  int rb, sb;       // stages of the raw and the token ring
+  uint32_t raw_pitch, raw_stage;  // bytes per row and per stage
+  // gate/up tokens: row of the token matrix behind grouped row `pos`
+  const int* pair_of_pos;   // null: the rows are grouped already
+  const int* seg_off;       // [n_seg_routed] = grouped rows ahead of the shared expert's
+  int n_seg_routed, n_used;
+};
+
+// Job i of this CTA: rounds of gridDim.x jobs, every other round dealt out backwards (the tiles' cost falls along the list).
+__device__ __forceinline__ int wt_job(int i) {
+  return i * (int)gridDim.x + ((i & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+}
+
+// Lane of an operand tile -> weight row: gate/up rows go in the order 0,2,1,3 inside every four, so that the
+// activations come out in the K order of the down kernel's operands.
+__device__ __forceinline__ int wt_row_of_lane(int mode, int l) { return mode == 0 ? ((l & ~3) | ((l & 1) << 1) | ((l >> 1) & 1)) : l; }
+
+template <int MODE, int FMT>
+__global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant__ WtParams w, const __grid_constant__ CUtensorMap tm_w0,
+                                                         const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__ CUtensorMap tm_s0,
+                                                         const __grid_constant__ CUtensorMap tm_s1) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) WtBars bars;
+  __shared__ uint32_t s_tmem;
+  constexpr int RAW_WARP = wt_raw_warp(MODE), RAW_WARPS = wt_raw_warps(MODE);
+  const GroupedParams& p = w.g;
+  unsigned char* b_ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  unsigned char* raw_ring = b_ring + (size_t)w.sb * W_B_STAGE;
+  unsigned char* patches = raw_ring + (size_t)w.rb * w.raw_stage;
+  // (shuffles and votes mark what is the same in the whole warp: the MMA operands then stay in uniform registers)
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
+  const int n_jobs = __shfl_sync(0xFFFFFFFFu, *p.n_tiles * w.n_blk, 0);
+  if (wt_job(0) >= n_jobs) return;
+
+  if (tid == 0) {
+    for (int s = 0; s < W_A_STAGES; ++s) {
+      mbar_init(&bars.full_a[s], 8);
+      mbar_init(&bars.empty_a[s], 1);
+    }
+    for (int s = 0; s < W_MAX_RING; ++s) {
+      mbar_init(&bars.full_b[s], MODE == 0 ? 64 : 1);
+      mbar_init(&bars.empty_b[s], 1);
+      mbar_init(&bars.full_raw[s], wt_tiled(FMT) ? 1 : RAW_WARPS * 32);
+      mbar_init(&bars.empty_raw[s], W_PRODUCERS / 32);
+    }
+    mbar_init(&bars.done, 1);
+    mbar_init(&bars.drained, W_PRODUCERS / 32);
+    mbar_fence_init();
+  }
+  if (warp == W_MMA_WARP) umma::tmem_alloc(&s_tmem, 512);
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  constexpr uint32_t tmem = 0;  // the whole of tensor memory is this CTA's: it starts at column 0
+  const int kb = w.k_blocks;
+  bool ok = true;
+
+  if (warp < W_PRODUCERS / 32) {
+    // ---- producers: unpack, then drain ----
+    const int g = warp >> 3, role = (warp >> 2) & 1, q = warp & 3;
+    const int slot = role * 128 + wt_row_of_lane(MODE, q * 32 + lane);  // row of the raw stage
+    const int dt = MODE == 1 ? p.down_dt : (role ? p.up_dt : p.gate_dt);
+    const int half_word = (int)(row_bytes(dt, 256) & 2);  // blocks of an odd number of half-words: every other one is off a word boundary
+    const uint32_t a_addr = tmem + ((uint32_t)(q * 32) << 16) + W_A_COL + 32u * role;
+    unsigned char* patch = patches + (size_t)warp * W_PATCH;
+    const uint32_t patch_u = smem_u32(patch);
+    RingPos rp, ap;  // raw blocks; A stages
+    if (g) ap.next(W_A_STAGES);
+    uint32_t d_phase = 0;
+    for (int it = 0; ok; ++it) {
+      const int job = wt_job(it);
+      if (job >= n_jobs) break;
+      const int tile = job / w.n_blk, blk0 = job - tile * w.n_blk;
+      const int e = p.tile_expert[tile], row0 = p.tile_row0[tile], rows_valid = p.tile_rows[tile];
+      const int wrow = MODE == 0 ? blk0 * 128 + (slot & 127) : blk0 * WR + slot;
+      for (int blk = 0; blk < kb; ++blk) {
+        if (!wt_wait(&bars.full_raw[rp.s], rp.phase)) { ok = false; break; }
+        const unsigned char* row = raw_ring + (size_t)rp.s * w.raw_stage + (size_t)slot * w.raw_pitch;
+        const int mis = ((wrow * kb + blk) & 1) * half_word;  // bytes of the stage's first word ahead of the block
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t o[32];
+          const int j = 2 * h + g;
+          const uint32_t* row32 = reinterpret_cast<const uint32_t*>(row);
+          if (FMT == WT_Q4K) {
+            unpack_q4k(row, j, o);
+          } else if (FMT == WT_Q5K) {
+            unpack_q5k_row(row, j, o);
+          } else if (FMT == WT_Q80) {
+            if (g) h ? unpack_q80_row<3>(row, o) : unpack_q80_row<1>(row, o);
+            else h ? unpack_q80_row<2>(row, o) : unpack_q80_row<0>(row, o);
+          } else if (FMT == WT_Q6K || dt == INFR_CUDA_DT_Q6K) {
+            unpack_q6k(row32, mis * 8, h, g, o);
+          } else if (dt == INFR_CUDA_DT_Q8_0) {
+            unpack_q80([&](int i) { return row32[17 * j + i]; }, o);
+          } else if (dt == INFR_CUDA_DT_Q5K) {
+            unpack_k45_words<true>(row32, j, o);
+          } else if (dt == INFR_CUDA_DT_Q4K) {
+            unpack_k45_words<false>(row32, j, o);
+          } else {
+            unpack_codes(dt, row + mis, j, o);
+          }
+          if (h == 1) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars.empty_raw[rp.s]);
+          }
+          if (!wt_wait(&bars.empty_a[ap.s], ap.phase ^ 1)) { ok = false; break; }
+          umma::fence_after_sync();
+          tmem_st_32x32(a_addr + 64u * ap.s, o);
+          umma::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars.full_a[ap.s]);
+          ap.next(W_A_STAGES);
+          ap.next(W_A_STAGES);
+        }
+        if (!ok) break;
+        rp.next(w.rb);
+      }
+      if (!ok) break;
+      if (!wt_wait(&bars.done, d_phase)) { ok = false; break; }
+      d_phase ^= 1;
+      umma::fence_after_sync();
+      const float clamp = e < p.n_expert ? p.clamp : 0.f;  // the shared expert's segment is not clamped
+      // the down kernel's operand: [K step][rows of the tile][128 B], swizzled like its image in shared memory
+      unsigned char* act = reinterpret_cast<unsigned char*>(p.act) + (size_t)row0 * p.nff * 2 + (size_t)(2 * blk0 + (q >> 1)) * rows_valid * 128;
+      // warps of one lane quarter share the tile's tokens, 16 at a time
+      for (int t0 = 16 * (warp >> 2); t0 < rows_valid; t0 += 64) {
+        const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)t0;
+        float v[2][2][8];  // [accumulator][16 lanes][fragment]
+        tmem_ld_16x16_quad(tq, tq + (16u << 16), tq + WN, tq + WN + (16u << 16), v[0][0], v[0][1], v[1][0], v[1][1]);
+        if (MODE == 0) {
+          if (p.act_kind == INFR_CUDA_ACT_SILU && clamp == 0.f) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              // accumulators are 256 x the products: SiLU(g) u = g u / (1 + 2^(-log2(e) g))
+              float& ga = v[0][i >> 3][i & 7];
+              const float ex = exp2_approx(ga * (-1.44269504f * W_POSTSCALE));
+              ga = __fdividef(ga * W_POSTSCALE, 1.0f + ex) * (v[1][i >> 3][i & 7] * W_POSTSCALE);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              v[0][i >> 3][i & 7] = gated_act_general(p.act_kind, clamp, v[0][i >> 3][i & 7] * W_POSTSCALE, v[1][i >> 3][i & 7] * W_POSTSCALE);
+          }
+          const int mi = lane >> 3;  // transposed on the way out: a patch row is a token's 32 positions of this lane quarter
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            stmatrix_x4_trans(patch_u + ((lane & 7) + 8 * (mi >> 1)) * 80 + (2 * h + (mi & 1)) * 16, f16x2_sat(v[0][h][0], v[0][h][1]),
+                              f16x2_sat(v[0][h][2], v[0][h][3]), f16x2_sat(v[0][h][4], v[0][h][5]), f16x2_sat(v[0][h][6], v[0][h][7]));
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int t = (lane >> 2) + 8 * i, c = lane & 3;
+            const uint4 x = *reinterpret_cast<const uint4*>(patch + t * 80 + c * 16);
+            if (t0 + t < rows_valid) *reinterpret_cast<uint4*>(act + (size_t)(t0 + t) * 128 + (((4 * (q & 1) + c) ^ (t & 7)) << 4)) = x;
+          }
+          __syncwarp();
+        } else {
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            const int f0 = blk0 * WR + m * 128 + q * 32;  // first of the 32 output features of this lane quarter
+            if (p.y_packed) {
+              // the combine kernel is the only reader: this thread's four outputs of a token (8 features apart) as one item
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {  // tokens 8 (k >> 1) + 2 (lane % 4) + (k & 1)
+                const int i0 = 4 * (k >> 1) + (k & 1), t = t0 + 8 * (k >> 1) + 2 * (lane & 3) + (k & 1);
+                const uint2 item = pack_y4(v[m][0][i0], v[m][0][i0 + 2], v[m][1][i0], v[m][1][i0 + 2]);
+                if (t < rows_valid) reinterpret_cast<uint2*>(p.y)[((size_t)(row0 + t) * p.ne + f0) / 4 + (lane >> 2)] = item;
+              }
+            } else {
+#pragma unroll
+              for (int cg = 0; cg < 2; ++cg) {  // eight tokens at a time
+                float* pf = reinterpret_cast<float*>(patch);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                  for (int i = 0; i < 4; ++i)
+                    pf[(2 * (lane & 3) + (i & 1)) * 36 + h * 16 + (i >> 1) * 8 + (lane >> 2)] = v[m][h][4 * cg + i] * W_POSTSCALE;
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                  const int t = (lane >> 3) + 4 * i, c = lane & 7;
+                  const float4 x = *reinterpret_cast<const float4*>(pf + t * 36 + c * 4);
+                  if (t0 + 8 * cg + t < rows_valid)
+                    *reinterpret_cast<float4*>(p.y + (size_t)(row0 + t0 + 8 * cg + t) * p.ne + f0 + c * 4) = x;
+                }
+                __syncwarp();
+              }
+            }
+          }
+        }
+      }
+      umma::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars.drained);
+    }
+    if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
+  } else if (warp == W_MMA_WARP) {
+    // ---- MMA issue: the warp waits, one elected lane issues ----
+    const uint64_t db0 = umma::smem_desc_k_major_swz128(b_ring, 0);
+    RingPos bp, ap;
+    uint32_t r_phase = 1;
+    for (int it = 0; ok; ++it) {
+      const int job = wt_job(it);
+      if (job >= n_jobs) break;
+      const uint32_t idesc = umma::idesc_f16_f32(128, (__shfl_sync(0xFFFFFFFFu, p.tile_rows[job / w.n_blk], 0) + 15) & ~15);
+      ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.drained, r_phase));
+      if (!ok) break;
+      r_phase ^= 1;
+      for (int step = 0; step < 4 * kb; ++step) {
+        ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.full_b[bp.s], bp.phase) && wt_wait(&bars.full_a[ap.s], ap.phase));
+        if (!ok) break;
+        umma::fence_after_sync();
+        if (elect_one()) {
+          const uint64_t db = db0 + (uint64_t)(bp.s * (W_B_STAGE >> 4));
+          const uint32_t a = W_A_COL + 64u * ap.s, acc = step > 0;
+          if (MODE == 0) umma::fence_proxy_async();  // the copies behind full_b were cp.async
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            mma_f16_ta(tmem, a + 8 * k, db + 2 * k, idesc, k > 0 ? 1u : acc);
+            mma_f16_ta(tmem + WN, a + 32 + 8 * k, db + 2 * k, idesc, k > 0 ? 1u : acc);
+          }
+          umma::commit(&bars.empty_a[ap.s]);
+          umma::commit(&bars.empty_b[bp.s]);
+          if (step == 4 * kb - 1) umma::commit(&bars.done);
+        }
+        __syncwarp();
+        bp.next(w.sb);
+        ap.next(W_A_STAGES);
+      }
+    }
+    if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
+  } else if (warp < RAW_WARP) {
+    // ---- token operand ----
+    RingPos bp;
+    if (MODE == 1) {
+      // the tile's activations: [K step][rows of the tile][128 B], swizzled - one copy per step (past the tile's last row
+      // it reads on into the next step: columns of the accumulators that nothing looks at)
+      for (int it = 0; ok; ++it) {
+        const int job = wt_job(it);
+        if (job >= n_jobs) break;
+        const int tile = job / w.n_blk, rows_valid = p.tile_rows[tile];
+        const uint32_t bytes = (uint32_t)((rows_valid + 15) & ~15) * 128u;
+        const unsigned char* src = reinterpret_cast<const unsigned char*>(p.act) + (size_t)p.tile_row0[tile] * p.nff * 2;
+        for (int step = 0; step < 4 * kb; ++step) {
+          if (!wt_wait(&bars.empty_b[bp.s], bp.phase ^ 1)) { ok = false; break; }
+          if (elect_one()) {
+            mbar_arrive_expect_tx(&bars.full_b[bp.s], bytes);
+            bulk_g2s(b_ring + (size_t)bp.s * W_B_STAGE, src + (size_t)step * rows_valid * 128, bytes, &bars.full_b[bp.s]);
+          }
+          __syncwarp();
+          bp.next(w.sb);
+        }
+      }
+    } else {
+      // Token rows from where they are: eight lanes per row and K step, 16 bytes each, straight into the swizzled operand
+      // image; two warps share a step (four rows out of every eight each), the two pairs alternate.  (Gathering TMA
+      // copies, four rows each, took 18 cycles per row: twice the tensor-core time of the step.)
+      const int tw = warp - W_TOK_WARP, r8 = (tw & 1) * 4 + (lane >> 3), c = lane & 7;
+      const uint32_t dst0 = smem_u32(b_ring) + (uint32_t)r8 * 128u + (uint32_t)((c ^ r8) << 4);
+      const uint4* tok = reinterpret_cast<const uint4*>(p.xg) + c;
+      const int n_sorted = w.seg_off[w.n_seg_routed];
+      if (tw & 2) bp.next(w.sb);
+      for (int it = 0; ok; ++it) {
+        const int job = wt_job(it);
+        if (job >= n_jobs) break;
+        const int tile = job / w.n_blk;
+        const int row0 = p.tile_row0[tile], rows_valid = p.tile_rows[tile], ni = ((rows_valid + 15) & ~15) >> 3;
+        uint32_t src[WN / 8];  // rows 8 i + r8, in units of 16 bytes
+#pragma unroll
+        for (int i = 0; i < WN / 8; ++i) {
+          if (i < ni) {
+            const int pos = row0 + min(8 * i + r8, rows_valid - 1);  // past the end: the last row once more
+            const int t = w.pair_of_pos == nullptr ? pos : pos < n_sorted ? w.pair_of_pos[pos] / w.n_used : pos - n_sorted;
+            src[i] = (uint32_t)t * (uint32_t)(p.ne >> 3);
+          }
+        }
+        for (int step = tw >> 1; step < 4 * kb; step += 2) {
+          if (!wt_wait(&bars.empty_b[bp.s], bp.phase ^ 1)) { ok = false; break; }
+          const uint32_t dst = dst0 + (uint32_t)bp.s * W_B_STAGE;
+          const uint4* ts = tok + step * 8;
+#pragma unroll
+          for (int i = 0; i < WN / 8; ++i)
+            if (i < ni) cp_async16(dst + i * 1024, ts + src[i]);
+          cp_async_arrive(&bars.full_b[bp.s]);
+          bp.next(w.sb);
+          bp.next(w.sb);
+        }
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
+  } else if (warp < RAW_WARP + RAW_WARPS) {
+    // ---- raw blocks ----
+    RingPos rp;
+    for (int it = 0; ok; ++it) {
+      const int job = wt_job(it);
+      if (job >= n_jobs) break;
+      const int tile = job / w.n_blk, blk0 = job - tile * w.n_blk, e = p.tile_expert[tile];
+      const bool shared_seg = e >= p.n_expert;
+      if (wt_tiled(FMT)) {
+        if (warp != RAW_WARP || lane != 0) break;  // one thread issues the tiled copies
+        // rows of one expert in the bank: nff, or 2 nff where gate and up share a bank (the up map then starts nff rows in)
+        const int r0 = MODE == 0 ? (shared_seg ? 0 : e * p.gu_rows) + blk0 * 128 : (shared_seg ? 0 : e * p.ne) + blk0 * WR;
+        for (int blk = 0; blk < kb; ++blk) {
+          if (!wt_wait(&bars.empty_raw[rp.s], rp.phase ^ 1)) { ok = false; break; }
+          unsigned char* dst = raw_ring + (size_t)rp.s * w.raw_stage;
+          const int x = blk * (int)(w.raw_pitch >> 1);  // in half-words
+          mbar_arrive_expect_tx(&bars.full_raw[rp.s], w.raw_stage);
+          tma_load_2d(dst, shared_seg ? &tm_s0 : &tm_w0, x, r0, &bars.full_raw[rp.s]);
+          tma_load_2d(dst + 128 * w.raw_pitch, shared_seg ? &tm_s1 : &tm_w1, x, r0 + (MODE == 0 ? 0 : 128), &bars.full_raw[rp.s]);
+          rp.next(w.rb);
+        }
+      } else {
+        // Whole words over a block's bytes: a block off a word boundary takes the half-word ahead of it, one that ends off
+        // a word boundary the half-word behind it (inside the bank: its block count is even).  One instruction per row and
+        // 32 words; the words left over of as many rows as fit share one.
+        const int lw = warp - RAW_WARP;
+        for (int blk = 0; blk < kb; ++blk) {
+          if (!wt_wait(&bars.empty_raw[rp.s], rp.phase ^ 1)) { ok = false; break; }
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {  // gate and up rows, or the two halves of the output features
+            const int dt = MODE == 1 ? p.down_dt : half ? p.up_dt : p.gate_dt;
+            const uint8_t* bank = MODE == 1 ? (shared_seg ? p.sh_down : p.down + (size_t)e * p.down_stride)
+                                            : half ? (shared_seg ? p.sh_up : p.up + (size_t)e * p.up_stride)
+                                                   : (shared_seg ? p.sh_gate : p.gate + (size_t)e * p.gate_stride);
+            const uint32_t chunk = FMT == WT_Q6K ? Q6K_BLOCK_BYTES : (uint32_t)row_bytes(dt, 256);
+            const uint32_t words = (chunk + 2) >> 2, full = words >> 5, tail = words & 31u, tail_rows = tail ? 32u / tail : 1u;
+            const size_t pitch = (size_t)chunk * kb;
+            const uint32_t dst0 = smem_u32(raw_ring) + rp.s * w.raw_stage + (uint32_t)half * 128u * w.raw_pitch;
+            const uintptr_t src = reinterpret_cast<uintptr_t>(bank + (size_t)(MODE == 0 ? blk0 * 128 : blk0 * WR + half * 128) * pitch + (size_t)blk * chunk);
+            if (full) {
+              uintptr_t a = src + lw * pitch + 4 * lane;
+              uint32_t d = dst0 + lw * w.raw_pitch + 4 * lane;
+#pragma unroll 4
+              for (int r = lw; r < 128; r += RAW_WARPS, a += RAW_WARPS * pitch, d += RAW_WARPS * w.raw_pitch) {
+                cp_async4(d, reinterpret_cast<const void*>(a & ~(uintptr_t)3));
+                if (full > 1) cp_async4(d + 128, reinterpret_cast<const void*>((a & ~(uintptr_t)3) + 128));
+              }
+            }
+            if (tail) {
+              const uint32_t t_row = lane / tail + lw * tail_rows, t_word = 32u * full + lane % tail, stride = RAW_WARPS * tail_rows;
+              const bool on = lane < tail_rows * tail;
+              uintptr_t a = src + t_row * pitch + 4 * t_word;
+              uint32_t d = dst0 + t_row * w.raw_pitch + 4 * t_word;
+#pragma unroll 4
+              for (uint32_t r = t_row; r < 128 + stride; r += stride, a += stride * pitch, d += stride * w.raw_pitch)
+                if (on && r < 128) cp_async4(d, reinterpret_cast<const void*>(a & ~(uintptr_t)3));
+            }
+          }
+          cp_async_arrive(&bars.full_raw[rp.s]);
+          rp.next(w.rb);
+        }
+      }
+    }
+    if (!wt_tiled(FMT)) asm volatile("cp.async.wait_all;" ::: "memory");
+    if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  if (warp == W_MMA_WARP) umma::tmem_dealloc(s_tmem, 512);
+}
+
+// A bank as a 2-D tensor of half-words [rows][row bytes / 2]; box: 256 weights (`chunk` bytes) of 128 rows.
+bool raw_rows_map(CUtensorMap* tm, const uint8_t* base, size_t rows, size_t row_bytes, uint32_t chunk) {
+  EncodeTiledFn enc = encode_tiled_fn();
+  if (!enc) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)row_bytes / 2, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
+  const cuuint32_t box[2] = {chunk / 2, 128};
+  const cuuint32_t estr[2] = {1, 1};
+  return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<uint8_t*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+int wt_format(int dt0, int dt1, bool down) {
+  if (dt0 == dt1) {
+    if (dt0 == INFR_CUDA_DT_Q4K) return WT_Q4K;
+    if (dt0 == INFR_CUDA_DT_Q5K) return WT_Q5K;
+    if (dt0 == INFR_CUDA_DT_Q8_0) return WT_Q80;
+    if (dt0 == INFR_CUDA_DT_Q6K && down) return WT_Q6K;
+  }
+  return WT_ANY;
+}
+
+// Bytes of 256 weights of a row in the raw stage.
+uint32_t raw_pitch_of(int fmt, int dt) {
+  if (wt_tiled(fmt)) return (uint32_t)row_bytes(dt, 256);  // 36, 44 or 68 words: 16-byte pieces of eight rows in different banks
+  const uint32_t words = ((uint32_t)row_bytes(dt, 256) + 2 + 3) / 4;  // room for the half-word ahead
+  return (words | 1) * 4;
+}
+
+template <int MODE, int FMT>
+int32_t launch_wt(infr_cuda_ctx* ctx, WtParams w, const CUtensorMap (&tm)[4], int max_tiles) {
+  // as many stages as fit: two raw stages at least, then up to four token stages, then more raw stages
+  const size_t patches = (size_t)(W_PRODUCERS / 32) * W_PATCH;
+  const size_t room = 227 * 1024 - 1024 - 1024 - patches;  // alignment slack, static shared memory
+  w.rb = 2;
+  w.sb = W_MAX_RING;
+  while (w.sb > 2 && (size_t)w.rb * w.raw_stage + (size_t)w.sb * W_B_STAGE > room) --w.sb;
+  while (w.rb < W_MAX_RING && (size_t)(w.rb + 1) * w.raw_stage + (size_t)w.sb * W_B_STAGE <= room) ++w.rb;
+  const size_t rings = (size_t)w.rb * w.raw_stage + (size_t)w.sb * W_B_STAGE;
+  if (rings > room) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "grouped GEMM: blocks too large for the raw ring");
+  const size_t smem = 1024 + rings + patches;
+  cudaError_t e = ensure_smem(reinterpret_cast<const void*>(k_wt_gemm<MODE, FMT>), smem);
+  if (e != cudaSuccess) return check_cuda(ctx, e, "grouped GEMM: shared-memory attribute");
+  const long long jobs = (long long)max_tiles * w.n_blk;
+  k_wt_gemm<MODE, FMT><<<(unsigned)std::min<long long>(jobs, ctx->sm_count), W_THREADS, smem, ctx->stream>>>(w, tm[0], tm[1], tm[2], tm[3]);
+  ctx->launches += 1;
+  return check_cuda(ctx, cudaGetLastError(), "grouped GEMM launch");
+}
+
+}  // namespace
+
+int wt_tile_rows() { return WN; }
+
+int32_t launch_wt_grouped(infr_cuda_ctx* ctx, const GroupedParams& p, const WtTokens& t, int max_tiles) {
+  WtParams w = {};
+  w.g = p;
+  w.pair_of_pos = t.pair_of_pos;
+  w.seg_off = t.seg_off;
+  w.n_seg_routed = t.n_seg_routed;
+  w.n_used = t.n_used;
+  CUtensorMap tm[4] = {};
+  bool ok = true;
+
+  // gate / up.  A bank's rows are one 2-D tensor; with gate and up in one bank an expert has 2 nff rows and the up map
+  // starts nff rows in (and ends with the bank)
+  w.n_blk = p.nff / 128;
+  w.k_blocks = p.ne / 256;
+  int fmt = wt_format(p.gate_dt, p.up_dt, false);
+  w.raw_pitch = std::max(raw_pitch_of(fmt, p.gate_dt), raw_pitch_of(fmt, p.up_dt));
+  w.raw_stage = WR * w.raw_pitch;
+  if (wt_tiled(fmt)) {
+    const size_t rb = row_bytes(p.gate_dt, p.ne), bank_rows = (size_t)p.n_expert * p.gu_rows;
+    ok = raw_rows_map(&tm[0], p.gate, bank_rows, rb, w.raw_pitch) && raw_rows_map(&tm[1], p.up, bank_rows - ((size_t)p.gu_rows - p.nff), rb, w.raw_pitch);
+    if (ok && p.sh_gate) ok = raw_rows_map(&tm[2], p.sh_gate, p.nff, rb, w.raw_pitch) && raw_rows_map(&tm[3], p.sh_up, p.nff, rb, w.raw_pitch);
+    if (!ok) return fail(ctx, INFR_CUDA_ERR_CUDA, "grouped GEMM: the driver refused a tensor map for the expert banks");
+  }
+  int32_t rc = fmt == WT_Q4K   ? launch_wt<0, WT_Q4K>(ctx, w, tm, max_tiles)
+               : fmt == WT_Q5K ? launch_wt<0, WT_Q5K>(ctx, w, tm, max_tiles)
+               : fmt == WT_Q80 ? launch_wt<0, WT_Q80>(ctx, w, tm, max_tiles)
+                               : launch_wt<0, WT_ANY>(ctx, w, tm, max_tiles);
+  if (rc) return rc;
+
+  // down
+  w.n_blk = p.ne / WR;
+  w.k_blocks = p.nff / 256;
+  fmt = wt_format(p.down_dt, p.down_dt, true);
+  w.raw_pitch = raw_pitch_of(fmt, p.down_dt);
+  w.raw_stage = WR * w.raw_pitch;
+  if (wt_tiled(fmt)) {
+    const size_t rb = row_bytes(p.down_dt, p.nff);
+    ok = raw_rows_map(&tm[0], p.down, (size_t)p.n_expert * p.ne, rb, w.raw_pitch);
+    if (ok && p.sh_down) ok = raw_rows_map(&tm[2], p.sh_down, p.ne, rb, w.raw_pitch);
+    tm[1] = tm[0];
+    tm[3] = tm[2];
+    if (!ok) return fail(ctx, INFR_CUDA_ERR_CUDA, "grouped GEMM: the driver refused a tensor map for the down bank");
+  }
+  return fmt == WT_Q4K   ? launch_wt<1, WT_Q4K>(ctx, w, tm, max_tiles)
+         : fmt == WT_Q5K ? launch_wt<1, WT_Q5K>(ctx, w, tm, max_tiles)
+         : fmt == WT_Q80 ? launch_wt<1, WT_Q80>(ctx, w, tm, max_tiles)
+         : fmt == WT_Q6K ? launch_wt<1, WT_Q6K>(ctx, w, tm, max_tiles)
+                         : launch_wt<1, WT_ANY>(ctx, w, tm, max_tiles);
+}
+
+cudaError_t publish_codebooks_tmem(const unsigned char* const* tables) { return publish_codebooks(tables); }
+
+}  // namespace infr

@@ -98,22 +98,17 @@ struct EmParams {
 // Device-side view of one grouped-GEMM launch (see grouped_ffn.cu).
 struct GroupedParams {
   const int *tile_expert, *tile_row0, *tile_rows, *n_tiles;  // tile table built on the device
-  // token rows grouped by expert, f16, K order 0,2,1,3 per four.  Legacy tiles: [rows, ne] and
-  // [rows, nff] row-major.  tcgen05 tiles: [tile][K step][256 rows][64] with swizzled 128-byte lines.
+  // f16, K order 0,2,1,3 per four.  mma.sync tiles: rows grouped by expert, row-major.  tcgen05 tiles: xg as the call has
+  // the tokens; act per tile as [K step][rows of the tile][128 B], swizzled
   const __half* xg;
   __half* act;
-  float* y;          // [rows, ne] raw down outputs: f32, or f16 in the same buffer when y_f16 is set
-  int y_f16;         // the combine kernel is the only reader (tcgen05 tiles): rows as f16 with one power-of-two
-                     // scale per 32 outputs of a row (y_scale), half the bytes both ways
-  float* y_scale;    // [rows, ne / 32]: in the unused half of the y buffer
+  float* y;          // [rows, ne] raw down outputs: f32, or with y_packed items of 8 bytes per four outputs of a row (the
+  int y_packed;      // combine kernel is the only reader; pack_y4): features 32 g + j + 8 i, i = 0..3, at item 8 g + j
   const uint8_t *gate, *up, *down;
   const uint8_t *sh_gate, *sh_up, *sh_down;  // segment index n_expert = the shared expert
   size_t gate_stride, up_stride, down_stride;
   DeviceStatus* status;
-  unsigned long long* trace;  // optional phase stamps
-  int trace_tile;             // tile whose first CTA writes them
   int ne, nff, n_expert;
-  int down_q4k;               // the down banks are Q4_K instead of Q6_K (tcgen05 kernels only)
   int gate_dt, up_dt, down_dt;  // INFR_CUDA_DT_* of the banks (the generic-format tiles read these)
   int act_kind;               // INFR_CUDA_ACT_*
   int gu_rows;                // rows of one expert in the gate bank: nff, or 2 nff where gate and up share a bank
@@ -146,9 +141,14 @@ struct GroupedCall {
   const float* down_scale; // [n_expert] or null
 };
 
-bool umma_grouped_supported(int ne, int nff);
-int umma_tile_rows();
-int32_t launch_umma_grouped(infr_cuda_ctx* ctx, const GroupedParams& p, int max_tiles);
+// Where the token rows of a grouped call are (grouped_tmem.cu).
+struct WtTokens {
+  const int* pair_of_pos;  // pair behind every grouped row, or null: `xg` is in grouped order itself
+  const int* seg_off;      // [n_seg_routed] = grouped rows ahead of the shared expert's, which follow in token order
+  int n_seg_routed, n_used;
+};
+int wt_tile_rows();
+int32_t launch_wt_grouped(infr_cuda_ctx* ctx, const GroupedParams& p, const WtTokens& t, int max_tiles);
 size_t grouped_scratch_bytes(int rows_total, int n_pairs, int n_seg, int ne, int nff);
 int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c);
 int32_t launch_combine(infr_cuda_ctx* ctx, const float* y, const int* pos_of_pair, const float* wts, const float* sh_logit,
@@ -205,6 +205,7 @@ int32_t launch_store_host(infr_cuda_ctx* ctx, const void* src, void* dst_dev_vie
 cudaError_t publish_codebooks_dense(const unsigned char* const* tables);
 cudaError_t publish_codebooks_anyfmt(const unsigned char* const* tables);
 cudaError_t publish_codebooks_grouped(const unsigned char* const* tables);
+cudaError_t publish_codebooks_tmem(const unsigned char* const* tables);
 int32_t launch_fetch_host_gated(infr_cuda_ctx* ctx, const void* src_dev_view, void* dst, size_t bytes, const unsigned long long* bell,
                                 unsigned long long ticket, unsigned long long limit_ns);
 int32_t launch_host_signal(infr_cuda_ctx* ctx, unsigned long long* done, unsigned long long ticket);
