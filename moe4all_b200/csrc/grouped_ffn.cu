@@ -21,6 +21,7 @@
 // K order: unpacking a 32-bit word of codes yields pairs (e0,e2),(e1,e3); tiles therefore hold
 // every aligned group of four K elements in the order 0,2,1,3, and the token-side arrays (xg,
 // act) are written in the same order.
+#include <cooperative_groups.h>
 #include <mma.h>
 
 #include <algorithm>
@@ -32,6 +33,8 @@
 namespace infr {
 
 namespace {
+
+namespace cg = cooperative_groups;
 
 constexpr int TM = 64;       // weight rows per role and CTA
 constexpr int TN = 64;       // tokens per CTA
@@ -111,19 +114,12 @@ __device__ __forceinline__ int tile_height(int cnt, int tn) {
   return ((cnt + n - 1) / n + 15) & ~15;
 }
 
-// Exclusive scan of the per-expert counts (thread e holds the count of segment e), the tile table
-// (the shared expert's rows appended as segment n_expert) and the segment offsets, by the 1024 threads
-// of one CTA.  Offsets stay in s_off for the caller.  Segments are listed by falling tile height, so
-// that the GEMM kernels' last round of jobs is made of the light ones.
-__device__ __forceinline__ void segment_tables(int cnt, int n_expert, int shared_rows, int tn, int* __restrict__ seg_off,
-                                               int* __restrict__ tile_expert, int* __restrict__ tile_row0,
-                                               int* __restrict__ tile_rows, int* __restrict__ n_tiles, int* s_cnt, int* s_off,
-                                               int* s_toff, int* s_ws) {
-  const int tid = threadIdx.x;
-  const int n_seg = n_expert + (shared_rows > 0 ? 1 : 0);
-  auto tiles_of = [&](int c) { const int h = tile_height(c, tn); return (c + h - 1) / h; };
-  int off = cnt, nt = tiles_of(cnt), total = 0, total_t = 0;  // rows ahead of this segment
-  block_scan2(off, nt, total, total_t, s_ws);
+// Exclusive scan of the per-expert counts (thread e holds the count of segment e; the shared expert's rows appended as
+// segment n_expert) by the 1024 threads of one CTA: counts and offsets in s_cnt, s_off; returns the rows in total.
+__device__ __forceinline__ int segment_offsets(int cnt, int n_expert, int shared_rows, int* s_cnt, int* s_off, int* s_ws) {
+  const int tid = threadIdx.x, n_seg = n_expert + (shared_rows > 0 ? 1 : 0);
+  int off = cnt, unused = 0, total = 0, total_unused = 0;
+  block_scan2(off, unused, total, total_unused, s_ws);
   if (tid < n_seg) {
     s_cnt[tid] = cnt;
     s_off[tid] = off;
@@ -134,28 +130,48 @@ __device__ __forceinline__ void segment_tables(int cnt, int n_expert, int shared
       s_off[1024] = total;
     }
     total += shared_rows;
-    total_t += tiles_of(shared_rows);
   }
-  if (tid == 0) {
-    s_off[n_seg] = total;
-    *n_tiles = total_t;
-    seg_off[n_expert + 1] = total;  // total grouped rows, with or without a shared segment
+  if (tid == 0) s_off[n_seg] = total;
+  __syncthreads();
+  return total;
+}
+
+// The tile table and the segment offsets.  Tiles are listed by falling height (in classes of 16 rows), so that the GEMM
+// kernels' last round of jobs is made of the light ones; the order inside a class is whatever it comes out as.
+__device__ __forceinline__ void segment_tables(int n_expert, int shared_rows, int total, int tn, int* __restrict__ seg_off,
+                                               int* __restrict__ tile_expert, int* __restrict__ tile_row0,
+                                               int* __restrict__ tile_rows, int* __restrict__ n_tiles, const int* s_cnt, const int* s_off,
+                                               int* s_cls) {
+  const int tid = threadIdx.x, n_seg = n_expert + (shared_rows > 0 ? 1 : 0);
+  if (tid < 32) s_cls[tid] = 0;
+  __syncthreads();
+  auto height = [&](int c) { return min(c, tile_height(c, tn)); };
+  for (int e = tid; e < n_seg; e += 1024) {
+    const int c = s_cnt[e];
+    if (c) atomicAdd(&s_cls[31 - ((height(c) + 15) >> 4)], (c + height(c) - 1) / height(c));
   }
   __syncthreads();
-  for (int e = tid; e < n_seg; e += 1024)  // (height, tiles) of every segment
-    s_toff[e] = (min(s_cnt[e], tile_height(s_cnt[e], tn)) << 20) | tiles_of(s_cnt[e]);
+  if (tid < 32) {  // class 31 - h: the highest tiles first
+    const int v = s_cls[tid];
+    int t = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xFFFFFFFFu, t, o);
+      if (tid >= o) t += u;
+    }
+    s_cls[tid] = t - v;
+    if (tid == 31) {
+      *n_tiles = t;
+      seg_off[n_expert + 1] = total;  // total grouped rows, with or without a shared segment
+    }
+  }
   __syncthreads();
   for (int e = tid; e <= n_seg; e += 1024) seg_off[e] = s_off[e];
   for (int e = tid; e < n_seg; e += 1024) {
-    const int c = s_cnt[e], mine = s_toff[e] >> 20;
+    const int c = s_cnt[e];
     if (!c) continue;
-    int t = 0;  // tiles of the segments with higher tiles, or as high in an earlier segment
-#pragma unroll 8
-    for (int o = 0; o < n_seg; ++o) {
-      const int v = s_toff[o], h = v >> 20;
-      t += (h > mine || (h == mine && o < e)) ? (v & 0xFFFFF) : 0;
-    }
-    const int h = tile_height(c, tn);
+    const int h = height(c);
+    int t = atomicAdd(&s_cls[31 - ((h + 15) >> 4)], (c + h - 1) / h);
     for (int r = 0; r < c; r += h, ++t) {
       tile_expert[t] = e;
       tile_row0[t] = s_off[e] + r;
@@ -169,16 +185,21 @@ __global__ void __launch_bounds__(1024) k_segment_scan(const int* __restrict__ c
                                                        int* __restrict__ seg_off, int* __restrict__ fill,
                                                        int* __restrict__ tile_expert, int* __restrict__ tile_row0,
                                                        int* __restrict__ tile_rows, int* __restrict__ n_tiles) {
-  __shared__ int s_cnt[1025], s_off[1026], s_toff[1026], s_ws[66];
+  __shared__ int s_cnt[1025], s_off[1026], s_cls[32], s_ws[66];
   const int tid = threadIdx.x;
   const int n_seg = n_expert + (shared_rows > 0 ? 1 : 0);
   const int cnt = tid < n_seg ? (tid < n_expert ? counts[tid] : shared_rows) : 0;
-  segment_tables(cnt, n_expert, shared_rows, tn, seg_off, tile_expert, tile_row0, tile_rows, n_tiles, s_cnt, s_off, s_toff, s_ws);
+  const int total = segment_offsets(cnt, n_expert, shared_rows, s_cnt, s_off, s_ws);
+  segment_tables(n_expert, shared_rows, total, tn, seg_off, tile_expert, tile_row0, tile_rows, n_tiles, s_cnt, s_off, s_cls);
   for (int e = tid; e < n_expert; e += 1024) fill[e] = 0;
 }
 
-// Calls of up to a few hundred thousand pairs: count, scan and scatter by one CTA with the
-// histogram and the cursors in shared memory - one launch instead of a memset and three kernels.
+// Calls of up to 64 K pairs: count, scan and scatter by one cluster of eight CTAs, histograms and cursors in shared memory
+// (a single CTA, one launch as well, spent 25 us on 32 K pairs: 32 rounds of dependent shared-memory atomics per thread).
+// A CTA counts its eighth of the pairs, adds up the eight histograms through distributed shared memory and places its
+// own pairs behind those of the CTAs before it; the pairs' ids stay in registers in between.
+constexpr int BK_CTAS = 8, BK_PER_THREAD = 8;
+constexpr int BK_MAX_PAIRS = BK_CTAS * BK_PER_THREAD * 1024;
 __device__ __forceinline__ int bucket_of(int e, int n_expert, uint32_t ep_lo, uint32_t ep_n, DeviceStatus* status) {
   if (e < 0) return -1;  // a negative id marks a pair another rank serves
   if (e >= n_expert) status->bad_index = 1;  // served as the last expert, reported at the next sync
@@ -186,52 +207,54 @@ __device__ __forceinline__ int bucket_of(int e, int n_expert, uint32_t ep_lo, ui
   if (ep_n && ((uint32_t)e < ep_lo || (uint32_t)e >= ep_lo + ep_n)) return -1;
   return e;
 }
-__global__ void __launch_bounds__(1024) k_bucket_fused(const int32_t* __restrict__ ids, int n_pairs, int n_expert, uint32_t ep_lo,
-                                                       uint32_t ep_n, int shared_rows, int tn, int* __restrict__ seg_off,
-                                                       int* __restrict__ tile_expert, int* __restrict__ tile_row0,
-                                                       int* __restrict__ tile_rows, int* __restrict__ n_tiles,
-                                                       int* __restrict__ pos_of_pair, int* __restrict__ pair_of_pos,
-                                                       DeviceStatus* status) {
-  __shared__ int s_cnt[1025], s_off[1026], s_toff[1026], s_ws[66], s_hist[1024];
-  const int tid = threadIdx.x;
+__global__ void __cluster_dims__(BK_CTAS, 1, 1) __launch_bounds__(1024)
+    k_bucket_fused(const int32_t* __restrict__ ids, int n_pairs, int n_expert, uint32_t ep_lo, uint32_t ep_n, int shared_rows, int tn,
+                   int* __restrict__ seg_off, int* __restrict__ tile_expert, int* __restrict__ tile_row0, int* __restrict__ tile_rows,
+                   int* __restrict__ n_tiles, int* __restrict__ pos_of_pair, int* __restrict__ pair_of_pos, DeviceStatus* status) {
+  __shared__ int s_hist[1024], s_cur[1024], s_cnt[1025], s_off[1026], s_cls[32], s_ws[66];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x, rank = (int)cluster.block_rank();
+  const int slice = (n_pairs + BK_CTAS - 1) / BK_CTAS, p_lo = rank * slice, p_hi = min(n_pairs, p_lo + slice);
   s_hist[tid] = 0;
   __syncthreads();
-  // eight ids per thread in flight: the loop is a chain of global-memory latencies otherwise
-  for (int p0 = tid; p0 < n_pairs; p0 += 8 * 1024) {
-    int idv[8];
+  int e[BK_PER_THREAD];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) idv[u] = p0 + u * 1024 < n_pairs ? ids[p0 + u * 1024] : -1;
+  for (int u = 0; u < BK_PER_THREAD; ++u) e[u] = p_lo + u * 1024 + tid < p_hi ? ids[p_lo + u * 1024 + tid] : -1;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int e = bucket_of(idv[u], n_expert, ep_lo, ep_n, status);
-      if (e >= 0) atomicAdd(&s_hist[e], 1);
+  for (int u = 0; u < BK_PER_THREAD; ++u) {
+    e[u] = bucket_of(e[u], n_expert, ep_lo, ep_n, status);
+    if (e[u] >= 0) atomicAdd(&s_hist[e[u]], 1);
+  }
+  cluster.sync();
+  int cnt = 0, before = 0;
+  if (tid < n_expert) {
+#pragma unroll
+    for (int c = 0; c < BK_CTAS; ++c) {
+      const int v = cluster.map_shared_rank(s_hist, c)[tid];
+      cnt += v;
+      before += c < rank ? v : 0;
+    }
+  } else if (tid == n_expert) {
+    cnt = shared_rows;
+  }
+  cluster.sync();  // no CTA's histogram goes away while another reads it
+  const int total = segment_offsets(cnt, n_expert, shared_rows, s_cnt, s_off, s_ws);
+  if (tid < n_expert) s_cur[tid] = s_off[tid] + before;
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < BK_PER_THREAD; ++u) {
+    const int p = p_lo + u * 1024 + tid;
+    if (p >= p_hi) break;
+    if (e[u] < 0) {
+      pos_of_pair[p] = -1;
+    } else {
+      const int pos = atomicAdd(&s_cur[e[u]], 1);
+      pos_of_pair[p] = pos;
+      pair_of_pos[pos] = p;
     }
   }
-  __syncthreads();
-  const int n_seg = n_expert + (shared_rows > 0 ? 1 : 0);
-  const int cnt = tid < n_seg ? (tid < n_expert ? s_hist[tid] : shared_rows) : 0;
-  __syncthreads();
-  s_hist[tid] = 0;  // now the fill cursors
-  segment_tables(cnt, n_expert, shared_rows, tn, seg_off, tile_expert, tile_row0, tile_rows, n_tiles, s_cnt, s_off, s_toff, s_ws);
-  __syncthreads();
-  for (int p0 = tid; p0 < n_pairs; p0 += 8 * 1024) {
-    int idv[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) idv[u] = p0 + u * 1024 < n_pairs ? ids[p0 + u * 1024] : -1;
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int p = p0 + u * 1024;
-      if (p >= n_pairs) break;
-      const int e = bucket_of(idv[u], n_expert, ep_lo, ep_n, status);
-      if (e < 0) {
-        pos_of_pair[p] = -1;
-      } else {
-        const int pos = s_off[e] + atomicAdd(&s_hist[e], 1);
-        pos_of_pair[p] = pos;
-        pair_of_pos[pos] = p;
-      }
-    }
-  }
+  if (rank == BK_CTAS - 1)
+    segment_tables(n_expert, shared_rows, total, tn, seg_off, tile_expert, tile_row0, tile_rows, n_tiles, s_cnt, s_off, s_cls);
 }
 
 __global__ void k_pair_scatter(const int32_t* __restrict__ ids, int n_pairs, int n_expert, uint32_t ep_lo, uint32_t ep_n,
@@ -807,8 +830,8 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
   const float* row_w = c.weight_before ? c.wts : nullptr;
   if (c.ids) {
     // routed call: bucket the pairs
-    if (c.n_pairs <= (1 << 16)) {
-      k_bucket_fused<<<1, 1024, 0, st>>>(c.ids, c.n_pairs, c.n_expert, c.ep_lo, c.ep_n, c.shared_rows, tn, seg_off, tile_expert, tile_row0,
+    if (c.n_pairs <= BK_MAX_PAIRS) {
+      k_bucket_fused<<<BK_CTAS, 1024, 0, st>>>(c.ids, c.n_pairs, c.n_expert, c.ep_lo, c.ep_n, c.shared_rows, tn, seg_off, tile_expert, tile_row0,
                                          tile_rows, n_tiles, pos_of_pair, pair_of_pos, ctx->status);
       ctx->launches += 1;
     } else {
