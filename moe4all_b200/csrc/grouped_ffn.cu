@@ -697,8 +697,9 @@ __device__ __forceinline__ float4 unpack_y4(uint2 v) {
 }
 constexpr float YP_POSTSCALE = W_POSTSCALE * (8192.0f / 8191.0f);
 
-// The shared segment starts right after the routed rows: its address is only known on the device.  A thread makes four
-// outputs of a token: four consecutive ones from f32 rows, four of every eighth (of 32) from packed rows.
+// The shared segment starts right after the routed rows: its address is only known on the device.  A thread makes eight
+// outputs of a token: from f32 rows eight consecutive ones, from packed rows two neighbours of every eighth (of 32), i.e.
+// 16 bytes of every slot's row, all slots' requested together.
 template <bool PACKED>
 __global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __restrict__ y, const int* __restrict__ pos_of_pair,
                                                                const float* __restrict__ wts, const float* __restrict__ sh_logit,
@@ -706,15 +707,26 @@ __global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __re
                                                                int rows, int n_used, int ne, const float* residual,
                                                                const int32_t* __restrict__ ids, const float* __restrict__ down_scale,
                                                                int weight_before, float* dst) {
-  const int item = blockIdx.x * 256 + threadIdx.x;
-  if (item * 4 >= ne) return;
-  const int c = PACKED ? (item >> 3) * 32 + (item & 7) : item * 4;
-  auto y4 = [&](size_t pos) {
-    if (!PACKED) return *reinterpret_cast<const float4*>(y + pos * ne + c);
-    return unpack_y4(__ldg(reinterpret_cast<const uint2*>(y) + pos * (ne / 4) + item));
-  };
+  const int q = blockIdx.x * 256 + threadIdx.x;
+  if (q * 8 >= ne) return;
+  const int c = PACKED ? (q >> 2) * 32 + 2 * (q & 3) : q * 8;
+  const int n_sorted = has_shared ? seg_off[n_seg_routed] : 0;
   for (int t = blockIdx.y; t < rows; t += gridDim.y) {  // the grid's y extent stops at 65535
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    // o[i], o[i + 4]: outputs c + i, c + i + 4; packed: c + 8 i, c + 8 i + 1
+    float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    auto take = [&](int pos, float w) {
+      float4 a, b;
+      if (PACKED) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(y) + (size_t)pos * (ne / 8) + q);
+        a = unpack_y4(make_uint2(v.x, v.y));
+        b = unpack_y4(make_uint2(v.z, v.w));
+      } else {
+        a = __ldg(reinterpret_cast<const float4*>(y + (size_t)pos * ne) + 2 * q);
+        b = __ldg(reinterpret_cast<const float4*>(y + (size_t)pos * ne) + 2 * q + 1);
+      }
+      o[0] += w * a.x; o[1] += w * a.y; o[2] += w * a.z; o[3] += w * a.w;
+      o[4] += w * b.x; o[5] += w * b.y; o[6] += w * b.z; o[7] += w * b.w;
+    };
 #pragma unroll 8
     for (int s = 0; s < n_used; ++s) {
       const int pos = pos_of_pair[(size_t)t * n_used + s];
@@ -724,29 +736,35 @@ __global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __re
       // y = raw * scale[e], then the weighted sum (Op::MoeFfn::down_scale); ids may be the caller's: same clamp as the
       // bucketing, which also reported the bad id
       if (down_scale != nullptr) w *= down_scale[min(max(ids[(size_t)t * n_used + s], 0), n_seg_routed - 1)];
-      const float4 v = y4((size_t)pos);
-      o.x += w * v.x; o.y += w * v.y; o.z += w * v.z; o.w += w * v.w;
+      take(pos, w);
     }
     if (has_shared) {
-      float gsh = sh_logit ? 1.0f / (1.0f + __expf(-sh_logit[t])) : 1.0f;
-      if (PACKED) gsh *= YP_POSTSCALE;
-      const float4 v = y4((size_t)(seg_off[n_seg_routed] + t));
-      o.x += gsh * v.x; o.y += gsh * v.y; o.z += gsh * v.z; o.w += gsh * v.w;
+      const float gsh = sh_logit ? 1.0f / (1.0f + __expf(-sh_logit[t])) : 1.0f;
+      take(n_sorted + t, PACKED ? gsh * YP_POSTSCALE : gsh);
     }
     // MoeFfn -> Add; may alias dst: each element is read, then written, by this thread
+    float* d = dst + (size_t)t * ne + c;
+    const float* h = residual != nullptr ? residual + (size_t)t * ne + c : nullptr;
     if (PACKED) {
-      float* d = dst + (size_t)t * ne + c;
-      if (residual != nullptr) {
-        const float* h = residual + (size_t)t * ne + c;
-        o.x += h[0]; o.y += h[8]; o.z += h[16]; o.w += h[24];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float2 v = make_float2(o[i], o[i + 4]);
+        if (h != nullptr) {
+          const float2 r = *reinterpret_cast<const float2*>(h + 8 * i);
+          v.x += r.x; v.y += r.y;
+        }
+        *reinterpret_cast<float2*>(d + 8 * i) = v;
       }
-      d[0] = o.x; d[8] = o.y; d[16] = o.z; d[24] = o.w;
     } else {
-      if (residual != nullptr) {
-        const float4 h = *reinterpret_cast<const float4*>(residual + (size_t)t * ne + c);
-        o.x += h.x; o.y += h.y; o.z += h.z; o.w += h.w;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        float4 v = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+        if (h != nullptr) {
+          const float4 r = *reinterpret_cast<const float4*>(h + 4 * i);
+          v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
+        }
+        *reinterpret_cast<float4*>(d + 4 * i) = v;
       }
-      *reinterpret_cast<float4*>(dst + (size_t)t * ne + c) = o;
     }
   }
 }
@@ -911,7 +929,7 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
   }
   if (c.dst) {
     auto comb = p.y_packed ? k_unpermute_combine_seg<true> : k_unpermute_combine_seg<false>;
-    comb<<<dim3((c.ne / 4 + 255) / 256, std::min(c.rows, 65535)), 256, 0, st>>>(y, pos_of_pair, c.wts, c.sh_logit, seg_off, n_seg_routed,
+    comb<<<dim3((c.ne / 8 + 255) / 256, std::min(c.rows, 65535)), 256, 0, st>>>(y, pos_of_pair, c.wts, c.sh_logit, seg_off, n_seg_routed,
                                                                                  c.shared_rows > 0 ? 1 : 0, c.rows, c.n_used, c.ne, c.residual, c.ids, c.down_scale,
                                                                                  c.weight_before, c.dst);
     ctx->launches += 1;
