@@ -383,6 +383,30 @@ __device__ __forceinline__ float q4k_dot64_i8(const uint4& hdr, const uint32_t (
   return d * (float)sv - dmin * (float)mv;
 }
 
+// The same for a Q5_K block: h = the block's 32 bytes of fifth bits (bit 2j of a byte belongs to the low nibbles of step j,
+// bit 2j + 1 to the high ones).  A 5-bit sub-block sum times its scale just fits int32, so the two are added as floats.
+__device__ __forceinline__ float q5k_dot64_i8(const uint4& hdr, const uint32_t (&q)[8], const uint32_t (&h)[8], const int (&xl)[16],
+                                              const int (&xh)[16], int sx0, int sx1, int j) {
+  int a_ll = 0, a_lh = 0, a_hl = 0, a_hh = 0;
+  const int rl = (4 - 2 * j) & 31, rh = (3 - 2 * j) & 31;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const unsigned lo = (__funnelshift_l(h[i], h[i], rl) & 0x10101010u) | (q[i] & 0x0F0F0F0Fu);
+    const unsigned hi = (__funnelshift_l(h[i], h[i], rh) & 0x10101010u) | ((q[i] >> 4) & 0x0F0F0F0Fu);
+    a_ll = dp4a_us(lo, xl[i], a_ll);
+    a_lh = dp4a_us(lo, xh[i], a_lh);
+    a_hl = dp4a_us(hi, xl[8 + i], a_hl);
+    a_hh = dp4a_us(hi, xh[8 + i], a_hh);
+  }
+  // |v| <= 32 * 31 * 32639 < 2^25, times a 6-bit scale < 2^31
+  const int v0 = a_lh * 256 + a_ll, v1 = a_hh * 256 + a_hl;
+  uint32_t scp, mp;
+  q4k_scale_min_pair(hdr.y, hdr.z, hdr.w, j, scp, mp);
+  const float sv = (float)((int)(scp & 0xFFu) * v0) + (float)((int)(scp >> 8) * v1);
+  const int mv = (int)(mp & 0xFFu) * sx0 + (int)(mp >> 8) * sx1;
+  return f16_bits_to_f32(hdr.x) * sv - f16_bits_to_f32(hdr.x >> 16) * (float)mv;
+}
+
 #endif  // __CUDACC__
 
 }  // namespace infr

@@ -16,6 +16,7 @@
 // activations arrive as 16-bit fixed point in two signed 8-bit limbs, the 4-bit (6-bit) codes are
 // masked in place and multiplied with integer dot-product instructions (exact integer sums), block
 // scales are applied per 32 (16) elements in f32, and row sums finish with warp shuffles.
+#include "formats.cuh"
 #include "kernels.cuh"
 
 namespace infr {
@@ -43,13 +44,15 @@ __device__ __forceinline__ bool in_band(const DecodeParams& p, int e) {
 // dependent integer ops and only other warps hide its latency.
 // Lane L owns the 64-element groups g = L, L+32, ... of the input (for ne = 2048 exactly one, so
 // its 64 activations stay in registers for the whole tile).
-template <int NG>
-__global__ void __maxnreg__(56) k_decode_gateup(DecodeParams p, int n_chunks) {
+// FIVE: the banks are Q5_K (176-byte blocks, 32 bytes of fifth bits behind the header) instead of Q4_K.
+template <int NG, bool FIVE>
+__global__ void __maxnreg__(FIVE ? 80 : 56) k_decode_gateup(DecodeParams p, int n_chunks) {
+  constexpr int BB = FIVE ? (int)Q5K_BLOCK_BYTES : (int)Q4K_BLOCK_BYTES, QS = FIVE ? 48 : 16;  // block bytes, offset of the code bytes
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[GU_MAX_CHUNKS];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int rb = p.ne / 256 * (int)Q4K_BLOCK_BYTES;  // bytes per weight row
+  const int rb = p.ne / 256 * BB;  // bytes per weight row
   const int GW = blockDim.x >> 5;  // warps = weight rows per chunk and role
   const int TR = GW * n_chunks;
   const int tiles = p.nff / TR, sh_tiles = p.sh_ff / TR;
@@ -163,19 +166,25 @@ __global__ void __maxnreg__(56) k_decode_gateup(DecodeParams p, int n_chunks) {
       if (g < n_groups) {
         if (NG > 1) load_x(g);
         const int blk = g >> 2, j = g & 3;
-        const uint4 gh = *reinterpret_cast<const uint4*>(grow + blk * Q4K_BLOCK_BYTES);
-        const uint4 uh = *reinterpret_cast<const uint4*>(urow + blk * Q4K_BLOCK_BYTES);
+        const unsigned char *gb = grow + blk * BB, *ub = urow + blk * BB;
+        auto words = [](const unsigned char* b, uint32_t (&w)[8]) {
+          const uint4 a = reinterpret_cast<const uint4*>(b)[0], c = reinterpret_cast<const uint4*>(b)[1];
+          w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = c.x; w[5] = c.y; w[6] = c.z; w[7] = c.w;
+        };
+        const uint4 gh = *reinterpret_cast<const uint4*>(gb), uh = *reinterpret_cast<const uint4*>(ub);
         uint32_t gq[8], uq[8];
-        {
-          const uint4 a = *reinterpret_cast<const uint4*>(grow + blk * Q4K_BLOCK_BYTES + 16 + 32 * j);
-          const uint4 b = *reinterpret_cast<const uint4*>(grow + blk * Q4K_BLOCK_BYTES + 32 + 32 * j);
-          gq[0] = a.x; gq[1] = a.y; gq[2] = a.z; gq[3] = a.w; gq[4] = b.x; gq[5] = b.y; gq[6] = b.z; gq[7] = b.w;
-          const uint4 c4 = *reinterpret_cast<const uint4*>(urow + blk * Q4K_BLOCK_BYTES + 16 + 32 * j);
-          const uint4 d4 = *reinterpret_cast<const uint4*>(urow + blk * Q4K_BLOCK_BYTES + 32 + 32 * j);
-          uq[0] = c4.x; uq[1] = c4.y; uq[2] = c4.z; uq[3] = c4.w; uq[4] = d4.x; uq[5] = d4.y; uq[6] = d4.z; uq[7] = d4.w;
+        words(gb + QS + 32 * j, gq);
+        words(ub + QS + 32 * j, uq);
+        if constexpr (FIVE) {
+          uint32_t g5[8], u5[8];
+          words(gb + 16, g5);
+          words(ub + 16, u5);
+          gsum += q5k_dot64_i8(gh, gq, g5, xl, xh, sx0, sx1, j);
+          usum += q5k_dot64_i8(uh, uq, u5, xl, xh, sx0, sx1, j);
+        } else {
+          gsum += q4k_dot64_i8(gh, gq, xl, xh, sx0, sx1, j);
+          usum += q4k_dot64_i8(uh, uq, xl, xh, sx0, sx1, j);
         }
-        gsum += q4k_dot64_i8(gh, gq, xl, xh, sx0, sx1, j);
-        usum += q4k_dot64_i8(uh, uq, xl, xh, sx0, sx1, j);
       }
     }
     gsum = warp_sum(gsum) * q_scale;
@@ -449,16 +458,17 @@ __global__ void __maxnreg__(56) k_decode_down(DecodeParams p, int TI) {
   }
 }
 
-size_t gateup_smem(int ne, int n_chunks, int gw = GU_WARPS) {
-  return (size_t)n_chunks * 2 * gw * (ne / 256 * Q4K_BLOCK_BYTES) + (size_t)(ne / 64) * GU_XQPITCH;
+size_t gateup_smem(int ne, int n_chunks, size_t gbb, int gw = GU_WARPS) {
+  return (size_t)n_chunks * 2 * gw * (ne / 256 * gbb) + (size_t)(ne / 64) * GU_XQPITCH;
 }
 
-int pick_chunks(int ne, int nff, int sh_ff) {
+// Chunks per CTA for gate/up banks of gbb bytes per block.
+int pick_chunks(int ne, int nff, int sh_ff, size_t gbb) {
   for (int c = 2; c >= 1; c >>= 1) {
     const int TR = GU_WARPS * c;
     if (nff % TR) continue;
     if (sh_ff && sh_ff % TR) continue;
-    if (gateup_smem(ne, c) <= 200 * 1024) return c;
+    if (gateup_smem(ne, c, gbb) <= 200 * 1024) return c;
   }
   return 0;
 }
@@ -499,7 +509,7 @@ bool decode_ffn_supported(const infr_cuda_ctx*, int ne, int nff, int sh_ff, int 
     if (why) *why = "small-m path: n_used larger than 32 is not covered";
     return false;
   }
-  if (!pick_chunks(ne, nff, sh_ff) || !pick_down_tile(ne, nff, sh_ff, n_used, down_q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES)) {
+  if (!pick_chunks(ne, nff, sh_ff, Q4K_BLOCK_BYTES) || !pick_down_tile(ne, nff, sh_ff, n_used, down_q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES)) {
     if (why) *why = "small-m path: tile does not fit shared memory for these dims";
     return false;
   }
@@ -507,15 +517,27 @@ bool decode_ffn_supported(const infr_cuda_ctx*, int ne, int nff, int sh_ff, int 
 }
 
 int32_t launch_decode_ffn(infr_cuda_ctx* ctx, const DecodeParams& p, bool pdl, uint32_t stages) {
-  if (!BankTypes{p.gate_dt, p.up_dt, p.down_dt}.tuned()) return launch_anyfmt_decode(ctx, p, pdl, stages);
   const bool has_sh = p.sh_gate != nullptr;
   const int sh_ff = has_sh ? p.sh_ff : 0;
-  const int n_chunks = pick_chunks(p.ne, p.nff, sh_ff);
-  const size_t dbb = p.down_q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
-  const int TI = pick_down_tile(p.ne, p.nff, sh_ff, p.n_used, dbb);
-  if (!n_chunks || !TI) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "small-m path: tile does not fit shared memory");
+  const BankTypes bt = {p.gate_dt, p.up_dt, p.down_dt};
+  // The two stages meet in f32 activations, so each takes the kernel written for its own banks (gate and up both Q4_K or
+  // both Q5_K; down Q6_K or Q4_K) and the generic one otherwise: two streams of a Q5_K / Q5_K / Q6_K layer took 50 us on
+  // the generic pair.
+  const bool five = p.gate_dt == INFR_CUDA_DT_Q5K;
+  const size_t gbb = five ? Q5K_BLOCK_BYTES : Q4K_BLOCK_BYTES, dbb = p.down_q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
+  const int n_chunks = pick_chunks(p.ne, p.nff, sh_ff, gbb), TI = pick_down_tile(p.ne, p.nff, sh_ff, p.n_used, dbb);
+  const bool wide_ok = bt.tuned() || p.ne / 64 <= 32 * 4;
+  const bool gu_own = p.gate_dt == p.up_dt && (five || p.gate_dt == INFR_CUDA_DT_Q4K) && n_chunks && wide_ok;
+  const bool dn_own = (p.down_q4k || p.down_dt == INFR_CUDA_DT_Q6K) && TI;
+  if (bt.tuned() && !(gu_own && dn_own)) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "small-m path: tile does not fit shared memory");
+  if (!gu_own && (stages & 2u)) {
+    const int32_t rc = launch_anyfmt_decode(ctx, p, pdl, 2u);
+    if (rc) return rc;
+    stages &= ~2u;
+  }
+  if (!dn_own && !(stages & 2u)) return (stages & 4u) ? launch_anyfmt_decode(ctx, p, pdl, 4u) : INFR_CUDA_OK;
   int gw = GU_WARPS;
-  int TR = gw * n_chunks;
+  int TR = gw * std::max(n_chunks, 1);
   int jobs = p.rows * p.n_used * (p.nff / TR) + (has_sh ? p.rows * (sh_ff / TR) : 0);
   int n_chunks_gu = n_chunks;
   {
@@ -531,7 +553,7 @@ int32_t launch_decode_ffn(infr_cuda_ctx* ctx, const DecodeParams& p, bool pdl, u
       jobs = p.rows * p.n_used * (p.nff / TR) + (has_sh ? p.rows * (sh_ff / TR) : 0);
     }
   }
-  size_t smem_gu = gateup_smem(p.ne, n_chunks_gu, gw);
+  size_t smem_gu = gateup_smem(p.ne, n_chunks_gu, gbb, gw);
   // A grid that fits the device one CTA per SM is spread that way: gate/up CTAs start while the
   // router's CTAs still hold some SMs and would otherwise pair up on the free ones, halving their
   // copy bandwidth and leaving no room for the down kernel's CTAs to start beside them.  A request
@@ -546,15 +568,16 @@ int32_t launch_decode_ffn(infr_cuda_ctx* ctx, const DecodeParams& p, bool pdl, u
   };
   if (stages & 2u) {
     if (ng == 1)
-      e = run_gu(k_decode_gateup<1>);
+      e = five ? run_gu(k_decode_gateup<1, true>) : run_gu(k_decode_gateup<1, false>);
     else if (ng == 2)
-      e = run_gu(k_decode_gateup<2>);
+      e = five ? run_gu(k_decode_gateup<2, true>) : run_gu(k_decode_gateup<2, false>);
     else
-      e = run_gu(k_decode_gateup<4>);
+      e = five ? run_gu(k_decode_gateup<4, true>) : run_gu(k_decode_gateup<4, false>);
     ctx->launches += 1;
     if (e != cudaSuccess) return check_cuda(ctx, e, "k_decode_gateup launch");
   }
   if (!(stages & 4u)) return INFR_CUDA_OK;
+  if (!dn_own) return launch_anyfmt_decode(ctx, p, pdl, 4u);
 
   const size_t smem_dn = down_smem(TI, p.nff, sh_ff, p.n_used, dbb);
   e = ensure_smem(reinterpret_cast<const void*>(k_decode_down), smem_dn);

@@ -29,10 +29,9 @@ namespace infr {
 namespace {
 
 constexpr int EM_FEAT = 32;         // gate/up: features per CTA
-constexpr int EM_GU_WARPS = 4;      // consumer warps: two 16-feature groups x two block parities
 constexpr int EM_MAX_STAGES = 4;
-constexpr int EM_DN_WARPS = 4;      // down: 16 output rows per warp (or fewer rows and a split of the blocks)
 constexpr int EM_SEG = 8;           // token rows per segment = the N extent of one MMA
+constexpr int EM_NARROW = 4;        // segments of up to this many: both limbs of a token as columns of one MMA
 
 __device__ __forceinline__ void mma_u8s8_k32(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -152,11 +151,94 @@ __global__ void __launch_bounds__(1024) k_em_bucket(EmParams p, int seg_cap) {
 // ---------------------------------------------------------------------------------------------
 // gate/up + activation
 // ---------------------------------------------------------------------------------------------
+// One 256-weight block of a warp's rows (gate g, gate g + 8, up g, up g + 8 of its feature group: `w`, eight rows on, `box`
+// bytes on) against the segment's tokens, added to fg, fu.
+//   wide: the 8 MMA columns are 8 tokens, one MMA per limb (x, x + xh); a thread ends with rows g, g + 8 of tokens 2t, 2t + 1.
+//   NARROW (at most four tokens, which is most segments of a decode batch): the columns are the two limbs of four
+//   tokens side by side, so a sub-block takes one MMA per role and a thread ends with the low and high sums of rows g,
+//   g + 8 of token t: half the MMAs, fragment loads and scale multiplies.
+template <bool NARROW>
+__device__ __forceinline__ void gateup_block(const unsigned char* w, uint32_t box, const unsigned char* x, uint32_t xh, const int* sum0, int sum_step,
+                                             int b, float (&fg)[4], float (&fu)[4]) {
+  constexpr int NT = NARROW ? 1 : 2;  // tokens of a thread
+  const int t = threadIdx.x & 3;
+  const unsigned char* rows4[4] = {w, w + 8 * Q4K_BLOCK_BYTES, w + box, w + box + 8 * Q4K_BLOCK_BYTES};
+  uint4 hdr[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) hdr[r] = *reinterpret_cast<const uint4*>(rows4[r]);
+  int svl[4][NT], svh[4][NT], mv[4][NT];  // [row][token]
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int k = 0; k < NT; ++k) svl[r][k] = svh[r][k] = mv[r][k] = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t wA[4], wB[4], scp[4], mp[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const unsigned char* q = rows4[r] + 16 + 32 * j + 4 * t;
+      wA[r] = *reinterpret_cast<const uint32_t*>(q);
+      wB[r] = *reinterpret_cast<const uint32_t*>(q + 16);
+      q4k_scale_min_pair(hdr[r].y, hdr[r].z, hdr[r].w, j, scp[r], mp[r]);
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int lsb = b * 8 + 2 * j + half;  // sub-block index inside the stage
+      const uint32_t b0 = *reinterpret_cast<const uint32_t*>(x + lsb * 32), b1 = *reinterpret_cast<const uint32_t*>(x + lsb * 32 + 16);
+      uint32_t a[4][2];
+      int sc[4], mn[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        a[r][0] = (wA[r] >> (4 * half)) & 0x0F0F0F0Fu;
+        a[r][1] = (wB[r] >> (4 * half)) & 0x0F0F0F0Fu;
+        sc[r] = (int)((scp[r] >> (8 * half)) & 0xFFu);
+        mn[r] = (int)((mp[r] >> (8 * half)) & 0xFFu);
+      }
+      int c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
+      mma_u8s8_k32(c0, a[0][0], a[1][0], a[0][1], a[1][1], b0, b1);
+      mma_u8s8_k32(c1, a[2][0], a[3][0], a[2][1], a[3][1], b0, b1);
+      if (NARROW) {
+        const int sx = sum0[lsb];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          svl[r][0] += sc[r] * (r < 2 ? c0[2 * (r & 1)] : c1[2 * (r & 1)]);
+          svh[r][0] += sc[r] * (r < 2 ? c0[2 * (r & 1) + 1] : c1[2 * (r & 1) + 1]);
+          mv[r][0] += mn[r] * sx;
+        }
+      } else {
+        const uint32_t b0h = *reinterpret_cast<const uint32_t*>(x + xh + lsb * 32), b1h = *reinterpret_cast<const uint32_t*>(x + xh + lsb * 32 + 16);
+        int h0[4] = {0, 0, 0, 0}, h1[4] = {0, 0, 0, 0};
+        mma_u8s8_k32(h0, a[0][0], a[1][0], a[0][1], a[1][1], b0h, b1h);
+        mma_u8s8_k32(h1, a[2][0], a[3][0], a[2][1], a[3][1], b0h, b1h);
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int k = 0; k < NT; ++k) {
+            const int i = 2 * (r & 1) + k;
+            svl[r][k] += sc[r] * (r < 2 ? c0[i] : c1[i]);
+            svh[r][k] += sc[r] * (r < 2 ? h0[i] : h1[i]);
+            mv[r][k] += mn[r] * sum0[lsb + k * sum_step];
+          }
+      }
+    }
+  }
+  // once per block: value = d * sum(sc * sum(q X)) - dmin * sum(m * sum(X)), X = 256 hi + lo
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const float d = f16_bits_to_f32(hdr[r].x), dm = f16_bits_to_f32(hdr[r].x >> 16);
+#pragma unroll
+    for (int k = 0; k < NT; ++k) {
+      const float v = d * fmaf(256.f, (float)svh[r][k], (float)svl[r][k]) - dm * (float)mv[r][k];
+      (r < 2 ? fg : fu)[2 * (r & 1) + k] += v;
+    }
+  }
+}
+
 // Job = (segment of up to 8 token rows, tile of EM_FEAT features, both roles); the CTAs are persistent
-// and take jobs blockIdx.x, blockIdx.x + gridDim.x, ...  Four consumer warps: warp (fw, ks) owns features
-// 16 fw .. 16 fw + 15 and every second block of the row (ks = block parity); MMA rows are the 16 gate rows
+// and take jobs blockIdx.x, blockIdx.x + gridDim.x, ...  2 KS consumer warps: warp (fw, ks) owns features
+// 16 fw .. 16 fw + 15 and every KS-th block of the row; MMA rows are the 16 gate rows
 // and, in a second accumulator set, the 16 up rows, so a thread ends with gate and up of the same
-// (feature, token).  The fifth warp is the producer: per stage it streams KB blocks of every weight row
+// (feature, token).  The last warp is the producer: per stage it streams KB blocks of every weight row
 // (one tiled TMA copy per block and role: a box of 32 rows x 144 bytes out of rows a whole row apart), the
 // same K range of the tokens' fixed-point limbs and their sub-block sums (1-D bulk copies), through a
 // ring of S stages that runs on across jobs, so the next job's weights arrive while this one is
@@ -164,14 +246,25 @@ __global__ void __launch_bounds__(1024) k_em_bucket(EmParams p, int seg_cap) {
 // consecutive words) conflict-free.
 // Scales are applied in integers: per block a thread accumulates sc * (limb sums) and m * sum(X) in int32
 // (bounded: 8 sub-blocks x 63 x 32 x 15 x 128 < 2^31) and converts once per block.
-__global__ void __launch_bounds__((EM_GU_WARPS + 1) * 32) k_em_gateup(EmParams p, int KB, int S, int xpitch, int gu_rows,
-                                                                      const __grid_constant__ CUtensorMap tm_gate,
-                                                                      const __grid_constant__ CUtensorMap tm_up,
-                                                                      const __grid_constant__ CUtensorMap tm_sh_gate,
-                                                                      const __grid_constant__ CUtensorMap tm_sh_up) {
+// What the consumers need of a job, put beside its first stage by the producer, which looks it up a job ahead (the lookups
+// are a chain of three L2 reads; made by every warp at both ends of a job they cost as much as a third of it).
+struct EmJob {
+  int job, e, cnt;  // job < 0: no more
+  int pair[8];
+  float xs[8], wp[8];  // value of one step of the token's fixed-point row; weight on the expert's input
+};
+
+template <int KS>
+__global__ void __launch_bounds__((2 * KS + 1) * 32, 2) k_em_gateup(EmParams p, int KB, int S, int xpitch, int gu_rows,
+                                                                    const __grid_constant__ CUtensorMap tm_gate,
+                                                                    const __grid_constant__ CUtensorMap tm_up,
+                                                                    const __grid_constant__ CUtensorMap tm_sh_gate,
+                                                                    const __grid_constant__ CUtensorMap tm_sh_up) {
+  constexpr int EM_GU_WARPS = 2 * KS;  // consumer warps
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_full[EM_MAX_STAGES], s_empty[EM_MAX_STAGES];
-  __shared__ float s_red[2][2][32][8];  // [job parity][feature group][lane][gate 4 | up 4]
+  __shared__ float s_red[2][2][32][8];  // [slot][feature group][lane][gate 4 | up 4]
+  __shared__ EmJob s_job[2];            // two suffice: the ring holds no more stages than a job has
   __shared__ int s_abort;               // a consumer warp's bounded wait ran out: all consumers leave together
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -199,37 +292,85 @@ __global__ void __launch_bounds__((EM_GU_WARPS + 1) * 32) k_em_gateup(EmParams p
 
   if (warp == EM_GU_WARPS) {
     bool ok = true;
-    for (int job = blockIdx.x; job < n_jobs && ok; job += gridDim.x) {
+    // the next job at or after j that has rows in its tile
+    const int both = p.sh_ff ? min(p.nff, p.sh_ff) : p.nff;  // rows that every segment has
+    int e_n = 0, cnt_n = 0, off_n = 0;
+    auto seek = [&](int j) {
+      for (; j < n_jobs; j += gridDim.x) {
+        const int seg = j / tiles_max, tile = j - seg * tiles_max;
+        e_n = __ldcg(p.seg_expert + seg);
+        cnt_n = __ldcg(p.seg_cnt + seg);
+        off_n = __ldcg(p.seg_off + seg);
+        if (tile * EM_FEAT < both || tile * EM_FEAT < (e_n >= p.n_expert ? p.sh_ff : p.nff)) break;
+      }
+      return j;
+    };
+    int pr_n = 0, row_n = 0;
+    float xs_n = 0.f, wp_n = 1.f;
+    auto pair_of = [&] { pr_n = (lane & 7) < cnt_n ? __ldcg(p.seg_pairs + off_n + (lane & 7)) : 0; };
+    auto token_of = [&] {
+      row_n = pr_n >= P ? pr_n - P : pr_n / p.n_used;
+      xs_n = __ldcg(p.xscale + row_n);
+      wp_n = (p.weight_before && e_n < p.n_expert) ? __ldcg(p.wts + pr_n) : 1.0f;
+    };
+    int job_n = seek(blockIdx.x);
+    if (job_n < n_jobs) {
+      pair_of();
+      token_of();
+    }
+    for (int k = 0; ok; ++k) {
+      const int job = job_n, e = e_n, cnt = cnt_n, pr = pr_n, row = row_n;
+      const float xs = xs_n, wp = wp_n;
+      const bool last = job >= n_jobs;
       const int seg = job / tiles_max, tile = job - seg * tiles_max;
-      const int e = __ldcg(p.seg_expert + seg), cnt = __ldcg(p.seg_cnt + seg), off = __ldcg(p.seg_off + seg);
       const bool shared_seg = e >= p.n_expert;
-      if (tile * EM_FEAT >= (shared_seg ? p.sh_ff : p.nff)) continue;
       const CUtensorMap* tmg = shared_seg ? &tm_sh_gate : &tm_gate;
       const CUtensorMap* tmu = shared_seg ? &tm_sh_up : &tm_up;
       const int bank_row0 = (shared_seg ? 0 : e * gu_rows) + tile * EM_FEAT;  // with gate and up in one bank the up map starts n_ff_exp rows in
-      // lanes 8-23: a limb row of token (lane & 7); lanes 24-31: its sums.  A padding slot reads row 0; its results are dropped.
-      int row = 0;
-      if (lane >= 8 && (lane & 7) < cnt) {
-        const int pr = __ldcg(p.seg_pairs + off + (lane & 7));
-        row = pr >= P ? pr - P : pr / p.n_used;
-      }
+      // lanes 8-23: a limb row of token (lane & 7); lanes 24-31: its sums.  A padding slot keeps what it held; its results are dropped.
+      // In a narrow segment (see gateup_block) the high limbs follow the low ones four rows on.
+      const bool mine = (lane & 7) < cnt;
+      const uint32_t x_slot = lane < 16 ? lane - 8 : (cnt <= EM_NARROW ? EM_NARROW : 8) + (lane & 7);
+      if (!last) job_n = seek(job + gridDim.x);
       for (int kc = 0; kc < n_kc; ++kc, ++it) {
         const int s = it % S;
         if (it >= (uint32_t)S && !mbar_wait_bounded(&s_empty[s], ((it / S) - 1) & 1)) { ok = false; break; }
         unsigned char* st = smem + (size_t)s * stage_bytes;
+        if (kc == 0) {
+          // free: with a stage of this job the consumers have left the job before last
+          EmJob& d = s_job[k & 1];
+          if (lane == 0) {
+            d.job = last ? -1 : job;
+            d.e = e;
+            d.cnt = cnt;
+          }
+          if (lane < 8) {
+            d.pair[lane] = pr;
+            d.xs[lane] = xs;
+            d.wp[lane] = wp;
+          }
+          __syncwarp();
+          if (last) {
+            if (lane == 0) mbar_arrive(&s_full[s]);
+            break;
+          }
+        }
         if (lane == 0)
-          mbar_arrive_expect_tx(&s_full[s], (uint32_t)(2 * EM_FEAT) * KB * Q4K_BLOCK_BYTES + (uint32_t)16 * KB * 256 + (uint32_t)8 * KB * 32);
+          mbar_arrive_expect_tx(&s_full[s], (uint32_t)(2 * EM_FEAT) * KB * Q4K_BLOCK_BYTES + (uint32_t)cnt * KB * (2 * 256 + 32));
         __syncwarp();
         if (lane < 2 * KB) {
           const int b = lane >> 1, role = lane & 1;
           tma_load_2d(st + (size_t)lane * BOX, role ? tmu : tmg, (kc * KB + b) * (int)Q4K_BLOCK_BYTES, bank_row0, &s_full[s]);
-        } else if (lane >= 8 && lane < 24) {
+        } else if (lane >= 8 && lane < 24 && mine) {
           const int8_t* src = ((lane >= 16) ? p.xq_hi : p.xq_lo) + (size_t)row * p.ne + (size_t)kc * KB * 256;
-          bulk_g2s(st + w_bytes + (size_t)(lane - 8) * xpitch, src, (uint32_t)KB * 256, &s_full[s]);
-        } else if (lane >= 24) {
+          bulk_g2s(st + w_bytes + (size_t)x_slot * xpitch, src, (uint32_t)KB * 256, &s_full[s]);
+        } else if (lane >= 24 && mine) {
           bulk_g2s(st + w_bytes + x_bytes + (size_t)(lane - 24) * spitch * 4, p.xsum + (size_t)row * nsb + (size_t)kc * KB * 8, (uint32_t)KB * 32, &s_full[s]);
         }
+        if (kc == 0 && job_n < n_jobs) pair_of();
       }
+      if (last) break;
+      if (job_n < n_jobs) token_of();
     }
     if (!ok && lane == 0) atomicExch(&p.status->timeout, 7);
     return;
@@ -237,122 +378,79 @@ __global__ void __launch_bounds__((EM_GU_WARPS + 1) * 32) k_em_gateup(EmParams p
 
   // consumers
   const int fw = warp & 1, ks = warp >> 1;
-  bool ok = true;
   int jpar = 0;
-  for (int job = blockIdx.x; job < n_jobs && ok; job += gridDim.x) {
-    const int seg = job / tiles_max, tile = job - seg * tiles_max;
-    const int e = __ldcg(p.seg_expert + seg), cnt = __ldcg(p.seg_cnt + seg), off = __ldcg(p.seg_off + seg);
-    const bool shared_seg = e >= p.n_expert;
-    if (tile * EM_FEAT >= (shared_seg ? p.sh_ff : p.nff)) continue;
+  bool ok = true;
+  for (int k = 0; ok; ++k) {
+    const EmJob& d = s_job[k & 1];
+    bool narrow = false;
     float fg[4] = {0.f, 0.f, 0.f, 0.f}, fu[4] = {0.f, 0.f, 0.f, 0.f};
     for (int kc = 0; kc < n_kc; ++kc, ++it) {
       const int s = it % S;
       if (!mbar_wait_bounded(&s_full[s], (it / S) & 1)) { ok = false; break; }
+      if (kc == 0) {
+        if (d.job < 0) return;
+        narrow = d.cnt <= EM_NARROW;
+      }
       const unsigned char* st = smem + (size_t)s * stage_bytes;
-      const unsigned char* xlo = st + w_bytes + (size_t)g * xpitch + 4 * t;  // B fragments: token g
-      const unsigned char* xhi = xlo + (size_t)8 * xpitch;
-      const int* sum0 = reinterpret_cast<const int*>(st + w_bytes + x_bytes) + (2 * t) * spitch;  // accumulator columns 2t, 2t + 1
-      const int* sum1 = sum0 + spitch;
-      for (int b = ks; b < KB; b += 2) {
-        // this block's rows: gate g, gate g + 8, up g, up g + 8 of the warp's feature group
-        const unsigned char* wst = st + (size_t)b * 2 * BOX + (size_t)(fw * 16 + g) * Q4K_BLOCK_BYTES;
-        const unsigned char* rows4[4] = {wst, wst + 8 * Q4K_BLOCK_BYTES, wst + BOX, wst + BOX + 8 * Q4K_BLOCK_BYTES};
-        uint4 hdr[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) hdr[r] = *reinterpret_cast<const uint4*>(rows4[r]);
-        int svh_g[4] = {0, 0, 0, 0}, svl_g[4] = {0, 0, 0, 0}, mv_g[4] = {0, 0, 0, 0};
-        int svh_u[4] = {0, 0, 0, 0}, svl_u[4] = {0, 0, 0, 0}, mv_u[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint32_t wA[4], wB[4], scp[4], mp[4];
-#pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            const unsigned char* q = rows4[r] + 16 + 32 * j + 4 * t;
-            wA[r] = *reinterpret_cast<const uint32_t*>(q);
-            wB[r] = *reinterpret_cast<const uint32_t*>(q + 16);
-            q4k_scale_min_pair(hdr[r].y, hdr[r].z, hdr[r].w, j, scp[r], mp[r]);
-          }
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int lsb = b * 8 + 2 * j + half;  // sub-block index inside the stage
-            const uint32_t b0l = *reinterpret_cast<const uint32_t*>(xlo + lsb * 32), b1l = *reinterpret_cast<const uint32_t*>(xlo + lsb * 32 + 16),
-                           b0h = *reinterpret_cast<const uint32_t*>(xhi + lsb * 32), b1h = *reinterpret_cast<const uint32_t*>(xhi + lsb * 32 + 16);
-            const int sx0 = sum0[lsb], sx1 = sum1[lsb];
-            uint32_t a[4][2];
-            int sc[4], mn[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-              a[r][0] = (wA[r] >> (4 * half)) & 0x0F0F0F0Fu;
-              a[r][1] = (wB[r] >> (4 * half)) & 0x0F0F0F0Fu;
-              sc[r] = (int)((scp[r] >> (8 * half)) & 0xFFu);
-              mn[r] = (int)((mp[r] >> (8 * half)) & 0xFFu);
-            }
-            int cgl[4] = {0, 0, 0, 0}, cgh[4] = {0, 0, 0, 0}, cul[4] = {0, 0, 0, 0}, cuh[4] = {0, 0, 0, 0};
-            mma_u8s8_k32(cgl, a[0][0], a[1][0], a[0][1], a[1][1], b0l, b1l);
-            mma_u8s8_k32(cgh, a[0][0], a[1][0], a[0][1], a[1][1], b0h, b1h);
-            mma_u8s8_k32(cul, a[2][0], a[3][0], a[2][1], a[3][1], b0l, b1l);
-            mma_u8s8_k32(cuh, a[2][0], a[3][0], a[2][1], a[3][1], b0h, b1h);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int r = i >> 1, sx = (i & 1) ? sx1 : sx0;  // accumulator rows g (i < 2) and g + 8; columns 2t, 2t + 1
-              svl_g[i] += sc[r] * cgl[i];
-              svh_g[i] += sc[r] * cgh[i];
-              mv_g[i] += mn[r] * sx;
-              svl_u[i] += sc[2 + r] * cul[i];
-              svh_u[i] += sc[2 + r] * cuh[i];
-              mv_u[i] += mn[2 + r] * sx;
-            }
-          }
-        }
-        // once per block: value = d * sum(sc * sum(q X)) - dmin * sum(m * sum(X)), X = 256 hi + lo
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = i >> 1;
-          const float dg = f16_bits_to_f32(hdr[r].x), dmg = f16_bits_to_f32(hdr[r].x >> 16);
-          const float du = f16_bits_to_f32(hdr[2 + r].x), dmu = f16_bits_to_f32(hdr[2 + r].x >> 16);
-          fg[i] += dg * fmaf(256.f, (float)svh_g[i], (float)svl_g[i]) - dmg * (float)mv_g[i];
-          fu[i] += du * fmaf(256.f, (float)svh_u[i], (float)svl_u[i]) - dmu * (float)mv_u[i];
-        }
+      const unsigned char* wst = st + (size_t)(fw * 16 + g) * Q4K_BLOCK_BYTES;
+      const unsigned char* x0 = st + w_bytes;
+      const int* sums = reinterpret_cast<const int*>(st + w_bytes + x_bytes);
+      for (int b = ks; b < KB; b += KS) {
+        if (narrow)
+          gateup_block<true>(wst + (size_t)b * 2 * BOX, BOX, x0 + (size_t)((g & 1) * EM_NARROW + (g >> 1)) * xpitch + 4 * t, 0, sums + t * spitch, 0, b, fg, fu);
+        else
+          gateup_block<false>(wst + (size_t)b * 2 * BOX, BOX, x0 + (size_t)g * xpitch + 4 * t, (uint32_t)8 * xpitch, sums + 2 * t * spitch, spitch, b, fg, fu);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_empty[s]);  // (arrivals after the producer's last wait complete phases nobody waits for)
     }
-    // the two block-parity halves of a feature group meet in shared memory (consumer warps only: named
-    // barrier 1).  The buffer alternates with the job, so the next job's writes cannot overtake this job's reads.
-    if (ks == 1) {
+    // the warps of a feature group add their sums up through two slots of shared memory (consumer warps only: named barrier 1).
+    // Four: 2 and 3 onto 0 and 1, then 1 onto 0.  Two: the jobs take the slots in turn.
+    if (!ok) s_abort = 1;
+    auto put = [&](int slot) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        s_red[jpar][fw][lane][i] = fg[i];
-        s_red[jpar][fw][lane][4 + i] = fu[i];
+        s_red[slot][fw][lane][i] = fg[i];
+        s_red[slot][fw][lane][4 + i] = fu[i];
       }
-    }
-    if (!ok) s_abort = 1;
-    asm volatile("bar.sync 1, %0;" ::"n"(EM_GU_WARPS * 32) : "memory");
+    };
+    auto add = [&](int slot) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        fg[i] += s_red[slot][fw][lane][i];
+        fu[i] += s_red[slot][fw][lane][4 + i];
+      }
+    };
+    auto meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(EM_GU_WARPS * 32) : "memory"); };
+    if (KS == 4 ? ks >= 2 : ks == 1) put(KS == 4 ? ks - 2 : jpar);
+    meet();
     if (*reinterpret_cast<volatile int*>(&s_abort)) {
       ok = false;
       break;
     }
+    if (KS == 4) {
+      if (ks < 2) add(ks);
+      if (ks == 1) put(1);  // (slot 1 was this warp's own to read)
+      meet();
+      if (ks == 0) add(1);
+      meet();  // the slots are free for the next job
+    } else {
+      if (ks == 0) add(jpar);
+      jpar ^= 1;
+    }
     if (ks == 0) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        fg[i] += s_red[jpar][fw][lane][i];
-        fu[i] += s_red[jpar][fw][lane][4 + i];
-      }
       // epilogue: act[pair, feature] = act_fn(gate) * up, f32
-      const float clamp = shared_seg ? 0.f : p.clamp;
-      const int f0 = tile * EM_FEAT + fw * 16;
+      const float clamp = d.e >= p.n_expert ? 0.f : p.clamp;
+      const int f0 = d.job % tiles_max * EM_FEAT + fw * 16, cnt = d.cnt;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int tk = 2 * t + (i & 1);
-        if (tk >= cnt) continue;
-        const int pr = __ldcg(p.seg_pairs + off + tk);
-        const int row = pr >= P ? pr - P : pr / p.n_used;
-        const float xs = __ldcg(p.xscale + row);
-        const float wp = (p.weight_before && !shared_seg) ? __ldcg(p.wts + pr) : 1.0f;
-        p.act[(size_t)pr * nffmax + f0 + g + 8 * (i >> 1)] = gated_act(p.act_kind, clamp, wp * (fg[i] * xs), wp * (fu[i] * xs));
+        // wide: rows g (i < 2) and g + 8 of tokens 2 t, 2 t + 1; narrow: rows g (i = 0) and g + 8 (i = 2) of token t
+        const int tk = narrow ? t : 2 * t + (i & 1);
+        if (tk >= cnt || (narrow && (i & 1))) continue;
+        const float xs = d.xs[tk], wp = d.wp[tk];
+        p.act[(size_t)d.pair[tk] * nffmax + f0 + g + 8 * (i >> 1)] = gated_act(p.act_kind, clamp, wp * (fg[i] * xs), wp * (fu[i] * xs));
       }
     }
-    jpar ^= 1;
   }
   if (!ok && lane == 0) atomicExch(&p.status->timeout, 7);
 }
@@ -360,6 +458,144 @@ __global__ void __launch_bounds__((EM_GU_WARPS + 1) * 32) k_em_gateup(EmParams p
 // ---------------------------------------------------------------------------------------------
 // down
 // ---------------------------------------------------------------------------------------------
+// One 256-weight block of a warp's 16 output rows (rows g and g + 8) against the segment's tokens, added to acc (rows
+// g: 0, 1; g + 8: 2, 3; wide: tokens 2t, 2t + 1; narrow: token t in 0 and 2).
+//
+// Q4_K: header (d, dmin, 12 scale bytes), then per 64 weights 32 code bytes whose low nibbles are the first 32-element
+// group and high nibbles the second.
+template <bool NARROW>
+__device__ __forceinline__ void down_block_q4(const unsigned char* blk0, const unsigned char* blk1, const unsigned char* alo, const unsigned char* ahi,
+                                              const int* sum0, const int* sum1, int b, float (&acc)[4]) {
+  constexpr int NT = NARROW ? 1 : 2;
+  const int t = threadIdx.x & 3;
+  const unsigned char* blk[2] = {blk0, blk1};
+  const uint4 hdr[2] = {*reinterpret_cast<const uint4*>(blk[0]), *reinterpret_cast<const uint4*>(blk[1])};
+  int svl[2][NT], svh[2][NT], mv[2][NT];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int k = 0; k < NT; ++k) svl[r][k] = svh[r][k] = mv[r][k] = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t scp[2], mp[2], w0[2], w1[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      q4k_scale_min_pair(hdr[r].y, hdr[r].z, hdr[r].w, j, scp[r], mp[r]);
+      w0[r] = *reinterpret_cast<const uint32_t*>(blk[r] + 16 + 32 * j + 4 * t);       // k = 4 t .. 4 t + 3 of a group
+      w1[r] = *reinterpret_cast<const uint32_t*>(blk[r] + 32 + 32 * j + 4 * t);       // k = 16 + 4 t ..
+    }
+#pragma unroll
+    for (int hn = 0; hn < 2; ++hn) {
+      const int k0 = b * 256 + j * 64 + hn * 32, grp = k0 >> 4;
+      const uint32_t a00 = (w0[0] >> (4 * hn)) & 0x0F0F0F0Fu, a10 = (w0[1] >> (4 * hn)) & 0x0F0F0F0Fu,
+                     a01 = (w1[0] >> (4 * hn)) & 0x0F0F0F0Fu, a11 = (w1[1] >> (4 * hn)) & 0x0F0F0F0Fu;
+      int cl[4] = {0, 0, 0, 0}, ch[4] = {0, 0, 0, 0};
+      mma_u8s8_k32(cl, a00, a10, a01, a11, *reinterpret_cast<const uint32_t*>(alo + k0), *reinterpret_cast<const uint32_t*>(alo + k0 + 16));
+      if (!NARROW) mma_u8s8_k32(ch, a00, a10, a01, a11, *reinterpret_cast<const uint32_t*>(ahi + k0), *reinterpret_cast<const uint32_t*>(ahi + k0 + 16));
+      const int m[2] = {sum0[grp] + sum0[grp + 1], NARROW ? 0 : sum1[grp] + sum1[grp + 1]};
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int sc = (int)((scp[r] >> (8 * hn)) & 0xFFu), mn = (int)((mp[r] >> (8 * hn)) & 0xFFu);
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          svl[r][k] += sc * cl[2 * r + k];
+          svh[r][k] += sc * (NARROW ? cl[2 * r + 1] : ch[2 * r + k]);
+          mv[r][k] += mn * m[k];
+        }
+      }
+    }
+  }
+  // sum over the block of d sc sum(q X) - dmin m sum(X), X = 256 hi + lo
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const float d = f16_bits_to_f32(hdr[r].x), dmin = f16_bits_to_f32(hdr[r].x >> 16);
+#pragma unroll
+    for (int k = 0; k < NT; ++k)
+      acc[2 * r + k] = fmaf(d, fmaf(256.f, (float)svh[r][k], (float)svl[r][k]), fmaf(-dmin, (float)mv[r][k], acc[2 * r + k]));
+  }
+}
+
+// Byte `i` of w as a signed integer, by one byte permute that replicates the sign.
+__device__ __forceinline__ int sext_byte(uint32_t w, int i) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(w), "r"((uint32_t)(i * 0x1111) | 0x8880u));
+  return (int)r;
+}
+
+// Q6_K: the slab starts on a 16-byte boundary, the rows' blocks at byte offsets ro0, ro1 on 2-byte ones.
+template <bool NARROW>
+__device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_t ro0, uint32_t ro1, const unsigned char* alo, const unsigned char* ahi,
+                                              const int* sum0, const int* sum1, int b, float (&acc)[4]) {
+  constexpr int NT = NARROW ? 1 : 2;
+  const int t = threadIdx.x & 3;
+  // per row: aligned view of the block, the shift that realigns it, d and the 16 scales
+  const uint32_t* wq[2];
+  uint32_t sh[2];
+  float d[2];
+  uint32_t sc[2][4];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const uint32_t ro = r ? ro1 : ro0;
+    sh[r] = (ro & 3u) * 8;
+    wq[r] = reinterpret_cast<const uint32_t*>(slab + (ro & ~3u));
+    d[r] = f16_bits_to_f32(*reinterpret_cast<const unsigned short*>(slab + ro + 208));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sc[r][i] = __funnelshift_r(wq[r][48 + i], wq[r][49 + i], sh[r]);
+  }
+  int svl[2][NT], svh[2][NT], mv[2][NT];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int k = 0; k < NT; ++k) svl[r][k] = svh[r][k] = mv[r][k] = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int lh = 0; lh < 2; ++lh) {
+      // words of ql (two 32-byte runs) and qh that hold l = 16 lh + 4 t .. + 3 of this half
+      uint32_t A[2], B[2], H[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int o = 16 * h + 4 * lh + t;
+        A[r] = __funnelshift_r(wq[r][o], wq[r][o + 1], sh[r]);
+        B[r] = __funnelshift_r(wq[r][o + 8], wq[r][o + 9], sh[r]);
+        const int oh = 32 + 8 * h + 4 * lh + t;
+        H[r] = __funnelshift_r(wq[r][oh], wq[r][oh + 1], sh[r]);
+      }
+#pragma unroll
+      for (int qd = 0; qd < 4; ++qd) {
+        uint32_t a[2];
+        int scv[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const uint32_t nib = (qd & 1) ? B[r] : A[r];
+          a[r] = (((qd & 2) ? (nib >> 4) : nib) & 0x0F0F0F0Fu) | ((qd < 2 ? H[r] << (4 - 2 * qd) : H[r] >> (2 * qd - 4)) & 0x30303030u);
+          const int si = 8 * h + 2 * qd + lh;  // scale index inside the block
+          scv[r] = sext_byte(sc[r][si >> 2], si & 3);
+        }
+        const int k0 = b * 256 + h * 128 + qd * 32 + lh * 16, grp = k0 >> 4;
+        int cl[4] = {0, 0, 0, 0}, ch[4] = {0, 0, 0, 0};
+        mma_u8s8_k16(cl, a[0], a[1], *reinterpret_cast<const uint32_t*>(alo + k0));
+        if (!NARROW) mma_u8s8_k16(ch, a[0], a[1], *reinterpret_cast<const uint32_t*>(ahi + k0));
+        const int m[2] = {sum0[grp], NARROW ? 0 : sum1[grp]};
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int k = 0; k < NT; ++k) {
+            svl[r][k] += scv[r] * cl[2 * r + k];
+            svh[r][k] += scv[r] * (NARROW ? cl[2 * r + 1] : ch[2 * r + k]);
+            mv[r][k] += scv[r] * m[k];
+          }
+      }
+    }
+  }
+  // sum over the block of sc * (sum(q X) - 32 sum(X)), X = 256 hi + lo
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int k = 0; k < NT; ++k)
+      acc[2 * r + k] = fmaf(d[r], fmaf(256.f, (float)svh[r][k], (float)svl[r][k]) - 32.f * (float)mv[r][k], acc[2 * r + k]);
+}
+
 // Job = (segment of up to 8 token rows, tile of `rows_cta` output features).  CTAs are persistent and take a
 // contiguous range of jobs, so consecutive jobs mostly share their segment.  A job's rows are one contiguous
 // slab of the expert's down matrix and arrive by one bulk copy into one of two buffers; the next job's slab
@@ -372,15 +608,15 @@ __global__ void __launch_bounds__((EM_GU_WARPS + 1) * 32) k_em_gateup(EmParams p
 // Q4 = the down banks are Q4_K (the other half of the layers of a Q4_K_M file): 144-byte blocks on 16-byte
 // boundaries, so fragment words are plain loads; a 32-element scale group is one m16n8k32 MMA per limb, its
 // 6-bit scale and min applied in integers (8 groups x 32 x 15 x 63 x 128 and 8 x 63 x 32 x 32639, both < 2^31).
-template <bool Q4>
-__global__ void __launch_bounds__(EM_DN_WARPS * 32) k_em_down(EmParams p, int rows_cta, int apitch, uint32_t slab_pitch) {
+// WARPS: 16 output rows per warp, or fewer rows (or more warps) and a split of the blocks over the warps.
+template <bool Q4, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta, int apitch, uint32_t slab_pitch) {
   constexpr uint32_t DBB = Q4 ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ int s_pair[8];
   __shared__ float s_xs[8];
-  __shared__ float s_wmax[EM_DN_WARPS];
-  __shared__ float s_dred[3 * 128];
+  __shared__ float s_dred[(WARPS - 1) * 128];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int tiles = p.ne / rows_cta;
@@ -393,8 +629,7 @@ __global__ void __launch_bounds__(EM_DN_WARPS * 32) k_em_down(EmParams p, int ro
   pdl_trigger();
   // the segment table is final (the gate/up kernel, ahead in the stream, only started after it)
   const int n_jobs = __ldcg(p.n_seg) * tiles;
-  const int per = (n_jobs + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int job0 = blockIdx.x * per, job1 = min(job0 + per, n_jobs);
+  const int job0 = (int)((long long)blockIdx.x * n_jobs / gridDim.x), job1 = (int)((long long)(blockIdx.x + 1) * n_jobs / gridDim.x);
   if (job0 >= job1) return;
   const int ngrp = (p.nffmax >> 4) + 4;  // ints per token of the sums: tokens 2t land in different banks
   // shared memory: activation limbs [2][8 tokens][apitch] | sums [8][ngrp] ints | two slab buffers
@@ -403,71 +638,78 @@ __global__ void __launch_bounds__(EM_DN_WARPS * 32) k_em_down(EmParams p, int ro
   unsigned char* slab_area = reinterpret_cast<unsigned char*>(s_sum + 8 * ngrp);
   slab_area += (128u - (smem_u32(slab_area) & 127u)) & 127u;
 
-  auto job_src = [&](int job, int& nff_e) {
-    const int seg = job / tiles, tile = job - seg * tiles;
-    const int e = __ldcg(p.seg_expert + seg);
-    const bool shared_seg = e >= p.n_expert;
-    nff_e = shared_seg ? p.sh_ff : p.nff;
-    return (shared_seg ? p.sh_down : p.down + (size_t)e * p.down_stride) + (size_t)tile * rows_cta * (nff_e / 256 * (int)DBB);
+  auto width_of = [&](int e) { return e >= p.n_expert ? p.sh_ff : p.nff; };
+  auto src_of = [&](int e, int tile) {
+    return (e >= p.n_expert ? p.sh_down : p.down + (size_t)e * p.down_stride) + (size_t)tile * rows_cta * (width_of(e) / 256 * (int)DBB);
   };
   // a slab lands at its source's offset inside a 128-byte line
-  auto request = [&](int job, int buf) {
-    int nff_e;
-    const uint8_t* src = job_src(job, nff_e);
-    const uint32_t bytes = (uint32_t)rows_cta * (nff_e / 256 * DBB);
+  auto request = [&](int e, int tile, int buf) {
+    const uint8_t* src = src_of(e, tile);
+    const uint32_t bytes = (uint32_t)rows_cta * (width_of(e) / 256 * DBB);
     mbar_arrive_expect_tx(&s_bar[buf], bytes);
     bulk_g2s(slab_area + (size_t)buf * slab_pitch + (uint32_t)(reinterpret_cast<uintptr_t>(src) & 127u), src, bytes, &s_bar[buf]);
   };
-  if (tid == 0) request(job0, 0);
+  // segment table entries of the current segment and of the one after it, read a segment ahead
+  int seg = job0 / tiles, tile = job0 - seg * tiles;
+  const int last_seg = (job1 - 1) / tiles;
+  int e = 0, cnt = 0, off = 0;
+  int e_n = __ldcg(p.seg_expert + seg), cnt_n = __ldcg(p.seg_cnt + seg), off_n = __ldcg(p.seg_off + seg);
+  if (tid == 0) request(e_n, tile, 0);
+  bool fresh = true;
+  int my_pair = tid < 8 && tid < cnt_n ? __ldcg(p.seg_pairs + off_n + tid) : -1;
   pdl_wait();  // activations come from the gate/up kernel
 
-  int cur_seg = -1, cnt = 0;
-  for (int job = job0; job < job1; ++job) {
+  for (int job = job0; job < job1; ++job, fresh = ++tile == tiles, seg += fresh, tile = fresh ? 0 : tile) {
     const int buf = (job - job0) & 1;
-    const int seg = job / tiles, tile = job - seg * tiles;
-    int nff_e;
-    const uint8_t* src = job_src(job, nff_e);
-    const unsigned char* slab = slab_area + (size_t)buf * slab_pitch + (uint32_t)(reinterpret_cast<uintptr_t>(src) & 127u);
+    if (fresh) {
+      e = e_n;
+      cnt = cnt_n;
+      off = off_n;
+      if (seg < last_seg) {
+        e_n = __ldcg(p.seg_expert + seg + 1);
+        cnt_n = __ldcg(p.seg_cnt + seg + 1);
+        off_n = __ldcg(p.seg_off + seg + 1);
+      }
+    }
+    const int nff_e = width_of(e);
+    const unsigned char* slab = slab_area + (size_t)buf * slab_pitch + (uint32_t)(reinterpret_cast<uintptr_t>(src_of(e, tile)) & 127u);
     const int drb = nff_e / 256 * (int)DBB;
     __syncthreads();  // every warp is done with the previous job: its slab buffer (the other one) and the limbs may be reused
-    if (tid == 0 && job + 1 < job1) request(job + 1, buf ^ 1);
-    if (seg != cur_seg) {
-      cur_seg = seg;
-      cnt = __ldcg(p.seg_cnt + seg);
-      const int off = __ldcg(p.seg_off + seg);
-      if (tid < 8) s_pair[tid] = tid < cnt ? __ldcg(p.seg_pairs + off + tid) : -1;
+    if (tid == 0 && job + 1 < job1) request(tile + 1 == tiles ? e_n : e, tile + 1 == tiles ? 0 : tile + 1, buf ^ 1);
+    if (fresh) {
+      if (job != job0) my_pair = tid < cnt ? __ldcg(p.seg_pairs + off + tid) : -1;
+      if (tid < 8) s_pair[tid] = my_pair;
       __syncthreads();
-      // fixed point: X = round(a * 32639 / max|a|) per row, limbs X = 256 hi + lo, sums per 16 elements
+      // fixed point: X = round(a * 32639 / max|a|) per row, limbs X = 256 hi + lo, sums per 16 elements.  A warp takes whole
+      // rows, so no barrier stands between a row's maximum and its rounding (rows one after the other with all warps
+      // on each made a segment of eight wait for sixteen of them).
       const int n4 = nff_e / 4;
-      for (int tk = 0; tk < cnt; ++tk) {
+      for (int tk = warp; tk < cnt; tk += WARPS) {
         const float4* arow = reinterpret_cast<const float4*>(p.act + (size_t)s_pair[tk] * p.nffmax);
         float m = 0.f;
-        for (int i = tid; i < n4; i += EM_DN_WARPS * 32) {
+#pragma unroll 4
+        for (int i = lane; i < n4; i += 32) {
           const float4 v = __ldcg(arow + i);
           m = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(m, fmaxf(fabsf(v.z), fabsf(v.w))));
         }
         m = warp_max(m);
-        if (lane == 0) s_wmax[warp] = m;
-        __syncthreads();
-        m = 0.f;
-#pragma unroll
-        for (int w = 0; w < EM_DN_WARPS; ++w) m = fmaxf(m, s_wmax[w]);
         const float inv = m > 0.f ? 32639.f / m : 0.f;
-        if (tid == 0) s_xs[tk] = m / 32639.f;
-        for (int i = tid; i < n4; i += EM_DN_WARPS * 32) {
+        if (lane == 0) s_xs[tk] = m / 32639.f;
+#pragma unroll 4
+        for (int i = lane; i < n4; i += 32) {
           const float4 v = __ldcg(arow + i);
           const int X[4] = {__float2int_rn(v.x * inv), __float2int_rn(v.y * inv), __float2int_rn(v.z * inv), __float2int_rn(v.w * inv)};
           uint32_t lo, hi;
           pack_limbs4(X, lo, hi);
           *reinterpret_cast<uint32_t*>(s_act + (size_t)tk * apitch + 4 * i) = lo;
-          *reinterpret_cast<uint32_t*>(s_act + (size_t)(8 + tk) * apitch + 4 * i) = hi;
-          int sx = (X[0] + X[1]) + (X[2] + X[3]);  // 16 elements = four neighbouring threads (n4 is a multiple of 64: whole warps)
+          *reinterpret_cast<uint32_t*>(s_act + (size_t)((cnt <= EM_NARROW ? EM_NARROW : 8) + tk) * apitch + 4 * i) = hi;
+          int sx = (X[0] + X[1]) + (X[2] + X[3]);  // 16 elements = four neighbouring lanes (n4 is a multiple of 64: whole warps)
           sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 1);
           sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 2);
           if ((i & 3) == 0) s_sum[tk * ngrp + (i >> 2)] = sx;
         }
-        __syncthreads();
       }
+      __syncthreads();
     }
     if (!mbar_wait_bounded(&s_bar[buf], ((job - job0) >> 1) & 1)) {
       if (lane == 0) atomicExch(&p.status->timeout, 8);
@@ -476,117 +718,21 @@ __global__ void __launch_bounds__(EM_DN_WARPS * 32) k_em_down(EmParams p, int ro
     const int nb = nff_e / 256;
     // 16-row tiles of this job: one per warp, or (fewer rows per CTA) several warps per tile, each taking
     // every ksplit-th block, their partial sums added through shared memory
-    const int n_rt = rows_cta / 16, ksplit = EM_DN_WARPS / n_rt;
-    const unsigned char* alo = s_act + (size_t)g * apitch + 4 * t;  // B fragments: token g
+    const int n_rt = rows_cta / 16, ksplit = WARPS / n_rt;
+    // B fragments: wide - token g, limbs eight rows apart; narrow (see gateup_block) - limb g & 1 of token g / 2
+    const bool narrow = cnt <= EM_NARROW;
+    const unsigned char* alo = s_act + (size_t)(narrow ? (g & 1) * EM_NARROW + (g >> 1) : g) * apitch + 4 * t;
     const unsigned char* ahi = alo + (size_t)8 * apitch;
-    const int* sum0 = s_sum + (2 * t) * ngrp;
+    const int* sum0 = s_sum + (narrow ? t : 2 * t) * ngrp;
     const int* sum1 = sum0 + ngrp;
     const int rt = warp % n_rt, ks = warp / n_rt;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     const uint32_t rofs[2] = {(uint32_t)(rt * 16 + g) * drb, (uint32_t)(rt * 16 + g + 8) * drb};
-    for (int b = ks; Q4 && b < nb; b += ksplit) {
-      // rows g and g + 8 of the tile: header (d, dmin, 12 scale bytes), then per 64 weights 32 code bytes whose
-      // low nibbles are the first 32-element group and high nibbles the second
-      const unsigned char* blk[2] = {slab + rofs[0] + (uint32_t)b * Q4K_BLOCK_BYTES, slab + rofs[1] + (uint32_t)b * Q4K_BLOCK_BYTES};
-      const uint4 hdr[2] = {*reinterpret_cast<const uint4*>(blk[0]), *reinterpret_cast<const uint4*>(blk[1])};
-      int svl[4] = {0, 0, 0, 0}, svh[4] = {0, 0, 0, 0}, mv[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        uint32_t scp[2], mp[2], w0[2], w1[2];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          q4k_scale_min_pair(hdr[r].y, hdr[r].z, hdr[r].w, j, scp[r], mp[r]);
-          w0[r] = *reinterpret_cast<const uint32_t*>(blk[r] + 16 + 32 * j + 4 * t);       // k = 4 t .. 4 t + 3 of a group
-          w1[r] = *reinterpret_cast<const uint32_t*>(blk[r] + 32 + 32 * j + 4 * t);       // k = 16 + 4 t ..
-        }
-#pragma unroll
-        for (int hn = 0; hn < 2; ++hn) {
-          const int k0 = b * 256 + j * 64 + hn * 32, grp = k0 >> 4;
-          const uint32_t a00 = (w0[0] >> (4 * hn)) & 0x0F0F0F0Fu, a10 = (w0[1] >> (4 * hn)) & 0x0F0F0F0Fu,
-                         a01 = (w1[0] >> (4 * hn)) & 0x0F0F0F0Fu, a11 = (w1[1] >> (4 * hn)) & 0x0F0F0F0Fu;
-          const uint32_t b0l = *reinterpret_cast<const uint32_t*>(alo + k0), b1l = *reinterpret_cast<const uint32_t*>(alo + k0 + 16);
-          const uint32_t b0h = *reinterpret_cast<const uint32_t*>(ahi + k0), b1h = *reinterpret_cast<const uint32_t*>(ahi + k0 + 16);
-          int cl[4] = {0, 0, 0, 0}, ch[4] = {0, 0, 0, 0};
-          mma_u8s8_k32(cl, a00, a10, a01, a11, b0l, b1l);
-          mma_u8s8_k32(ch, a00, a10, a01, a11, b0h, b1h);
-          const int m0 = sum0[grp] + sum0[grp + 1], m1 = sum1[grp] + sum1[grp + 1];
-          const int scv[2] = {(int)((scp[0] >> (8 * hn)) & 0xFFu), (int)((scp[1] >> (8 * hn)) & 0xFFu)};
-          const int mnv[2] = {(int)((mp[0] >> (8 * hn)) & 0xFFu), (int)((mp[1] >> (8 * hn)) & 0xFFu)};
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            svl[i] += scv[i >> 1] * cl[i];
-            svh[i] += scv[i >> 1] * ch[i];
-            mv[i] += mnv[i >> 1] * ((i & 1) ? m1 : m0);
-          }
-        }
-      }
-      // sum over the block of d sc sum(q X) - dmin m sum(X), X = 256 hi + lo
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float d = f16_bits_to_f32(hdr[i >> 1].x), dmin = f16_bits_to_f32(hdr[i >> 1].x >> 16);
-        acc[i] = fmaf(d, fmaf(256.f, (float)svh[i], (float)svl[i]), fmaf(-dmin, (float)mv[i], acc[i]));
-      }
-    }
-    for (int b = ks; !Q4 && b < nb; b += ksplit) {
-      // per row: aligned view of the block, the shift that realigns it, d and the 16 scales
-      const uint32_t* wq[2];
-      uint32_t sh[2];
-      float d[2];
-      uint32_t sc[2][4];
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const uint32_t ro = rofs[r] + (uint32_t)b * Q6K_BLOCK_BYTES;  // the slab starts on a 16-byte boundary
-        sh[r] = (ro & 3u) * 8;
-        wq[r] = reinterpret_cast<const uint32_t*>(slab + (ro & ~3u));
-        d[r] = f16_bits_to_f32(*reinterpret_cast<const unsigned short*>(slab + ro + 208));
-#pragma unroll
-        for (int i = 0; i < 4; ++i) sc[r][i] = __funnelshift_r(wq[r][48 + i], wq[r][49 + i], sh[r]);
-      }
-      int svl[4] = {0, 0, 0, 0}, svh[4] = {0, 0, 0, 0}, mv[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int lh = 0; lh < 2; ++lh) {
-          // words of ql (two 32-byte runs) and qh that hold l = 16 lh + 4 t .. + 3 of this half
-          uint32_t A[2], B[2], H[2];
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const int o = 16 * h + 4 * lh + t;
-            A[r] = __funnelshift_r(wq[r][o], wq[r][o + 1], sh[r]);
-            B[r] = __funnelshift_r(wq[r][o + 8], wq[r][o + 9], sh[r]);
-            const int oh = 32 + 8 * h + 4 * lh + t;
-            H[r] = __funnelshift_r(wq[r][oh], wq[r][oh + 1], sh[r]);
-          }
-#pragma unroll
-          for (int qd = 0; qd < 4; ++qd) {
-            uint32_t a[2];
-            int scv[2];
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              const uint32_t nib = (qd & 1) ? B[r] : A[r];
-              a[r] = (((qd & 2) ? (nib >> 4) : nib) & 0x0F0F0F0Fu) | (((H[r] >> (2 * qd)) << 4) & 0x30303030u);
-              const int si = 8 * h + 2 * qd + lh;  // scale index inside the block
-              scv[r] = (int)(signed char)((sc[r][si >> 2] >> (8 * (si & 3))) & 0xFFu);
-            }
-            const int k0 = b * 256 + h * 128 + qd * 32 + lh * 16, grp = k0 >> 4;
-            const uint32_t bl = *reinterpret_cast<const uint32_t*>(alo + k0), bh = *reinterpret_cast<const uint32_t*>(ahi + k0);
-            const int m0 = sum0[grp], m1 = sum1[grp];
-            int cl[4] = {0, 0, 0, 0}, ch[4] = {0, 0, 0, 0};
-            mma_u8s8_k16(cl, a[0], a[1], bl);
-            mma_u8s8_k16(ch, a[0], a[1], bh);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              svl[i] += scv[i >> 1] * cl[i];
-              svh[i] += scv[i >> 1] * ch[i];
-              mv[i] += scv[i >> 1] * ((i & 1) ? m1 : m0);
-            }
-          }
-        }
-      }
-      // sum over the block of sc * (sum(q X) - 32 sum(X)), X = 256 hi + lo
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        acc[i] = fmaf(d[i >> 1], fmaf(256.f, (float)svh[i], (float)svl[i]) - 32.f * (float)mv[i], acc[i]);
+    for (int b = ks; b < nb; b += ksplit) {
+      if (Q4 && narrow) down_block_q4<true>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
+      if (Q4 && !narrow) down_block_q4<false>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
+      if (!Q4 && narrow) down_block_q6<true>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
+      if (!Q4 && !narrow) down_block_q6<false>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
     }
     if (ksplit > 1) {
       if (ks > 0) {
@@ -604,8 +750,8 @@ __global__ void __launch_bounds__(EM_DN_WARPS * 32) k_em_down(EmParams p, int ro
       const int i0 = tile * rows_cta + rt * 16;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int tk = 2 * t + (i & 1);
-        if (tk < cnt) p.y[(size_t)s_pair[tk] * p.ne + i0 + g + 8 * (i >> 1)] = acc[i] * s_xs[tk];
+        const int tk = narrow ? t : 2 * t + (i & 1);
+        if (tk < cnt && !(narrow && (i & 1))) p.y[(size_t)s_pair[tk] * p.ne + i0 + g + 8 * (i >> 1)] = acc[i] * s_xs[tk];
       }
     }
   }
@@ -672,6 +818,10 @@ void gateup_shape(int ne, int* KB, int* S, int* xpitch, size_t* stage_bytes) {
 
 // Rows of the down matrix per job: 64 (one 16-row tile per warp) while two slab buffers and the activation
 // limbs leave room for two CTAs per SM, else 32 or 16 with the blocks split over the warps.
+// Eight warps where a row has at least three blocks to split (64 rows, 28 MB experts: the layer 1511 -> 1384 us), four for
+// shorter rows, whose jobs the extra barrier costs more than it gives (32 rows, 512-wide experts: 153 -> 168 us).
+int down_warps(int nffmax) { return nffmax >= 768 ? 8 : 4; }
+
 int down_rows(int ne, int nffmax, size_t dbb, int* apitch, size_t* slab_pitch, size_t* smem) {
   *apitch = nffmax + 16;  // 4 (mod 32) words
   const size_t fixed = (size_t)16 * *apitch + (size_t)8 * (nffmax / 16 + 4) * 4 + 256;
@@ -679,8 +829,7 @@ int down_rows(int ne, int nffmax, size_t dbb, int* apitch, size_t* slab_pitch, s
   const int nb = nffmax / 256;
   for (int rows : {64, 32, 16}) {
     if (ne % rows) continue;
-    const int ksplit = EM_DN_WARPS / (rows / 16);
-    if (nb % ksplit) continue;
+    if (nb == 1 && rows < 64) continue;  // (fewer rows only spread the blocks over more warps)
     *slab_pitch = align_up((size_t)rows * drb + 8, 128) + 128;
     *smem = fixed + 2 * *slab_pitch;
     if (*smem <= 110 * 1024 || rows == 16) return *smem <= 200 * 1024 ? rows : 0;
@@ -770,10 +919,16 @@ int32_t launch_em_ffn(infr_cuda_ctx* ctx, const DecodeParams& dp, void* scratch,
     if (!ok) return fail(ctx, INFR_CUDA_ERR_CUDA, "expert-major gate/up kernel: the driver refused a tensor map for the expert banks");
     // persistent CTAs: two per SM (the shared-memory request allows no more), never more than there are jobs
     const unsigned jobs_bound = (unsigned)n_seg_bound * (unsigned)(nffmax / EM_FEAT);
-    e = ensure_smem(reinterpret_cast<const void*>(k_em_gateup), smem);
-    if (e == cudaSuccess)
-      e = launch_ex(k_em_gateup, dim3(std::min(jobs_bound, 2u * (unsigned)ctx->sm_count)), dim3((EM_GU_WARPS + 1) * 32), smem, ctx->stream, true,
-                    p, KB, S, xpitch, (int)rows_per_expert, tm_gate, tm_up, tm_sh_gate, tm_sh_up);
+    auto run_gu = [&](auto kern, unsigned threads) {
+      cudaError_t ee = ensure_smem(reinterpret_cast<const void*>(kern), smem);
+      if (ee == cudaSuccess)
+        ee = launch_ex(kern, dim3(std::min(jobs_bound, 2u * (unsigned)ctx->sm_count)), dim3(threads), smem, ctx->stream, true, p, KB, S, xpitch,
+                       (int)rows_per_expert, tm_gate, tm_up, tm_sh_gate, tm_sh_up);
+      return ee;
+    };
+    // A long row keeps four warps per feature group busy and hides the tree of sums at its end (7168 wide, 64 rows: 1511 us a
+    // layer with two, 1384 with four); rows of 8 blocks are done too soon for it (2048 wide, 32 rows: 152 against 153 us).
+    e = dp.ne >= 4096 ? run_gu(k_em_gateup<4>, 9 * 32) : run_gu(k_em_gateup<2>, 5 * 32);
     ctx->launches += 1;
     if (e != cudaSuccess) return check_cuda(ctx, e, "k_em_gateup launch");
   }
@@ -785,14 +940,16 @@ int32_t launch_em_ffn(infr_cuda_ctx* ctx, const DecodeParams& dp, void* scratch,
     if (!rows_cta) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "expert-major down kernel: tile does not fit shared memory");
     const unsigned jobs_bound = (unsigned)n_seg_bound * (unsigned)(dp.ne / rows_cta);
     const unsigned per_sm = (unsigned)std::max<size_t>(1, std::min<size_t>(4, (200 * 1024) / smem));
+    const int warps = down_warps((int)nffmax);
     auto run_dn = [&](auto kern) {
       cudaError_t ee = ensure_smem(reinterpret_cast<const void*>(kern), smem);
       if (ee == cudaSuccess)
-        ee = launch_ex(kern, dim3(std::min(jobs_bound, per_sm * (unsigned)ctx->sm_count)), dim3(EM_DN_WARPS * 32), smem, ctx->stream, true, p,
+        ee = launch_ex(kern, dim3(std::min(jobs_bound, per_sm * (unsigned)ctx->sm_count)), dim3(warps * 32), smem, ctx->stream, true, p,
                        rows_cta, apitch, (uint32_t)slab_pitch);
       return ee;
     };
-    e = dp.down_q4k ? run_dn(k_em_down<true>) : run_dn(k_em_down<false>);
+    e = warps == 8 ? (dp.down_q4k ? run_dn(k_em_down<true, 8>) : run_dn(k_em_down<false, 8>))
+                   : (dp.down_q4k ? run_dn(k_em_down<true, 4>) : run_dn(k_em_down<false, 4>));
     ctx->launches += 1;
     if (e != cudaSuccess) return check_cuda(ctx, e, "k_em_down launch");
   }

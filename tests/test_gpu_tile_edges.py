@@ -1,0 +1,82 @@
+"""Sizes at which the tiles of the batched and expert-major kernels begin, end and split, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from moe4all_b200 import synth
+
+from helpers import GpuLayer, assert_close, near_tie_rows, oracle_layer
+
+pytestmark = pytest.mark.gpu
+
+Q8_0, Q4K, Q5K, Q6K = 8, 12, 13, 14
+
+
+def ids_of(counts, seed):
+    """One expert id per row, experts in mixed order, expert e chosen counts[e] times."""
+    return np.random.default_rng(seed).permutation(np.repeat(np.arange(len(counts), dtype=np.int32), counts)).reshape(-1, 1)
+
+
+@pytest.mark.parametrize("mix", [(Q4K, Q4K, Q6K), (Q5K, Q5K, Q4K), (Q8_0, Q8_0, Q8_0), (Q6K, Q4K, Q5K)])
+@pytest.mark.parametrize("ne,nff", [(512, 256), (768, 768)])
+def test_grouped_token_tiles(backend, mix, ne, nff):
+    # an expert's tokens go in tiles of 160, the MMA's extent in steps of 16
+    counts = [1, 15, 16, 17, 0, 33, 143, 144, 145, 159, 160, 161, 176, 321, 0, 2]
+    L = synth.make_layer(51, ne, len(counts), nff, sh_ff=nff, router_std=0.05, dtypes=mix)
+    ids = ids_of(counts, 3)
+    x = synth.activations(81, len(ids), ne)
+    out, _, _ = GpuLayer(backend, L).run(x, 1, path=2, expert_ids=ids)
+    assert_close(out, oracle_layer(L, x, 1, expert_ids=ids).dst)
+
+
+@pytest.mark.parametrize("rows", [8191, 8192, 8193, 16400])
+def test_bucket_slices(backend, rows):
+    # pairs are counted in slices over the CTAs of a cluster: just below, at and past 65536 and 131072 of them
+    L = synth.make_layer(52, 256, 16, 256, router_std=0.05)
+    x = synth.activations(82, rows, 256)
+    out, ids, _ = GpuLayer(backend, L).run(x, 8)
+    sel = np.unique(np.r_[0:8, rows // 2 : rows // 2 + 8, rows - 8 : rows])
+    ref = oracle_layer(L, x[sel], 8)
+    keep = [i for i in range(len(sel)) if i not in set(near_tie_rows(ref, 8).tolist())]
+    assert np.array_equal(ids[sel[keep]], ref.ids[keep])
+    assert_close(out[sel[keep]], ref.dst[keep])
+
+
+@pytest.mark.parametrize("rows", [8, 9, 17, 63, 64, 65])
+def test_router_of_wide_rows(backend, rows):
+    # token rows stream through the router's stages from 9 rows on; 40 experts are not a whole tile
+    L = synth.make_layer(53, 7168, 40, 256, router_std=0.05)
+    x = synth.activations(83, rows, 7168)
+    out, ids, _ = GpuLayer(backend, L).run(x, 4)
+    ref = oracle_layer(L, x, 4)
+    keep = [i for i in range(rows) if i not in set(near_tie_rows(ref, 4).tolist())]
+    assert np.array_equal(ids[keep], ref.ids[keep])
+    assert_close(out[keep], ref.dst[keep])
+
+
+@pytest.mark.parametrize("down_q4k", [False, True])
+@pytest.mark.parametrize("ne,nff", [(512, 256), (2048, 768), (4096, 512), (4352, 1024)])
+def test_expert_major_segments(backend, ne, nff, down_q4k):
+    # up to four tokens of a segment share one MMA with both limbs, more take one per limb; a segment holds eight
+    counts = [1, 3, 4, 5, 0, 7, 8, 9, 12, 13]
+    L = synth.make_layer(54, ne, len(counts), nff, sh_ff=nff, router_std=0.05, down_q4k=down_q4k)
+    ids = ids_of(counts, 4)
+    x = synth.activations(84, len(ids), ne)
+    backend.set_config(expert_major=2)
+    try:
+        out, _, _ = GpuLayer(backend, L).run(x, 1, path=1, expert_ids=ids)
+    finally:
+        backend.set_config(expert_major=0)
+    assert_close(out, oracle_layer(L, x, 1, expert_ids=ids).dst)
+
+
+@pytest.mark.parametrize("ne,nff,sh_ff", [(256, 256, 0), (2048, 512, 512), (4096, 256, 768), (8192, 256, 0)])
+@pytest.mark.parametrize("mix", [(Q5K, Q5K, Q6K), (Q5K, Q5K, Q8_0), (Q4K, Q5K, Q6K), (Q8_0, Q8_0, Q4K)])
+def test_decode_stage_mixes(backend, mix, ne, nff, sh_ff):
+    # per-pair decode: each stage takes the kernel of its own banks or the generic one
+    L = synth.make_layer(55, ne, 8, nff, sh_ff=sh_ff, router_std=0.05, dtypes=mix)
+    x = synth.activations(85, 3, ne)
+    out, ids, _ = GpuLayer(backend, L).run(x, 4, path=1)
+    ref = oracle_layer(L, x, 4)
+    keep = [i for i in range(3) if i not in set(near_tie_rows(ref, 4).tolist())]
+    assert np.array_equal(ids[keep], ref.ids[keep])
+    assert_close(out[keep], ref.dst[keep])
