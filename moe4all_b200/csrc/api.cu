@@ -598,13 +598,16 @@ int32_t validate_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d, ui
 //   experts of 28 MB:  2 rows pp 290 / em 196 / gg 385 us; 64: 8190 / 2247 / 4083; 256: 32770 / 3785 / 4649
 // The expert-major form's time grows with the rows per expert, the grouped GEMM's hardly at all: they cross
 // near 11 (token, expert) pairs per expert.
-// Per-pair against expert-major: the second reads an expert's blocks once for all its rows but takes two more launches and a
-// pass over f32 rows (us per layer, 2048 wide, pp / em; 256 experts of 512: Q6_K down 20 rows 120 / 127, 24 rows 138 / 134;
-// Q4_K down 10 rows 68 / 70, 12 rows 75 / 74, 32 rows 157 / 102; 128 experts of 768: Q6_K 10 rows 96 / 92, 16 rows 136 / 116;
-// Q4_K 8 rows 70 / 70, 16 rows 112 / 89).
-bool em_preferred(uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff, bool down_q4k) {
-  const bool big = (uint64_t)ne * nff >= (1ull << 23);  // experts of tens of megabytes
-  return big ? rows >= 2 : (uint64_t)rows * n_used * 100 >= (uint64_t)n_expert * (down_q4k ? 35 : 65) + 1300;
+// Per-pair against expert-major: the second reads an expert's blocks once for all its rows (about pairs^2 / (2 experts) fewer
+// reads of an expert) but takes two more launches and a pass over f32 rows, so what it saves has to reach some size; for experts
+// so small that it never does, two pairs per expert (us per layer, pp / em; 2048 wide, 256 experts of 512, Q4_K down: 13 rows
+// 78 / 76, 16 rows 91 / 83, 32 rows 155 / 112; Q6_K: 16 rows 100 / 93, 24 rows 134 / 107; 128 experts of 768, Q6_K: 8 rows
+// 75 / 75, 10 rows 93 / 82; Q4_K: 8 rows 64 / 69, 10 rows 77 / 76; 1024 wide, 32 experts of 256: 8 rows of 4 18 / 29, 12 rows
+// 26 / 31, 24 rows 50 / 34).
+bool em_preferred(uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff) {
+  const uint64_t size = (uint64_t)ne * nff, pairs = (uint64_t)rows * n_used;
+  if (size >= (1ull << 23)) return rows >= 2;  // experts of tens of megabytes
+  return pairs >= 2 * (uint64_t)n_expert || pairs * pairs * (size >> 10) >= (uint64_t)n_expert * 51200;
 }
 
 uint32_t choose_moe_path(const infr_cuda_ctx* ctx, uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff,
@@ -730,7 +733,7 @@ int32_t infr_cuda_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d) {
   // (small) launches.
   const bool use_em = path == 1 && em_ok &&
                       (ctx->cfg.expert_major == 2 || !small_ok ||
-                       (ctx->cfg.expert_major == 0 && em_preferred(d->rows, d->n_used, d->n_expert, d->ne, d->n_ff_exp, down_q4k)));
+                       (ctx->cfg.expert_major == 0 && em_preferred(d->rows, d->n_used, d->n_expert, d->ne, d->n_ff_exp)));
   if (path == 1) {
     if (!small_ok && !use_em) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, why);
     // Where the whole-row router kernel covers the call it also normalises x and makes its

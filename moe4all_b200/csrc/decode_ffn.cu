@@ -47,12 +47,13 @@ __device__ __forceinline__ bool in_band(const DecodeParams& p, int e) {
 // FIVE: the banks are Q5_K (176-byte blocks, 32 bytes of fifth bits behind the header) instead of Q4_K.
 template <int NG, bool FIVE>
 __global__ void __maxnreg__(FIVE ? 80 : 56) k_decode_gateup(DecodeParams p, int n_chunks) {
-  constexpr int BB = FIVE ? (int)Q5K_BLOCK_BYTES : (int)Q4K_BLOCK_BYTES, QS = FIVE ? 48 : 16;  // block bytes, offset of the code bytes
+  constexpr uint32_t BB = FIVE ? Q5K_BLOCK_BYTES : Q4K_BLOCK_BYTES;
+  constexpr int QS = FIVE ? 48 : 16;  // block bytes, offset of the code bytes
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[GU_MAX_CHUNKS];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int rb = p.ne / 256 * BB;  // bytes per weight row
+  const int rb = p.ne / 256 * (int)BB;  // bytes per weight row
   const int GW = blockDim.x >> 5;  // warps = weight rows per chunk and role
   const int TR = GW * n_chunks;
   const int tiles = p.nff / TR, sh_tiles = p.sh_ff / TR;
@@ -166,19 +167,23 @@ __global__ void __maxnreg__(FIVE ? 80 : 56) k_decode_gateup(DecodeParams p, int 
       if (g < n_groups) {
         if (NG > 1) load_x(g);
         const int blk = g >> 2, j = g & 3;
-        const unsigned char *gb = grow + blk * BB, *ub = urow + blk * BB;
-        auto words = [](const unsigned char* b, uint32_t (&w)[8]) {
-          const uint4 a = reinterpret_cast<const uint4*>(b)[0], c = reinterpret_cast<const uint4*>(b)[1];
-          w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = c.x; w[5] = c.y; w[6] = c.z; w[7] = c.w;
-        };
-        const uint4 gh = *reinterpret_cast<const uint4*>(gb), uh = *reinterpret_cast<const uint4*>(ub);
+        const uint4 gh = *reinterpret_cast<const uint4*>(grow + blk * BB);
+        const uint4 uh = *reinterpret_cast<const uint4*>(urow + blk * BB);
         uint32_t gq[8], uq[8];
-        words(gb + QS + 32 * j, gq);
-        words(ub + QS + 32 * j, uq);
+        {
+          const uint4 a = *reinterpret_cast<const uint4*>(grow + blk * BB + QS + 32 * j);
+          const uint4 b = *reinterpret_cast<const uint4*>(grow + blk * BB + QS + 16 + 32 * j);
+          gq[0] = a.x; gq[1] = a.y; gq[2] = a.z; gq[3] = a.w; gq[4] = b.x; gq[5] = b.y; gq[6] = b.z; gq[7] = b.w;
+          const uint4 c4 = *reinterpret_cast<const uint4*>(urow + blk * BB + QS + 32 * j);
+          const uint4 d4 = *reinterpret_cast<const uint4*>(urow + blk * BB + QS + 16 + 32 * j);
+          uq[0] = c4.x; uq[1] = c4.y; uq[2] = c4.z; uq[3] = c4.w; uq[4] = d4.x; uq[5] = d4.y; uq[6] = d4.z; uq[7] = d4.w;
+        }
         if constexpr (FIVE) {
           uint32_t g5[8], u5[8];
-          words(gb + 16, g5);
-          words(ub + 16, u5);
+          const uint4 a = *reinterpret_cast<const uint4*>(grow + blk * BB + 16), b = *reinterpret_cast<const uint4*>(grow + blk * BB + 32);
+          g5[0] = a.x; g5[1] = a.y; g5[2] = a.z; g5[3] = a.w; g5[4] = b.x; g5[5] = b.y; g5[6] = b.z; g5[7] = b.w;
+          const uint4 c4 = *reinterpret_cast<const uint4*>(urow + blk * BB + 16), d4 = *reinterpret_cast<const uint4*>(urow + blk * BB + 32);
+          u5[0] = c4.x; u5[1] = c4.y; u5[2] = c4.z; u5[3] = c4.w; u5[4] = d4.x; u5[5] = d4.y; u5[6] = d4.z; u5[7] = d4.w;
           gsum += q5k_dot64_i8(gh, gq, g5, xl, xh, sx0, sx1, j);
           usum += q5k_dot64_i8(uh, uq, u5, xl, xh, sx0, sx1, j);
         } else {

@@ -609,8 +609,12 @@ __device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_
 // boundaries, so fragment words are plain loads; a 32-element scale group is one m16n8k32 MMA per limb, its
 // 6-bit scale and min applied in integers (8 groups x 32 x 15 x 63 x 128 and 8 x 63 x 32 x 32639, both < 2^31).
 // WARPS: 16 output rows per warp, or fewer rows (or more warps) and a split of the blocks over the warps.
+// NBUF slab buffers: two where a job is long.  The short jobs of four warps have one and, in the memory that this frees, more
+// CTAs per SM to fill each other's waits (at 24 rows, Q6_K, 512 wide, a scheduler had 2.8 warps and no instruction in 44 % of
+// its cycles: 113 -> 107 us a layer).
 template <bool Q4, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta, int apitch, uint32_t slab_pitch) {
+  constexpr int NBUF = WARPS == 8 ? 2 : 1;
   constexpr uint32_t DBB = Q4 ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[2];
@@ -632,7 +636,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
   const int job0 = (int)((long long)blockIdx.x * n_jobs / gridDim.x), job1 = (int)((long long)(blockIdx.x + 1) * n_jobs / gridDim.x);
   if (job0 >= job1) return;
   const int ngrp = (p.nffmax >> 4) + 4;  // ints per token of the sums: tokens 2t land in different banks
-  // shared memory: activation limbs [2][8 tokens][apitch] | sums [8][ngrp] ints | two slab buffers
+  // shared memory: activation limbs [2][8 tokens][apitch] | sums [8][ngrp] ints | NBUF slab buffers
   unsigned char* s_act = smem;
   int* s_sum = reinterpret_cast<int*>(smem + (size_t)16 * apitch);
   unsigned char* slab_area = reinterpret_cast<unsigned char*>(s_sum + 8 * ngrp);
@@ -660,7 +664,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
   pdl_wait();  // activations come from the gate/up kernel
 
   for (int job = job0; job < job1; ++job, fresh = ++tile == tiles, seg += fresh, tile = fresh ? 0 : tile) {
-    const int buf = (job - job0) & 1;
+    const int buf = NBUF == 2 ? (job - job0) & 1 : 0;
     if (fresh) {
       e = e_n;
       cnt = cnt_n;
@@ -675,7 +679,11 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
     const unsigned char* slab = slab_area + (size_t)buf * slab_pitch + (uint32_t)(reinterpret_cast<uintptr_t>(src_of(e, tile)) & 127u);
     const int drb = nff_e / 256 * (int)DBB;
     __syncthreads();  // every warp is done with the previous job: its slab buffer (the other one) and the limbs may be reused
-    if (tid == 0 && job + 1 < job1) request(tile + 1 == tiles ? e_n : e, tile + 1 == tiles ? 0 : tile + 1, buf ^ 1);
+    if (NBUF == 2) {
+      if (tid == 0 && job + 1 < job1) request(tile + 1 == tiles ? e_n : e, tile + 1 == tiles ? 0 : tile + 1, buf ^ 1);
+    } else if (tid == 0 && job != job0) {
+      request(e, tile, 0);
+    }
     if (fresh) {
       if (job != job0) my_pair = tid < cnt ? __ldcg(p.seg_pairs + off + tid) : -1;
       if (tid < 8) s_pair[tid] = my_pair;
@@ -711,7 +719,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
       }
       __syncthreads();
     }
-    if (!mbar_wait_bounded(&s_bar[buf], ((job - job0) >> 1) & 1)) {
+    if (!mbar_wait_bounded(&s_bar[buf], (NBUF == 2 ? (job - job0) >> 1 : job - job0) & 1)) {
       if (lane == 0) atomicExch(&p.status->timeout, 8);
       return;
     }
@@ -816,7 +824,7 @@ void gateup_shape(int ne, int* KB, int* S, int* xpitch, size_t* stage_bytes) {
   *S = s;
 }
 
-// Rows of the down matrix per job: 64 (one 16-row tile per warp) while two slab buffers and the activation
+// Rows of the down matrix per job: 64 (one 16-row tile per warp) while the slab buffers and the activation
 // limbs leave room for two CTAs per SM, else 32 or 16 with the blocks split over the warps.
 // Eight warps where a row has at least three blocks to split (64 rows, 28 MB experts: the layer 1511 -> 1384 us), four for
 // shorter rows, whose jobs the extra barrier costs more than it gives (32 rows, 512-wide experts: 153 -> 168 us).
@@ -831,7 +839,7 @@ int down_rows(int ne, int nffmax, size_t dbb, int* apitch, size_t* slab_pitch, s
     if (ne % rows) continue;
     if (nb == 1 && rows < 64) continue;  // (fewer rows only spread the blocks over more warps)
     *slab_pitch = align_up((size_t)rows * drb + 8, 128) + 128;
-    *smem = fixed + 2 * *slab_pitch;
+    *smem = fixed + (down_warps(nffmax) == 8 ? 2 : 1) * *slab_pitch;
     if (*smem <= 110 * 1024 || rows == 16) return *smem <= 200 * 1024 ? rows : 0;
   }
   return 0;
@@ -939,7 +947,7 @@ int32_t launch_em_ffn(infr_cuda_ctx* ctx, const DecodeParams& dp, void* scratch,
     const int rows_cta = down_rows(dp.ne, (int)nffmax, dp.down_q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES, &apitch, &slab_pitch, &smem);
     if (!rows_cta) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "expert-major down kernel: tile does not fit shared memory");
     const unsigned jobs_bound = (unsigned)n_seg_bound * (unsigned)(dp.ne / rows_cta);
-    const unsigned per_sm = (unsigned)std::max<size_t>(1, std::min<size_t>(4, (200 * 1024) / smem));
+    const unsigned per_sm = (unsigned)std::max<size_t>(1, std::min<size_t>(6, (215 * 1024) / (smem + 3072)));
     const int warps = down_warps((int)nffmax);
     auto run_dn = [&](auto kern) {
       cudaError_t ee = ensure_smem(reinterpret_cast<const void*>(kern), smem);
