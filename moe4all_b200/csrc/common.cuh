@@ -18,6 +18,7 @@ namespace infr {
 // ---------------------------------------------------------------------------------------------
 
 constexpr uint32_t Q4K_BLOCK_BYTES = 144;  // 256 weights: f16 d, f16 dmin, 12 B scales, 128 B nibbles
+constexpr uint32_t Q5K_BLOCK_BYTES = 176;  // 256 weights: f16 d, f16 dmin, 12 B scales, 32 B high bits, 128 B nibbles
 constexpr uint32_t Q6K_BLOCK_BYTES = 210;  // 256 weights: 128 B ql, 64 B qh, 16 i8 scales, f16 d
 constexpr uint32_t QK = 256;
 

@@ -47,7 +47,6 @@
 
 namespace infr {
 
-constexpr uint32_t Q5K_BLOCK_BYTES = 176;  // 256 weights: f16 d, f16 dmin, 12 B scales, 32 B high bits, 128 B nibbles
 constexpr uint32_t Q80_BLOCK_BYTES = 34;   // 32 weights: f16 d, 32 int8
 constexpr uint32_t IQ4NL_BLOCK_BYTES = 18;   // 32 weights: f16 d, 16 B nibbles (elements j and j + 16 share a byte)
 constexpr uint32_t IQ4XS_BLOCK_BYTES = 136;  // 256 weights: f16 d, u16 scale high bits, 4 B scale low nibbles, 128 B nibbles
