@@ -609,12 +609,12 @@ __device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_
 // boundaries, so fragment words are plain loads; a 32-element scale group is one m16n8k32 MMA per limb, its
 // 6-bit scale and min applied in integers (8 groups x 32 x 15 x 63 x 128 and 8 x 63 x 32 x 32639, both < 2^31).
 // WARPS: 16 output rows per warp, or fewer rows (or more warps) and a split of the blocks over the warps.
-// NBUF slab buffers: two where a job is long.  The short jobs of four warps have one and, in the memory that this frees, more
-// CTAs per SM to fill each other's waits (at 24 rows, Q6_K, 512 wide, a scheduler had 2.8 warps and no instruction in 44 % of
-// its cycles: 113 -> 107 us a layer).
-template <bool Q4, int WARPS>
+// NBUF slab buffers.  The short jobs of four warps have one and, in the memory that this frees, more CTAs per SM to fill each
+// other's waits (at 24 rows, Q6_K, 512 wide, a scheduler had 2.8 warps and no instruction in 44 % of its cycles: 113 -> 107 us
+// a layer).  Eight warps have two (768 wide, 16 rows: 103 us against 115 with one) unless two leave room for 16 rows only:
+// one of 32 then halves the jobs and their barriers (2048 wide, 64 rows: 1372 -> 1312 us).
+template <bool Q4, int WARPS, int NBUF>
 __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta, int apitch, uint32_t slab_pitch) {
-  constexpr int NBUF = WARPS == 8 ? 2 : 1;
   constexpr uint32_t DBB = Q4 ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[2];
@@ -830,17 +830,22 @@ void gateup_shape(int ne, int* KB, int* S, int* xpitch, size_t* stage_bytes) {
 // shorter rows, whose jobs the extra barrier costs more than it gives (32 rows, 512-wide experts: 153 -> 168 us).
 int down_warps(int nffmax) { return nffmax >= 768 ? 8 : 4; }
 
-int down_rows(int ne, int nffmax, size_t dbb, int* apitch, size_t* slab_pitch, size_t* smem) {
+int down_rows(int ne, int nffmax, size_t dbb, int* apitch, size_t* slab_pitch, size_t* smem, int* nbuf) {
   *apitch = nffmax + 16;  // 4 (mod 32) words
   const size_t fixed = (size_t)16 * *apitch + (size_t)8 * (nffmax / 16 + 4) * 4 + 256;
   const size_t drb = (size_t)nffmax / 256 * dbb;
   const int nb = nffmax / 256;
+  const int most = down_warps(nffmax) == 8 ? 2 : 1;
   for (int rows : {64, 32, 16}) {
     if (ne % rows) continue;
     if (nb == 1 && rows < 64) continue;  // (fewer rows only spread the blocks over more warps)
     *slab_pitch = align_up((size_t)rows * drb + 8, 128) + 128;
-    *smem = fixed + (down_warps(nffmax) == 8 ? 2 : 1) * *slab_pitch;
-    if (*smem <= 110 * 1024 || rows == 16) return *smem <= 200 * 1024 ? rows : 0;
+    for (*nbuf = most; *nbuf >= 1; --*nbuf) {
+      *smem = fixed + *nbuf * *slab_pitch;
+      if (rows == 16) return *smem <= 200 * 1024 ? rows : 0;
+      if (*smem <= 110 * 1024) return rows;
+      if (rows != 32) break;
+    }
   }
   return 0;
 }
@@ -863,8 +868,9 @@ size_t em_scratch_bytes(int rows, int n_used, int ne, int nff, int sh_ff) {
 bool em_supported(int ne, int nff, int sh_ff, int n_expert, BankTypes bt) {
   if (!bt.tuned() || ne % 256 || nff % 256 || sh_ff % 256 || n_expert > 1024) return false;
   int apitch;
+  int nbuf;
   size_t slab_pitch, smem;
-  return down_rows(ne, std::max(nff, sh_ff), bt.down_q4k() ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES, &apitch, &slab_pitch, &smem) != 0;
+  return down_rows(ne, std::max(nff, sh_ff), bt.down_q4k() ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES, &apitch, &slab_pitch, &smem, &nbuf) != 0;
 }
 
 int32_t launch_em_ffn(infr_cuda_ctx* ctx, const DecodeParams& dp, void* scratch, uint32_t stages) {
@@ -942,9 +948,9 @@ int32_t launch_em_ffn(infr_cuda_ctx* ctx, const DecodeParams& dp, void* scratch,
   }
   if (!(stages & 4u)) return INFR_CUDA_OK;
   {
-    int apitch;
+    int apitch, nbuf;
     size_t slab_pitch, smem;
-    const int rows_cta = down_rows(dp.ne, (int)nffmax, dp.down_q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES, &apitch, &slab_pitch, &smem);
+    const int rows_cta = down_rows(dp.ne, (int)nffmax, dp.down_q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES, &apitch, &slab_pitch, &smem, &nbuf);
     if (!rows_cta) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "expert-major down kernel: tile does not fit shared memory");
     const unsigned jobs_bound = (unsigned)n_seg_bound * (unsigned)(dp.ne / rows_cta);
     const unsigned per_sm = (unsigned)std::max<size_t>(1, std::min<size_t>(6, (215 * 1024) / (smem + 3072)));
@@ -956,8 +962,12 @@ int32_t launch_em_ffn(infr_cuda_ctx* ctx, const DecodeParams& dp, void* scratch,
                        rows_cta, apitch, (uint32_t)slab_pitch);
       return ee;
     };
-    e = warps == 8 ? (dp.down_q4k ? run_dn(k_em_down<true, 8>) : run_dn(k_em_down<false, 8>))
-                   : (dp.down_q4k ? run_dn(k_em_down<true, 4>) : run_dn(k_em_down<false, 4>));
+    if (warps == 4)
+      e = dp.down_q4k ? run_dn(k_em_down<true, 4, 1>) : run_dn(k_em_down<false, 4, 1>);
+    else if (nbuf == 2)
+      e = dp.down_q4k ? run_dn(k_em_down<true, 8, 2>) : run_dn(k_em_down<false, 8, 2>);
+    else
+      e = dp.down_q4k ? run_dn(k_em_down<true, 8, 1>) : run_dn(k_em_down<false, 8, 1>);
     ctx->launches += 1;
     if (e != cudaSuccess) return check_cuda(ctx, e, "k_em_down launch");
   }
