@@ -838,6 +838,7 @@ int32_t infr_cuda_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d) {
     if ((rc = ensure_scratch(ctx, sz.total + gbytes + hn_bytes))) return rc;
     Scratch s = carve(ctx->scratch, d, false);
     RouteParams rp = route_params(ctx, d, s, true);
+    rp.batched = 1;
     const float* x_eff = static_cast<const float*>(d->x->ptr);
     if (d->norm_weight) {
       // RmsNorm -> MoeFfn: the batched kernels read the normed rows from scratch

@@ -225,6 +225,12 @@ inline cudaError_t launch_ex(K kernel, dim3 grid, dim3 block, size_t smem, cudaS
 // ---- programmatic dependent launch ------------------------------------------------------------
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A pointer to what an earlier kernel wrote, for use after pdl_wait(): read-only loads through it cannot move above the wait.
+template <typename T>
+__device__ __forceinline__ T* after_wait(T* ptr) {
+  asm volatile("" : "+l"(ptr)::"memory");
+  return ptr;
+}
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- optional phase stamps (latency analysis) ---------------------------------------------------

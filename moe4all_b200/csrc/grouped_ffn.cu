@@ -212,6 +212,9 @@ __global__ void __cluster_dims__(BK_CTAS, 1, 1) __launch_bounds__(1024)
                    int* __restrict__ seg_off, int* __restrict__ tile_expert, int* __restrict__ tile_row0, int* __restrict__ tile_rows,
                    int* __restrict__ n_tiles, int* __restrict__ pos_of_pair, int* __restrict__ pair_of_pos, DeviceStatus* status) {
   __shared__ int s_hist[1024], s_cur[1024], s_cnt[1025], s_off[1026], s_cls[32], s_ws[66];
+  pdl_wait();     // the ids come from the kernel ahead in the stream, and an earlier call may still have read the tables
+  pdl_trigger();
+  const int32_t* ids_now = after_wait(ids);
   cg::cluster_group cluster = cg::this_cluster();
   const int tid = threadIdx.x, rank = (int)cluster.block_rank();
   const int slice = (n_pairs + BK_CTAS - 1) / BK_CTAS, p_lo = rank * slice, p_hi = min(n_pairs, p_lo + slice);
@@ -219,7 +222,7 @@ __global__ void __cluster_dims__(BK_CTAS, 1, 1) __launch_bounds__(1024)
   __syncthreads();
   int e[BK_PER_THREAD];
 #pragma unroll
-  for (int u = 0; u < BK_PER_THREAD; ++u) e[u] = p_lo + u * 1024 + tid < p_hi ? ids[p_lo + u * 1024 + tid] : -1;
+  for (int u = 0; u < BK_PER_THREAD; ++u) e[u] = p_lo + u * 1024 + tid < p_hi ? ids_now[p_lo + u * 1024 + tid] : -1;
 #pragma unroll
   for (int u = 0; u < BK_PER_THREAD; ++u) {
     e[u] = bucket_of(e[u], n_expert, ep_lo, ep_n, status);
@@ -305,13 +308,18 @@ __global__ void __launch_bounds__(256) k_gather_rows(const float* __restrict__ x
   }
 }
 
-// Token rows -> f16 where they are (the tcgen05 kernels gather rows themselves), eight elements per thread.
+// Token rows -> f16 where they are (the tcgen05 kernels gather rows themselves), eight elements per thread.  Runs beside the
+// bucketing kernel ahead of it, which starts it only after everything before the bucketing is complete; this kernel in turn
+// completes only after the bucketing.
 __global__ void __launch_bounds__(256) k_rows_f16(const float* __restrict__ x, size_t n8, __half* __restrict__ xh) {
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= n8) return;
-  const float4 a = __ldg(reinterpret_cast<const float4*>(x) + 2 * i), b = __ldg(reinterpret_cast<const float4*>(x) + 2 * i + 1);
-  const __half2 h[4] = {__floats2half2_rn(a.x, a.z), __floats2half2_rn(a.y, a.w), __floats2half2_rn(b.x, b.z), __floats2half2_rn(b.y, b.w)};
-  reinterpret_cast<uint4*>(xh)[i] = *reinterpret_cast<const uint4*>(h);
+  pdl_trigger();
+  if (i < n8) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(x) + 2 * i), b = __ldg(reinterpret_cast<const float4*>(x) + 2 * i + 1);
+    const __half2 h[4] = {__floats2half2_rn(a.x, a.z), __floats2half2_rn(a.y, a.w), __floats2half2_rn(b.x, b.z), __floats2half2_rn(b.y, b.w)};
+    reinterpret_cast<uint4*>(xh)[i] = *reinterpret_cast<const uint4*>(h);
+  }
+  pdl_wait();
 }
 
 // ---- tensor-core tile helpers ----------------------------------------------------------------------
@@ -701,12 +709,16 @@ constexpr float YP_POSTSCALE = W_POSTSCALE * (8192.0f / 8191.0f);
 // outputs of a token: from f32 rows eight consecutive ones, from packed rows two neighbours of every eighth (of 32), i.e.
 // 16 bytes of every slot's row, all slots' requested together.
 template <bool PACKED>
-__global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __restrict__ y, const int* __restrict__ pos_of_pair,
-                                                               const float* __restrict__ wts, const float* __restrict__ sh_logit,
-                                                               const int* __restrict__ seg_off, int n_seg_routed, int has_shared,
+__global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __restrict__ y_in, const int* __restrict__ pos_of_pair_in,
+                                                               const float* __restrict__ wts_in, const float* __restrict__ sh_logit_in,
+                                                               const int* __restrict__ seg_off_in, int n_seg_routed, int has_shared,
                                                                int rows, int n_used, int ne, const float* residual,
-                                                               const int32_t* __restrict__ ids, const float* __restrict__ down_scale,
+                                                               const int32_t* __restrict__ ids_in, const float* __restrict__ down_scale,
                                                                int weight_before, float* dst) {
+  pdl_wait();  // the expert rows come from the down kernel
+  const float *y = after_wait(y_in), *wts = after_wait(wts_in), *sh_logit = after_wait(sh_logit_in);
+  const int *pos_of_pair = after_wait(pos_of_pair_in), *seg_off = after_wait(seg_off_in);
+  const int32_t* ids = after_wait(ids_in);
   const int q = blockIdx.x * 256 + threadIdx.x;
   if (q * 8 >= ne) return;
   const int c = PACKED ? (q >> 2) * 32 + 2 * (q & 3) : q * 8;
@@ -849,8 +861,9 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
   if (c.ids) {
     // routed call: bucket the pairs
     if (c.n_pairs <= BK_MAX_PAIRS) {
-      k_bucket_fused<<<BK_CTAS, 1024, 0, st>>>(c.ids, c.n_pairs, c.n_expert, c.ep_lo, c.ep_n, c.shared_rows, tn, seg_off, tile_expert, tile_row0,
-                                         tile_rows, n_tiles, pos_of_pair, pair_of_pos, ctx->status);
+      const cudaError_t e = launch_ex(k_bucket_fused, dim3(BK_CTAS), dim3(1024), 0, st, true, c.ids, c.n_pairs, c.n_expert, c.ep_lo, c.ep_n,
+                                      c.shared_rows, tn, seg_off, tile_expert, tile_row0, tile_rows, n_tiles, pos_of_pair, pair_of_pos, ctx->status);
+      if (e != cudaSuccess) return check_cuda(ctx, e, "k_bucket_fused launch");
       ctx->launches += 1;
     } else {
       cudaError_t e = cudaMemsetAsync(counts, 0, (size_t)(n_seg + 2) * 4, st);
@@ -861,9 +874,12 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
                                                                pos_of_pair, pair_of_pos);
       ctx->launches += 3;
     }
-    if (use_wt && !row_w)
-      k_rows_f16<<<(unsigned)(((size_t)c.rows * c.ne / 8 + 255) / 256), 256, 0, st>>>(c.x, (size_t)c.rows * c.ne / 8, xg);
-    else
+    if (use_wt && !row_w) {
+      // (beside the fused bucketing kernel; the three-kernel form releases nothing early)
+      const cudaError_t e = launch_ex(k_rows_f16, dim3((unsigned)(((size_t)c.rows * c.ne / 8 + 255) / 256)), dim3(256), 0, st, c.n_pairs <= BK_MAX_PAIRS,
+                                      c.x, (size_t)c.rows * c.ne / 8, xg);
+      if (e != cudaSuccess) return check_cuda(ctx, e, "k_rows_f16 launch");
+    } else
       k_gather_rows<<<(rows_total + 7) / 8, 256, 0, st>>>(c.x, pair_of_pos, row_w, seg_off, n_seg_routed, c.n_used, rows_total, c.ne, xg);
     ctx->launches += 1;
   } else {
@@ -929,9 +945,10 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
   }
   if (c.dst) {
     auto comb = p.y_packed ? k_unpermute_combine_seg<true> : k_unpermute_combine_seg<false>;
-    comb<<<dim3((c.ne / 8 + 255) / 256, std::min(c.rows, 65535)), 256, 0, st>>>(y, pos_of_pair, c.wts, c.sh_logit, seg_off, n_seg_routed,
-                                                                                 c.shared_rows > 0 ? 1 : 0, c.rows, c.n_used, c.ne, c.residual, c.ids, c.down_scale,
-                                                                                 c.weight_before, c.dst);
+    const cudaError_t e = launch_ex(comb, dim3((c.ne / 8 + 255) / 256, std::min(c.rows, 65535)), dim3(256), 0, st, use_wt, y, pos_of_pair, c.wts,
+                                    c.sh_logit, seg_off, n_seg_routed, c.shared_rows > 0 ? 1 : 0, c.rows, c.n_used, c.ne, c.residual, c.ids,
+                                    c.down_scale, c.weight_before, c.dst);
+    if (e != cudaSuccess) return check_cuda(ctx, e, "combine launch");
     ctx->launches += 1;
   }
   return check_cuda(ctx, cudaGetLastError(), "grouped ffn launch");

@@ -392,6 +392,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
   unsigned char* patches = raw_ring + (size_t)w.rb * w.raw_stage;
   // (shuffles and votes mark what is the same in the whole warp: the MMA operands then stay in uniform registers)
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
+  pdl_wait();  // tiles, rows and activations come from the kernels ahead in the stream
+  pdl_trigger();
   const int n_jobs = __shfl_sync(0xFFFFFFFFu, *p.n_tiles * w.n_blk, 0);
   if (wt_job(0) >= n_jobs) return;
 
@@ -768,7 +770,9 @@ int32_t launch_wt(infr_cuda_ctx* ctx, WtParams w, const CUtensorMap (&tm)[4], in
   cudaError_t e = ensure_smem(reinterpret_cast<const void*>(k_wt_gemm<MODE, FMT>), smem);
   if (e != cudaSuccess) return check_cuda(ctx, e, "grouped GEMM: shared-memory attribute");
   const long long jobs = (long long)max_tiles * w.n_blk;
-  k_wt_gemm<MODE, FMT><<<(unsigned)std::min<long long>(jobs, ctx->sm_count), W_THREADS, smem, ctx->stream>>>(w, tm[0], tm[1], tm[2], tm[3]);
+  e = launch_ex(k_wt_gemm<MODE, FMT>, dim3((unsigned)std::min<long long>(jobs, ctx->sm_count)), dim3(W_THREADS), smem, ctx->stream, true, w, tm[0],
+                tm[1], tm[2], tm[3]);
+  if (e != cudaSuccess) return check_cuda(ctx, e, "grouped GEMM launch");
   ctx->launches += 1;
   return check_cuda(ctx, cudaGetLastError(), "grouped GEMM launch");
 }

@@ -36,6 +36,7 @@ struct RouteParams {
   int rows, ne, n_expert, n_used;
   float scale;
   int gating, norm_w, n_groups, n_groups_used;
+  int batched;               // the next kernel in the stream is one of the batched path: it may start beside the top-k
 };
 
 // Formats of a call's expert banks (INFR_CUDA_DT_*); the shared expert's tensors follow the same three.
