@@ -156,8 +156,10 @@ __global__ void k_shared_add(const float* __restrict__ moe, const float* __restr
 
 // One CTA per row; Σx² is accumulated in double so that the row scale agrees with the sequential
 // f32 sum of the CPU to within an ulp or two whatever the order.
-__global__ void __launch_bounds__(256) k_rmsnorm(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void __launch_bounds__(256) k_rmsnorm(const float* __restrict__ x_in, const float* __restrict__ w_in,
                                                  float* __restrict__ dst, int dim, float eps) {
+  pdl_wait();
+  const float *x = after_wait(x_in), *w = after_wait(w_in);
   __shared__ double s_part[8];
   __shared__ float s_scale;
   const float* xr = x + (size_t)blockIdx.x * dim;
@@ -271,7 +273,8 @@ int32_t launch_shared_add(infr_cuda_ctx* ctx, const float* moe, const float* she
 }
 
 int32_t launch_rmsnorm(infr_cuda_ctx* ctx, const float* x, const float* w, float* dst, int rows, int dim, float eps) {
-  k_rmsnorm<<<rows, 256, 0, ctx->stream>>>(x, w, dst, dim, eps);
+  const cudaError_t e = launch_ex(k_rmsnorm, dim3(rows), dim3(256), 0, ctx->stream, true, x, w, dst, dim, eps);
+  if (e != cudaSuccess) return check_cuda(ctx, e, "k_rmsnorm launch");
   ctx->launches += 1;
   return check_cuda(ctx, cudaGetLastError(), "k_rmsnorm launch");
 }

@@ -392,10 +392,15 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
   unsigned char* patches = raw_ring + (size_t)w.rb * w.raw_stage;
   // (shuffles and votes mark what is the same in the whole warp: the MMA operands then stay in uniform registers)
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
-  pdl_wait();  // tiles, rows and activations come from the kernels ahead in the stream
+  // Tiles and rows come from the kernels ahead in the stream.  The down kernel starts when the gate/up kernel already has them:
+  // only its token copies wait (for the activations), its weights are on their way and unpacked by then.
+  if (MODE == 0) pdl_wait();
   pdl_trigger();
   const int n_jobs = __shfl_sync(0xFFFFFFFFu, *p.n_tiles * w.n_blk, 0);
-  if (wt_job(0) >= n_jobs) return;
+  if (wt_job(0) >= n_jobs) {
+    if (MODE == 1) pdl_wait();
+    return;
+  }
 
   if (tid == 0) {
     for (int s = 0; s < W_A_STAGES; ++s) {
@@ -601,6 +606,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     if (MODE == 1) {
       // the tile's activations: [K step][rows of the tile][128 B], swizzled - one copy per step (past the tile's last row
       // it reads on into the next step: columns of the accumulators that nothing looks at)
+      pdl_wait();
       for (int it = 0; ok; ++it) {
         const int job = wt_job(it);
         if (job >= n_jobs) break;
