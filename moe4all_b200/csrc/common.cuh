@@ -225,7 +225,9 @@ inline cudaError_t launch_ex(K kernel, dim3 grid, dim3 block, size_t smem, cudaS
 // ---- programmatic dependent launch ------------------------------------------------------------
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// A pointer to what an earlier kernel wrote, for use after pdl_wait(): read-only loads through it cannot move above the wait.
+// A pointer to what an earlier kernel wrote, for use after pdl_wait(): loads through it cannot move above the wait.  Kernels
+// that start beside their predecessors read such data past L1 (__ldcg): no kernel boundary has emptied it since it may last
+// have held the same addresses.
 template <typename T>
 __device__ __forceinline__ T* after_wait(T* ptr) {
   asm volatile("" : "+l"(ptr)::"memory");

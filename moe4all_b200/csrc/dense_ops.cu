@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm(const float* __restrict__ x_in,
   const float* xr = x + (size_t)blockIdx.x * dim;
   double acc = 0.0;
   for (int i = threadIdx.x; i < dim; i += 256) {
-    const float v = xr[i];
+    const float v = __ldcg(xr + i);
     acc += (double)(v * v);
   }
 #pragma unroll
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(256) k_rmsnorm(const float* __restrict__ x_in,
   __syncthreads();
   const float s = s_scale;
   float* dr = dst + (size_t)blockIdx.x * dim;
-  for (int i = threadIdx.x; i < dim; i += 256) dr[i] = xr[i] * s * w[i];
+  for (int i = threadIdx.x; i < dim; i += 256) dr[i] = __ldcg(xr + i) * s * __ldcg(w + i);
 }
 
 // Rows of x in 16-bit fixed point for the small-m expert kernels: X = round(x * 32639 / max|x|)

@@ -222,7 +222,7 @@ __global__ void __cluster_dims__(BK_CTAS, 1, 1) __launch_bounds__(1024)
   __syncthreads();
   int e[BK_PER_THREAD];
 #pragma unroll
-  for (int u = 0; u < BK_PER_THREAD; ++u) e[u] = p_lo + u * 1024 + tid < p_hi ? ids_now[p_lo + u * 1024 + tid] : -1;
+  for (int u = 0; u < BK_PER_THREAD; ++u) e[u] = p_lo + u * 1024 + tid < p_hi ? __ldcg(ids_now + p_lo + u * 1024 + tid) : -1;
 #pragma unroll
   for (int u = 0; u < BK_PER_THREAD; ++u) {
     e[u] = bucket_of(e[u], n_expert, ep_lo, ep_n, status);
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(256) k_rows_f16(const float* __restrict__ x, s
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   pdl_trigger();
   if (i < n8) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(x) + 2 * i), b = __ldg(reinterpret_cast<const float4*>(x) + 2 * i + 1);
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(x) + 2 * i), b = __ldcg(reinterpret_cast<const float4*>(x) + 2 * i + 1);
     const __half2 h[4] = {__floats2half2_rn(a.x, a.z), __floats2half2_rn(a.y, a.w), __floats2half2_rn(b.x, b.z), __floats2half2_rn(b.y, b.w)};
     reinterpret_cast<uint4*>(xh)[i] = *reinterpret_cast<const uint4*>(h);
   }
@@ -709,16 +709,12 @@ constexpr float YP_POSTSCALE = W_POSTSCALE * (8192.0f / 8191.0f);
 // outputs of a token: from f32 rows eight consecutive ones, from packed rows two neighbours of every eighth (of 32), i.e.
 // 16 bytes of every slot's row, all slots' requested together.
 template <bool PACKED>
-__global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __restrict__ y_in, const int* __restrict__ pos_of_pair_in,
-                                                               const float* __restrict__ wts_in, const float* __restrict__ sh_logit_in,
-                                                               const int* __restrict__ seg_off_in, int n_seg_routed, int has_shared,
+__global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __restrict__ y, const int* __restrict__ pos_of_pair,
+                                                               const float* __restrict__ wts, const float* __restrict__ sh_logit,
+                                                               const int* __restrict__ seg_off, int n_seg_routed, int has_shared,
                                                                int rows, int n_used, int ne, const float* residual,
-                                                               const int32_t* __restrict__ ids_in, const float* __restrict__ down_scale,
+                                                               const int32_t* __restrict__ ids, const float* __restrict__ down_scale,
                                                                int weight_before, float* dst) {
-  pdl_wait();  // the expert rows come from the down kernel
-  const float *y = after_wait(y_in), *wts = after_wait(wts_in), *sh_logit = after_wait(sh_logit_in);
-  const int *pos_of_pair = after_wait(pos_of_pair_in), *seg_off = after_wait(seg_off_in);
-  const int32_t* ids = after_wait(ids_in);
   const int q = blockIdx.x * 256 + threadIdx.x;
   if (q * 8 >= ne) return;
   const int c = PACKED ? (q >> 2) * 32 + 2 * (q & 3) : q * 8;
@@ -945,7 +941,8 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
   }
   if (c.dst) {
     auto comb = p.y_packed ? k_unpermute_combine_seg<true> : k_unpermute_combine_seg<false>;
-    const cudaError_t e = launch_ex(comb, dim3((c.ne / 8 + 255) / 256, std::min(c.rows, 65535)), dim3(256), 0, st, use_wt, y, pos_of_pair, c.wts,
+    // an ordinary launch: this kernel reads through L1, which a kernel boundary empties
+    const cudaError_t e = launch_ex(comb, dim3((c.ne / 8 + 255) / 256, std::min(c.rows, 65535)), dim3(256), 0, st, false, y, pos_of_pair, c.wts,
                                     c.sh_logit, seg_off, n_seg_routed, c.shared_rows > 0 ? 1 : 0, c.rows, c.n_used, c.ne, c.residual, c.ids,
                                     c.down_scale, c.weight_before, c.dst);
     if (e != cudaSuccess) return check_cuda(ctx, e, "combine launch");

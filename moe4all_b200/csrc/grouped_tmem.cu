@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
   // only its token copies wait (for the activations), its weights are on their way and unpacked by then.
   if (MODE == 0) pdl_wait();
   pdl_trigger();
-  const int n_jobs = __shfl_sync(0xFFFFFFFFu, *p.n_tiles * w.n_blk, 0);
+  const int n_jobs = __shfl_sync(0xFFFFFFFFu, __ldcg(p.n_tiles) * w.n_blk, 0);
   if (wt_job(0) >= n_jobs) {
     if (MODE == 1) pdl_wait();
     return;
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       const int job = wt_job(it);
       if (job >= n_jobs) break;
       const int tile = job / w.n_blk, blk0 = job - tile * w.n_blk;
-      const int e = p.tile_expert[tile], row0 = p.tile_row0[tile], rows_valid = p.tile_rows[tile];
+      const int e = __ldcg(p.tile_expert + tile), row0 = __ldcg(p.tile_row0 + tile), rows_valid = __ldcg(p.tile_rows + tile);
       const int wrow = MODE == 0 ? blk0 * 128 + (slot & 127) : blk0 * WR + slot;
       for (int blk = 0; blk < kb; ++blk) {
         if (!wt_wait(&bars.full_raw[rp.s], rp.phase)) { ok = false; break; }
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     for (int it = 0; ok; ++it) {
       const int job = wt_job(it);
       if (job >= n_jobs) break;
-      const uint32_t idesc = umma::idesc_f16_f32(128, (__shfl_sync(0xFFFFFFFFu, p.tile_rows[job / w.n_blk], 0) + 15) & ~15);
+      const uint32_t idesc = umma::idesc_f16_f32(128, (__shfl_sync(0xFFFFFFFFu, __ldcg(p.tile_rows + job / w.n_blk), 0) + 15) & ~15);
       ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.drained, r_phase));
       if (!ok) break;
       r_phase ^= 1;
@@ -610,9 +610,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       for (int it = 0; ok; ++it) {
         const int job = wt_job(it);
         if (job >= n_jobs) break;
-        const int tile = job / w.n_blk, rows_valid = p.tile_rows[tile];
+        const int tile = job / w.n_blk, rows_valid = __ldcg(p.tile_rows + tile);
         const uint32_t bytes = (uint32_t)((rows_valid + 15) & ~15) * 128u;
-        const unsigned char* src = reinterpret_cast<const unsigned char*>(p.act) + (size_t)p.tile_row0[tile] * p.nff * 2;
+        const unsigned char* src = reinterpret_cast<const unsigned char*>(p.act) + (size_t)__ldcg(p.tile_row0 + tile) * p.nff * 2;
         for (int step = 0; step < 4 * kb; ++step) {
           if (!wt_wait(&bars.empty_b[bp.s], bp.phase ^ 1)) { ok = false; break; }
           if (elect_one()) {
@@ -630,19 +630,19 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       const int tw = warp - W_TOK_WARP, r8 = (tw & 1) * 4 + (lane >> 3), c = lane & 7;
       const uint32_t dst0 = smem_u32(b_ring) + (uint32_t)r8 * 128u + (uint32_t)((c ^ r8) << 4);
       const uint4* tok = reinterpret_cast<const uint4*>(p.xg) + c;
-      const int n_sorted = w.seg_off[w.n_seg_routed];
+      const int n_sorted = __ldcg(w.seg_off + w.n_seg_routed);
       if (tw & 2) bp.next(w.sb);
       for (int it = 0; ok; ++it) {
         const int job = wt_job(it);
         if (job >= n_jobs) break;
         const int tile = job / w.n_blk;
-        const int row0 = p.tile_row0[tile], rows_valid = p.tile_rows[tile], ni = ((rows_valid + 15) & ~15) >> 3;
+        const int row0 = __ldcg(p.tile_row0 + tile), rows_valid = __ldcg(p.tile_rows + tile), ni = ((rows_valid + 15) & ~15) >> 3;
         uint32_t src[WN / 8];  // rows 8 i + r8, in units of 16 bytes
 #pragma unroll
         for (int i = 0; i < WN / 8; ++i) {
           if (i < ni) {
             const int pos = row0 + min(8 * i + r8, rows_valid - 1);  // past the end: the last row once more
-            const int t = w.pair_of_pos == nullptr ? pos : pos < n_sorted ? w.pair_of_pos[pos] / w.n_used : pos - n_sorted;
+            const int t = w.pair_of_pos == nullptr ? pos : pos < n_sorted ? __ldcg(w.pair_of_pos + pos) / w.n_used : pos - n_sorted;
             src[i] = (uint32_t)t * (uint32_t)(p.ne >> 3);
           }
         }
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     for (int it = 0; ok; ++it) {
       const int job = wt_job(it);
       if (job >= n_jobs) break;
-      const int tile = job / w.n_blk, blk0 = job - tile * w.n_blk, e = p.tile_expert[tile];
+      const int tile = job / w.n_blk, blk0 = job - tile * w.n_blk, e = __ldcg(p.tile_expert + tile);
       const bool shared_seg = e >= p.n_expert;
       if (wt_tiled(FMT)) {
         if (warp != RAW_WARP || lane != 0) break;  // one thread issues the tiled copies

@@ -80,3 +80,29 @@ def test_decode_stage_mixes(backend, mix, ne, nff, sh_ff):
     keep = [i for i in range(3) if i not in set(near_tie_rows(ref, 4).tolist())]
     assert np.array_equal(ids[keep], ref.ids[keep])
     assert_close(out[keep], ref.dst[keep])
+
+
+@pytest.mark.parametrize("gated", [False, True])
+def test_batched_calls_back_to_back(backend, gated):
+    # the kernels of a call start beside their predecessors, those of the next call too: enqueued without a pause, with
+    # other rows and other weights in the same scratch, calls give what they give alone
+    from moe4all_b200 import MoeFfn
+    be, calls = backend, []
+    for i, rows in enumerate((300, 97, 641, 1200)):
+        L = synth.make_layer(60 + i, 512, 32, 256, sh_ff=256, gated_shared=gated, router_std=0.05)
+        g, x = GpuLayer(be, L), be.from_host(synth.activations(90 + i, rows, 512))
+        norm = be.from_host(np.linspace(0.5, 1.5, 512).astype(np.float32)) if i % 2 else None
+        dst = [be.alloc(rows * 512 * 4) for _ in range(2)]
+        op = [MoeFfn(x=x, router=g.router, gate_exps=g.gate, up_exps=g.up, down_exps=g.down, dst=d, rows=rows, ne=512, n_expert=32, n_used=4,
+                     n_ff_exp=256, sh_gate=g.sh_gate, sh_up=g.sh_up, sh_down=g.sh_down, sh_gate_inp=g.sh_gate_inp, sh_ff=256,
+                     norm_weight=norm, path=2) for d in dst]
+        calls.append((g, op, dst))
+    for _, op, _ in calls:
+        be.moe_ffn(op[0])
+        be.sync()
+    for rep in range(25):
+        for _, op, _ in calls:
+            be.moe_ffn(op[1])
+        be.sync()
+        for _, _, dst in calls:
+            assert np.array_equal(be.download(dst[0], np.float32), be.download(dst[1], np.float32))
