@@ -97,7 +97,7 @@ typedef struct infr_cuda_config {
                                     (default 12); 0 = no cap                                              */
   uint32_t upload_by_copy;       /* 1: small pinned-memory copies of the *_async calls go through the copy
                                     engine instead of a fetch kernel (default 0)                          */
-  uint32_t trace_tile;           /* tile whose CTAs write phase stamps in the tcgen05 kernels (default 0)  */
+  uint32_t trace_tile;           /* no effect: the tcgen05 kernels write no phase stamps                  */
   uint32_t expert_major;         /* small-m path, who owns a CTA: 0 = choose by rows (default), 1 = always
                                     one (token, expert) pair per CTA, 2 = always one expert with all of
                                     its tokens per CTA (int8 tensor-core tiles)                           */
