@@ -767,44 +767,53 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
 
 // dst[r, :] = sum over ranks (rank order) of w * (y[pair] * down_scale[e]), then the shared expert's row
 // (sigmoid-gated when its logit is given), then the residual - the order of the per-pair kernels.
-__global__ void __launch_bounds__(256) k_em_combine(EmParams p, const float* sh_logit, const float* residual, float* dst) {
-  pdl_wait();
-  const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
+// A chain of three L2 reads behind the down kernel (8 us of 32 rows): the routing was complete before the down kernel started,
+// so ids, weights and the residual are read while it still runs, and CTAs of 128 threads spread the rows over the device.
+constexpr int EM_COMBINE_T = 128;
+__global__ void __launch_bounds__(EM_COMBINE_T) k_em_combine(EmParams p, const float* sh_logit, const float* residual, float* dst) {
+  const int c = (blockIdx.x * EM_COMBINE_T + threadIdx.x) * 4;
   if (c >= p.ne) return;
   const int P = p.rows * p.n_used;
+  bool waited = false;
   for (int r = blockIdx.y; r < p.rows; r += gridDim.y) {
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f), h = o;
+    if (residual != nullptr) h = __ldcg(reinterpret_cast<const float4*>(residual + (size_t)r * p.ne + c));  // may alias dst: each element is read, then written, by this thread
+    const float gsh = (p.sh_ff && sh_logit) ? 1.0f / (1.0f + __expf(-__ldcg(sh_logit + r))) : 1.0f;
     for (int s0 = 0; s0 < p.n_used; s0 += 8) {
-      // eight ranks at a time: ids, weights and rows are requested together, then added in rank order
-      float w[8];
+      // eight ranks at a time: ids and weights, then rows are requested together, then added in rank order
+      float w[8], ds[8];
+      bool on[8];
       float4 v[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int pr = r * p.n_used + s0 + j;
-        w[j] = 0.f;
-        v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (s0 + j >= p.n_used) continue;
-        int e = __ldcg(p.ids + pr);
-        if (e < 0) continue;
+        const bool in = s0 + j < p.n_used;
+        int e = in ? __ldcg(p.ids + pr) : -1;
+        on[j] = e >= 0;
         e = min(e, p.n_expert - 1);
-        if (p.ep_n != 0 && ((uint32_t)e < p.ep_lo || (uint32_t)e >= p.ep_lo + p.ep_n)) continue;
-        const float ds = p.down_scale ? __ldg(p.down_scale + e) : 1.0f;
-        w[j] = p.weight_before ? 1.0f : __ldcg(p.wts + pr);
-        v[j] = __ldcg(reinterpret_cast<const float4*>(p.y + (size_t)pr * p.ne + c));
-        v[j].x *= ds; v[j].y *= ds; v[j].z *= ds; v[j].w *= ds;
+        if (p.ep_n != 0 && ((uint32_t)e < p.ep_lo || (uint32_t)e >= p.ep_lo + p.ep_n)) on[j] = false;
+        ds[j] = (on[j] && p.down_scale) ? __ldg(p.down_scale + e) : 1.0f;
+        w[j] = on[j] ? (p.weight_before ? 1.0f : __ldcg(p.wts + pr)) : 0.f;
+      }
+      if (!waited) {
+        pdl_wait();  // the rows come from the down kernel
+        waited = true;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[j] = on[j] ? __ldcg(reinterpret_cast<const float4*>(p.y + (size_t)(r * p.n_used + s0 + j) * p.ne + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {  // a skipped rank adds 0 * 0: the sum is the one over the served ranks, in order
+        v[j].x *= ds[j]; v[j].y *= ds[j]; v[j].z *= ds[j]; v[j].w *= ds[j];
         o.x += w[j] * v[j].x; o.y += w[j] * v[j].y; o.z += w[j] * v[j].z; o.w += w[j] * v[j].w;
       }
     }
     if (p.sh_ff) {
-      const float gsh = sh_logit ? 1.0f / (1.0f + __expf(-__ldcg(sh_logit + r))) : 1.0f;
       const float4 v = __ldcg(reinterpret_cast<const float4*>(p.y + (size_t)(P + r) * p.ne + c));
       o.x += gsh * v.x; o.y += gsh * v.y; o.z += gsh * v.z; o.w += gsh * v.w;
     }
-    if (residual != nullptr) {  // may alias dst: each element is read, then written, by this thread
-      const float4 h = __ldcg(reinterpret_cast<const float4*>(residual + (size_t)r * p.ne + c));
+    if (residual != nullptr) {
       o.x += h.x; o.y += h.y; o.z += h.z; o.w += h.w;
     }
     *reinterpret_cast<float4*>(dst + (size_t)r * p.ne + c) = o;
@@ -971,7 +980,7 @@ int32_t launch_em_ffn(infr_cuda_ctx* ctx, const DecodeParams& dp, void* scratch,
     ctx->launches += 1;
     if (e != cudaSuccess) return check_cuda(ctx, e, "k_em_down launch");
   }
-  e = launch_ex(k_em_combine, dim3((dp.ne / 4 + 255) / 256, std::min(rows, 65535)), dim3(256), 0, ctx->stream, true, p, dp.sh_logit,
+  e = launch_ex(k_em_combine, dim3((dp.ne / 4 + EM_COMBINE_T - 1) / EM_COMBINE_T, std::min(rows, 65535)), dim3(EM_COMBINE_T), 0, ctx->stream, true, p, dp.sh_logit,
                 dp.residual, dp.dst);
   ctx->launches += 1;
   return check_cuda(ctx, e, "k_em_combine launch");
