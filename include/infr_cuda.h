@@ -104,10 +104,10 @@ typedef struct infr_cuda_config {
   uint32_t sync_timeout_ms;      /* expert-parallel contexts: how long infr_cuda_sync waits for the stream
                                     before it aborts the communicator and returns INFR_CUDA_ERR_NCCL
                                     (default 60000)                                                       */
-  uint32_t raw_rows_f32;         /* batched path on the tcgen05 tiles: 1 = the experts' raw output rows cross memory
-                                    as f32 between the down and the combine kernel instead of f16 with a scale
-                                    per 32 outputs (twice the bytes, no rounding before the sum over a token's
-                                    experts; default 0)                                                    */
+  uint32_t raw_rows_f32;         /* batched path on the tcgen05 tiles, Q4_K gate/up with Q4_K or Q6_K down: 1 = the
+                                    experts' raw output rows cross memory as f32 between the down and the combine
+                                    kernel instead of the upper 24 bits of each (4 / 3 of the bytes, no rounding
+                                    before the sum over a token's experts; default 0)                      */
   uint32_t gate_timeout_ms;      /* host-paced plans: how long a gated fetch waits for its ticket, and
                                     infr_cuda_host_await for its own, before giving up with
                                     INFR_CUDA_ERR_TIMEOUT (default 2000)                                  */

@@ -691,23 +691,15 @@ __global__ void __launch_bounds__(256) k_unpermute_combine(const float* __restri
   }
 }
 
-// Four outputs packed by the tcgen05 down kernel, times 2^8 / (1 - 2^-13) of what they stand for (see YP_POSTSCALE).
-__device__ __forceinline__ float4 unpack_y4(uint2 v) {
-  const uint32_t e = v.y >> 24;
-  const uint32_t q[4] = {v.x, v.x >> 14, __funnelshift_r(v.x, v.y, 28), v.y >> 10};
-  if (e == 255u)  // an infinite or NaN output among them: the top bits of each
-    return make_float4(__uint_as_float(q[0] << 18), __uint_as_float(q[1] << 18), __uint_as_float(q[2] << 18), __uint_as_float(q[3] << 18));
-  const float sc = __uint_as_float((e - 12u) << 23);
-  float f[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) f[i] = (__uint_as_float(((q[i] & 0x3FFFu) ^ 0x2000u) | 0x4B000000u) - 8396800.0f) * sc;
-  return make_float4(f[0], f[1], f[2], f[3]);
+// Four outputs packed by the tcgen05 down kernel (pack_y4), times 2^8.
+__device__ __forceinline__ float4 unpack_y4(uint2 hi, uint32_t lo) {
+  return make_float4(__uint_as_float(__byte_perm(hi.x, lo, 0x1044) & 0xFFFFFF00u), __uint_as_float(__byte_perm(hi.x, lo, 0x3255) & 0xFFFFFF00u),
+                     __uint_as_float(__byte_perm(hi.y, lo, 0x1066) & 0xFFFFFF00u), __uint_as_float(__byte_perm(hi.y, lo, 0x3277) & 0xFFFFFF00u));
 }
-constexpr float YP_POSTSCALE = W_POSTSCALE * (8192.0f / 8191.0f);
 
 // The shared segment starts right after the routed rows: its address is only known on the device.  A thread makes eight
 // outputs of a token: from f32 rows eight consecutive ones, from packed rows two neighbours of every eighth (of 32), i.e.
-// 16 bytes of every slot's row, all slots' requested together.
+// 16 + 8 bytes of every slot's row, all slots' requested together.
 template <bool PACKED>
 __global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __restrict__ y, const int* __restrict__ pos_of_pair,
                                                                const float* __restrict__ wts, const float* __restrict__ sh_logit,
@@ -725,9 +717,11 @@ __global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __re
     auto take = [&](int pos, float w) {
       float4 a, b;
       if (PACKED) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(y) + (size_t)pos * (ne / 8) + q);
-        a = unpack_y4(make_uint2(v.x, v.y));
-        b = unpack_y4(make_uint2(v.z, v.w));
+        const unsigned char* row = reinterpret_cast<const unsigned char*>(y) + (size_t)pos * ne * 3;
+        const uint4 hi = __ldg(reinterpret_cast<const uint4*>(row) + q);
+        const uint2 lo = __ldg(reinterpret_cast<const uint2*>(row + 2 * ne) + q);
+        a = unpack_y4(make_uint2(hi.x, hi.y), lo.x);
+        b = unpack_y4(make_uint2(hi.z, hi.w), lo.y);
       } else {
         a = __ldg(reinterpret_cast<const float4*>(y + (size_t)pos * ne) + 2 * q);
         b = __ldg(reinterpret_cast<const float4*>(y + (size_t)pos * ne) + 2 * q + 1);
@@ -740,7 +734,7 @@ __global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __re
       const int pos = pos_of_pair[(size_t)t * n_used + s];
       if (pos < 0) continue;
       float w = weight_before ? 1.0f : wts[(size_t)t * n_used + s];
-      if (PACKED) w *= YP_POSTSCALE;
+      if (PACKED) w *= W_POSTSCALE;
       // y = raw * scale[e], then the weighted sum (Op::MoeFfn::down_scale); ids may be the caller's: same clamp as the
       // bucketing, which also reported the bad id
       if (down_scale != nullptr) w *= down_scale[min(max(ids[(size_t)t * n_used + s], 0), n_seg_routed - 1)];
@@ -748,7 +742,7 @@ __global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __re
     }
     if (has_shared) {
       const float gsh = sh_logit ? 1.0f / (1.0f + __expf(-sh_logit[t])) : 1.0f;
-      take(n_sorted + t, PACKED ? gsh * YP_POSTSCALE : gsh);
+      take(n_sorted + t, PACKED ? gsh * W_POSTSCALE : gsh);
     }
     // MoeFfn -> Add; may alias dst: each element is read, then written, by this thread
     float* d = dst + (size_t)t * ne + c;
@@ -910,8 +904,8 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
   p.ne = c.ne;
   p.nff = c.nff;
   p.n_expert = c.n_expert;
-  // tcgen05 tiles with the combine behind them: the raw rows cross memory packed (half the bytes out of the down kernel
-  // and into the combine) for the Q4_K / Q6_K banks; rows handed to the caller stay f32
+  // tcgen05 tiles with the combine behind them: the raw rows cross memory packed (three quarters of the bytes out of the
+  // down kernel and into the combine) for the Q4_K / Q6_K banks; rows handed to the caller stay f32
   p.y_packed = (use_wt && tuned && c.dst != nullptr && c.y_out == nullptr && !ctx->cfg.raw_rows_f32) ? 1 : 0;
   p.gate_dt = c.gate_dt;
   p.up_dt = c.up_dt;

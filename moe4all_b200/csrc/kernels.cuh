@@ -103,8 +103,8 @@ struct GroupedParams {
   // the tokens; act per tile as [K step][rows of the tile][128 B], swizzled
   const __half* xg;
   __half* act;
-  float* y;          // [rows, ne] raw down outputs: f32, or with y_packed items of 8 bytes per four outputs of a row (the
-  int y_packed;      // combine kernel is the only reader; pack_y4): features 32 g + j + 8 i, i = 0..3, at item 8 g + j
+  float* y;          // [rows, ne] raw down outputs: f32, or with y_packed (the combine kernel is the only reader) rows of
+  int y_packed;      // 3 ne bytes: item 8 g + j = features 32 g + j + 8 i, i = 0..3 (pack_y4), all items' hi, then their lo
   const uint8_t *gate, *up, *down;
   const uint8_t *sh_gate, *sh_up, *sh_down;  // segment index n_expert = the shared expert
   size_t gate_stride, up_stride, down_stride;

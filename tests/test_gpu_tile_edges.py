@@ -106,3 +106,50 @@ def test_batched_calls_back_to_back(backend, gated):
         be.sync()
         for _, _, dst in calls:
             assert np.array_equal(be.download(dst[0], np.float32), be.download(dst[1], np.float32))
+
+
+def scale_down_rows(L, scale_of_feature):
+    """Multiplies the f16 scales (d, and dmin of Q4_K) of every expert's down rows, feature by feature."""
+    nbytes, slots = synth.BLOCKS[L.down_dtype][1:]
+    for name, n in (("down", L.n_expert), ("sh_down", 1)):
+        if getattr(L, name) is None:
+            continue
+        blk = np.array(getattr(L, name), np.uint8).reshape(n, L.ne, -1, nbytes)
+        for o in slots:
+            d = np.ascontiguousarray(blk[..., o : o + 2]).view(np.float16).astype(np.float32) * scale_of_feature[None, :, None, None]
+            blk[..., o : o + 2] = d.astype(np.float16).view(np.uint8)
+        setattr(L, name, blk.reshape(-1))
+
+
+@pytest.mark.parametrize("down_q4k", [False, True])
+@pytest.mark.parametrize("with_nan", [False, True])
+def test_raw_rows_keep_each_outputs_precision(backend, with_nan, down_q4k):
+    # a few outputs a thousand times their neighbours (and two that are NaN): the others are as exact as alone
+    ne, rows = 768, 150
+    L = synth.make_layer(57, ne, 8, 256, sh_ff=256, router_std=0.05, down_q4k=down_q4k)
+    big = np.random.default_rng(5).random(ne) < 0.1
+    scale = np.where(big, 31.25, 0.03125).astype(np.float32)  # (the largest weights stay below 2^8, where f16 operands end)
+    if with_nan:
+        scale[[70, 401]] = np.nan
+    scale_down_rows(L, scale)
+    x = synth.activations(86, rows, ne)
+    g, out = GpuLayer(backend, L), {}
+    for f32 in (0, 1):
+        backend.set_config(raw_rows_f32=f32)
+        try:
+            out[f32] = g.run(x, 4, path=2)[0], g.run(x, 1, path=2, shared=False)[0]
+        finally:
+            backend.set_config(raw_rows_f32=0)
+    # one expert of weight 1 a row: an output is its raw value, rounded to 16 bits of mantissa (2^-16 of itself) at most
+    got, want = out[0][1], out[1][1]
+    finite = np.isfinite(want)
+    assert np.array_equal(finite, ~np.isnan(got)) and finite.sum() == rows * (ne - 2 * with_nan)
+    assert np.all(np.abs(got[finite] - want[finite]) <= 2.0**-16 * np.abs(want[finite]))
+    # four experts and the shared one, feature by feature: at most 2^-16 of the sum of the five terms' magnitudes, which in
+    # the 2-norm over the rows is about sqrt(5) times the sum's own; 2^-14 leaves 1.8 times that
+    got, want = (out[i][0][:, np.isfinite(scale)].astype(np.float64) for i in (0, 1))
+    assert np.all(np.linalg.norm(got - want, axis=0) <= 2.0**-14 * np.linalg.norm(want, axis=0))
+    if not with_nan:
+        ref = oracle_layer(L, x, 4)
+        keep = [i for i in range(rows) if i not in set(near_tie_rows(ref, 4).tolist())]
+        assert_close(out[0][0][keep], ref.dst[keep])
