@@ -97,7 +97,8 @@ typedef struct infr_cuda_config {
                                     (default 12); 0 = no cap                                              */
   uint32_t upload_by_copy;       /* 1: small pinned-memory copies of the *_async calls go through the copy
                                     engine instead of a fetch kernel (default 0)                          */
-  uint32_t trace_tile;           /* no effect: the tcgen05 kernels write no phase stamps                  */
+  uint32_t trace_tile;           /* tile whose job over the first weight rows writes phase stamps in the tcgen05
+                                    kernels while a trace buffer is set (default 0, the heaviest tile)     */
   uint32_t expert_major;         /* small-m path, who owns a CTA: 0 = choose by rows (default), 1 = always
                                     one (token, expert) pair per CTA, 2 = always one expert with all of
                                     its tokens per CTA (int8 tensor-core tiles)                           */
@@ -451,7 +452,9 @@ int32_t infr_cuda_umma_selftest(infr_cuda_ctx* ctx, const infr_cuda_buf* a, cons
 uint64_t infr_cuda_launch_count(const infr_cuda_ctx* ctx);
 /* Attach (or with NULL detach) a 4096-byte device buffer into which the decode kernels write
  * phase time stamps: pairs of u64 (global timer in ns, SM cycle counter), 16 pairs per kernel in
- * the order router, gate/up, down.  A profiling aid for latency work; the reference's analogue is
+ * the order router, gate/up, down.  The tcgen05 kernels of the batched path write those of one tile
+ * (`trace_tile`): pairs 40 - 43 job start, first weights there, accumulators complete and read for
+ * gate/up, 44 - 47 for down; 64 - 127 and 128 - 191 the first K steps of each.  A profiling aid for latency work; the reference's analogue is
  * the per-op `[prof-moe]` breakdown of crates/infr-cpu/src/lib.rs:4267-4285. */
 int32_t infr_cuda_set_trace(infr_cuda_ctx* ctx, infr_cuda_buf* buf);
 

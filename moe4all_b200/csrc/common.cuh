@@ -238,13 +238,16 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // ---- optional phase stamps (latency analysis) ---------------------------------------------------
 // When a trace buffer is attached to the context, thread 0 of selected CTAs records
 // (globaltimer ns, SM clock) pairs at phase boundaries.  Null pointer = no stores.
-__device__ __forceinline__ void trace_stamp(unsigned long long* tr, int slot) {
-  if (tr != nullptr && threadIdx.x == 0) {
+__device__ __forceinline__ void trace_write(unsigned long long* tr, int slot) {  // by the calling thread
+  if (tr != nullptr) {
     unsigned long long g;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g));
     tr[2 * slot] = g;
     tr[2 * slot + 1] = (unsigned long long)clock64();
   }
+}
+__device__ __forceinline__ void trace_stamp(unsigned long long* tr, int slot) {
+  if (threadIdx.x == 0) trace_write(tr, slot);
 }
 
 // Grid-wide extremes for the same buffer: earliest / latest time any CTA passed a point.

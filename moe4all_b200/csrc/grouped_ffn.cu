@@ -914,6 +914,8 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
   p.gu_rows = (int)(c.gate_stride / row_bytes(c.gate_dt, c.ne));
   p.clamp = c.clamp;
   p.status = ctx->status;
+  p.trace = ctx->trace;
+  p.trace_tile = (int)std::min<uint32_t>(ctx->cfg.trace_tile, (uint32_t)max_tiles);  // (past the last tile: none)
   if (use_wt) {
     WtTokens t = {};
     t.pair_of_pos = (c.ids && !row_w) ? pair_of_pos : nullptr;

@@ -372,7 +372,12 @@ __device__ __forceinline__ int wt_job(int i) {
 // activations come out in the K order of the down kernel's operands.
 __device__ __forceinline__ int wt_row_of_lane(int mode, int l) { return mode == 0 ? ((l & ~3) | ((l & 1) << 1) | ((l >> 1) & 1)) : l; }
 
-template <int MODE, int FMT>
+// TRACED: with a trace buffer attached, the job of tile p.trace_tile over the first weight rows writes phase stamps.  Gate/up
+// (down: 4 slots on): 40 the job's start, 41 its first raw blocks there, 42 accumulators complete, 43 drained.  Of its first 16
+// K steps (down: 64 slots on): 64 + 4 i the first producer warp looks for the raw blocks of step 2 i, 65 + 4 i has them, 66 + 4 i
+// has unpacked its weights, 67 + 4 i has stored them; 96 + 2 i the operands of step i are there, 97 + 2 i its MMAs are issued.
+// A variant of its own: the plain one has neither the pointer's registers nor a branch per step.
+template <int MODE, int FMT, bool TRACED>
 __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant__ WtParams w, const __grid_constant__ CUtensorMap tm_w0,
                                                          const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__ CUtensorMap tm_s0,
                                                          const __grid_constant__ CUtensorMap tm_s1) {
@@ -437,8 +442,13 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       const int tile = job / w.n_blk, blk0 = job - tile * w.n_blk;
       const int e = __ldcg(p.tile_expert + tile), row0 = __ldcg(p.tile_row0 + tile), rows_valid = __ldcg(p.tile_rows + tile);
       const int wrow = MODE == 0 ? blk0 * 128 + (slot & 127) : blk0 * WR + slot;
+      unsigned long long* tr = TRACED && tile == p.trace_tile && blk0 == 0 ? p.trace : nullptr;
+      if (TRACED) trace_stamp(tr, 40 + 4 * MODE);
       for (int blk = 0; blk < kb; ++blk) {
+        if (TRACED && blk < 4) trace_stamp(tr, 64 + 64 * MODE + 8 * blk);
         if (!wt_wait(&bars.full_raw[rp.s], rp.phase)) { ok = false; break; }
+        if (TRACED && blk == 0) trace_stamp(tr, 41 + 4 * MODE);
+        if (TRACED && blk < 4) trace_stamp(tr, 65 + 64 * MODE + 8 * blk);
         const unsigned char* row = raw_ring + (size_t)rp.s * w.raw_stage + (size_t)slot * w.raw_pitch;
         const int mis = ((wrow * kb + blk) & 1) * half_word;  // bytes of the stage's first word ahead of the block
 #pragma unroll
@@ -468,12 +478,18 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars.empty_raw[rp.s]);
           }
+          if (TRACED && blk < 4) trace_stamp(tr, 66 + 64 * MODE + 8 * blk + 4 * h);
           if (!wt_wait(&bars.empty_a[ap.s], ap.phase ^ 1)) { ok = false; break; }
           umma::fence_after_sync();
           tmem_st_32x32(a_addr + 64u * ap.s, o);
           umma::fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars.full_a[ap.s]);
+          if (TRACED && blk < 4) trace_stamp(tr, 67 + 64 * MODE + 8 * blk + 4 * h);
+          if (TRACED && blk < 4 && h == 0) {  // the block's second step has its raw blocks already
+            trace_stamp(tr, 68 + 64 * MODE + 8 * blk);
+            trace_stamp(tr, 69 + 64 * MODE + 8 * blk);
+          }
           ap.next(W_A_STAGES);
           ap.next(W_A_STAGES);
         }
@@ -484,6 +500,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       if (!wt_wait(&bars.done, d_phase)) { ok = false; break; }
       d_phase ^= 1;
       umma::fence_after_sync();
+      if (TRACED) trace_stamp(tr, 42 + 4 * MODE);
       const float clamp = e < p.n_expert ? p.clamp : 0.f;  // the shared expert's segment is not clamped
       // the down kernel's operand: [K step][rows of the tile][128 B], swizzled like its image in shared memory
       unsigned char* act = reinterpret_cast<unsigned char*>(p.act) + (size_t)row0 * p.nff * 2 + (size_t)(2 * blk0 + (q >> 1)) * rows_valid * 128;
@@ -563,6 +580,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       umma::fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars.drained);
+      if (TRACED) trace_stamp(tr, 43 + 4 * MODE);
     }
     if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
   } else if (warp == W_MMA_WARP) {
@@ -584,6 +602,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
         if (elect_one()) {
           const uint64_t db = db0 + (uint64_t)(bp.s * (W_B_STAGE >> 4));
           const uint32_t a = W_A_COL + 64u * ap.s, acc = step > 0;
+          unsigned long long* tr = TRACED && job == p.trace_tile * w.n_blk && step < 16 ? p.trace : nullptr;
+          if (TRACED) trace_write(tr, 96 + 64 * MODE + 2 * step);
           if (MODE == 0) umma::fence_proxy_async();  // the copies behind full_b were cp.async
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -593,6 +613,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           umma::commit(&bars.empty_a[ap.s]);
           umma::commit(&bars.empty_b[bp.s]);
           if (step == 4 * kb - 1) umma::commit(&bars.done);
+          if (TRACED) trace_write(tr, 97 + 64 * MODE + 2 * step);
         }
         __syncwarp();
         bp.next(w.sb);
@@ -773,10 +794,11 @@ int32_t launch_wt(infr_cuda_ctx* ctx, WtParams w, const CUtensorMap (&tm)[4], in
   const size_t rings = (size_t)w.rb * w.raw_stage + (size_t)w.sb * W_B_STAGE;
   if (rings > room) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "grouped GEMM: blocks too large for the raw ring");
   const size_t smem = 1024 + rings + patches;
-  cudaError_t e = ensure_smem(reinterpret_cast<const void*>(k_wt_gemm<MODE, FMT>), smem);
+  auto kern = w.g.trace != nullptr ? k_wt_gemm<MODE, FMT, true> : k_wt_gemm<MODE, FMT, false>;
+  cudaError_t e = ensure_smem(reinterpret_cast<const void*>(kern), smem);
   if (e != cudaSuccess) return check_cuda(ctx, e, "grouped GEMM: shared-memory attribute");
   const long long jobs = (long long)max_tiles * w.n_blk;
-  e = launch_ex(k_wt_gemm<MODE, FMT>, dim3((unsigned)std::min<long long>(jobs, ctx->sm_count)), dim3(W_THREADS), smem, ctx->stream, true, w, tm[0],
+  e = launch_ex(kern, dim3((unsigned)std::min<long long>(jobs, ctx->sm_count)), dim3(W_THREADS), smem, ctx->stream, true, w, tm[0],
                 tm[1], tm[2], tm[3]);
   if (e != cudaSuccess) return check_cuda(ctx, e, "grouped GEMM launch");
   ctx->launches += 1;

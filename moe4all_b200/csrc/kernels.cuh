@@ -113,6 +113,8 @@ struct GroupedParams {
   int gate_dt, up_dt, down_dt;  // INFR_CUDA_DT_* of the banks (the generic-format tiles read these)
   int act_kind;               // INFR_CUDA_ACT_*
   int gu_rows;                // rows of one expert in the gate bank: nff, or 2 nff where gate and up share a bank
+  unsigned long long* trace;  // optional phase stamps (tcgen05 tiles)
+  int trace_tile;             // tile whose job over the first weight rows writes them
   float clamp;                // > 0: routed tiles clamp gate (from above) and up (both sides) first
 };
 

@@ -197,3 +197,32 @@ def test_many_pairs(backend):
     ties = ids_match(ids, ref, 8)
     keep = [r for r in range(rows) if r not in ties]
     assert_close(out[keep], ref.dst[keep])
+
+
+@pytest.mark.parametrize("mix", [(12, 12, 14), (13, 13, 12), (8, 8, 8), (14, 12, 13)])
+def test_phase_stamps_of_one_tile(backend, mix):
+    # with a trace buffer set, the tcgen05 kernels stamp the phases of the chosen tile and compute what they do without
+    be = backend
+    L = synth.make_layer(63, 512, 8, 512, router_std=0.05, dtypes=mix)
+    x = synth.activations(24, 400, 512)
+    g = GpuLayer(be, L)
+    want, _, _ = g.run(x, 2, path=2)
+    for tile, there in ((0, True), (3, True), (4096, False)):
+        buf = be.alloc(4096)
+        be.set_trace(buf)
+        be.set_config(trace_tile=tile)
+        try:
+            out, _, _ = g.run(x, 2, path=2)
+        finally:
+            be.set_trace(None)
+            be.set_config(trace_tile=0)
+        assert np.array_equal(out, want)
+        ns = be.download(buf, np.uint64).reshape(256, 2)[:, 0].astype(np.int64)
+        if not there:
+            assert not ns[40:48].any() and not ns[64:192].any()
+            continue
+        assert (ns[40:48] > 0).all() and (np.diff(ns[40:44]) >= 0).all() and (np.diff(ns[44:48]) >= 0).all()
+        # 512 inputs are eight K steps: four of the first producer warp, eight issued by the MMA warp
+        for k in (64, 128):
+            assert (ns[k : k + 16] > 0).all() and (np.diff(ns[k : k + 16]) >= 0).all() and not ns[k + 16 : k + 32].any()
+            assert (ns[k + 32 : k + 48] > 0).all() and (np.diff(ns[k + 32 : k + 48]) >= 0).all() and not ns[k + 48 : k + 64].any()
