@@ -420,9 +420,11 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
-  constexpr uint32_t tmem = 0;  // the whole of tensor memory is this CTA's: it starts at column 0
+  // All 512 columns are this CTA's, so they start at column 0 of lane 0, and addresses below are constants.  Were it ever
+  // otherwise, every role would leave at once and the call report it.
+  constexpr uint32_t tmem = 0;
   const int kb = w.k_blocks;
-  bool ok = true;
+  bool ok = s_tmem == tmem;
 
   if (warp < W_PRODUCERS / 32) {
     // ---- producers: unpack, then drain ----
