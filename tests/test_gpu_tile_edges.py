@@ -153,3 +153,47 @@ def test_raw_rows_keep_each_outputs_precision(backend, with_nan, down_q4k):
         ref = oracle_layer(L, x, 4)
         keep = [i for i in range(rows) if i not in set(near_tie_rows(ref, 4).tolist())]
         assert_close(out[0][0][keep], ref.dst[keep])
+
+
+@pytest.mark.parametrize("recorded", [False, True])
+def test_forms_in_turn_on_the_same_rows(backend, recorded):
+    # every kernel family and format in turn, in place on the same rows and in the same scratch, each kernel starting beside
+    # its predecessors: enqueued without a pause, or replayed as one plan, the rows end up as with a pause after every call
+    from moe4all_b200 import DType, MoeFfn
+    be, ne, calls = backend, 512, []
+    forms = [((Q4K, Q4K, Q6K), 1200, 2, 0), ((Q4K, Q4K, Q6K), 4, 1, 1), ((Q5K, Q5K, Q6K), 300, 2, 0), ((Q5K, Q5K, Q6K), 2, 1, 0),
+             ((Q8_0, Q8_0, Q8_0), 641, 2, 0), ((Q4K, Q4K, Q4K), 24, 1, 2), ((39, 39, 39), 97, 2, 0), ((39, 39, 39), 9, 1, 0),
+             ((Q4K, Q4K, Q4K), 300, 2, 0), ((Q4K, Q4K, Q6K), 64, 1, 2), ((Q6K, Q4K, Q5K), 130, 2, 0), ((Q4K, Q4K, Q6K), 1, 1, 1)]
+    hidden = be.alloc(1200 * ne * 4)
+    for i, (mix, rows, path, em) in enumerate(forms):
+        L = synth.make_layer(70 + i, ne, 16, 256, sh_ff=256, gated_shared=bool(i % 2), router_std=0.05, dtypes=mix)
+        g, norm = GpuLayer(be, L), be.from_host(np.linspace(0.5, 1.5, ne).astype(np.float32))
+        op = MoeFfn(x=hidden, router=g.router, gate_exps=g.gate, up_exps=g.up, down_exps=g.down, dst=hidden, rows=rows, ne=ne, n_expert=16,
+                    n_used=4, n_ff_exp=256, sh_gate=g.sh_gate, sh_up=g.sh_up, sh_down=g.sh_down, sh_gate_inp=g.sh_gate_inp, sh_ff=256,
+                    norm_weight=norm, residual=hidden, path=path, gate_dtype=DType(mix[0]), up_dtype=DType(mix[1]), down_dtype=DType(mix[2]))
+        calls.append((op, em, g, norm))
+    h0 = synth.activations(95, 1200, ne)
+
+    def enqueue(pause=False):
+        for op, em, *_ in calls:
+            be.set_config(expert_major=em)
+            be.moe_ffn(op)
+            if pause:
+                be.sync()
+
+    try:
+        be.upload(hidden, h0)
+        enqueue(pause=True)
+        want = be.download(hidden, np.float32)
+        assert np.isfinite(want).all() and not np.array_equal(want, h0.reshape(-1))
+        if recorded:
+            be.graph_begin()
+            enqueue()
+            plan = be.graph_end()
+        for rep in range(25):
+            be.upload(hidden, h0)
+            be.execute(plan) if recorded else enqueue()
+            be.sync()
+            assert np.array_equal(be.download(hidden, np.float32), want)
+    finally:
+        be.set_config(expert_major=0)
