@@ -199,11 +199,6 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, u
       : "memory");
 }
 
-// L2 prefetch of a byte range (16-byte aligned address, size multiple of 16).
-__device__ __forceinline__ void bulk_prefetch_l2(const void* gmem_src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem_src), "r"(bytes) : "memory");
-}
-
 // Kernel launch with or without the programmatic-dependent-launch attribute (the launched kernel
 // may then start before the one ahead of it in the stream has finished; it waits with pdl_wait()).
 template <typename K, typename... Args>
