@@ -640,12 +640,13 @@ def run_ours(args):
     # ---- the step's three kernels, each replayed alone (stage masks: 1 router + top-k, 2 gate/up, 4 down) ----
     kernel_us = {}
     n_k = 200
-    # from n_expert / n_used rows on, the small-m path runs its expert-major kernels (the library's own rule)
-    em = banks_tuned() and N_EXPERT <= R * N_USED and R * N_USED * 8 < N_EXPERT * 88
+    n0 = be.launch_count()
+    be.moe_ffn(op_for(0, stages=2))
+    em = be.launch_count() - n0 == 2  # the expert-major kernels bucket the pairs first
     router = "k_router_mid" if 8 < R <= 64 else "k_router_small"  # (beyond 64 rows: the batched router's three kernels)
+    own_gu, own_dn = BANKS[0] == BANKS[1] and BANKS[0] in (12, 13), BANKS[2] in (12, 14)
     names = (router, "k_em_bucket + k_em_gateup", "k_em_down + k_em_combine") if em else \
-            (router, "k_decode_gateup", "k_decode_down") if banks_tuned() else \
-            (router, "k_anyfmt_gateup", "k_anyfmt_down")
+            (router, "k_decode_gateup" if own_gu else "k_anyfmt_gateup", "k_decode_down" if own_dn else "k_anyfmt_down")
     for name, mask in zip(names, (1, 2, 4)):
         for s in range(SETS):
             be.moe_ffn(op_for(s, stages=mask))
@@ -712,7 +713,8 @@ def run_ours(args):
     e2e_steps = (e2e_steps + PACED - 1) // PACED * PACED
     be.graph_begin()
     for s in range(PACED):
-        be.upload_ptr_gated(x_in, stage_ptr, nbytes, s + 1)
+        for off in range(0, nbytes, 256 << 10):  # at most 256 KB per gated fetch
+            be.upload_ptr_gated(x_in, stage_ptr + off, min(nbytes - off, 256 << 10), s + 1, offset=off)
         if host_dst is not None:
             be.moe_ffn(dataclasses.replace(op_for(s, xbuf=x_in), dst=host_dst))
         else:
