@@ -592,18 +592,24 @@ int32_t validate_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d, ui
   return INFR_CUDA_OK;
 }
 
-// Which kernels serve a call of `rows` rows (measured on B200, 256 experts top-8, experts of 2 MB and of
-// 28 MB; pp = one CTA per pair, em = expert-major integer tensor-core tiles, gg = grouped GEMM on tcgen05):
-//   experts of 2 MB:   32 rows pp 174 / em 168 / gg 313 us; 64: 330 / 227 / 420; 256: 1206 / 363 / 488
-//   experts of 28 MB:  2 rows pp 290 / em 196 / gg 385 us; 64: 8190 / 2247 / 4083; 256: 32770 / 3785 / 4649
-// The expert-major form's time grows with the rows per expert, the grouped GEMM's hardly at all: they cross
-// near 11 (token, expert) pairs per expert.
+// Which kernels serve a call of `rows` rows: pp = one CTA per pair, em = expert-major integer tensor-core tiles, gg = grouped
+// GEMM on tcgen05.  us per layer on B200, 256 experts top-8 and the shared one (2 MB: 2048 wide, 512; 28 MB: 7168 wide, 2048):
+//   em / gg   2 MB, Q6_K down:  64 rows 155 / 230, 192: 249 / 270, 256: 296 / 271, 352: 371 / 272
+//             2 MB, Q4_K down:  64 rows 135 / 181, 128: 190 / 214, 192: 221 / 214, 256: 262 / 217
+//             28 MB, Q6_K down: 64 rows 1652 / 2479, 192: 2510 / 2828, 256: 3107 / 2850
+//             28 MB, Q4_K down: 8 rows 508 / 504, 64: 1816 / 1637, 256: 3341 / 1970
+//   pp / gg   2 MB, Q5_K / Q6_K: 16 rows 111 / 146, 32: 193 / 212, 64: 357 / 260
+//             2 MB, Q8_0: 2 rows 51 / 52, 8: 135 / 96, 64: 815 / 205;  MXFP4: 16 rows 310 / 390, 32: 581 / 585, 64: 1121 / 754
+//             28 MB: 4 rows of Q8_0 1240 / 361, of Q5_K / Q6_K 581 / 492, of MXFP4 1674 / 1523
+// The lines below were drawn on earlier kernels: eleven pairs per expert between em and gg, 2.75 rows per expert (8 rows of
+// large ones) between pp and gg.  On today's, em and gg cross at six to seven pairs per expert (gg is level from 8 rows on for
+// large experts with Q4_K down), pp and gg between 0.1 rows per expert (Q8_0) and one (Q5_K, MXFP4).
 // Per-pair against expert-major: the second reads an expert's blocks once for all its rows (about pairs^2 / (2 experts) fewer
 // reads of an expert) but takes two more launches and a pass over f32 rows, so what it saves has to reach some size; for experts
-// so small that it never does, two pairs per expert (us per layer, pp / em; 2048 wide, 256 experts of 512, Q4_K down: 13 rows
-// 78 / 76, 16 rows 91 / 83, 32 rows 155 / 112; Q6_K: 16 rows 100 / 93, 24 rows 134 / 107; 128 experts of 768, Q6_K: 8 rows
-// 75 / 75, 10 rows 93 / 82; Q4_K: 8 rows 64 / 69, 10 rows 77 / 76; 1024 wide, 32 experts of 256: 8 rows of 4 18 / 29, 12 rows
-// 26 / 31, 24 rows 50 / 34).
+// so small that it never does, two pairs per expert (pp / em; 2048 wide, 256 experts of 512, Q4_K down: 8 rows 59 / 68, 12 rows
+// 74 / 69, 16 rows 91 / 81; Q6_K: 8 rows 62 / 71, 12 rows 80 / 77, 16 rows 99 / 88; 128 experts of 768, Q6_K: 8 rows 76 / 74,
+// 10 rows 94 / 78; Q4_K: 8 rows 66 / 68, 10 rows 78 / 71; 1024 wide, 32 experts of 256: 8 rows of 4 19 / 26, 12 rows 27 / 28,
+// 16 rows 30 / 29, 24 rows 37 / 32; 28 MB experts: 1 row 171 / 104, 2 rows 306 / 164).
 bool em_preferred(uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff) {
   const uint64_t size = (uint64_t)ne * nff, pairs = (uint64_t)rows * n_used;
   if (size >= (1ull << 23)) return rows >= 2;  // experts of tens of megabytes

@@ -610,8 +610,8 @@ __device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_
 // 6-bit scale and min applied in integers (8 groups x 32 x 15 x 63 x 128 and 8 x 63 x 32 x 32639, both < 2^31).
 // WARPS: 16 output rows per warp, or fewer rows (or more warps) and a split of the blocks over the warps.
 // NBUF slab buffers.  The short jobs of four warps have one and, in the memory that this frees, more CTAs per SM to fill each
-// other's waits (at 24 rows, Q6_K, 512 wide, a scheduler had 2.8 warps and no instruction in 44 % of its cycles: 113 -> 107 us
-// a layer).  Eight warps have two (768 wide, 16 rows: 103 us against 115 with one) unless two leave room for 16 rows only:
+// other's waits (24 rows, Q6_K, 512 wide: 113 -> 107 us a layer; a scheduler then has 4.4 warps and still nothing to issue in
+// 41 % of its cycles at 32 rows).  Eight warps have two (768 wide, 16 rows: 103 us against 115 with one) unless two leave room for 16 rows only:
 // one of 32 then halves the jobs and their barriers (2048 wide, 64 rows: 1372 -> 1312 us).
 template <bool Q4, int WARPS, int NBUF>
 __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta, int apitch, uint32_t slab_pitch) {

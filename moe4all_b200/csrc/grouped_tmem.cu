@@ -5,7 +5,7 @@
 //   act = silu(Wg x) * (Wu x)      (MODE 0, k_wt_gemm<0, ...>)
 //   y   = Wd act                   (MODE 1, k_wt_gemm<1, ...>)
 //
-// What bounds such a GEMM is the unpacking: every tile has to turn its blocks into f16 operands, whatever the number
+// What such a GEMM pays for is the unpacking: every tile has to turn its blocks into f16 operands, whatever the number
 // of tokens behind them, and the operand then crosses shared memory twice (written by the producers, read by the
 // MMAs).  So the weights are the A operand and A lives in tensor memory: a producer thread owns one weight row, unpacks
 // 64 of its weights into 32 registers and stores them with one tcgen05.st into its lane - no swizzle, no shared-memory
@@ -23,6 +23,11 @@
 //          whose rows of 256 weights are not whole 16-byte pieces word by word with cp.async (rows on an odd word pitch,
 //          free of bank conflicts)
 // All rings run on across jobs; every wait is bounded.
+//
+// Measured (phase stamps, SM cycles per step of 64 K elements): gate/up of full tiles 970, of which the eight MMAs are 640 and
+// the rest their hand-over - the producers wait for a free A stage more than half of their time; of light tiles 820, the
+// unpack.  Down with Q6_K 1130 - 1300, the unpack (1200 - 1800 per own step of a warp); reading out a full tile takes 7000
+// beside the 11000 of its K loop at 512 inputs, with the tensor core idle: there is one set of accumulators.
 #include <cuda.h>
 
 #include <algorithm>
