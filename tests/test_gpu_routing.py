@@ -1,0 +1,75 @@
+"""Routing of decode-sized calls against the oracle where the selection can go wrong: expert counts at the edges of the lanes'
+shares, every number of rows a CTA routes, ties, groups, selections made by the caller, and shapes the team form does not take."""
+import numpy as np
+import pytest
+
+from helpers import near_tie_rows
+from moe4all_b200 import MoeFfn, MoeGating
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+NE = 256
+
+
+def route(be, x, router, k, *, bias=None, gating=0, groups=0, groups_used=0, norm_w=True, scale=1.0, given=None):
+    rows, E = x.shape[0], router.shape[0]
+    ids, wts = be.alloc(rows * k * 4), be.alloc(rows * k * 4)
+    g = be.from_host(np.ascontiguousarray(given, np.int32)) if given is not None else None
+    b = be.from_host(bias) if bias is not None else None
+    be.moe_route(MoeFfn(x=be.from_host(x), router=be.from_host(router), gate_exps=None, up_exps=None, down_exps=None, dst=None, rows=rows, ne=NE,
+                        n_expert=E, n_used=k, n_ff_exp=256, gating=MoeGating(gating), norm_w=norm_w, scale=scale, exp_probs_b=b,
+                        n_expert_groups=groups, n_expert_groups_used=groups_used, ids_out=ids, wts_out=wts, expert_ids=g))
+    be.sync()
+    return be.download(ids, np.int32).reshape(rows, k), be.download(wts, np.float32).reshape(rows, k)
+
+
+def reference(x, router, k, *, bias=None, gating=0, groups=0, groups_used=0, norm_w=True, scale=1.0, given=None):
+    E = router.shape[0]
+    z = np.zeros(E * 256 * 144, np.uint8)  # expert blocks of zeros: only ids, weights and scores are looked at
+    return orc.moe_ffn(x, router, z, z, np.zeros(E * NE * 210, np.uint8), n_expert=E, n_used=k, n_ff_exp=256, gating=gating, bias=bias, groups=groups,
+                       groups_used=groups_used, norm_w=norm_w, scale=scale, expert_ids=given)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("E,k,gating,groups,used,bias", [
+    (4, 1, 0, 0, 0, False), (8, 8, 0, 0, 0, False), (36, 6, 1, 0, 0, True), (100, 8, 0, 0, 0, False), (128, 8, 0, 0, 0, False),
+    (130, 8, 0, 0, 0, False),                                   # not a multiple of four: the general form
+    (132, 8, 2, 0, 0, True), (256, 8, 0, 0, 0, False), (256, 9, 0, 0, 0, False), (256, 8, 1, 8, 4, True), (256, 8, 1, 2, 1, True),
+    (128, 8, 1, 16, 5, True), (256, 2, 0, 32, 3, False), (64, 4, 1, 32, 7, True), (260, 8, 0, 0, 0, False), (252, 6, 1, 3, 2, True)])
+def test_selection(backend, rows, E, k, gating, groups, used, bias):
+    rng = np.random.default_rng(E * 31 + rows)
+    x = rng.standard_normal((rows, NE)).astype(np.float32)
+    router = (rng.standard_normal((E, NE)) * 0.1).astype(np.float32)
+    kw = dict(bias=(rng.standard_normal(E) * 0.05).astype(np.float32) if bias else None, gating=gating, groups=groups, groups_used=used, scale=1.5)
+    ids, wts = route(backend, x, router, k, **kw)
+    ref = reference(x, router, k, **kw)
+    tied = near_tie_rows(ref, k)
+    same = (ids == ref.ids).all(axis=1)
+    assert set(np.where(~same)[0]) <= set(tied), (ids, ref.ids)
+    # the same operations on the same logits: only the last bit of exp can differ
+    np.testing.assert_allclose(wts[same], ref.wts[same], rtol=1e-6)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 4, 8])
+@pytest.mark.parametrize("E", [32, 128, 256])
+def test_ties_take_the_lower_index(backend, rows, E):
+    rng = np.random.default_rng(E + rows)
+    x = rng.standard_normal((rows, NE)).astype(np.float32)
+    base = (rng.standard_normal((4, NE)) * 0.1).astype(np.float32)
+    router = np.ascontiguousarray(base[np.arange(E) % 4])  # equal logits throughout: E / 4 experts share each score
+    ids, _ = route(backend, x, router, 8)
+    ref = reference(x, router, 8)
+    assert np.array_equal(ids, ref.ids)
+
+
+@pytest.mark.parametrize("rows", [1, 3])
+def test_given_selection_and_plain_weights(backend, rows):
+    rng = np.random.default_rng(rows)
+    x = rng.standard_normal((rows, NE)).astype(np.float32)
+    router = (rng.standard_normal((128, NE)) * 0.1).astype(np.float32)
+    given = np.stack([rng.permutation(128)[:6] for _ in range(rows)]).astype(np.int32)
+    for norm_w in (True, False):
+        ids, wts = route(backend, x, router, 6, given=given, norm_w=norm_w, scale=0.5)
+        ref = reference(x, router, 6, given=given, norm_w=norm_w, scale=0.5)
+        assert np.array_equal(ids, given)
+        np.testing.assert_allclose(wts, ref.wts, rtol=1e-6)
