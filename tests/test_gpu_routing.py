@@ -73,3 +73,25 @@ def test_given_selection_and_plain_weights(backend, rows):
         ref = reference(x, router, 6, given=given, norm_w=norm_w, scale=0.5)
         assert np.array_equal(ids, given)
         np.testing.assert_allclose(wts, ref.wts, rtol=1e-6)
+
+
+@pytest.mark.parametrize("ne,rows", [(256, 3), (768, 8), (1024, 8), (1280, 5), (2048, 1), (2048, 4), (2048, 5), (2304, 3), (4096, 2), (4096, 3),
+                                     (4352, 2), (7168, 3)])
+def test_rows_normed_in_the_router(backend, ne, rows):
+    # every share of a row per thread and every remainder of rows per pass; the ids are those of the oracle on normed rows
+    from helpers import assert_close
+    from moe4all_b200 import synth
+    L = synth.make_layer(ne + rows, ne, 16, 256, router_std=0.05)
+    rng = np.random.default_rng(ne)
+    x = (rng.standard_normal((rows, ne)) * rng.uniform(0.1, 10.0, (rows, 1))).astype(np.float32)
+    nw = (1.0 + 0.1 * rng.standard_normal(ne)).astype(np.float32)
+    b = {n: backend.from_host(getattr(L, n)) for n in ("router", "gate", "up", "down")}
+    dst, ids = backend.alloc(rows * ne * 4), backend.alloc(rows * 4 * 4)
+    backend.moe_ffn(MoeFfn(x=backend.from_host(x), dst=dst, norm_weight=backend.from_host(nw), norm_eps=1e-6, router=b["router"], gate_exps=b["gate"],
+                           up_exps=b["up"], down_exps=b["down"], rows=rows, ne=ne, n_expert=16, n_used=4, n_ff_exp=256, ids_out=ids, path=1))
+    backend.sync()
+    ref = orc.moe_ffn(orc.rmsnorm(x, nw, 1e-6), L.router, L.gate, L.up, L.down, n_expert=16, n_used=4, n_ff_exp=256)
+    keep = np.setdiff1d(np.arange(rows), near_tie_rows(ref, 4, ulps=64))  # the norm's own rounding moves a score by some ulps
+    assert len(keep) >= rows - 1
+    assert np.array_equal(backend.download(ids, np.int32).reshape(rows, 4)[keep], ref.ids[keep])
+    assert_close(backend.download(dst, np.float32).reshape(rows, ne)[keep], ref.dst[keep])
