@@ -30,7 +30,7 @@ def reference(x, router, k, *, bias=None, gating=0, groups=0, groups_used=0, nor
                        groups_used=groups_used, norm_w=norm_w, scale=scale, expert_ids=given)
 
 
-@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 8, 9, 21])  # from nine on: a selecting CTA per row, or one per eight
 @pytest.mark.parametrize("E,k,gating,groups,used,bias", [
     (4, 1, 0, 0, 0, False), (8, 8, 0, 0, 0, False), (36, 6, 1, 0, 0, True), (100, 8, 0, 0, 0, False), (128, 8, 0, 0, 0, False),
     (130, 8, 0, 0, 0, False),                                   # not a multiple of four: the general form
