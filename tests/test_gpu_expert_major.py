@@ -198,3 +198,14 @@ def test_bad_expert_id_is_reported(backend):
                       n_expert=32, n_used=4, n_ff_exp=256, ids_out=be.from_host(ids), wts_out=be.from_host(wts), stages=14, path=2))
     with pytest.raises(BackendError, match="expert id"):
         be.sync()
+
+
+@pytest.mark.parametrize("rows", [384, 385, 700])
+def test_more_pairs_than_the_bucketing_keeps_in_registers(em, rows):
+    # 8 pairs a row on one CTA of 1024 threads that keep three each: exactly full, one row more, nearly twice
+    L = synth.make_layer(29, 256, 16, 256, router_std=0.05)
+    x = synth.activations(300 + rows, rows, 256)
+    out, ids, _ = GpuLayer(em, L).run(x, 8, path=1)
+    ref = oracle_layer(L, x, 8)
+    keep = check_ids(ids, ref, 8)
+    assert_close(out[keep], ref.dst[keep])
