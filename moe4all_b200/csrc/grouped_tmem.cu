@@ -174,11 +174,11 @@ __device__ __forceinline__ void unpack_q4k(const unsigned char* row, int j, uint
   }
 }
 
-// Four codes (bytes) with one scale: code - off exactly, times s.
-template <uint32_t OFF>  // f16 bits of 1024 + off
+// Four signed bytes with one scale: 1024 + (byte + 128) in one operation (the sign bit flips with the exponent's bits), the
+// offset off exactly, times s.
 __device__ __forceinline__ void codes4_mul(uint32_t c, __half2 s, uint32_t& o02, uint32_t& o13) {
-  o02 = h2_as_u32(__hmul2(__hsub2(u32_as_h2((c & 0x00FF00FFu) | 0x64006400u), h2_const(OFF)), s));
-  o13 = h2_as_u32(__hmul2(__hsub2(u32_as_h2(((c >> 8) & 0x00FF00FFu) | 0x64006400u), h2_const(OFF)), s));
+  o02 = h2_as_u32(__hmul2(__hsub2(u32_as_h2((c & 0x00FF00FFu) ^ 0x64806480u), h2_const(0x6480u)), s));
+  o13 = h2_as_u32(__hmul2(__hsub2(u32_as_h2(((c >> 8) & 0x00FF00FFu) ^ 0x64806480u), h2_const(0x6480u)), s));
 }
 
 // Two int8 scales (bytes of `w` picked by the selector) times d: exact integers in f16, one rounding.
@@ -228,9 +228,9 @@ __device__ __forceinline__ void unpack_q80(Word w, uint32_t (&o)[32]) {
   const uint32_t mid = w(8);
   const __half2 d = __hmul2(u32_as_h2(__byte_perm(w(0), mid, 0x7610)), h2_const(0x5C00u));
 #pragma unroll
-  for (int i = 0; i < 8; ++i) codes4_mul<0x6480u>(__funnelshift_r(w(i), w(i + 1), 16) ^ 0x80808080u, __low2half2(d), o[2 * i], o[2 * i + 1]);
+  for (int i = 0; i < 8; ++i) codes4_mul(__funnelshift_r(w(i), w(i + 1), 16), __low2half2(d), o[2 * i], o[2 * i + 1]);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) codes4_mul<0x6480u>(w(9 + i) ^ 0x80808080u, __high2half2(d), o[16 + 2 * i], o[16 + 2 * i + 1]);
+  for (int i = 0; i < 8; ++i) codes4_mul(w(9 + i), __high2half2(d), o[16 + 2 * i], o[16 + 2 * i + 1]);
 }
 // The row on a 16-byte boundary: the words of step J are words J .. J + 16 of five 16-byte pieces.
 template <int J>
@@ -324,9 +324,10 @@ __device__ __noinline__ float gated_act_general(int act, float clamp, float g, f
 // A chunk of 4096 tokens, 2048 wide, eight experts of 256 and the shared one each: 560 us (8 bytes: 553; f32 rows: 573).
 __device__ __forceinline__ void pack_y4(float a, float b, float c, float d, uint2& hi, uint32_t& lo) {
   uint32_t q[4] = {__float_as_uint(a), __float_as_uint(b), __float_as_uint(c), __float_as_uint(d)};
+  // (sums of products of f16 stay below 2^50, so what is not finite is an infinity or the tensor core's NaN, 0x7FFFFFFF: the
+  // first keeps its upper bits under the addition, the second by the limit)
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if ((q[i] & 0x7FFFFFFFu) < 0x7F7FFF80u) q[i] += 0x80u;  // the last finite values, infinities and NaN keep their upper bits
+  for (int i = 0; i < 4; ++i) q[i] = (uint32_t)(min((int)q[i], 0x7FFFFF7F) + 0x80);
   hi = make_uint2(__byte_perm(q[0], q[1], 0x7632), __byte_perm(q[2], q[3], 0x7632));
   lo = __byte_perm(__byte_perm(q[0], q[1], 0x0051), __byte_perm(q[2], q[3], 0x0051), 0x5410);
 }

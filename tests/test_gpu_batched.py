@@ -226,3 +226,17 @@ def test_phase_stamps_of_one_tile(backend, mix):
         for k in (64, 128):
             assert (ns[k : k + 16] > 0).all() and (np.diff(ns[k : k + 16]) >= 0).all() and not ns[k + 16 : k + 32].any()
             assert (ns[k + 32 : k + 48] > 0).all() and (np.diff(ns[k + 32 : k + 48]) >= 0).all() and not ns[k + 48 : k + 64].any()
+
+
+@pytest.mark.parametrize("bits", [0x7C00, 0xFC00, 0x7E00, 0xFFFF], ids=["inf", "-inf", "nan", "-nan"])
+@pytest.mark.parametrize("q4k", [False, True])
+def test_outputs_that_are_not_finite_stay_so_between_down_and_combine(backend, bits, q4k):
+    # a scale that is not finite in one block of the down banks: the rows packed for the combine kernel keep that, in that feature only
+    L = synth.make_layer(46, 512, 8, 256, down_q4k=q4k, router_std=0.05)
+    block, at = (144, 0) if q4k else (210, 208)
+    bank = L.down.reshape(8, 512, block)
+    bank[:, 77, at], bank[:, 77, at + 1] = bits & 0xFF, bits >> 8
+    x = synth.activations(9, 96, 512)
+    out, _, _ = GpuLayer(backend, L).run(x, 8, path=2)  # every expert serves every row
+    assert not np.isfinite(out[:, 77]).any()
+    assert np.isfinite(np.delete(out, 77, axis=1)).all()
