@@ -209,3 +209,17 @@ def test_more_pairs_than_the_bucketing_keeps_in_registers(em, rows):
     ref = oracle_layer(L, x, 8)
     keep = check_ids(ids, ref, 8)
     assert_close(out[keep], ref.dst[keep])
+
+
+@pytest.mark.parametrize("down_q4k,rows,em_form", [(False, 5, False), (False, 6, True), (True, 7, False), (True, 8, True)])
+def test_line_between_the_small_m_forms(backend, down_q4k, rows, em_form):
+    # small experts: three pairs per two experts with Q6_K down banks, two per expert with Q4_K; either side of each line
+    L = synth.make_layer(33, 512, 16, 256, sh_ff=256, down_q4k=down_q4k, router_std=0.05)
+    x = synth.activations(40 + rows, rows, 512)
+    g = GpuLayer(backend, L)
+    n0 = backend.launch_count()
+    out, ids, _ = g.run(x, 4)
+    assert backend.launch_count() - n0 == (5 if em_form else 3)
+    ref = oracle_layer(L, x, 4)
+    keep = check_ids(ids, ref, 4)
+    assert_close(out[keep], ref.dst[keep], tol=2e-4)  # both forms round activations to 16 bits: far inside the bound on layers
