@@ -607,7 +607,7 @@ int32_t validate_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d, ui
 // Per-pair against expert-major: the second reads an expert's blocks once for all its rows, about pairs^2 / (2 experts) fewer
 // reads of an expert and rows - 1 fewer of the shared one, but takes two more launches and a pass over f32 rows, so what it saves
 // has to reach some size: the reads saved times the expert's weights, 18432 x 1024 of them (or three pairs per two experts, where
-// experts are so small that they never do).  With Q4_K down banks the expert-major kernels round activations per 256 and not per
+// experts are so small that they never do).  With Q4_K down banks the expert-major kernels round activations per row and not per
 // 128 as the per-pair ones (up to 1.05 times the error): there the line is where the reads saved of the routed experts alone
 // are 25600 x 1024 weights, or two pairs per expert.  pp / em around the line, us per layer, Q6_K down and (Q4_K down):
 //   2048 wide, 256 of 512, top-8, shared: 8 rows 68.2 / 72.9 (65.1 / 66.7), 9 rows 68.4 / 67.0 (64.7 / 62.3), 13 rows 86.4 / 77.1 (79.6 / 70.4)

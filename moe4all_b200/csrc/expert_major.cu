@@ -482,7 +482,7 @@ __global__ void __launch_bounds__((2 * KS + 1) * 32, 2) k_em_gateup(EmParams p, 
 // group and high nibbles the second.
 template <bool NARROW>
 __device__ __forceinline__ void down_block_q4(const unsigned char* blk0, const unsigned char* blk1, const unsigned char* alo, const unsigned char* ahi,
-                                              const int* sum0, const int* sum1, const float* xs0, const float* xs1, int b, float (&acc)[4]) {
+                                              const int* sum0, const int* sum1, int b, float (&acc)[4]) {
   constexpr int NT = NARROW ? 1 : 2;
   const int t = threadIdx.x & 3;
   const unsigned char* blk[2] = {blk0, blk1};
@@ -527,10 +527,8 @@ __device__ __forceinline__ void down_block_q4(const unsigned char* blk0, const u
   for (int r = 0; r < 2; ++r) {
     const float d = f16_bits_to_f32(hdr[r].x), dmin = f16_bits_to_f32(hdr[r].x >> 16);
 #pragma unroll
-    for (int k = 0; k < NT; ++k) {
-      const float u = k ? xs1[b] : xs0[b];  // the block's fixed-point unit
-      acc[2 * r + k] = fmaf(d * u, fmaf(256.f, (float)svh[r][k], (float)svl[r][k]), fmaf(-dmin * u, (float)mv[r][k], acc[2 * r + k]));
-    }
+    for (int k = 0; k < NT; ++k)
+      acc[2 * r + k] = fmaf(d, fmaf(256.f, (float)svh[r][k], (float)svl[r][k]), fmaf(-dmin, (float)mv[r][k], acc[2 * r + k]));
   }
 }
 
@@ -719,41 +717,50 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
       if (job != job0) my_pair = tid < cnt ? __ldcg(p.seg_pairs + off + tid) : -1;
       if (tid < 8) s_pair[tid] = my_pair;
       __syncthreads();
-      // fixed point: X = round(a * 32639 / max|a|) per 128 (Q6_K) or 256 (Q4_K) of a row, limbs X = 256 hi + lo, sums per 16
-      // elements.  A warp takes whole rows, a unit's elements at a time: one pass over them, no barrier between a maximum and its
-      // rounding.  One unit for the whole row (two passes) left 1.1 - 1.2 times the error of the per-pair kernels' 128 with Q6_K
-      // banks (7.1e-5 against 8.1e-5 of the result, 13 rows of 512) and was slower (32 rows 122 -> 119 us the layer); units of 128
-      // with Q4_K, whose errors are level with the row's, cost a conversion more per half block (32 rows 109 -> 114).
+      // fixed point: X = round(a * 32639 / max|a|) per 128 elements of a row (Q6_K) or per row (Q4_K), limbs X = 256 hi + lo, sums
+      // per 16 elements.  A warp takes whole rows: no barrier between a maximum and its rounding.  With Q6_K banks one unit for
+      // the whole row left 1.1 - 1.2 times the error of the per-pair kernels' 128 (7.1e-5 against 8.1e-5 of the result, 13 rows of
+      // 512) and was slower (32 rows 122 -> 119 us the layer); with Q4_K the errors are level, and a unit per block costs two
+      // multiplications for each of its results (427 rows of 2560, 512-wide experts: the kernel 76 us, 71 with one per row).
       const int n4 = nff_e / 4;
       for (int tk = warp; tk < cnt; tk += WARPS) {
         const float4* arow = reinterpret_cast<const float4*>(p.act + (size_t)s_pair[tk] * p.nffmax);
         if constexpr (Q4) {
-          constexpr int W = 2;  // 128 elements each
-#pragma unroll 2
-          for (int c = 0; c < n4; c += 32 * W) {
-            float4 v[W];
-            float m = 0.f;
-#pragma unroll
-            for (int u = 0; u < W; ++u) {
-              v[u] = __ldcg(arow + c + 32 * u + lane);
-              m = fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(m, fmaxf(fabsf(v[u].z), fabsf(v[u].w))));
-            }
+          auto top = [](float4 v, float m) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(m, fmaxf(fabsf(v.z), fabsf(v.w)))); };
+          float inv = 0.f;
+          auto unit = [&](float m) {
             m = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));
-            const float inv = m > 0.f ? 32639.f / m : 0.f;
-            if (lane == 0) s_xs[tk * nhalf + c / (32 * W)] = m / 32639.f;
+            inv = m > 0.f ? 32639.f / m : 0.f;
+            if (lane == 0) s_xs[tk * nhalf] = m / 32639.f;
+          };
+          auto limbs = [&](int i, float4 v) {  // (n4 is a multiple of 64: whole warps)
+            const int X[4] = {__float2int_rn(v.x * inv), __float2int_rn(v.y * inv), __float2int_rn(v.z * inv), __float2int_rn(v.w * inv)};
+            uint32_t lo, hi;
+            pack_limbs4(X, lo, hi);
+            *reinterpret_cast<uint32_t*>(s_act + (size_t)tk * apitch + 4 * i) = lo;
+            *reinterpret_cast<uint32_t*>(s_act + (size_t)((cnt <= EM_NARROW ? EM_NARROW : 8) + tk) * apitch + 4 * i) = hi;
+            int sx = (X[0] + X[1]) + (X[2] + X[3]);  // 16 elements = four neighbouring lanes
+            sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 1);
+            sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 2);
+            if ((i & 3) == 0) s_sum[tk * ngrp + (i >> 2)] = sx;
+          };
+          float m = 0.f;
+          if (n4 <= 128) {  // up to 512 wide: the row stays in registers
+            float4 v[4];
 #pragma unroll
-            for (int u = 0; u < W; ++u) {
-              const int i = c + 32 * u + lane;
-              const int X[4] = {__float2int_rn(v[u].x * inv), __float2int_rn(v[u].y * inv), __float2int_rn(v[u].z * inv), __float2int_rn(v[u].w * inv)};
-              uint32_t lo, hi;
-              pack_limbs4(X, lo, hi);
-              *reinterpret_cast<uint32_t*>(s_act + (size_t)tk * apitch + 4 * i) = lo;
-              *reinterpret_cast<uint32_t*>(s_act + (size_t)((cnt <= EM_NARROW ? EM_NARROW : 8) + tk) * apitch + 4 * i) = hi;
-              int sx = (X[0] + X[1]) + (X[2] + X[3]);  // 16 elements = four neighbouring lanes
-              sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 1);
-              sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 2);
-              if ((i & 3) == 0) s_sum[tk * ngrp + (i >> 2)] = sx;
-            }
+            for (int u = 0; u < 4; ++u) v[u] = lane + 32 * u < n4 ? __ldcg(arow + lane + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) m = top(v[u], m);
+            unit(m);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (lane + 32 * u < n4) limbs(lane + 32 * u, v[u]);
+          } else {
+#pragma unroll 4
+            for (int i = lane; i < n4; i += 32) m = top(__ldcg(arow + i), m);
+            unit(m);
+#pragma unroll 4
+            for (int i = lane; i < n4; i += 32) limbs(i, __ldcg(arow + i));
           }
         } else {
 #pragma unroll 4
@@ -797,8 +804,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     const uint32_t rofs[2] = {(uint32_t)(rt * 16 + g) * drb, (uint32_t)(rt * 16 + g + 8) * drb};
     for (int b = ks; b < nb; b += ksplit) {
-      if (Q4 && narrow) down_block_q4<true>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, xs0, xs1, b, acc);
-      if (Q4 && !narrow) down_block_q4<false>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, xs0, xs1, b, acc);
+      if (Q4 && narrow) down_block_q4<true>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
+      if (Q4 && !narrow) down_block_q4<false>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
       if (!Q4 && narrow) down_block_q6<true>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, xs0, xs1, b, acc);
       if (!Q4 && !narrow) down_block_q6<false>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, xs0, xs1, b, acc);
     }
@@ -819,7 +826,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int tk = narrow ? t : 2 * t + (i & 1);
-        if (tk < cnt && !(narrow && (i & 1))) p.y[(size_t)s_pair[tk] * p.ne + i0 + g + 8 * (i >> 1)] = acc[i];
+        if (tk < cnt && !(narrow && (i & 1)))
+          p.y[(size_t)s_pair[tk] * p.ne + i0 + g + 8 * (i >> 1)] = Q4 ? acc[i] * s_xs[tk * nhalf] : acc[i];
       }
     }
   }
