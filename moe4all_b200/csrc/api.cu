@@ -763,16 +763,13 @@ int32_t infr_cuda_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d) {
     Scratch s = carve(ctx->scratch, d, true);
     RouteParams rp = route_params(ctx, d, s, true);
     const uint32_t stages = d->stages ? d->stages : 7u;
-    bool xsum_ready = false;
+    // the expert-major kernels' sums of x (the first array of their scratch) come out of the pass that makes the fixed-point copy
+    int* const xsum = use_em && (stages & 9u) ? reinterpret_cast<int*>(static_cast<char*>(ctx->scratch) + sz.total + hn_bytes) : nullptr;
     if (few) {
       rp.xq_lo = s.xq_lo;
       rp.xq_hi = s.xq_hi;
       rp.xscale = s.xscale;
-      if (use_em && (stages & 1u)) {
-        // the expert-major kernels' sums of x (the first array of their scratch) come out of the same pass
-        rp.xsum = reinterpret_cast<int*>(static_cast<char*>(ctx->scratch) + sz.total + hn_bytes);
-        xsum_ready = true;
-      }
+      rp.xsum = xsum;
       rp.rms_w = d->norm_weight ? static_cast<const float*>(d->norm_weight->ptr) : nullptr;
       rp.rms_eps = d->norm_eps;
       if (stages & 1u) {
@@ -780,7 +777,7 @@ int32_t infr_cuda_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d) {
       } else if (stages & 8u) {
         // routing came from elsewhere: the router kernel, which would have made the fixed-point copy, does not run
         if (d->norm_weight) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "moe_ffn: stages without the router cannot apply norm_weight");
-        if ((rc = launch_quantize_rows(ctx, static_cast<const float*>(d->x->ptr), s.xq_lo, s.xq_hi, s.xscale, (int)d->rows, (int)d->ne))) return rc;
+        if ((rc = launch_quantize_rows(ctx, static_cast<const float*>(d->x->ptr), s.xq_lo, s.xq_hi, s.xscale, xsum, (int)d->rows, (int)d->ne))) return rc;
       }
     } else if (stages & 1u) {
       const float* x_eff = static_cast<const float*>(d->x->ptr);
@@ -792,11 +789,11 @@ int32_t infr_cuda_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d) {
         rp.x = hn;
       }
       if ((rc = launch_route(ctx, rp, false))) return rc;
-      if ((rc = launch_quantize_rows(ctx, x_eff, s.xq_lo, s.xq_hi, s.xscale, (int)d->rows, (int)d->ne))) return rc;
+      if ((rc = launch_quantize_rows(ctx, x_eff, s.xq_lo, s.xq_hi, s.xscale, xsum, (int)d->rows, (int)d->ne))) return rc;
     } else if (stages & 8u) {
       // routing came from elsewhere (ids_out / wts_out are inputs): only the fixed-point copy of x is made here
       if (d->norm_weight) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "moe_ffn: stages without the router cannot apply norm_weight");
-      if ((rc = launch_quantize_rows(ctx, static_cast<const float*>(d->x->ptr), s.xq_lo, s.xq_hi, s.xscale, (int)d->rows, (int)d->ne))) return rc;
+      if ((rc = launch_quantize_rows(ctx, static_cast<const float*>(d->x->ptr), s.xq_lo, s.xq_hi, s.xscale, xsum, (int)d->rows, (int)d->ne))) return rc;
     }
     DecodeParams dp = {};
     dp.xq_lo = s.xq_lo;
@@ -832,7 +829,7 @@ int32_t infr_cuda_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d) {
     dp.gate_dt = d->gate_dtype;
     dp.up_dt = d->up_dtype;
     dp.down_dt = d->down_dtype;
-    dp.xsum_ready = xsum_ready ? 1 : 0;
+    dp.xsum_ready = xsum != nullptr ? 1 : 0;
     dp.down_scale = d->down_scale ? static_cast<const float*>(d->down_scale->ptr) : nullptr;
     dp.act_kind = (int)d->act;
     dp.weight_before = d->weight_before ? 1 : 0;

@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(1024) k_em_bucket(EmParams p, int seg_cap) {
       pdl_wait();
       // sums of the fixed-point activations per 32-element sub-block (the Q4_K `min` term needs them).
       // xq_* come from the kernel before this one in the stream.
-      if (!p.xsum_ready) {  // (the whole-row router kernels make them with the fixed-point copy)
+      if (!p.xsum_ready) {  // (a call that only runs the expert stages: no kernel of its own made the fixed-point copy)
         const int nsb = p.ne / 32, total = p.rows * nsb;
         for (int i = tid; i < total; i += 1024) {
           const int r = i / nsb, sb = i - r * nsb;

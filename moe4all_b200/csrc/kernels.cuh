@@ -67,7 +67,7 @@ struct DecodeParams {
   uint32_t ep_lo, ep_n;  // band (ep_n == 0: off)
   int down_q4k;          // the down banks (routed and shared) are Q4_K instead of Q6_K
   int gate_dt, up_dt, down_dt;  // INFR_CUDA_DT_* of the banks (the generic-format kernels read these)
-  int xsum_ready;        // the router kernel already made the expert-major kernels' sums of x (first array of their scratch)
+  int xsum_ready;        // the expert-major kernels' sums of x (first array of their scratch) were made with the fixed-point copy
   const float* down_scale;  // [n_expert] scale on a routed expert's down output, or null
   int act_kind;          // INFR_CUDA_ACT_*
   int weight_before;     // routing weight on gate and up before the activation, none on the output
@@ -80,7 +80,7 @@ struct EmParams {
   const int8_t *xq_lo, *xq_hi;   // [rows, ne] fixed-point limbs of x
   const float* xscale;           // [rows]
   int* xsum;                     // [rows, ne/32] integer sums of x per 32-element sub-block
-  int xsum_ready;                // made by the router kernel with the fixed-point copy: the bucket kernel skips them
+  int xsum_ready;                // made with the fixed-point copy: the bucket kernel skips them
   const int32_t* ids;            // [rows, n_used]
   const float* wts;              // [rows, n_used]
   int *n_seg, *seg_expert, *seg_off, *seg_cnt, *seg_pairs;  // segment table, built on the device
@@ -199,7 +199,7 @@ int32_t launch_gated_act(infr_cuda_ctx* ctx, const float* gate, const float* up,
 int32_t launch_shared_add(infr_cuda_ctx* ctx, const float* moe, const float* shexp, const float* gate, float* dst,
                           int rows, int n);
 int32_t launch_rmsnorm(infr_cuda_ctx* ctx, const float* x, const float* w, float* dst, int rows, int dim, float eps);
-int32_t launch_quantize_rows(infr_cuda_ctx* ctx, const float* x, int8_t* lo, int8_t* hi, float* scale, int rows, int dim);
+int32_t launch_quantize_rows(infr_cuda_ctx* ctx, const float* x, int8_t* lo, int8_t* hi, float* scale, int* xsum, int rows, int dim);
 int32_t launch_add(infr_cuda_ctx* ctx, const float* a, const float* b, float* dst, size_t n);
 // dst[0, bytes) = the pinned host range whose device view is src_dev_view (16-byte aligned, bytes % 16 == 0).
 int32_t launch_fetch_host(infr_cuda_ctx* ctx, const void* src_dev_view, void* dst, size_t bytes);
