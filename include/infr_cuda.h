@@ -450,6 +450,9 @@ void infr_cuda_graph_free(infr_cuda_ctx* ctx, infr_cuda_graph* graph);
 int32_t infr_cuda_umma_selftest(infr_cuda_ctx* ctx, const infr_cuda_buf* a, const infr_cuda_buf* b, infr_cuda_buf* c, uint32_t n);
 /* Number of kernel launches this context has issued since creation (host-side count). */
 uint64_t infr_cuda_launch_count(const infr_cuda_ctx* ctx);
+/* CTAs per SM that the expert-major down kernel is launched with for layers of these sizes (down_dtype Q4_K or Q6_K);
+ * 0 where those kernels do not take the sizes.  Test aid, no reference counterpart. */
+uint32_t infr_cuda_em_down_ctas_per_sm(const infr_cuda_ctx* ctx, uint32_t ne, uint32_t n_ff_exp, uint32_t sh_ff, uint32_t down_dtype);
 /* Attach (or with NULL detach) a 4096-byte device buffer into which the decode kernels write
  * phase time stamps: pairs of u64 (global timer in ns, SM cycle counter), 16 pairs per kernel in
  * the order router, gate/up, down.  The tcgen05 kernels of the batched path write those of one tile

@@ -31,7 +31,7 @@ EXPORTS = [
     "infr_cuda_gguf_meta_u64", "infr_cuda_gguf_meta_f64", "infr_cuda_gguf_meta_str", "infr_cuda_gguf_upload",
     "infr_cuda_sync", "infr_cuda_moe_ffn", "infr_cuda_moe_route", "infr_cuda_linear",
     "infr_cuda_gated_act", "infr_cuda_moe_shared_add", "infr_cuda_rmsnorm", "infr_cuda_add",
-    "infr_cuda_moe_expert_rows", "infr_cuda_launch_count",
+    "infr_cuda_moe_expert_rows", "infr_cuda_launch_count", "infr_cuda_em_down_ctas_per_sm",
     "infr_cuda_graph_begin", "infr_cuda_graph_end", "infr_cuda_graph_launch", "infr_cuda_graph_free", "infr_cuda_set_trace", "infr_cuda_moe_route_noalloc", "infr_cuda_moe_combine", "infr_cuda_umma_selftest",
     "infr_cuda_get_config", "infr_cuda_set_config",
     "infr_cuda_ep_unique_id", "infr_cuda_ep_init", "infr_cuda_ep_finalize", "infr_cuda_ep_last_phases",
@@ -208,6 +208,8 @@ def load_library(path: Optional[str] = None):
     L.infr_cuda_ep_last_phases.argtypes = [vp, C.POINTER(C.c_float)]
     L.infr_cuda_launch_count.argtypes = [vp]
     L.infr_cuda_launch_count.restype = C.c_uint64
+    L.infr_cuda_em_down_ctas_per_sm.argtypes = [vp, u32, u32, u32, u32]
+    L.infr_cuda_em_down_ctas_per_sm.restype = u32
     for name in EXPORTS:
         f = getattr(L, name)
         if f.restype is C.c_int:  # default: every remaining entry point returns an int32 status

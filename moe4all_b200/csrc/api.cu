@@ -5,6 +5,7 @@
 #include <map>
 #include <mutex>
 #include <new>
+#include <tuple>
 
 #include "formats.cuh"
 #include "kernels.cuh"
@@ -58,6 +59,25 @@ cudaError_t ensure_smem(const void* kernel, size_t bytes) {
   if (e == cudaSuccess && bytes > 40 * 1024)
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e == cudaSuccess) g = bytes > 40 * 1024 ? bytes : 40 * 1024;
+  return e;
+}
+
+cudaError_t resident_ctas(const void* kernel, int threads, size_t bytes, int* ctas) {
+  cudaError_t e = ensure_smem(kernel, bytes);
+  if (e != cudaSuccess) return e;
+  // what the driver answers depends on these values alone: asked once for each
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void*, int, size_t>, int> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  int& n = known[{dev, kernel, threads, bytes}];
+  if (n == 0) {
+    int v = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, threads, bytes);
+    if (e == cudaSuccess) n = v > 1 ? v : 1;
+  }
+  *ctas = n;
   return e;
 }
 
@@ -436,6 +456,14 @@ int32_t infr_cuda_sync(infr_cuda_ctx* ctx) {
 }
 
 uint64_t infr_cuda_launch_count(const infr_cuda_ctx* ctx) { return ctx ? ctx->launches : 0; }
+
+uint32_t infr_cuda_em_down_ctas_per_sm(const infr_cuda_ctx* ctx, uint32_t ne, uint32_t n_ff_exp, uint32_t sh_ff, uint32_t down_dtype) {
+  if (!ctx || ne == 0 || ne % 256 || n_ff_exp == 0 || n_ff_exp % 256 || sh_ff % 256 || (down_dtype != INFR_CUDA_DT_Q4K && down_dtype != INFR_CUDA_DT_Q6K) ||
+      ne > (1u << 20) || n_ff_exp > (1u << 20) || sh_ff > (1u << 20))
+    return 0;
+  DeviceGuard guard(ctx->device);
+  return (uint32_t)em_down_ctas_per_sm((int)ne, (int)n_ff_exp, (int)sh_ff, down_dtype == INFR_CUDA_DT_Q4K);
+}
 
 int32_t infr_cuda_set_trace(infr_cuda_ctx* ctx, infr_cuda_buf* buf) {
   if (!ctx) return INFR_CUDA_ERR_INVALID_ARG;

@@ -84,6 +84,8 @@ int32_t ensure_scratch(infr_cuda_ctx* ctx, size_t bytes);
 
 // Raise a kernel's dynamic shared-memory limit once per (device, kernel) instead of on every launch.
 cudaError_t ensure_smem(const void* kernel, size_t bytes);
+// *ctas = CTAs of that many threads and bytes of dynamic shared memory that an SM holds (at least 1); grants the bytes first.
+cudaError_t resident_ctas(const void* kernel, int threads, size_t bytes, int* ctas);
 
 #ifdef __CUDACC__
 #define INFR_HD __host__ __device__

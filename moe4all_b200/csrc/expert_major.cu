@@ -907,24 +907,45 @@ void gateup_shape(int ne, int* KB, int* S, int* xpitch, size_t* stage_bytes) {
 // shorter rows, whose jobs the extra barrier costs more than it gives (32 rows, 512-wide experts: 153 -> 168 us).
 int down_warps(int nffmax) { return nffmax >= 768 ? 8 : 4; }
 
-int down_rows(int ne, int nffmax, size_t dbb, int* apitch, size_t* slab_pitch, size_t* smem, int* nbuf) {
-  *apitch = nffmax + 16;  // 4 (mod 32) words
-  const size_t fixed = (size_t)16 * *apitch + (size_t)8 * (nffmax / 16 + 4) * 4 + (size_t)8 * (nffmax / 128 + 1) * 4 + 256;
+using DownKernel = void (*)(EmParams, int, int, uint32_t);
+
+struct DownShape {
+  int rows, apitch, nbuf, warps;  // rows 0: no tile fits shared memory
+  size_t slab_pitch, smem;
+  DownKernel kernel;
+};
+
+DownShape down_shape(int ne, int nffmax, bool q4k) {
+  DownShape d = {};
+  d.apitch = nffmax + 16;  // 4 (mod 32) words
+  const size_t dbb = q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
+  const size_t fixed = (size_t)16 * d.apitch + (size_t)8 * (nffmax / 16 + 4) * 4 + (size_t)8 * (nffmax / 128 + 1) * 4 + 256;
   const size_t drb = (size_t)nffmax / 256 * dbb;
   const int nb = nffmax / 256;
-  const int most = down_warps(nffmax) == 8 ? 2 : 1;
-  for (int rows : {64, 32, 16}) {
-    if (ne % rows) continue;
-    if (nb == 1 && rows < 64) continue;  // (fewer rows only spread the blocks over more warps)
-    *slab_pitch = align_up((size_t)rows * drb + 8, 128) + 128;
-    for (*nbuf = most; *nbuf >= 1; --*nbuf) {
-      *smem = fixed + *nbuf * *slab_pitch;
-      if (rows == 16) return *smem <= 200 * 1024 ? rows : 0;
-      if (*smem <= 110 * 1024) return rows;
-      if (rows != 32) break;
+  d.warps = down_warps(nffmax);
+  const int most = d.warps == 8 ? 2 : 1;
+  auto choose = [&]() {
+    for (int rows : {64, 32, 16}) {
+      if (ne % rows) continue;
+      if (nb == 1 && rows < 64) continue;  // (fewer rows only spread the blocks over more warps)
+      d.slab_pitch = align_up((size_t)rows * drb + 8, 128) + 128;
+      for (d.nbuf = most; d.nbuf >= 1; --d.nbuf) {
+        d.smem = fixed + d.nbuf * d.slab_pitch;
+        if (rows == 16) return d.smem <= 200 * 1024 ? rows : 0;
+        if (d.smem <= 110 * 1024) return rows;
+        if (rows != 32) break;
+      }
     }
-  }
-  return 0;
+    return 0;
+  };
+  d.rows = choose();
+  if (d.warps == 4)
+    d.kernel = q4k ? k_em_down<true, 4, 1> : k_em_down<false, 4, 1>;
+  else if (d.nbuf == 2)
+    d.kernel = q4k ? k_em_down<true, 8, 2> : k_em_down<false, 8, 2>;
+  else
+    d.kernel = q4k ? k_em_down<true, 8, 1> : k_em_down<false, 8, 1>;
+  return d;
 }
 
 }  // namespace
@@ -944,10 +965,13 @@ size_t em_scratch_bytes(int rows, int n_used, int ne, int nff, int sh_ff) {
 
 bool em_supported(int ne, int nff, int sh_ff, int n_expert, BankTypes bt) {
   if (!bt.tuned() || ne % 256 || nff % 256 || sh_ff % 256 || n_expert > 1024) return false;
-  int apitch;
-  int nbuf;
-  size_t slab_pitch, smem;
-  return down_rows(ne, std::max(nff, sh_ff), bt.down_q4k() ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES, &apitch, &slab_pitch, &smem, &nbuf) != 0;
+  return down_shape(ne, std::max(nff, sh_ff), bt.down_q4k()).rows != 0;
+}
+
+int em_down_ctas_per_sm(int ne, int nff, int sh_ff, bool q4k) {
+  const DownShape d = down_shape(ne, std::max(nff, sh_ff), q4k);
+  int n = 0;
+  return d.rows != 0 && resident_ctas(reinterpret_cast<const void*>(d.kernel), d.warps * 32, d.smem, &n) == cudaSuccess ? n : 0;
 }
 
 int32_t launch_em_ffn(infr_cuda_ctx* ctx, const DecodeParams& dp, void* scratch, uint32_t stages) {
@@ -1025,26 +1049,18 @@ int32_t launch_em_ffn(infr_cuda_ctx* ctx, const DecodeParams& dp, void* scratch,
   }
   if (!(stages & 4u)) return INFR_CUDA_OK;
   {
-    int apitch, nbuf;
-    size_t slab_pitch, smem;
-    const int rows_cta = down_rows(dp.ne, (int)nffmax, dp.down_q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES, &apitch, &slab_pitch, &smem, &nbuf);
-    if (!rows_cta) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "expert-major down kernel: tile does not fit shared memory");
-    const unsigned jobs_bound = (unsigned)n_seg_bound * (unsigned)(dp.ne / rows_cta);
-    const unsigned per_sm = (unsigned)std::max<size_t>(1, std::min<size_t>(6, (215 * 1024) / (smem + 3072)));
-    const int warps = down_warps((int)nffmax);
-    auto run_dn = [&](auto kern) {
-      cudaError_t ee = ensure_smem(reinterpret_cast<const void*>(kern), smem);
-      if (ee == cudaSuccess)
-        ee = launch_ex(kern, dim3(std::min(jobs_bound, per_sm * (unsigned)ctx->sm_count)), dim3(warps * 32), smem, ctx->stream, true, p,
-                       rows_cta, apitch, (uint32_t)slab_pitch);
-      return ee;
-    };
-    if (warps == 4)
-      e = dp.down_q4k ? run_dn(k_em_down<true, 4, 1>) : run_dn(k_em_down<false, 4, 1>);
-    else if (nbuf == 2)
-      e = dp.down_q4k ? run_dn(k_em_down<true, 8, 2>) : run_dn(k_em_down<false, 8, 2>);
-    else
-      e = dp.down_q4k ? run_dn(k_em_down<true, 8, 1>) : run_dn(k_em_down<false, 8, 1>);
+    const DownShape d = down_shape(dp.ne, (int)nffmax, dp.down_q4k != 0);
+    if (!d.rows) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "expert-major down kernel: tile does not fit shared memory");
+    const unsigned jobs_bound = (unsigned)n_seg_bound * (unsigned)(dp.ne / d.rows);
+    // as many CTAs as an SM holds of them: with fewer, SMs are half used, or idle where two of a grid's CTAs land on one; with more,
+    // the last ones, whose share of the jobs is as large as the others', run behind them.  Asked of the driver: by 215 KB over the
+    // request + 3 KB it was two of three (Q4_K, 128 experts of 1280, 32 rows: the layer 179 -> 157 us; of 768 116 -> 105), one of two
+    // (Q6_K, 1536: 274 -> 203) and six of five (Q6_K, 256: 65.4 -> 61.5)
+    int per_sm = 0;
+    e = resident_ctas(reinterpret_cast<const void*>(d.kernel), d.warps * 32, d.smem, &per_sm);
+    if (e == cudaSuccess)
+      e = launch_ex(d.kernel, dim3(std::min(jobs_bound, (unsigned)(per_sm * ctx->sm_count))), dim3(d.warps * 32), d.smem, ctx->stream, true, p,
+                    d.rows, d.apitch, (uint32_t)d.slab_pitch);
     ctx->launches += 1;
     if (e != cudaSuccess) return check_cuda(ctx, e, "k_em_down launch");
   }

@@ -183,6 +183,7 @@ int route_small_group(const infr_cuda_ctx* ctx, int rows, int ne, int n_expert);
 int32_t launch_decode_ffn(infr_cuda_ctx* ctx, const DecodeParams& p, bool pdl, uint32_t stages);
 // The expert-major form of the same stages (2: bucket + gate/up, 4: down + combine); `scratch` holds em_scratch_bytes(...).
 bool em_supported(int ne, int nff, int sh_ff, int n_expert, BankTypes bt);
+int em_down_ctas_per_sm(int ne, int nff, int sh_ff, bool q4k);  // of the down kernel's launch; 0: not supported
 size_t em_scratch_bytes(int rows, int n_used, int ne, int nff, int sh_ff);
 int32_t launch_em_ffn(infr_cuda_ctx* ctx, const DecodeParams& p, void* scratch, uint32_t stages);
 // Whether the small-m kernels cover this shape (dims, shared-memory budget).

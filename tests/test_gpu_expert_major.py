@@ -223,3 +223,9 @@ def test_line_between_the_small_m_forms(backend, down_q4k, rows, em_form):
     ref = oracle_layer(L, x, 4)
     keep = check_ids(ids, ref, 4)
     assert_close(out[keep], ref.dst[keep], tol=2e-4)  # both forms round activations to 16 bits: far inside the bound on layers
+
+
+@pytest.mark.parametrize("dtype,nff,ctas", [(12, 768, 3), (12, 1024, 2), (12, 1280, 3), (14, 768, 2), (14, 1280, 2), (14, 1536, 2), (14, 3072, 1)])
+def test_down_kernel_fills_an_sm(backend, dtype, nff, ctas):
+    # widths whose CTAs only just fit an SM's shared memory (Q4_K 768 and 1280: three, Q6_K 1536: two) and others
+    assert backend._lib.infr_cuda_em_down_ctas_per_sm(backend._ctx, 2048, nff, 0, dtype) == ctas
