@@ -647,6 +647,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ int s_pair[8];
+  __shared__ float s_unit[8];  // Q4_K: a token's fixed-point unit
   __shared__ float s_dred[(WARPS - 1) * 128];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -663,12 +664,12 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
   const int job0 = (int)((long long)blockIdx.x * n_jobs / gridDim.x), job1 = (int)((long long)(blockIdx.x + 1) * n_jobs / gridDim.x);
   if (job0 >= job1) return;
   const int ngrp = (p.nffmax >> 4) + 4;  // ints per token of the sums: tokens 2t land in different banks
-  const int nhalf = (p.nffmax >> 7) + 1;  // room for a token's fixed-point units
-  // shared memory: activation limbs [2][8 tokens][apitch] | sums [8][ngrp] ints | units [8][nhalf] | NBUF slab buffers
+  const int nhalf = (p.nffmax >> 7) + 1;  // room for a token's fixed-point units (Q6_K)
+  // shared memory: activation limbs [2][8 tokens][apitch] | sums [8][ngrp] ints | Q6_K: units [8][nhalf] | NBUF slab buffers
   unsigned char* s_act = smem;
   int* s_sum = reinterpret_cast<int*>(smem + (size_t)16 * apitch);
   float* s_xs = reinterpret_cast<float*>(s_sum + 8 * ngrp);
-  unsigned char* slab_area = reinterpret_cast<unsigned char*>(s_xs + 8 * nhalf);
+  unsigned char* slab_area = reinterpret_cast<unsigned char*>(Q4 ? s_xs : s_xs + 8 * nhalf);
   slab_area += (128u - (smem_u32(slab_area) & 127u)) & 127u;
 
   auto width_of = [&](int e) { return e >= p.n_expert ? p.sh_ff : p.nff; };
@@ -731,7 +732,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
           auto unit = [&](float m) {
             m = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));
             inv = m > 0.f ? 32639.f / m : 0.f;
-            if (lane == 0) s_xs[tk * nhalf] = m / 32639.f;
+            if (lane == 0) s_unit[tk] = m / 32639.f;
           };
           auto limbs = [&](int i, float4 v) {  // (n4 is a multiple of 64: whole warps)
             const int X[4] = {__float2int_rn(v.x * inv), __float2int_rn(v.y * inv), __float2int_rn(v.z * inv), __float2int_rn(v.w * inv)};
@@ -827,7 +828,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
       for (int i = 0; i < 4; ++i) {
         const int tk = narrow ? t : 2 * t + (i & 1);
         if (tk < cnt && !(narrow && (i & 1)))
-          p.y[(size_t)s_pair[tk] * p.ne + i0 + g + 8 * (i >> 1)] = Q4 ? acc[i] * s_xs[tk * nhalf] : acc[i];
+          p.y[(size_t)s_pair[tk] * p.ne + i0 + g + 8 * (i >> 1)] = Q4 ? acc[i] * s_unit[tk] : acc[i];
       }
     }
   }
@@ -919,7 +920,7 @@ DownShape down_shape(int ne, int nffmax, bool q4k) {
   DownShape d = {};
   d.apitch = nffmax + 16;  // 4 (mod 32) words
   const size_t dbb = q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
-  const size_t fixed = (size_t)16 * d.apitch + (size_t)8 * (nffmax / 16 + 4) * 4 + (size_t)8 * (nffmax / 128 + 1) * 4 + 256;
+  const size_t fixed = (size_t)16 * d.apitch + (size_t)8 * (nffmax / 16 + 4) * 4 + (q4k ? 0 : (size_t)8 * (nffmax / 128 + 1) * 4) + 256;
   const size_t drb = (size_t)nffmax / 256 * dbb;
   const int nb = nffmax / 256;
   d.warps = down_warps(nffmax);

@@ -225,7 +225,19 @@ def test_line_between_the_small_m_forms(backend, down_q4k, rows, em_form):
     assert_close(out[keep], ref.dst[keep], tol=2e-4)  # both forms round activations to 16 bits: far inside the bound on layers
 
 
-@pytest.mark.parametrize("dtype,nff,ctas", [(12, 768, 3), (12, 1024, 2), (12, 1280, 3), (14, 768, 2), (14, 1280, 2), (14, 1536, 2), (14, 3072, 1)])
+@pytest.mark.parametrize("dtype,nff,ctas", [(12, 768, 3), (12, 1024, 2), (12, 1280, 3), (12, 2048, 2), (12, 3072, 2), (14, 768, 2), (14, 1280, 2), (14, 1536, 2), (14, 3072, 1)])
 def test_down_kernel_fills_an_sm(backend, dtype, nff, ctas):
-    # widths whose CTAs only just fit an SM's shared memory (Q4_K 768 and 1280: three, Q6_K 1536: two) and others
+    # widths whose CTAs only just fit an SM's shared memory (Q4_K 768 and 1280: three, 2048 and 3072: two, Q6_K 1536: two) and others
     assert backend._lib.infr_cuda_em_down_ctas_per_sm(backend._ctx, 2048, nff, 0, dtype) == ctas
+
+
+def test_widest_q4k_down_banks(em):
+    # 5632: the widest whose 16-row jobs fit shared memory
+    L = synth.make_layer(35, 512, 8, 5632, down_q4k=True, router_std=0.05)
+    x = synth.activations(41, 5, 512)
+    n0 = em.launch_count()
+    out, ids, _ = GpuLayer(em, L).run(x, 2, path=1)
+    assert em.launch_count() - n0 == 5  # the expert-major kernels ran
+    ref = oracle_layer(L, x, 2)
+    keep = check_ids(ids, ref, 2)
+    assert_close(out[keep], ref.dst[keep])
