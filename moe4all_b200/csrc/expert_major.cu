@@ -542,7 +542,7 @@ __device__ __forceinline__ int sext_byte(uint32_t w, int i) {
 // Q6_K: the slab starts on a 16-byte boundary, the rows' blocks at byte offsets ro0, ro1 on 2-byte ones.
 template <bool NARROW>
 __device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_t ro0, uint32_t ro1, const unsigned char* alo, const unsigned char* ahi,
-                                              const int* sum0, const int* sum1, const float* xs0, const float* xs1, int b, float (&acc)[4]) {
+                                              const int* sum0, const int* sum1, int b, float (&acc)[4]) {
   constexpr int NT = NARROW ? 1 : 2;
   const int t = threadIdx.x & 3;
   // per row: aligned view of the block, the shift that realigns it, d and the 16 scales
@@ -560,14 +560,10 @@ __device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_
     for (int i = 0; i < 4; ++i) sc[r][i] = __funnelshift_r(wq[r][48 + i], wq[r][49 + i], sh[r]);
   }
   int svl[2][NT], svh[2][NT], mv[2][NT];
-  float part[2][NT];
 #pragma unroll
   for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int k = 0; k < NT; ++k) {
-      svl[r][k] = svh[r][k] = mv[r][k] = 0;
-      part[r][k] = 0.f;
-    }
+    for (int k = 0; k < NT; ++k) svl[r][k] = svh[r][k] = mv[r][k] = 0;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
 #pragma unroll
@@ -608,20 +604,13 @@ __device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_
           }
       }
     }
-    // half a block (128 activations share a fixed-point unit): sc * (sum(q X) - 32 sum(X)), X = 256 hi + lo
-    const float xs[2] = {xs0[2 * b + h], NARROW ? 0.f : xs1[2 * b + h]};
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-      for (int k = 0; k < NT; ++k) {
-        part[r][k] = fmaf(xs[k], fmaf(256.f, (float)svh[r][k], (float)svl[r][k]) - 32.f * (float)mv[r][k], part[r][k]);
-        svl[r][k] = svh[r][k] = mv[r][k] = 0;
-      }
   }
+  // sum over the block of sc * (sum(q X) - 32 sum(X)), X = 256 hi + lo
 #pragma unroll
   for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int k = 0; k < NT; ++k) acc[2 * r + k] = fmaf(d[r], part[r][k], acc[2 * r + k]);
+    for (int k = 0; k < NT; ++k)
+      acc[2 * r + k] = fmaf(d[r], fmaf(256.f, (float)svh[r][k], (float)svl[r][k]) - 32.f * (float)mv[r][k], acc[2 * r + k]);
 }
 
 // Job = (segment of up to 8 token rows, tile of `rows_cta` output features).  CTAs are persistent and take a
@@ -641,13 +630,16 @@ __device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_
 // other's waits (24 rows, Q6_K, 512 wide: 113 -> 107 us a layer; a scheduler then has 4.4 warps and still nothing to issue in
 // 41 % of its cycles at 32 rows).  Eight warps have two (768 wide, 16 rows: 103 us against 115 with one) unless two leave room for 16 rows only:
 // one of 32 then halves the jobs and their barriers (2048 wide, 64 rows: 1372 -> 1312 us).
+// Two CTAs per SM asked of the compiler where eight warps read Q6_K: left alone it takes 97 registers, told of them 118, with more
+// loads ahead of their use (128 experts of 1024, 32 rows: the layer 154 -> 148 us; of 768 121 -> 117).  Not with Q4_K, of which three
+// fit at 74 registers, nor with four warps (80 registers and spills: 512 wide, 32 rows 86 -> 89).
 template <bool Q4, int WARPS, int NBUF>
-__global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta, int apitch, uint32_t slab_pitch) {
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 && !Q4 ? 2 : 0) k_em_down(EmParams p, int rows_cta, int apitch, uint32_t slab_pitch) {
   constexpr uint32_t DBB = Q4 ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ int s_pair[8];
-  __shared__ float s_unit[8];  // Q4_K: a token's fixed-point unit
+  __shared__ float s_unit[8];  // a token's fixed-point unit
   __shared__ float s_dred[(WARPS - 1) * 128];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -664,12 +656,10 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
   const int job0 = (int)((long long)blockIdx.x * n_jobs / gridDim.x), job1 = (int)((long long)(blockIdx.x + 1) * n_jobs / gridDim.x);
   if (job0 >= job1) return;
   const int ngrp = (p.nffmax >> 4) + 4;  // ints per token of the sums: tokens 2t land in different banks
-  const int nhalf = (p.nffmax >> 7) + 1;  // room for a token's fixed-point units (Q6_K)
-  // shared memory: activation limbs [2][8 tokens][apitch] | sums [8][ngrp] ints | Q6_K: units [8][nhalf] | NBUF slab buffers
+  // shared memory: activation limbs [2][8 tokens][apitch] | sums [8][ngrp] ints | NBUF slab buffers
   unsigned char* s_act = smem;
   int* s_sum = reinterpret_cast<int*>(smem + (size_t)16 * apitch);
-  float* s_xs = reinterpret_cast<float*>(s_sum + 8 * ngrp);
-  unsigned char* slab_area = reinterpret_cast<unsigned char*>(Q4 ? s_xs : s_xs + 8 * nhalf);
+  unsigned char* slab_area = reinterpret_cast<unsigned char*>(s_sum + 8 * ngrp);
   slab_area += (128u - (smem_u32(slab_area) & 127u)) & 127u;
 
   auto width_of = [&](int e) { return e >= p.n_expert ? p.sh_ff : p.nff; };
@@ -718,69 +708,48 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
       if (job != job0) my_pair = tid < cnt ? __ldcg(p.seg_pairs + off + tid) : -1;
       if (tid < 8) s_pair[tid] = my_pair;
       __syncthreads();
-      // fixed point: X = round(a * 32639 / max|a|) per 128 elements of a row (Q6_K) or per row (Q4_K), limbs X = 256 hi + lo, sums
-      // per 16 elements.  A warp takes whole rows: no barrier between a maximum and its rounding.  With Q6_K banks one unit for
-      // the whole row left 1.1 - 1.2 times the error of the per-pair kernels' 128 (7.1e-5 against 8.1e-5 of the result, 13 rows of
-      // 512) and was slower (32 rows 122 -> 119 us the layer); with Q4_K the errors are level, and a unit per block costs two
-      // multiplications for each of its results (427 rows of 2560, 512-wide experts: the kernel 76 us, 71 with one per row).
+      // fixed point: X = round(a * 32639 / max|a|) per row, limbs X = 256 hi + lo, sums per 16 elements.  A warp takes whole rows: no
+      // barrier between a row's maximum and its rounding.  One unit per 128 elements, as in the per-pair kernels, has a little less
+      // error (Q6_K, 13 rows of 512: 7.1e-5 of the result against 8.1e-5; Q4_K level) but costs two multiplications and a conversion
+      // more for each of its results (Q4_K, 427 rows of 2560 over 512-wide experts: the kernel 76 us, 71 with one per row).
       const int n4 = nff_e / 4;
       for (int tk = warp; tk < cnt; tk += WARPS) {
         const float4* arow = reinterpret_cast<const float4*>(p.act + (size_t)s_pair[tk] * p.nffmax);
-        if constexpr (Q4) {
-          auto top = [](float4 v, float m) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(m, fmaxf(fabsf(v.z), fabsf(v.w)))); };
-          float inv = 0.f;
-          auto unit = [&](float m) {
-            m = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));
-            inv = m > 0.f ? 32639.f / m : 0.f;
-            if (lane == 0) s_unit[tk] = m / 32639.f;
-          };
-          auto limbs = [&](int i, float4 v) {  // (n4 is a multiple of 64: whole warps)
-            const int X[4] = {__float2int_rn(v.x * inv), __float2int_rn(v.y * inv), __float2int_rn(v.z * inv), __float2int_rn(v.w * inv)};
-            uint32_t lo, hi;
-            pack_limbs4(X, lo, hi);
-            *reinterpret_cast<uint32_t*>(s_act + (size_t)tk * apitch + 4 * i) = lo;
-            *reinterpret_cast<uint32_t*>(s_act + (size_t)((cnt <= EM_NARROW ? EM_NARROW : 8) + tk) * apitch + 4 * i) = hi;
-            int sx = (X[0] + X[1]) + (X[2] + X[3]);  // 16 elements = four neighbouring lanes
-            sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 1);
-            sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 2);
-            if ((i & 3) == 0) s_sum[tk * ngrp + (i >> 2)] = sx;
-          };
-          float m = 0.f;
-          if (n4 <= 128) {  // up to 512 wide: the row stays in registers
-            float4 v[4];
+        auto top = [](float4 v, float m) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(m, fmaxf(fabsf(v.z), fabsf(v.w)))); };
+        float inv = 0.f;
+        auto unit = [&](float m) {
+          m = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));
+          inv = m > 0.f ? 32639.f / m : 0.f;
+          if (lane == 0) s_unit[tk] = m / 32639.f;
+        };
+        auto limbs = [&](int i, float4 v) {  // (n4 is a multiple of 64: whole warps)
+          const int X[4] = {__float2int_rn(v.x * inv), __float2int_rn(v.y * inv), __float2int_rn(v.z * inv), __float2int_rn(v.w * inv)};
+          uint32_t lo, hi;
+          pack_limbs4(X, lo, hi);
+          *reinterpret_cast<uint32_t*>(s_act + (size_t)tk * apitch + 4 * i) = lo;
+          *reinterpret_cast<uint32_t*>(s_act + (size_t)((cnt <= EM_NARROW ? EM_NARROW : 8) + tk) * apitch + 4 * i) = hi;
+          int sx = (X[0] + X[1]) + (X[2] + X[3]);  // 16 elements = four neighbouring lanes
+          sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 1);
+          sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 2);
+          if ((i & 3) == 0) s_sum[tk * ngrp + (i >> 2)] = sx;
+        };
+        float m = 0.f;
+        if (n4 <= 128) {  // up to 512 wide: the row stays in registers
+          float4 v[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = lane + 32 * u < n4 ? __ldcg(arow + lane + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int u = 0; u < 4; ++u) v[u] = lane + 32 * u < n4 ? __ldcg(arow + lane + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) m = top(v[u], m);
-            unit(m);
+          for (int u = 0; u < 4; ++u) m = top(v[u], m);
+          unit(m);
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (lane + 32 * u < n4) limbs(lane + 32 * u, v[u]);
-          } else {
-#pragma unroll 4
-            for (int i = lane; i < n4; i += 32) m = top(__ldcg(arow + i), m);
-            unit(m);
-#pragma unroll 4
-            for (int i = lane; i < n4; i += 32) limbs(i, __ldcg(arow + i));
-          }
+          for (int u = 0; u < 4; ++u)
+            if (lane + 32 * u < n4) limbs(lane + 32 * u, v[u]);
         } else {
 #pragma unroll 4
-          for (int i = lane; i < n4; i += 32) {
-            const float4 v = __ldcg(arow + i);
-            float m = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(0.f, fmaxf(fabsf(v.z), fabsf(v.w))));
-            m = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));
-            const float inv = m > 0.f ? 32639.f / m : 0.f;
-            if (lane == 0) s_xs[tk * nhalf + (i >> 5)] = m / 32639.f;
-            const int X[4] = {__float2int_rn(v.x * inv), __float2int_rn(v.y * inv), __float2int_rn(v.z * inv), __float2int_rn(v.w * inv)};
-            uint32_t lo, hi;
-            pack_limbs4(X, lo, hi);
-            *reinterpret_cast<uint32_t*>(s_act + (size_t)tk * apitch + 4 * i) = lo;
-            *reinterpret_cast<uint32_t*>(s_act + (size_t)((cnt <= EM_NARROW ? EM_NARROW : 8) + tk) * apitch + 4 * i) = hi;
-            int sx = (X[0] + X[1]) + (X[2] + X[3]);  // 16 elements = four neighbouring lanes (n4 is a multiple of 64: whole warps)
-            sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 1);
-            sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 2);
-            if ((i & 3) == 0) s_sum[tk * ngrp + (i >> 2)] = sx;
-          }
+          for (int i = lane; i < n4; i += 32) m = top(__ldcg(arow + i), m);
+          unit(m);
+#pragma unroll 4
+          for (int i = lane; i < n4; i += 32) limbs(i, __ldcg(arow + i));
         }
       }
       __syncthreads();
@@ -799,16 +768,14 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
     const unsigned char* ahi = alo + (size_t)8 * apitch;
     const int* sum0 = s_sum + (narrow ? t : 2 * t) * ngrp;
     const int* sum1 = sum0 + ngrp;
-    const float* xs0 = s_xs + (narrow ? t : 2 * t) * nhalf;
-    const float* xs1 = xs0 + nhalf;
     const int rt = warp % n_rt, ks = warp / n_rt;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     const uint32_t rofs[2] = {(uint32_t)(rt * 16 + g) * drb, (uint32_t)(rt * 16 + g + 8) * drb};
     for (int b = ks; b < nb; b += ksplit) {
       if (Q4 && narrow) down_block_q4<true>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
       if (Q4 && !narrow) down_block_q4<false>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
-      if (!Q4 && narrow) down_block_q6<true>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, xs0, xs1, b, acc);
-      if (!Q4 && !narrow) down_block_q6<false>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, xs0, xs1, b, acc);
+      if (!Q4 && narrow) down_block_q6<true>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
+      if (!Q4 && !narrow) down_block_q6<false>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
     }
     if (ksplit > 1) {
       if (ks > 0) {
@@ -827,8 +794,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_em_down(EmParams p, int rows_cta
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int tk = narrow ? t : 2 * t + (i & 1);
-        if (tk < cnt && !(narrow && (i & 1)))
-          p.y[(size_t)s_pair[tk] * p.ne + i0 + g + 8 * (i >> 1)] = Q4 ? acc[i] * s_unit[tk] : acc[i];
+        if (tk < cnt && !(narrow && (i & 1))) p.y[(size_t)s_pair[tk] * p.ne + i0 + g + 8 * (i >> 1)] = acc[i] * s_unit[tk];
       }
     }
   }
@@ -920,7 +886,7 @@ DownShape down_shape(int ne, int nffmax, bool q4k) {
   DownShape d = {};
   d.apitch = nffmax + 16;  // 4 (mod 32) words
   const size_t dbb = q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
-  const size_t fixed = (size_t)16 * d.apitch + (size_t)8 * (nffmax / 16 + 4) * 4 + (q4k ? 0 : (size_t)8 * (nffmax / 128 + 1) * 4) + 256;
+  const size_t fixed = (size_t)16 * d.apitch + (size_t)8 * (nffmax / 16 + 4) * 4 + 256;
   const size_t drb = (size_t)nffmax / 256 * dbb;
   const int nb = nffmax / 256;
   d.warps = down_warps(nffmax);

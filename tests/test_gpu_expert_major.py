@@ -241,3 +241,41 @@ def test_widest_q4k_down_banks(em):
     ref = oracle_layer(L, x, 2)
     keep = check_ids(ids, ref, 2)
     assert_close(out[keep], ref.dst[keep])
+
+
+def identity_bank(n, dtype):
+    """[n, n] weights in raw blocks: 1 on the diagonal, 0 elsewhere."""
+    i = np.arange(n)
+    b, e = i // 256, i % 256  # block of the row and element of the block
+    if dtype == 12:
+        out = np.zeros((n, n // 256, 144), np.uint8)
+        out[..., 1] = 0x3C  # d = 1.0
+        out[..., 4:8] = 1  # six-bit scales of sub-blocks 0 - 3 (mins 0) ...
+        out[..., 12:16] = 1  # ... and 4 - 7
+        out[i, b, 16 + 32 * (e // 64) + e % 32] = np.where(e % 64 < 32, 0x01, 0x10)
+    else:
+        out = np.zeros((n, n // 256, 210), np.uint8)
+        out[..., 128:192] = 0xAA  # q = 32 everywhere: weight 0
+        out[i, b, 192 + e // 16] = 1  # the other groups' scales stay 0: a group's integer sums stay below 2^24
+        out[..., 209] = 0x3C
+        out[i, b, 64 * (e // 128) + e % 64] = np.where(e % 128 < 64, 0x01, 0x10)  # q = 33
+    return out.reshape(-1)
+
+
+@pytest.mark.parametrize("dtype", [12, 14])
+@pytest.mark.parametrize("nff", [256, 512, 768])  # one row of activations in registers, and read twice by eight warps
+@pytest.mark.parametrize("rows", [3, 24])
+def test_activations_have_one_unit_per_row(em, dtype, nff, rows):
+    # Down banks that pass the activations through show their fixed-point form: every element of a row is a whole multiple of the row's
+    # largest / 32639.  A finer unit is as correct but gives other bits, after which a row of a chain of layers can take another expert.
+    L = synth.make_layer(37, nff, 4, nff, router_std=0.05, dtypes=(12, 12, dtype))
+    L.down = np.tile(identity_bank(nff, dtype), 4)
+    x = synth.activations(43 + rows, rows, nff)
+    out, ids, _ = GpuLayer(em, L).run(x, 1, path=1)
+    ref = oracle_layer(L, x, 1)
+    keep = check_ids(ids, ref, 1)
+    assert_close(out[keep], ref.dst[keep])
+    out = out.astype(np.float64)
+    q = out / (np.abs(out).max(axis=1, keepdims=True) / 32639)
+    # the unit, its product with a whole number of at most 32639 and the same of the largest: up to four roundings of 2^-24
+    assert np.abs(q - np.rint(q)).max() <= 4 * 32639 * 2.0**-24
