@@ -632,27 +632,20 @@ int32_t validate_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d, ui
 // The lines below were drawn on earlier kernels: eleven pairs per expert between em and gg, 2.75 rows per expert (8 rows of
 // large ones) between pp and gg.  On today's, em and gg cross at six to seven pairs per expert (gg is level from 8 rows on for
 // large experts with Q4_K down), pp and gg between 0.1 rows per expert (Q8_0) and one (Q5_K, MXFP4).
-// Per-pair against expert-major: the second reads an expert's blocks once for all its rows, about pairs^2 / (2 experts) fewer
-// reads of an expert and rows - 1 fewer of the shared one, but takes two more launches and a pass over f32 rows, so what it saves
-// has to reach some size: the reads saved times the expert's weights, 18432 x 1024 of them (or three pairs per two experts, where
-// experts are so small that they never do).  With Q4_K down banks the expert-major kernels round activations per row and not per
-// 128 as the per-pair ones (up to 1.05 times the error): there the line is where the reads saved of the routed experts alone
-// are 25600 x 1024 weights, or two pairs per expert.  pp / em around the line, us per layer, Q6_K down and (Q4_K down):
+// Per-pair against expert-major: the second reads an expert's blocks once for all its rows (about pairs^2 / (2 experts) fewer
+// reads of an expert) but takes two more launches and a pass over f32 rows, so what it saves has to reach some size, 25600 x 1024
+// weights; for experts so small that it never does, two pairs per expert.  The expert-major kernels round activations per row and
+// not per 128 as the per-pair ones (up to 1.2 times the error with Q6_K down banks, 1.05 with Q4_K), so the line is not drawn
+// where the times cross but behind it.  pp / em around the line, us per layer, Q6_K down and (Q4_K down):
 //   2048 wide, 256 of 512, top-8, shared: 8 rows 68.2 / 72.9 (65.1 / 66.7), 9 rows 68.4 / 67.0 (64.7 / 62.3), 13 rows 86.4 / 77.1 (79.6 / 70.4)
 //   2048 wide, 128 of 768, top-8: 6 rows 68.3 / 69.9 (58.7 / 62.9), 7 rows 77.5 / 72.1 (67.5 / 63.9), 8 rows 83.2 / 76.1 (72.4 / 70.4)
 //   2048 wide, 64 of 1024, top-8: 4 rows 63.1 / 58.7 (50.0 / 53.4), 5 rows 84.4 / 66.8 (67.9 / 63.3)
-//   3072 wide, 128 of 768, top-8, shared: 4 rows 87.3 / 69.2 (81.4 / 64.3), 5 rows 106 / 84 (100 / 73): the line is at 5
 //   4096 wide, 96 of 1536, top-4: 5 rows 106 / 112 (94 / 84), 6 rows 120 / 123 (108 / 94), 8 rows 150 / 146 (135 / 112)
-//   2560 wide, 160 of 512, top-6, shared: 8 rows 77.4 / 73.5 (68.7 / 66.3), 10 rows 88.3 / 71.4 (80.1 / 67.4): the line is at 9
 //   1024 wide, 32 of 256, top-4: 10 rows 27.8 / 27.2, 12 rows 28.4 / 26.9, 16 rows 31.2 / 28.5;  28 MB experts: 1 row 171 / 104, 2 rows 306 / 164
-bool em_preferred(uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff, uint32_t sh_ff, bool down_q4k) {
+bool em_preferred(uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff) {
   const uint64_t size = (uint64_t)ne * nff, pairs = (uint64_t)rows * n_used;
   if (size >= (1ull << 23)) return rows >= 2;  // experts of tens of megabytes
-  if (down_q4k) return pairs >= 2 * (uint64_t)n_expert || pairs * pairs * (size >> 10) >= (uint64_t)n_expert * 51200;
-  if (2 * pairs >= 3 * (uint64_t)n_expert) return true;
-  // twice the weights not read again, both terms over n_expert
-  const uint64_t saved = pairs * pairs * size + 2 * (uint64_t)(rows - 1) * ne * sh_ff * n_expert;
-  return saved >= 2 * (uint64_t)n_expert * (18432ull << 10);
+  return pairs >= 2 * (uint64_t)n_expert || pairs * pairs * (size >> 10) >= (uint64_t)n_expert * 51200;
 }
 
 uint32_t choose_moe_path(const infr_cuda_ctx* ctx, uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff,
@@ -778,7 +771,7 @@ int32_t infr_cuda_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d) {
   // (small) launches.
   const bool use_em = path == 1 && em_ok &&
                       (ctx->cfg.expert_major == 2 || !small_ok ||
-                       (ctx->cfg.expert_major == 0 && em_preferred(d->rows, d->n_used, d->n_expert, d->ne, d->n_ff_exp, (uint32_t)sh_ff_eff, down_q4k)));
+                       (ctx->cfg.expert_major == 0 && em_preferred(d->rows, d->n_used, d->n_expert, d->ne, d->n_ff_exp)));
   if (path == 1) {
     if (!small_ok && !use_em) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, why);
     // Where the whole-row router kernel covers the call it also normalises x and makes its

@@ -165,7 +165,7 @@ int32_t validate_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d, ui
 // expert-major kernels are ahead of the per-pair ones.
 uint32_t choose_moe_path(const infr_cuda_ctx* ctx, uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff,
                          uint32_t sh_ff, BankTypes bt);
-bool em_preferred(uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff, uint32_t sh_ff, bool down_q4k);
+bool em_preferred(uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff);
 
 size_t small_path_scratch_need(const infr_cuda_moe_ffn_desc* d);
 
