@@ -196,6 +196,18 @@ def test_wide_hidden(backend):
     assert_close(out, ref.dst)
 
 
+@pytest.mark.parametrize("rows,ne", [(1, 8448), (2, 8448), (1, 12288)])
+@pytest.mark.parametrize("dtypes", [(12, 12, 14), (8, 8, 8)])
+def test_rows_wider_than_a_ctas_registers(backend, rows, ne, dtypes):
+    # past 8192 the expert-major and the generic kernels serve small calls; the router kernel makes their fixed-point copy of x
+    L = synth.make_layer(13, ne, 4, 256, router_std=0.05, dtypes=dtypes)
+    x = synth.activations(90 + rows, rows, ne)
+    out, ids, wts = GpuLayer(backend, L).run(x, 2)
+    ref = oracle_layer(L, x, 2)
+    check_ids(ids, wts, ref, 2)
+    assert_close(out, ref.dst)
+
+
 @pytest.mark.parametrize("rows,ne", [(6, 7168), (16, 2048), (33, 1024), (64, 512)])
 def test_router_row_groups(backend, rows, ne):
     # calls of more rows than one router CTA holds run as groups of tokens (one selecting CTA and
