@@ -16,7 +16,7 @@ def route(be, x, router, k, *, bias=None, gating=0, groups=0, groups_used=0, nor
     ids, wts = be.alloc(rows * k * 4), be.alloc(rows * k * 4)
     g = be.from_host(np.ascontiguousarray(given, np.int32)) if given is not None else None
     b = be.from_host(bias) if bias is not None else None
-    be.moe_route(MoeFfn(x=be.from_host(x), router=be.from_host(router), gate_exps=None, up_exps=None, down_exps=None, dst=None, rows=rows, ne=NE,
+    be.moe_route(MoeFfn(x=be.from_host(x), router=be.from_host(router), gate_exps=None, up_exps=None, down_exps=None, dst=None, rows=rows, ne=x.shape[1],
                         n_expert=E, n_used=k, n_ff_exp=256, gating=MoeGating(gating), norm_w=norm_w, scale=scale, exp_probs_b=b,
                         n_expert_groups=groups, n_expert_groups_used=groups_used, ids_out=ids, wts_out=wts, expert_ids=g))
     be.sync()
@@ -25,8 +25,9 @@ def route(be, x, router, k, *, bias=None, gating=0, groups=0, groups_used=0, nor
 
 def reference(x, router, k, *, bias=None, gating=0, groups=0, groups_used=0, norm_w=True, scale=1.0, given=None):
     E = router.shape[0]
-    z = np.zeros(E * 256 * 144, np.uint8)  # expert blocks of zeros: only ids, weights and scores are looked at
-    return orc.moe_ffn(x, router, z, z, np.zeros(E * NE * 210, np.uint8), n_expert=E, n_used=k, n_ff_exp=256, gating=gating, bias=bias, groups=groups,
+    ne = x.shape[1]
+    z = np.zeros(E * ne * 144, np.uint8)  # expert blocks of zeros: only ids, weights and scores are looked at
+    return orc.moe_ffn(x, router, z, z, np.zeros(E * ne * 210, np.uint8), n_expert=E, n_used=k, n_ff_exp=256, gating=gating, bias=bias, groups=groups,
                        groups_used=groups_used, norm_w=norm_w, scale=scale, expert_ids=given)
 
 
@@ -47,6 +48,22 @@ def test_selection(backend, rows, E, k, gating, groups, used, bias):
     same = (ids == ref.ids).all(axis=1)
     assert set(np.where(~same)[0]) <= set(tied), (ids, ref.ids)
     # the same operations on the same logits: only the last bit of exp can differ
+    np.testing.assert_allclose(wts[same], ref.wts[same], rtol=1e-6)
+
+
+@pytest.mark.parametrize("rows", [3, 4, 7])
+@pytest.mark.parametrize("groups,used", [(0, 0), (2, 1), (4, 2)])
+def test_groups_of_rows_of_unlike_sizes(backend, rows, groups, used):
+    # three rows of 10240 fit a CTA, so four and seven leave one for the last group: teams of two warps and of four; with two expert
+    # groups of 64 the larger team's lanes hold too few of them, and neither group of rows goes to teams
+    rng = np.random.default_rng(rows * 7 + groups)
+    x = rng.standard_normal((rows, 10240)).astype(np.float32)
+    router = (rng.standard_normal((128, 10240)) * 0.02).astype(np.float32)
+    kw = dict(gating=1, groups=groups, groups_used=used)
+    ids, wts = route(backend, x, router, 8, **kw)
+    ref = reference(x, router, 8, **kw)
+    same = (ids == ref.ids).all(axis=1)
+    assert set(np.where(~same)[0]) <= set(near_tie_rows(ref, 8)), (ids, ref.ids)
     np.testing.assert_allclose(wts[same], ref.wts[same], rtol=1e-6)
 
 
