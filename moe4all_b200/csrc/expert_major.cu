@@ -56,7 +56,8 @@ __global__ void __launch_bounds__(1024) k_em_bucket(EmParams p, int seg_cap) {
   pdl_trigger();
   // Two passes over the same code: the first, while the router still runs, without pairs and without stores, has the second find
   // its instructions cached.  A thread keeps its pairs' experts and their ranks inside them (the count before its own) in
-  // registers (32 rows, top-8 of 256: 3.2 - 5.5 -> 2.8 us behind the router).
+  // registers (32 rows, top-8 of 256: 3.2 - 5.5 -> 2.8 us behind the router).  With these the kernel has 58 registers and fits beside no
+  // CTA of the router; held to 32, which does, it made the layer 0 - 3 us slower from 33 to 64 rows (40 rows 124.9 -> 128.1).
   constexpr int KEEP = 3;  // covers eleven pairs per expert of 256; more are read again
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
