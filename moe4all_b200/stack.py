@@ -29,7 +29,9 @@ class MoeStack:
         self.hidden = torch.zeros(rows, ne, device=dev)
         self.hn = torch.zeros(rows, ne, device=dev)
         self.sub = torch.zeros(rows, ne, device=dev)
-        self.ids = torch.zeros(len(layers), rows, n_used, dtype=torch.int32, device=dev)
+        # each layer's ids on a 16-byte boundary, as the library wants its buffers
+        per_layer = (rows * n_used + 3) // 4 * 4
+        self.ids = torch.zeros(len(layers), per_layer, dtype=torch.int32, device=dev)[:, : rows * n_used].unflatten(1, (rows, n_used))
         self._nw = norm_weights
         self.b_hidden, self.b_hn, self.b_sub = be.wrap_tensor(self.hidden), be.wrap_tensor(self.hn), be.wrap_tensor(self.sub)
         self.b_nw = [be.wrap_tensor(w) for w in norm_weights]

@@ -67,6 +67,32 @@ def test_stack_teacher_forced_and_replay(backend, fused):
             be.set_stream(None)
 
 
+@pytest.mark.parametrize("rows,k", [(1, 6), (5, 3), (25, 6)])
+def test_ids_of_a_layer_may_end_anywhere(backend, rows, k):
+    # rows x k ids that are no multiple of 16 bytes: every layer's are its own, and those of the layer alone
+    be = backend
+    # (norm weights of 0.04 with routers of 1 / 0.04: sub-layers that add a fraction of the stream, scores as far apart as without)
+    layers = [DeviceLayer(be, 400 + i, NE, E, NFF, router_std=0.05 / 0.04) for i in range(3)]
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    nws = [0.04 * (1.0 + 0.1 * torch.randn(NE, generator=gen, device="cuda")) for _ in layers]
+    torch.cuda.synchronize()
+    st = MoeStack(be, layers, nws, rows, NE, E, k, NFF)
+    assert tuple(st.ids.shape) == (3, rows, k)
+    h = torch.randn(rows, NE, generator=gen, device="cuda")
+    st.hidden.copy_(h)
+    torch.cuda.synchronize()
+    st.step()
+    be.sync()
+    h = h.cpu().numpy()
+    for li, L in enumerate(layers):
+        H = L.host()
+        res = orc.moe_ffn(orc.rmsnorm(h, nws[li].cpu().numpy(), 1e-6), H.router, H.gate, H.up, H.down, n_expert=E, n_used=k, n_ff_exp=NFF)
+        keep = np.setdiff1d(np.arange(rows), near_tie_rows(res, k, ulps=4096))  # the stream itself is the GPU's in the layers behind
+        assert len(keep) >= rows - 2
+        assert np.array_equal(st.ids[li].cpu().numpy()[keep], res.ids[keep])
+        h = orc.add(h, res.dst)
+
+
 @pytest.mark.parametrize("rows,path", [(2, 1), (40, 2)])
 def test_fused_norm_and_residual_one_op(backend, rows, path):
     # RmsNorm -> MoeFfn -> Add folded into one call, in place on the hidden state, both paths
