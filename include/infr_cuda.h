@@ -434,7 +434,7 @@ int32_t infr_cuda_gguf_upload(infr_cuda_ctx* ctx, const infr_cuda_gguf* g, const
  * on the context's stream.  Buffers named by the recorded calls must stay alive and keep their
  * addresses; new inputs are written into the same buffers before each replay.  Calls that need
  * to grow the context's scratch memory fail with INVALID_ARG while recording: run the same calls
- * once un-recorded first. */
+ * once un-recorded first.  Buffers and plans freed while recording go when the recording ends. */
 typedef struct infr_cuda_graph infr_cuda_graph;
 int32_t infr_cuda_graph_begin(infr_cuda_ctx* ctx);
 int32_t infr_cuda_graph_end(infr_cuda_ctx* ctx, infr_cuda_graph** out);

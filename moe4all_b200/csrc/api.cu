@@ -96,6 +96,40 @@ struct DeviceGuard {
   }
 };
 
+// Frees of one context must not end another one's recording on the same thread.
+struct CaptureRelaxed {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+void destroy_graph(infr_cuda_graph* gr) {
+  if (gr->exec) cudaGraphExecDestroy(gr->exec);
+  if (gr->graph) cudaGraphDestroy(gr->graph);
+  delete gr;
+}
+
+// Whether the release is put off to the recording's end.  (Without memory for the note it is never freed: the recording matters more.)
+template <class T>
+bool put_off(infr_cuda_ctx* ctx, std::vector<T>& late, T what) {
+  if (!ctx->capturing) return false;
+  try {
+    late.push_back(what);
+  } catch (const std::bad_alloc&) {
+  }
+  return true;
+}
+
+void free_late(infr_cuda_ctx* ctx, cudaStream_t after) {
+  if (ctx->late_bufs.empty() && ctx->late_graphs.empty()) return;
+  CaptureRelaxed relaxed;
+  cudaStreamSynchronize(after);
+  for (infr_cuda_graph* gr : ctx->late_graphs) destroy_graph(gr);
+  for (void* p : ctx->late_bufs) cudaFree(p);
+  ctx->late_graphs.clear();
+  ctx->late_bufs.clear();
+}
+
 bool fits(const infr_cuda_buf* b, size_t need) { return b && b->ptr && b->bytes >= need; }
 
 // Device copies of the grid tables, per device (see infr_cuda_set_codebook).
@@ -197,8 +231,10 @@ int32_t infr_cuda_create(int32_t device, infr_cuda_ctx** out) {
 void infr_cuda_destroy(infr_cuda_ctx* ctx) {
   if (!ctx) return;
   DeviceGuard g(ctx->device);
+  CaptureRelaxed relaxed;
   if (ctx->ep) ep_release(ctx, false);
   if (ctx->own_stream) cudaStreamSynchronize(ctx->own_stream);
+  free_late(ctx, ctx->own_stream);  // (a stream of the caller's may be gone)
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->status_host) cudaFreeHost(ctx->status_host);
   if (ctx->route_logits) cudaFree(ctx->route_logits);
@@ -276,8 +312,12 @@ void infr_cuda_free(infr_cuda_ctx* ctx, infr_cuda_buf* buf) {
   if (buf->owned && buf->ptr) {
     if (ctx) {
       DeviceGuard g(ctx->device);
-      cudaStreamSynchronize(ctx->stream);
-      cudaFree(buf->ptr);
+      std::lock_guard<std::mutex> lock(ctx->free_mu);
+      if (!put_off(ctx, ctx->late_bufs, buf->ptr)) {
+        CaptureRelaxed relaxed;
+        cudaStreamSynchronize(ctx->stream);
+        cudaFree(buf->ptr);
+      }
     } else {
       cudaFree(buf->ptr);
     }
@@ -476,6 +516,7 @@ int32_t infr_cuda_graph_begin(infr_cuda_ctx* ctx) {
   if (!ctx) return INFR_CUDA_ERR_INVALID_ARG;
   if (ctx->capturing) return fail(ctx, INFR_CUDA_ERR_INVALID_ARG, "graph_begin: already recording");
   DeviceGuard g(ctx->device);
+  std::lock_guard<std::mutex> lock(ctx->free_mu);
   cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return check_cuda(ctx, e, "graph_begin");
   ctx->capturing = true;
@@ -488,9 +529,14 @@ int32_t infr_cuda_graph_end(infr_cuda_ctx* ctx, infr_cuda_graph** out) {
   *out = nullptr;
   if (!ctx->capturing) return fail(ctx, INFR_CUDA_ERR_INVALID_ARG, "graph_end: not recording");
   DeviceGuard g(ctx->device);
-  ctx->capturing = false;
   cudaGraph_t graph = nullptr;
-  cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
+  cudaError_t e;
+  {
+    std::lock_guard<std::mutex> lock(ctx->free_mu);
+    e = cudaStreamEndCapture(ctx->stream, &graph);
+    ctx->capturing = false;
+    free_late(ctx, ctx->stream);
+  }
   if (e != cudaSuccess || !graph) return check_cuda(ctx, e == cudaSuccess ? cudaErrorUnknown : e, "graph_end");
   cudaGraphExec_t exec = nullptr;
   e = cudaGraphInstantiate(&exec, graph, 0);
@@ -522,13 +568,13 @@ int32_t infr_cuda_graph_launch(infr_cuda_ctx* ctx, infr_cuda_graph* graph) {
 
 void infr_cuda_graph_free(infr_cuda_ctx* ctx, infr_cuda_graph* graph) {
   if (!graph) return;
-  if (ctx) {
-    DeviceGuard g(ctx->device);
-    cudaStreamSynchronize(ctx->stream);
-  }
-  if (graph->exec) cudaGraphExecDestroy(graph->exec);
-  if (graph->graph) cudaGraphDestroy(graph->graph);
-  delete graph;
+  if (!ctx) return destroy_graph(graph);
+  DeviceGuard g(ctx->device);
+  std::lock_guard<std::mutex> lock(ctx->free_mu);
+  if (put_off(ctx, ctx->late_graphs, graph)) return;
+  CaptureRelaxed relaxed;
+  cudaStreamSynchronize(ctx->stream);
+  destroy_graph(graph);
 }
 
 // ---- Op::MoeFfn ---------------------------------------------------------------------------------

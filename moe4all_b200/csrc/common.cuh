@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -55,6 +56,11 @@ struct infr_cuda_ctx {
   uint64_t launches = 0;
   bool capturing = false;
   uint64_t capture_launches = 0;  // launches recorded since graph_begin
+  // Buffers and plans freed while recording (by a collector, on any thread): the wait and the free would end the recording, so they
+  // are kept until graph_end.  The mutex orders frees with the two ends of a recording.
+  std::mutex free_mu;
+  std::vector<void*> late_bufs;
+  std::vector<infr_cuda_graph*> late_graphs;
   // scratch grown on demand (never inside a launch sequence that could be captured)
   void* scratch = nullptr;
   size_t scratch_bytes = 0;

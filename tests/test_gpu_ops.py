@@ -151,3 +151,39 @@ def test_record_replay_matches_eager(backend):
     be.sync()
     assert_close(be.download(dst).reshape(2, 512), oracle_layer(L, x2, 4).dst)
     plan.free()
+
+
+def test_buffers_plans_and_contexts_may_go_while_recording(backend):
+    # as a collector frees them: nothing of it may end the recording, and the memory is back when the recording ends
+    import torch
+    from moe4all_b200 import CudaBackend
+    be = backend
+    L = synth.make_layer(31, 512, 16, 256, sh_ff=256)
+    g = GpuLayer(be, L)
+    x = synth.activations(8, 2, 512)
+    eager, _, _ = g.run(x, 4)
+    xb, dst = be.from_host(x), be.alloc(2 * 512 * 4)
+    op = MoeFfn(x=xb, router=g.router, gate_exps=g.gate, up_exps=g.up, down_exps=g.down, dst=dst, rows=2, ne=512,
+                n_expert=16, n_used=4, n_ff_exp=256, sh_gate=g.sh_gate, sh_up=g.sh_up, sh_down=g.sh_down,
+                sh_gate_inp=g.sh_gate_inp, sh_ff=256)
+    be.graph_begin()
+    be.moe_ffn(op)
+    old = be.graph_end()
+    other = CudaBackend(0)
+    foreign = other.alloc(1 << 20)
+    before = torch.cuda.mem_get_info()[0]
+    spare = be.alloc(256 << 20)
+    be.sync()
+    be.graph_begin()
+    be.moe_ffn(op)
+    spare.free()
+    old.free()
+    foreign.free()
+    other.close()
+    be.moe_ffn(op)
+    plan = be.graph_end()
+    assert torch.cuda.mem_get_info()[0] >= before - (64 << 20)
+    be.execute(plan)
+    be.sync()
+    assert np.array_equal(be.download(dst).reshape(2, 512), eager)
+    plan.free()
