@@ -712,7 +712,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 && !Q4 ? 2 : 0) k_em_do
       // fixed point: X = round(a * 32639 / max|a|) per row, limbs X = 256 hi + lo, sums per 16 elements.  A warp takes whole rows: no
       // barrier between a row's maximum and its rounding.  One unit per 128 elements, as in the per-pair kernels, has a little less
       // error (Q6_K, 13 rows of 512: 7.1e-5 of the result against 8.1e-5; Q4_K level) but costs two multiplications and a conversion
-      // more for each of its results (Q4_K, 427 rows of 2560 over 512-wide experts: the kernel 76 us, 71 with one per row).
+      // more for each of its results (Q4_K, 427 rows of 2560 over 512-wide experts: the kernel 76 us, 71 with one per row).  Another
+      // unit also moves a layer's result by 6e-5, after which rows of a chain of layers now and then take another expert.
       const int n4 = nff_e / 4;
       for (int tk = warp; tk < cnt; tk += WARPS) {
         const float4* arow = reinterpret_cast<const float4*>(p.act + (size_t)s_pair[tk] * p.nffmax);
