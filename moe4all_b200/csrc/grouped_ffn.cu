@@ -706,13 +706,14 @@ __global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __re
                                                                const int* __restrict__ seg_off, int n_seg_routed, int has_shared,
                                                                int rows, int n_used, int ne, const float* residual,
                                                                const int32_t* __restrict__ ids, const float* __restrict__ down_scale,
-                                                               int weight_before, float* dst) {
+                                                               int weight_before, int y_shift, float* dst) {
   const int q = blockIdx.x * 256 + threadIdx.x;
   if (q * 8 >= ne) return;
-  const int c = PACKED ? (q >> 2) * 32 + 2 * (q & 3) : q * 8;
+  // packed: items 2 q and 2 q + 1, whose first outputs are 2^y_shift features apart
+  const int c = PACKED ? ((((q >> 2) >> y_shift) * 32 + 2 * (q & 3)) << y_shift) + ((q >> 2) & ((1 << y_shift) - 1)) : q * 8;
   const int n_sorted = has_shared ? seg_off[n_seg_routed] : 0;
   for (int t = blockIdx.y; t < rows; t += gridDim.y) {  // the grid's y extent stops at 65535
-    // o[i], o[i + 4]: outputs c + i, c + i + 4; packed: c + 8 i, c + 8 i + 1
+    // o[i], o[i + 4]: outputs c + i, c + i + 4; packed: c + 8 i, c + 8 i + 1 (times 2^y_shift)
     float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     auto take = [&](int pos, float w) {
       float4 a, b;
@@ -747,7 +748,13 @@ __global__ void __launch_bounds__(256) k_unpermute_combine_seg(const float* __re
     // MoeFfn -> Add; may alias dst: each element is read, then written, by this thread
     float* d = dst + (size_t)t * ne + c;
     const float* h = residual != nullptr ? residual + (size_t)t * ne + c : nullptr;
-    if (PACKED) {
+    if (PACKED && y_shift) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int at = (8 * (i & 3) + (i >> 2)) << y_shift;
+        d[at] = h != nullptr ? o[i] + h[at] : o[i];
+      }
+    } else if (PACKED) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float2 v = make_float2(o[i], o[i + 4]);
@@ -907,6 +914,7 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
   // tcgen05 tiles with the combine behind them: the raw rows cross memory packed (three quarters of the bytes out of the
   // down kernel and into the combine) for the Q4_K / Q6_K banks; rows handed to the caller stay f32
   p.y_packed = (use_wt && tuned && c.dst != nullptr && c.y_out == nullptr && !ctx->cfg.raw_rows_f32) ? 1 : 0;
+  p.y_shift = use_wt ? wt_y_shift(c.down_dt, c.nff) : 0;
   p.gate_dt = c.gate_dt;
   p.up_dt = c.up_dt;
   p.down_dt = c.down_dt;
@@ -940,7 +948,7 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
     // an ordinary launch: this kernel reads through L1, which a kernel boundary empties
     const cudaError_t e = launch_ex(comb, dim3((c.ne / 8 + 255) / 256, std::min(c.rows, 65535)), dim3(256), 0, st, false, y, pos_of_pair, c.wts,
                                     c.sh_logit, seg_off, n_seg_routed, c.shared_rows > 0 ? 1 : 0, c.rows, c.n_used, c.ne, c.residual, c.ids,
-                                    c.down_scale, c.weight_before, c.dst);
+                                    c.down_scale, c.weight_before, p.y_shift, c.dst);
     if (e != cudaSuccess) return check_cuda(ctx, e, "combine launch");
     ctx->launches += 1;
   }

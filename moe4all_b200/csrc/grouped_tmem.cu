@@ -19,15 +19,17 @@
 //   16     issues the MMAs (one elected lane)
 //   then   token loaders: gate/up - four warps bring rows of the f16 token matrix straight from where the tokens are
 //          (cp.async), two of them per K step; down - one warp, one bulk copy per K step of the tile's activations
-//   last   raw-block loaders: 256 weights of 256 rows at a time, into a ring: Q4_K, Q5_K and Q8_0 by tiled copies, formats
-//          whose rows of 256 weights are not whole 16-byte pieces word by word with cp.async (rows on an odd word pitch,
-//          free of bank conflicts)
+//   last   raw-block loaders: 256 weights of 256 rows at a time, into a ring: Q4_K, Q5_K, Q8_0 and the down banks' Q6_K by
+//          tiled copies, other formats word by word with cp.async (rows on an odd word pitch, free of bank conflicts)
 // All rings run on across jobs; every wait is bounded.
 //
 // Measured (phase stamps, SM cycles per step of 64 K elements): gate/up of full tiles 970, of which the eight MMAs are 640 and
 // the rest their hand-over - the producers wait for a free A stage more than half of their time; of light tiles 820, the
-// unpack.  Down with Q6_K 1130 - 1300, the unpack (1200 - 1800 per own step of a warp); reading out a full tile takes 7000
-// beside the 11000 of its K loop at 512 inputs, with the tensor core idle: there is one set of accumulators.
+// unpack.  Reading out a full tile of the down kernel takes 7000 beside the 11000 of its K loop at 512 inputs, with the tensor core
+// idle: there is one set of accumulators.
+// Down with Q6_K, whose blocks are 210 bytes: as words by cp.async the copies were what everything waited for (without them 3704 ->
+// 2104 us, 8192 tokens of 28 MB experts).  Now a tiled copy brings the 240 bytes around a block, of one row in every 1, 2, 4 or 8
+// (row_shift), so that a warp's rows have one offset inside them: 3704 -> 2526 us, 4096 tokens of 2 MB experts 177 -> 142.
 #include <cuda.h>
 
 #include <algorithm>
@@ -221,6 +223,62 @@ __device__ __forceinline__ void unpack_q6k(const uint32_t* row, int mis, int h, 
   }
 }
 
+// Half h (128 weights, two steps) of a Q6_K block in 16-byte pieces, words realigned: the block starts WO words and `mis` (0 or 16)
+// bits into the 16-byte boundary `row`.
+struct Q6kHalf {
+  uint32_t ql[16], qh[8], sc[2], d;
+};
+template <int WO>
+__device__ __forceinline__ void fetch_q6k_half(const unsigned char* row, int h, int mis, Q6kHalf& r) {
+  {
+    uint32_t v[20];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const uint4 x = *reinterpret_cast<const uint4*>(row + 64 * h + 16 * i);
+      v[4 * i] = x.x, v[4 * i + 1] = x.y, v[4 * i + 2] = x.z, v[4 * i + 3] = x.w;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) r.ql[i] = __funnelshift_r(v[WO + i], v[WO + i + 1], mis);
+  }
+  {
+    uint32_t v[12];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const uint4 x = *reinterpret_cast<const uint4*>(row + 128 + 32 * h + 16 * i);
+      v[4 * i] = x.x, v[4 * i + 1] = x.y, v[4 * i + 2] = x.z, v[4 * i + 3] = x.w;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) r.qh[i] = __funnelshift_r(v[WO + i], v[WO + i + 1], mis);
+  }
+  const uint4 a = *reinterpret_cast<const uint4*>(row + 192), b = *reinterpret_cast<const uint4*>(row + 208);
+  const uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  const uint32_t s0 = h ? v[WO + 2] : v[WO], s1 = h ? v[WO + 3] : v[WO + 1], s2 = h ? v[WO + 4] : v[WO + 2];
+  r.sc[0] = __funnelshift_r(s0, s1, mis);
+  r.sc[1] = __funnelshift_r(s1, s2, mis);
+  r.d = v[WO + 4] >> mis;
+}
+
+// Step 2 h + G from the half.
+template <int G>
+__device__ __forceinline__ void unpack_q6k_half(const Q6kHalf& r, uint32_t (&o)[32]) {
+  const __half2 d = __hmul2(u32_as_h2(__byte_perm(r.d, 0u, 0x1010)), h2_const(0x5C00u));
+  const __half2 s01 = i8_scale_pair(r.sc[G], 0x4140, d), s23 = i8_scale_pair(r.sc[G], 0x4342, d);
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    const __half2 s_a = __low2half2(part ? s23 : s01), s_b = __high2half2(part ? s23 : s01);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t L = G ? r.ql[8 * part + i] >> 4 : r.ql[8 * part + i];
+      const uint32_t H = G ? (part ? r.qh[i] >> 2 : r.qh[i]) : (part ? r.qh[i] << 2 : r.qh[i] << 4);  // the code's bits 4, 5 in place
+      const uint32_t c = (H & 0x30303030u) | (L & 0x0F0F0F0Fu);
+      const uint32_t c02 = __byte_perm(c, 0x64u, 0x4240), c13 = __byte_perm(c, 0x64u, 0x4341);
+      const __half2 s = i < 4 ? s_a : s_b;
+      o[16 * part + 2 * i] = h2_as_u32(__hmul2(__hsub2(u32_as_h2(c02), h2_const(0x6420u)), s));
+      o[16 * part + 2 * i + 1] = h2_as_u32(__hmul2(__hsub2(u32_as_h2(c13), h2_const(0x6420u)), s));
+    }
+  }
+}
+
 // A step of eight Q8_0 blocks: 68 bytes = two blocks, the first on a word boundary, the second two bytes past one.
 // w(i): word i of the step.
 template <typename Word>
@@ -334,9 +392,12 @@ __device__ __forceinline__ void pack_y4(float a, float b, float c, float d, uint
 
 // ---- the kernel ---------------------------------------------------------------------------------------
 
-// Q4_K, Q5_K, Q8_0 (both roles): tiled copies, rows of whole 16-byte pieces; Q6_K, any: words, on an odd word pitch.
+// Q4_K, Q5_K, Q8_0 (both roles): tiled copies, rows of whole 16-byte pieces.  Q6_K (down): tiled copies of the 240 bytes around a
+// block of 210, over 2^row_shift rows at a time, whose bytes are whole 16-byte pieces.  Any: words, on an odd word pitch.
 enum WtFormat { WT_Q4K, WT_Q5K, WT_Q80, WT_Q6K, WT_ANY };
-__host__ __device__ constexpr bool wt_tiled(int fmt) { return fmt <= WT_Q80; }
+__host__ __device__ constexpr bool wt_tiled(int fmt) { return fmt <= WT_Q6K; }
+constexpr uint32_t W_Q6K_BOX = 240;  // 15 pieces of 16 bytes: 14 bytes of offset and 210 of block, rounded up; odd, so that eight
+                                     // rows' pieces are in different banks
 
 struct WtBars {
   uint64_t full_a[W_A_STAGES], empty_a[W_A_STAGES];      // A stages in tensor memory
@@ -363,6 +424,7 @@ struct WtParams {
   int k_blocks;     // 256-element blocks along K
   int rb, sb;       // stages of the raw and the token ring
   uint32_t raw_pitch, raw_stage;  // bytes per row and per stage
+  int row_shift;            // down: producer warp w holds the rows (32 (w >> row_shift) + lane) 2^row_shift + w % 2^row_shift
   // gate/up tokens: row of the token matrix behind grouped row `pos`
   const int* pair_of_pos;   // null: the rows are grouped already
   const int* seg_off;       // [n_seg_routed] = grouped rows ahead of the shared expert's
@@ -435,7 +497,10 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
   if (warp < W_PRODUCERS / 32) {
     // ---- producers: unpack, then drain ----
     const int g = warp >> 3, role = (warp >> 2) & 1, q = warp & 3;
-    const int slot = role * 128 + wt_row_of_lane(MODE, q * 32 + lane);  // row of the raw stage
+    const int w8 = warp & 7, sub = w8 & ((1 << w.row_shift) - 1);
+    // row of the raw stage (down: the rows of a warp have one offset from the 16-byte boundary)
+    const int slot = MODE == 0 ? role * 128 + wt_row_of_lane(MODE, q * 32 + lane)
+                               : (sub << (8 - w.row_shift)) + (w8 >> w.row_shift) * 32 + lane;
     const int dt = MODE == 1 ? p.down_dt : (role ? p.up_dt : p.gate_dt);
     const int half_word = (int)(row_bytes(dt, 256) & 2);  // blocks of an odd number of half-words: every other one is off a word boundary
     const uint32_t a_addr = tmem + ((uint32_t)(q * 32) << 16) + W_A_COL + 32u * role;
@@ -443,6 +508,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     const uint32_t patch_u = smem_u32(patch);
     RingPos rp, ap;  // raw blocks; A stages
     if (g) ap.next(W_A_STAGES);
+    if (g && FMT == WT_Q6K) ap.next(W_A_STAGES);
     uint32_t d_phase = 0;
     for (int it = 0; ok; ++it) {
       const int job = wt_job(it);
@@ -459,6 +525,20 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
         if (TRACED && blk < 4) trace_stamp(tr, 65 + 64 * MODE + 8 * blk);
         const unsigned char* row = raw_ring + (size_t)rp.s * w.raw_stage + (size_t)slot * w.raw_pitch;
         const int mis = ((wrow * kb + blk) & 1) * half_word;  // bytes of the stage's first word ahead of the block
+        Q6kHalf half;
+        if (FMT == WT_Q6K) {
+          // The group's two steps are one half of the block (the low and the high bits of the same code bytes), so its words are read
+          // and realigned once for both, and the stage is free as soon as they are in registers.
+          const int off = ((int)Q6K_BLOCK_BYTES * (sub * kb + blk)) & 15, bits = (off & 2) * 8;
+          switch (off >> 2) {
+            case 0: fetch_q6k_half<0>(row, g, bits, half); break;
+            case 1: fetch_q6k_half<1>(row, g, bits, half); break;
+            case 2: fetch_q6k_half<2>(row, g, bits, half); break;
+            default: fetch_q6k_half<3>(row, g, bits, half); break;
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars.empty_raw[rp.s]);
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint32_t o[32];
@@ -471,7 +551,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           } else if (FMT == WT_Q80) {
             if (g) h ? unpack_q80_row<3>(row, o) : unpack_q80_row<1>(row, o);
             else h ? unpack_q80_row<2>(row, o) : unpack_q80_row<0>(row, o);
-          } else if (FMT == WT_Q6K || dt == INFR_CUDA_DT_Q6K) {
+          } else if (FMT == WT_Q6K) {
+            h ? unpack_q6k_half<1>(half, o) : unpack_q6k_half<0>(half, o);
+          } else if (dt == INFR_CUDA_DT_Q6K) {
             unpack_q6k(row32, mis * 8, h, g, o);
           } else if (dt == INFR_CUDA_DT_Q8_0) {
             unpack_q80([&](int i) { return row32[17 * j + i]; }, o);
@@ -482,7 +564,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           } else {
             unpack_codes(dt, row + mis, j, o);
           }
-          if (h == 1) {
+          if (h == 1 && FMT != WT_Q6K) {
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars.empty_raw[rp.s]);
           }
@@ -499,7 +581,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
             trace_stamp(tr, 69 + 64 * MODE + 8 * blk);
           }
           ap.next(W_A_STAGES);
-          ap.next(W_A_STAGES);
+          if (FMT != WT_Q6K || h == 1) ap.next(W_A_STAGES);
+          if (FMT == WT_Q6K && h == 1) ap.next(W_A_STAGES);
         }
         if (!ok) break;
         rp.next(w.rb);
@@ -547,9 +630,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
         } else {
 #pragma unroll
           for (int m = 0; m < 2; ++m) {
-            const int f0 = blk0 * WR + m * 128 + q * 32;  // first of the 32 output features of this lane quarter
+            const int wq = m * 4 + q, f0 = blk0 * WR + wq * 32;  // first of the lane quarter's 32 places among the output features
             if (p.y_packed) {
-              // the combine kernel is the only reader: this thread's four outputs of a token (8 features apart) as one item
+              // the combine kernel is the only reader: this thread's four outputs of a token (8 places apart) as one item
 #pragma unroll
               for (int k = 0; k < 4; ++k) {  // tokens 8 (k >> 1) + 2 (lane % 4) + (k & 1)
                 const int i0 = 4 * (k >> 1) + (k & 1), t = t0 + 8 * (k >> 1) + 2 * (lane & 3) + (k & 1);
@@ -576,8 +659,16 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
                 for (int i = 0; i < 2; ++i) {
                   const int t = (lane >> 3) + 4 * i, c = lane & 7;
                   const float4 x = *reinterpret_cast<const float4*>(pf + t * 36 + c * 4);
-                  if (t0 + 8 * cg + t < rows_valid)
-                    *reinterpret_cast<float4*>(p.y + (size_t)(row0 + t0 + 8 * cg + t) * p.ne + f0 + c * 4) = x;
+                  float* y = p.y + (size_t)(row0 + t0 + 8 * cg + t) * p.ne;
+                  if (t0 + 8 * cg + t < rows_valid) {
+                    if (w.row_shift == 0) {
+                      *reinterpret_cast<float4*>(y + f0 + c * 4) = x;
+                    } else {
+                      const int sh = w.row_shift;
+                      y += blk0 * WR + (((wq >> sh) * 32 + c * 4) << sh) + (wq & ((1 << sh) - 1));
+                      y[0] = x.x; y[1 << sh] = x.y; y[2 << sh] = x.z; y[3 << sh] = x.w;
+                    }
+                  }
                 }
                 __syncwarp();
               }
@@ -705,6 +796,16 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
         for (int blk = 0; blk < kb; ++blk) {
           if (!wt_wait(&bars.empty_raw[rp.s], rp.phase ^ 1)) { ok = false; break; }
           unsigned char* dst = raw_ring + (size_t)rp.s * w.raw_stage;
+          if (FMT == WT_Q6K) {
+            // the rows of one place among 2^row_shift rows per copy, from the 16-byte boundary at or ahead of the block (a box that
+            // runs on past the last block's row is filled up with zeros)
+            mbar_arrive_expect_tx(&bars.full_raw[rp.s], w.raw_stage);
+            for (int i = 0; i < 1 << w.row_shift; ++i)
+              tma_load_2d(dst + i * (w.raw_stage >> w.row_shift), shared_seg ? &tm_s0 : &tm_w0, (((int)Q6K_BLOCK_BYTES * (i * kb + blk)) & ~15) >> 1,
+                          r0 >> w.row_shift, &bars.full_raw[rp.s]);
+            rp.next(w.rb);
+            continue;
+          }
           const int x = blk * (int)(w.raw_pitch >> 1);  // in half-words
           mbar_arrive_expect_tx(&bars.full_raw[rp.s], w.raw_stage);
           tma_load_2d(dst, shared_seg ? &tm_s0 : &tm_w0, x, r0, &bars.full_raw[rp.s]);
@@ -724,7 +825,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
             const uint8_t* bank = MODE == 1 ? (shared_seg ? p.sh_down : p.down + (size_t)e * p.down_stride)
                                             : half ? (shared_seg ? p.sh_up : p.up + (size_t)e * p.up_stride)
                                                    : (shared_seg ? p.sh_gate : p.gate + (size_t)e * p.gate_stride);
-            const uint32_t chunk = FMT == WT_Q6K ? Q6K_BLOCK_BYTES : (uint32_t)row_bytes(dt, 256);
+            const uint32_t chunk = (uint32_t)row_bytes(dt, 256);
             const uint32_t words = (chunk + 2) >> 2, full = words >> 5, tail = words & 31u, tail_rows = tail ? 32u / tail : 1u;
             const size_t pitch = (size_t)chunk * kb;
             const uint32_t dst0 = smem_u32(raw_ring) + rp.s * w.raw_stage + (uint32_t)half * 128u * w.raw_pitch;
@@ -761,13 +862,13 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
   if (warp == W_MMA_WARP) umma::tmem_dealloc(s_tmem, 512);
 }
 
-// A bank as a 2-D tensor of half-words [rows][row bytes / 2]; box: 256 weights (`chunk` bytes) of 128 rows.
-bool raw_rows_map(CUtensorMap* tm, const uint8_t* base, size_t rows, size_t row_bytes, uint32_t chunk) {
+// A bank as a 2-D tensor of half-words [rows][row bytes / 2]; box: 256 weights (`chunk` bytes) of `box_rows` rows.
+bool raw_rows_map(CUtensorMap* tm, const uint8_t* base, size_t rows, size_t row_bytes, uint32_t chunk, uint32_t box_rows = 128) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)row_bytes / 2, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
-  const cuuint32_t box[2] = {chunk / 2, 128};
+  const cuuint32_t box[2] = {chunk / 2, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<uint8_t*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -785,6 +886,7 @@ int wt_format(int dt0, int dt1, bool down) {
 
 // Bytes of 256 weights of a row in the raw stage.
 uint32_t raw_pitch_of(int fmt, int dt) {
+  if (fmt == WT_Q6K) return W_Q6K_BOX;
   if (wt_tiled(fmt)) return (uint32_t)row_bytes(dt, 256);  // 36, 44 or 68 words: 16-byte pieces of eight rows in different banks
   const uint32_t words = ((uint32_t)row_bytes(dt, 256) + 2 + 3) / 4;  // room for the half-word ahead
   return (words | 1) * 4;
@@ -816,6 +918,14 @@ int32_t launch_wt(infr_cuda_ctx* ctx, WtParams w, const CUtensorMap (&tm)[4], in
 }  // namespace
 
 int wt_tile_rows() { return WN; }
+
+// A Q6_K row of 256 k weights is 210 k bytes: 1, 2, 4 or 8 rows are whole 16-byte pieces.
+int wt_y_shift(int down_dt, int nff) {
+  if (wt_format(down_dt, down_dt, true) != WT_Q6K) return 0;
+  int sh = 0;
+  while ((row_bytes(down_dt, nff) << sh) % 16) ++sh;
+  return sh;
+}
 
 int32_t launch_wt_grouped(infr_cuda_ctx* ctx, const GroupedParams& p, const WtTokens& t, int max_tiles) {
   WtParams w = {};
@@ -852,10 +962,12 @@ int32_t launch_wt_grouped(infr_cuda_ctx* ctx, const GroupedParams& p, const WtTo
   fmt = wt_format(p.down_dt, p.down_dt, true);
   w.raw_pitch = raw_pitch_of(fmt, p.down_dt);
   w.raw_stage = WR * w.raw_pitch;
+  w.row_shift = p.y_shift;
   if (wt_tiled(fmt)) {
-    const size_t rb = row_bytes(p.down_dt, p.nff);
-    ok = raw_rows_map(&tm[0], p.down, (size_t)p.n_expert * p.ne, rb, w.raw_pitch);
-    if (ok && p.sh_down) ok = raw_rows_map(&tm[2], p.sh_down, p.ne, rb, w.raw_pitch);
+    const size_t rb = row_bytes(p.down_dt, p.nff) << w.row_shift;
+    const uint32_t box_rows = fmt == WT_Q6K ? (uint32_t)WR >> w.row_shift : 128u;
+    ok = raw_rows_map(&tm[0], p.down, (size_t)p.n_expert * p.ne >> w.row_shift, rb, w.raw_pitch, box_rows);
+    if (ok && p.sh_down) ok = raw_rows_map(&tm[2], p.sh_down, (size_t)p.ne >> w.row_shift, rb, w.raw_pitch, box_rows);
     tm[1] = tm[0];
     tm[3] = tm[2];
     if (!ok) return fail(ctx, INFR_CUDA_ERR_CUDA, "grouped GEMM: the driver refused a tensor map for the down bank");

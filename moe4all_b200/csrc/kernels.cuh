@@ -104,7 +104,8 @@ struct GroupedParams {
   const __half* xg;
   __half* act;
   float* y;          // [rows, ne] raw down outputs: f32, or with y_packed (the combine kernel is the only reader) rows of
-  int y_packed;      // 3 ne bytes: item 8 g + j = features 32 g + j + 8 i, i = 0..3 (pack_y4), all items' hi, then their lo
+  int y_packed;      // 3 ne bytes: item 8 g + j = places 32 g + j + 8 i, i = 0..3 (pack_y4), all items' hi, then their lo
+  int y_shift;       // place 32 g + l of a packed row = feature (32 (g >> y_shift) + l) 2^y_shift + g % 2^y_shift (wt_y_shift)
   const uint8_t *gate, *up, *down;
   const uint8_t *sh_gate, *sh_up, *sh_down;  // segment index n_expert = the shared expert
   size_t gate_stride, up_stride, down_stride;
@@ -151,6 +152,7 @@ struct WtTokens {
   int n_seg_routed, n_used;
 };
 int wt_tile_rows();
+int wt_y_shift(int down_dt, int nff);
 int32_t launch_wt_grouped(infr_cuda_ctx* ctx, const GroupedParams& p, const WtTokens& t, int max_tiles);
 size_t grouped_scratch_bytes(int rows_total, int n_pairs, int n_seg, int ne, int nff);
 int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c);

@@ -51,7 +51,7 @@ class GpuLayer:
 
     def run(self, x, n_used, *, router_x=None, scale=1.0, gating=MoeGating.Softmax, norm_w=True,
             groups=0, groups_used=0, ep_band=None, shared=True, path=0, expert_ids=None, down_scale=None,
-            act=0, weight_before=False, swiglu_clamp=0.0, fused_gate_up=False):
+            act=0, weight_before=False, swiglu_clamp=0.0, fused_gate_up=False, residual=None):
         be, L = self.be, self.L
         x = np.ascontiguousarray(x, np.float32)
         rows = x.shape[0]
@@ -77,7 +77,7 @@ class GpuLayer:
                     sh_ff=L.sh_ff if use_sh else 0, path=path, down_dtype=DType(getattr(L, "down_dtype", 14)),
                     gate_dtype=DType(getattr(L, "gate_dtype", 12)), up_dtype=DType(getattr(L, "up_dtype", 12)),
                     expert_ids=given, down_scale=dsc, act=act, weight_before=weight_before, swiglu_clamp=swiglu_clamp,
-                    fused_gate_up=fused_gate_up)
+                    fused_gate_up=fused_gate_up, residual=residual)
         be.moe_ffn(op)
         be.sync()
         out = be.download(dst, np.float32).reshape(rows, L.ne)

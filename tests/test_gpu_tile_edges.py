@@ -28,6 +28,23 @@ def test_grouped_token_tiles(backend, mix, ne, nff):
     assert_close(out, oracle_layer(L, x, 1, expert_ids=ids).dst)
 
 
+@pytest.mark.parametrize("raw_f32", [0, 1])
+@pytest.mark.parametrize("ne,nff", [(256, 256), (768, 512), (256, 1024), (512, 1536), (256, 2048)])
+def test_q6k_down_rows_by_offset(backend, ne, nff, raw_f32):
+    # Q6_K down rows of 210 nff / 256 bytes go to the operand's lanes 8, 4, 2, 4 and 1 apart; the outputs come back in order, packed
+    # or in f32, with the residual
+    counts = [1, 16, 17, 0, 160, 161, 33]
+    L = synth.make_layer(58, ne, len(counts), nff, sh_ff=nff, router_std=0.05)
+    ids = ids_of(counts, 5)
+    x, r = synth.activations(86, len(ids), ne), synth.activations(87, len(ids), ne)
+    backend.set_config(raw_rows_f32=raw_f32)
+    try:
+        out, _, _ = GpuLayer(backend, L).run(x, 1, path=2, expert_ids=ids, residual=backend.from_host(r))
+    finally:
+        backend.set_config(raw_rows_f32=0)
+    assert_close(out - r, oracle_layer(L, x, 1, expert_ids=ids).dst)
+
+
 @pytest.mark.parametrize("rows", [8191, 8192, 8193, 16400])
 def test_bucket_slices(backend, rows):
     # pairs are counted in slices over the CTAs of a cluster: just below, at and past 65536 and 131072 of them
