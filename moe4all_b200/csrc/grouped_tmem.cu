@@ -13,19 +13,23 @@
 // tensor-core time of a tile is proportional to its tokens.  Tensor memory: two accumulators of 160 columns (gate and
 // up rows, or the two halves of 256 output features) and three A stages of 64 columns (64 K elements of 256 rows).
 //
-// One persistent CTA per SM walks the jobs (tile, 256 weight rows), tiles listed heaviest first and dealt out in a
-// snake.  Warp roles (24 warps):
+// One persistent pair of CTAs per two SMs walks the jobs (tile, 2 x 256 weight rows, 256 of them in each CTA), tiles listed
+// heaviest first and dealt out in a snake.  The MMAs are the pair's (cta_group::2, M 256): each CTA unpacks its own rows into its
+// own tensor memory and brings half of the tile's tokens, and the tensor cores read both halves.  What it gives (us, gate/up /
+// down, one CTA by itself -> pairs): 777 tokens 58 / 56 -> 54 / 52, 4096 177 / 141 -> 150 / 133, 1024 of Q8_0 82 / 76 -> 74 / 69,
+// 8192 of 28 MB experts 4150 / 2470 -> 3610 / 2320.  Two things were in the way: the 16-byte asynchronous copies of the gathered
+// tokens (all their writes, not their latency: 20 KB a step, one copy instead of twenty a lane 177 -> 151; in a pair it is 10),
+// and the MMAs, which take 640 cycles of eight at 160 tokens in pairs and 740 - 790 in one CTA with a wait for a stage between them.
+// Warp roles (24 warps of each CTA):
 //   0-15   producers, two groups of eight on alternate K steps; afterwards they drain the accumulators
-//   16     issues the MMAs (one elected lane)
+//   16     first CTA: issues the MMAs (one elected lane); second: passes on that its tokens are there
 //   then   token loaders: gate/up - four warps bring rows of the f16 token matrix straight from where the tokens are
 //          (cp.async), two of them per K step; down - one warp, one bulk copy per K step of the tile's activations
 //   last   raw-block loaders: 256 weights of 256 rows at a time, into a ring: Q4_K, Q5_K, Q8_0 and the down banks' Q6_K by
 //          tiled copies, other formats word by word with cp.async (rows on an odd word pitch, free of bank conflicts)
 // All rings run on across jobs; every wait is bounded.
 //
-// Measured (phase stamps, SM cycles per step of 64 K elements): gate/up of full tiles 970, of which the eight MMAs are 640 and
-// the rest their hand-over - the producers wait for a free A stage more than half of their time; of light tiles 820, the
-// unpack.  Reading out a full tile of the down kernel takes 7000 beside the 11000 of its K loop at 512 inputs, with the tensor core
+// Reading out a full tile of the down kernel takes 7000 beside the 11000 of its K loop at 512 inputs, with the tensor core
 // idle: there is one set of accumulators.
 // Down with Q6_K, whose blocks are 210 bytes: as words by cp.async the copies were what everything waited for (without them 3704 ->
 // 2104 us, 8192 tokens of 28 MB experts).  Now a tiled copy brings the 240 bytes around a block, of one row in every 1, 2, 4 or 8
@@ -50,9 +54,10 @@ constexpr int W_MMA_WARP = 16, W_TOK_WARP = 17;
 __host__ __device__ constexpr int wt_tok_warps(int mode) { return mode == 0 ? 4 : 1; }
 __host__ __device__ constexpr int wt_raw_warp(int mode) { return W_TOK_WARP + wt_tok_warps(mode); }
 __host__ __device__ constexpr int wt_raw_warps(int mode) { return mode == 0 ? 3 : 4; }
-constexpr uint32_t W_B_STAGE = WN * 128;       // 64 K elements of the tile's tokens
+constexpr uint32_t W_B_STAGE = WN / 2 * 128;   // 64 K elements of half of the tile's tokens
 constexpr uint32_t W_PATCH = 1280;             // per warp: 16 rows x 80 B (f16) or 8 rows x 144 B (f32)
-constexpr int W_MAX_RING = 4;
+constexpr int W_B_STAGES = 6;                  // (four: the down kernel 2 - 3 % slower)
+constexpr int W_MAX_RAW = 4;
 constexpr int W_A_STAGES = 3;
 constexpr uint32_t W_A_COL = 2 * WN;           // first A column of tensor memory
 constexpr float W_PRESCALE = 256.0f;           // keeps block scales out of the f16 subnormals
@@ -94,14 +99,35 @@ __device__ __forceinline__ void tmem_ld_16x16_quad(uint32_t ta, uint32_t tb, uin
       : "memory");
 }
 
-// D[tmem] (+)= A[tmem] * B[smem]^T for one K = 16 slice; A: lane = row, a 32-bit column = two K elements.
+// D[tmem] (+)= A[tmem] * B[smem]^T for one K = 16 slice; A: lane = row, a 32-bit column = two K elements.  A and D: 128 rows in
+// each CTA of the pair, at the same columns; B: half of the rows (tokens) in each, at the same place of shared memory.
 __device__ __forceinline__ void mma_f16_ta(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(acc)
       : "memory");
+}
+// All MMAs issued so far by this thread arrive on `bar` of both CTAs when they have completed.
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+
+__device__ __forceinline__ uint32_t pair_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// One arrival on `bar` of the pair's first CTA.  What it tells of is in tensor memory, complete, or fenced for the tensor cores, so it
+// orders no other memory of the pair (released and acquired at cluster scope the gate/up kernel of 4096 tokens takes 243 us, not 150).
+__device__ __forceinline__ void arrive_first(uint64_t* bar) {
+  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\tmbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}"
+               ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void pair_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 // One lane of a converged warp.  Branching on this (and not on a lane number), in a branch the compiler knows to be
@@ -390,6 +416,15 @@ __device__ __forceinline__ void pack_y4(float a, float b, float c, float d, uint
   lo = __byte_perm(__byte_perm(q[0], q[1], 0x0051), __byte_perm(q[2], q[3], 0x0051), 0x5410);
 }
 
+// All 512 columns of both CTAs' tensor memory; one warp of each takes part.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(slot)) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(taddr) : "memory");
+}
+
 // ---- the kernel ---------------------------------------------------------------------------------------
 
 // Q4_K, Q5_K, Q8_0 (both roles): tiled copies, rows of whole 16-byte pieces.  Q6_K (down): tiled copies of the 240 bytes around a
@@ -401,8 +436,8 @@ constexpr uint32_t W_Q6K_BOX = 240;  // 15 pieces of 16 bytes: 14 bytes of offse
 
 struct WtBars {
   uint64_t full_a[W_A_STAGES], empty_a[W_A_STAGES];      // A stages in tensor memory
-  uint64_t full_b[W_MAX_RING], empty_b[W_MAX_RING];      // token stages
-  uint64_t full_raw[W_MAX_RING], empty_raw[W_MAX_RING];  // raw-block stages
+  uint64_t full_b[W_B_STAGES], empty_b[W_B_STAGES];      // token stages
+  uint64_t full_raw[W_MAX_RAW], empty_raw[W_MAX_RAW];    // raw-block stages
   uint64_t done, drained;                                // accumulators complete / read
 };
 
@@ -420,9 +455,9 @@ struct RingPos {
 
 struct WtParams {
   GroupedParams g;
-  int n_blk;        // jobs per tile
+  int n_blk, n_pair;  // blocks of 256 weight rows per tile; pairs of them
   int k_blocks;     // 256-element blocks along K
-  int rb, sb;       // stages of the raw and the token ring
+  int rb;           // stages of the raw ring
   uint32_t raw_pitch, raw_stage;  // bytes per row and per stage
   int row_shift;            // down: producer warp w holds the rows (32 (w >> row_shift) + lane) 2^row_shift + w % 2^row_shift
   // gate/up tokens: row of the token matrix behind grouped row `pos`
@@ -431,9 +466,24 @@ struct WtParams {
   int n_seg_routed, n_used;
 };
 
-// Job i of this CTA: rounds of gridDim.x jobs, every other round dealt out backwards (the tiles' cost falls along the list).
+// Job i of this pair of CTAs: rounds of as many jobs as there are pairs, every other round dealt out backwards (the tiles' cost
+// falls along the list).
 __device__ __forceinline__ int wt_job(int i) {
-  return i * (int)gridDim.x + ((i & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+  const int pairs = (int)gridDim.x >> 1, me = (int)blockIdx.x >> 1;
+  return i * pairs + ((i & 1) ? pairs - 1 - me : me);
+}
+// Weight rows of a job that are this CTA's; where the blocks are odd in number the last one's pair does it twice and keeps one.
+struct JobBlock {
+  int tile, blk0;
+  bool keep;
+};
+__device__ __forceinline__ JobBlock wt_block(int job, int n_pair, int n_blk, int rank) {
+  JobBlock j;
+  j.tile = job / n_pair;
+  const int b = 2 * (job - j.tile * n_pair) + rank;
+  j.keep = b < n_blk;
+  j.blk0 = min(b, n_blk - 1);
+  return j;
 }
 
 // Lane of an operand tile -> weight row: gate/up rows go in the order 0,2,1,3 inside every four, so that the
@@ -455,7 +505,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
   constexpr int RAW_WARP = wt_raw_warp(MODE), RAW_WARPS = wt_raw_warps(MODE);
   const GroupedParams& p = w.g;
   unsigned char* b_ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  unsigned char* raw_ring = b_ring + (size_t)w.sb * W_B_STAGE;
+  unsigned char* raw_ring = b_ring + W_B_STAGES * W_B_STAGE;
   unsigned char* patches = raw_ring + (size_t)w.rb * w.raw_stage;
   // (shuffles and votes mark what is the same in the whole warp: the MMA operands then stay in uniform registers)
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
@@ -463,7 +513,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
   // only its token copies wait (for the activations), its weights are on their way and unpacked by then.
   if (MODE == 0) pdl_wait();
   pdl_trigger();
-  const int n_jobs = __shfl_sync(0xFFFFFFFFu, __ldcg(p.n_tiles) * w.n_blk, 0);
+  const int rank = __shfl_sync(0xFFFFFFFFu, (int)pair_rank(), 0);
+  const int n_jobs = __shfl_sync(0xFFFFFFFFu, __ldcg(p.n_tiles) * w.n_pair, 0);
   if (wt_job(0) >= n_jobs) {
     if (MODE == 1) pdl_wait();
     return;
@@ -471,22 +522,24 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
 
   if (tid == 0) {
     for (int s = 0; s < W_A_STAGES; ++s) {
-      mbar_init(&bars.full_a[s], 8);
+      mbar_init(&bars.full_a[s], 16);
       mbar_init(&bars.empty_a[s], 1);
     }
-    for (int s = 0; s < W_MAX_RING; ++s) {
-      mbar_init(&bars.full_b[s], MODE == 0 ? 64 : 1);
+    for (int s = 0; s < W_B_STAGES; ++s) {
+      mbar_init(&bars.full_b[s], (MODE == 0 ? 64 : 1) + (rank == 0 ? 1 : 0));
       mbar_init(&bars.empty_b[s], 1);
+    }
+    for (int s = 0; s < W_MAX_RAW; ++s) {
       mbar_init(&bars.full_raw[s], wt_tiled(FMT) ? 1 : RAW_WARPS * 32);
       mbar_init(&bars.empty_raw[s], W_PRODUCERS / 32);
     }
     mbar_init(&bars.done, 1);
-    mbar_init(&bars.drained, W_PRODUCERS / 32);
+    mbar_init(&bars.drained, 2 * W_PRODUCERS / 32);
     mbar_fence_init();
   }
-  if (warp == W_MMA_WARP) umma::tmem_alloc(&s_tmem, 512);
+  if (warp == W_MMA_WARP) tmem_alloc_pair(&s_tmem);
   umma::fence_before_sync();
-  __syncthreads();
+  pair_sync();  // the other CTA's barriers are there, and both have their tensor memory
   umma::fence_after_sync();
   // All 512 columns are this CTA's, so they start at column 0 of lane 0, and addresses below are constants.  Were it ever
   // otherwise, every role would leave at once and the call report it.
@@ -513,10 +566,11 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     for (int it = 0; ok; ++it) {
       const int job = wt_job(it);
       if (job >= n_jobs) break;
-      const int tile = job / w.n_blk, blk0 = job - tile * w.n_blk;
+      const JobBlock jb = wt_block(job, w.n_pair, w.n_blk, rank);
+      const int tile = jb.tile, blk0 = jb.blk0;
       const int e = __ldcg(p.tile_expert + tile), row0 = __ldcg(p.tile_row0 + tile), rows_valid = __ldcg(p.tile_rows + tile);
       const int wrow = MODE == 0 ? blk0 * 128 + (slot & 127) : blk0 * WR + slot;
-      unsigned long long* tr = TRACED && tile == p.trace_tile && blk0 == 0 ? p.trace : nullptr;
+      unsigned long long* tr = TRACED && tile == p.trace_tile && blk0 == 0 && rank == 0 ? p.trace : nullptr;
       if (TRACED) trace_stamp(tr, 40 + 4 * MODE);
       for (int blk = 0; blk < kb; ++blk) {
         if (TRACED && blk < 4) trace_stamp(tr, 64 + 64 * MODE + 8 * blk);
@@ -574,7 +628,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           tmem_st_32x32(a_addr + 64u * ap.s, o);
           umma::fence_before_sync();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&bars.full_a[ap.s]);
+          if (lane == 0) arrive_first(&bars.full_a[ap.s]);
           if (TRACED && blk < 4) trace_stamp(tr, 67 + 64 * MODE + 8 * blk + 4 * h);
           if (TRACED && blk < 4 && h == 0) {  // the block's second step has its raw blocks already
             trace_stamp(tr, 68 + 64 * MODE + 8 * blk);
@@ -596,7 +650,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       // the down kernel's operand: [K step][rows of the tile][128 B], swizzled like its image in shared memory
       unsigned char* act = reinterpret_cast<unsigned char*>(p.act) + (size_t)row0 * p.nff * 2 + (size_t)(2 * blk0 + (q >> 1)) * rows_valid * 128;
       // warps of one lane quarter share the tile's tokens, 16 at a time
-      for (int t0 = 16 * (warp >> 2); t0 < rows_valid; t0 += 64) {
+      for (int t0 = 16 * (warp >> 2); t0 < rows_valid && jb.keep; t0 += 64) {
         const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)t0;
         float v[2][2][8];  // [accumulator][16 lanes][fragment]
         tmem_ld_16x16_quad(tq, tq + (16u << 16), tq + WN, tq + WN + (16u << 16), v[0][0], v[0][1], v[1][0], v[1][1]);
@@ -678,47 +732,65 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       }
       umma::fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars.drained);
+      if (lane == 0) arrive_first(&bars.drained);
       if (TRACED) trace_stamp(tr, 43 + 4 * MODE);
     }
     if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
   } else if (warp == W_MMA_WARP) {
-    // ---- MMA issue: the warp waits, one elected lane issues ----
-    const uint64_t db0 = umma::smem_desc_k_major_swz128(b_ring, 0);
+    // ---- MMA issue: the first CTA's warp waits, one elected lane issues for both; the other's passes on that its tokens are there ----
     RingPos bp, ap;
-    uint32_t r_phase = 1;
-    for (int it = 0; ok; ++it) {
-      const int job = wt_job(it);
-      if (job >= n_jobs) break;
-      const uint32_t idesc = umma::idesc_f16_f32(128, (__shfl_sync(0xFFFFFFFFu, __ldcg(p.tile_rows + job / w.n_blk), 0) + 15) & ~15);
-      ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.drained, r_phase));
-      if (!ok) break;
-      r_phase ^= 1;
-      for (int step = 0; step < 4 * kb; ++step) {
-        ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.full_b[bp.s], bp.phase) && wt_wait(&bars.full_a[ap.s], ap.phase));
-        if (!ok) break;
-        umma::fence_after_sync();
-        if (elect_one()) {
-          const uint64_t db = db0 + (uint64_t)(bp.s * (W_B_STAGE >> 4));
-          const uint32_t a = W_A_COL + 64u * ap.s, acc = step > 0;
-          unsigned long long* tr = TRACED && job == p.trace_tile * w.n_blk && step < 16 ? p.trace : nullptr;
-          if (TRACED) trace_write(tr, 96 + 64 * MODE + 2 * step);
-          if (MODE == 0) umma::fence_proxy_async();  // the copies behind full_b were cp.async
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            mma_f16_ta(tmem, a + 8 * k, db + 2 * k, idesc, k > 0 ? 1u : acc);
-            mma_f16_ta(tmem + WN, a + 32 + 8 * k, db + 2 * k, idesc, k > 0 ? 1u : acc);
+    if (rank != 0) {
+      for (int it = 0; ok && wt_job(it) < n_jobs; ++it)
+        for (int step = 0; step < 4 * kb; ++step) {
+          ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.full_b[bp.s], bp.phase));
+          if (!ok) break;
+          if (elect_one()) {
+            if (MODE == 0) umma::fence_proxy_async();  // the copies behind full_b were cp.async
+            arrive_first(&bars.full_b[bp.s]);
           }
-          umma::commit(&bars.empty_a[ap.s]);
-          umma::commit(&bars.empty_b[bp.s]);
-          if (step == 4 * kb - 1) umma::commit(&bars.done);
-          if (TRACED) trace_write(tr, 97 + 64 * MODE + 2 * step);
+          __syncwarp();
+          bp.next(W_B_STAGES);
+          ap.next(W_A_STAGES);
         }
-        __syncwarp();
-        bp.next(w.sb);
-        ap.next(W_A_STAGES);
+    } else {
+      const uint64_t db0 = umma::smem_desc_k_major_swz128(b_ring, 0);
+      uint32_t r_phase = 1;
+      for (int it = 0; ok; ++it) {
+        const int job = wt_job(it);
+        if (job >= n_jobs) break;
+        const uint32_t idesc = umma::idesc_f16_f32(256, (__shfl_sync(0xFFFFFFFFu, __ldcg(p.tile_rows + job / w.n_pair), 0) + 31) & ~31);
+        ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.drained, r_phase));
+        if (!ok) break;
+        r_phase ^= 1;
+        for (int step = 0; step < 4 * kb; ++step) {
+          ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.full_b[bp.s], bp.phase) && wt_wait(&bars.full_a[ap.s], ap.phase));
+          if (!ok) break;
+          umma::fence_after_sync();
+          if (elect_one()) {
+            const uint64_t db = db0 + (uint64_t)(bp.s * (W_B_STAGE >> 4));
+            const uint32_t a = W_A_COL + 64u * ap.s, acc = step > 0;
+            unsigned long long* tr = TRACED && job == p.trace_tile * w.n_pair && step < 16 ? p.trace : nullptr;
+            if (TRACED) trace_write(tr, 96 + 64 * MODE + 2 * step);
+            if (MODE == 0) umma::fence_proxy_async();
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              mma_f16_ta(tmem, a + 8 * k, db + 2 * k, idesc, k > 0 ? 1u : acc);
+              mma_f16_ta(tmem + WN, a + 32 + 8 * k, db + 2 * k, idesc, k > 0 ? 1u : acc);
+            }
+            commit_pair(&bars.empty_a[ap.s]);
+            commit_pair(&bars.empty_b[bp.s]);
+            if (step == 4 * kb - 1) commit_pair(&bars.done);
+            if (TRACED) trace_write(tr, 97 + 64 * MODE + 2 * step);
+          }
+          __syncwarp();
+          bp.next(W_B_STAGES);
+          ap.next(W_A_STAGES);
+        }
       }
     }
+    // every commit that this CTA was promised has arrived before either leaves
+    for (int i = 0; i < W_B_STAGES && ok; ++i, bp.next(W_B_STAGES)) ok = wt_wait(&bars.empty_b[bp.s], bp.phase ^ 1);
+    for (int i = 0; i < W_A_STAGES && ok; ++i, ap.next(W_A_STAGES)) ok = wt_wait(&bars.empty_a[ap.s], ap.phase ^ 1);
     if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
   } else if (warp < RAW_WARP) {
     // ---- token operand ----
@@ -730,9 +802,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       for (int it = 0; ok; ++it) {
         const int job = wt_job(it);
         if (job >= n_jobs) break;
-        const int tile = job / w.n_blk, rows_valid = __ldcg(p.tile_rows + tile);
-        const uint32_t bytes = (uint32_t)((rows_valid + 15) & ~15) * 128u;
-        const unsigned char* src = reinterpret_cast<const unsigned char*>(p.act) + (size_t)__ldcg(p.tile_row0 + tile) * p.nff * 2;
+        const int tile = job / w.n_pair, rows_valid = __ldcg(p.tile_rows + tile);
+        const uint32_t bytes = (uint32_t)((rows_valid + 31) & ~31) * 64u;
+        const unsigned char* src = reinterpret_cast<const unsigned char*>(p.act) + (size_t)__ldcg(p.tile_row0 + tile) * p.nff * 2 + rank * bytes;
         for (int step = 0; step < 4 * kb; ++step) {
           if (!wt_wait(&bars.empty_b[bp.s], bp.phase ^ 1)) { ok = false; break; }
           if (elect_one()) {
@@ -740,7 +812,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
             bulk_g2s(b_ring + (size_t)bp.s * W_B_STAGE, src + (size_t)step * rows_valid * 128, bytes, &bars.full_b[bp.s]);
           }
           __syncwarp();
-          bp.next(w.sb);
+          bp.next(W_B_STAGES);
         }
       }
     } else {
@@ -751,17 +823,17 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       const uint32_t dst0 = smem_u32(b_ring) + (uint32_t)r8 * 128u + (uint32_t)((c ^ r8) << 4);
       const uint4* tok = reinterpret_cast<const uint4*>(p.xg) + c;
       const int n_sorted = __ldcg(w.seg_off + w.n_seg_routed);
-      if (tw & 2) bp.next(w.sb);
+      if (tw & 2) bp.next(W_B_STAGES);
       for (int it = 0; ok; ++it) {
         const int job = wt_job(it);
         if (job >= n_jobs) break;
-        const int tile = job / w.n_blk;
-        const int row0 = __ldcg(p.tile_row0 + tile), rows_valid = __ldcg(p.tile_rows + tile), ni = ((rows_valid + 15) & ~15) >> 3;
-        uint32_t src[WN / 8];  // rows 8 i + r8, in units of 16 bytes
+        const int tile = job / w.n_pair;
+        const int row0 = __ldcg(p.tile_row0 + tile), rows_valid = __ldcg(p.tile_rows + tile), ni = ((rows_valid + 31) >> 5) * 2;
+        uint32_t src[WN / 16];  // rows 8 i + r8 of this CTA's half, in units of 16 bytes
 #pragma unroll
-        for (int i = 0; i < WN / 8; ++i) {
+        for (int i = 0; i < WN / 16; ++i) {
           if (i < ni) {
-            const int pos = row0 + min(8 * i + r8, rows_valid - 1);  // past the end: the last row once more
+            const int pos = row0 + min(8 * (rank * ni + i) + r8, rows_valid - 1);  // past the end: the last row once more
             const int t = w.pair_of_pos == nullptr ? pos : pos < n_sorted ? __ldcg(w.pair_of_pos + pos) / w.n_used : pos - n_sorted;
             src[i] = (uint32_t)t * (uint32_t)(p.ne >> 3);
           }
@@ -771,11 +843,11 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           const uint32_t dst = dst0 + (uint32_t)bp.s * W_B_STAGE;
           const uint4* ts = tok + step * 8;
 #pragma unroll
-          for (int i = 0; i < WN / 8; ++i)
+          for (int i = 0; i < WN / 16; ++i)
             if (i < ni) cp_async16(dst + i * 1024, ts + src[i]);
           cp_async_arrive(&bars.full_b[bp.s]);
-          bp.next(w.sb);
-          bp.next(w.sb);
+          bp.next(W_B_STAGES);
+          bp.next(W_B_STAGES);
         }
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
@@ -787,7 +859,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     for (int it = 0; ok; ++it) {
       const int job = wt_job(it);
       if (job >= n_jobs) break;
-      const int tile = job / w.n_blk, blk0 = job - tile * w.n_blk, e = __ldcg(p.tile_expert + tile);
+      const JobBlock jb = wt_block(job, w.n_pair, w.n_blk, rank);
+      const int blk0 = jb.blk0, e = __ldcg(p.tile_expert + jb.tile);
       const bool shared_seg = e >= p.n_expert;
       if (wt_tiled(FMT)) {
         if (warp != RAW_WARP || lane != 0) break;  // one thread issues the tiled copies
@@ -858,8 +931,10 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
   }
   umma::fence_before_sync();
-  __syncthreads();
-  if (warp == W_MMA_WARP) umma::tmem_dealloc(s_tmem, 512);
+  __syncwarp();
+  pair_sync();
+  __syncwarp();
+  if (warp == W_MMA_WARP) tmem_dealloc_pair(s_tmem);
 }
 
 // A bank as a 2-D tensor of half-words [rows][row bytes / 2]; box: 256 weights (`chunk` bytes) of `box_rows` rows.
@@ -894,22 +969,29 @@ uint32_t raw_pitch_of(int fmt, int dt) {
 
 template <int MODE, int FMT>
 int32_t launch_wt(infr_cuda_ctx* ctx, WtParams w, const CUtensorMap (&tm)[4], int max_tiles) {
-  // as many stages as fit: two raw stages at least, then up to four token stages, then more raw stages
+  // the token stages, and as many raw stages as fit beside them, two at least
   const size_t patches = (size_t)(W_PRODUCERS / 32) * W_PATCH;
-  const size_t room = 227 * 1024 - 1024 - 1024 - patches;  // alignment slack, static shared memory
-  w.rb = 2;
-  w.sb = W_MAX_RING;
-  while (w.sb > 2 && (size_t)w.rb * w.raw_stage + (size_t)w.sb * W_B_STAGE > room) --w.sb;
-  while (w.rb < W_MAX_RING && (size_t)(w.rb + 1) * w.raw_stage + (size_t)w.sb * W_B_STAGE <= room) ++w.rb;
-  const size_t rings = (size_t)w.rb * w.raw_stage + (size_t)w.sb * W_B_STAGE;
-  if (rings > room) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "grouped GEMM: blocks too large for the raw ring");
-  const size_t smem = 1024 + rings + patches;
+  const size_t room = 227 * 1024 - 1024 - 1024 - patches - W_B_STAGES * W_B_STAGE;  // alignment slack, static shared memory
+  w.rb = (int)std::min<size_t>(W_MAX_RAW, room / w.raw_stage);
+  if (w.rb < 2) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "grouped GEMM: blocks too large for the raw ring");
+  const size_t smem = 1024 + W_B_STAGES * W_B_STAGE + (size_t)w.rb * w.raw_stage + patches;
   auto kern = w.g.trace != nullptr ? k_wt_gemm<MODE, FMT, true> : k_wt_gemm<MODE, FMT, false>;
   cudaError_t e = ensure_smem(reinterpret_cast<const void*>(kern), smem);
   if (e != cudaSuccess) return check_cuda(ctx, e, "grouped GEMM: shared-memory attribute");
-  const long long jobs = (long long)max_tiles * w.n_blk;
-  e = launch_ex(kern, dim3((unsigned)std::min<long long>(jobs, ctx->sm_count)), dim3(W_THREADS), smem, ctx->stream, true, w, tm[0],
-                tm[1], tm[2], tm[3]);
+  const long long jobs = (long long)max_tiles * w.n_pair;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * (unsigned)std::min<long long>(jobs, ctx->sm_count / 2));
+  cfg.blockDim = dim3(W_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim = {2, 1, 1};
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  e = cudaLaunchKernelEx(&cfg, kern, w, tm[0], tm[1], tm[2], tm[3]);
   if (e != cudaSuccess) return check_cuda(ctx, e, "grouped GEMM launch");
   ctx->launches += 1;
   return check_cuda(ctx, cudaGetLastError(), "grouped GEMM launch");
@@ -940,6 +1022,7 @@ int32_t launch_wt_grouped(infr_cuda_ctx* ctx, const GroupedParams& p, const WtTo
   // gate / up.  A bank's rows are one 2-D tensor; with gate and up in one bank an expert has 2 nff rows and the up map
   // starts nff rows in (and ends with the bank)
   w.n_blk = p.nff / 128;
+  w.n_pair = (w.n_blk + 1) / 2;
   w.k_blocks = p.ne / 256;
   int fmt = wt_format(p.gate_dt, p.up_dt, false);
   w.raw_pitch = std::max(raw_pitch_of(fmt, p.gate_dt), raw_pitch_of(fmt, p.up_dt));
@@ -958,6 +1041,7 @@ int32_t launch_wt_grouped(infr_cuda_ctx* ctx, const GroupedParams& p, const WtTo
 
   // down
   w.n_blk = p.ne / WR;
+  w.n_pair = (w.n_blk + 1) / 2;
   w.k_blocks = p.nff / 256;
   fmt = wt_format(p.down_dt, p.down_dt, true);
   w.raw_pitch = raw_pitch_of(fmt, p.down_dt);
