@@ -112,3 +112,19 @@ def test_rows_normed_in_the_router(backend, ne, rows):
     assert len(keep) >= rows - 1
     assert np.array_equal(backend.download(ids, np.int32).reshape(rows, 4)[keep], ref.ids[keep])
     assert_close(backend.download(dst, np.float32).reshape(rows, ne)[keep], ref.dst[keep])
+
+
+@pytest.mark.parametrize("ne", [256, 768])
+@pytest.mark.parametrize("rows,E", [(65, 40), (65, 256), (300, 256), (500, 256), (640, 256), (777, 256), (900, 250), (1024, 256), (1300, 256), (1700, 256),
+                                    (2368, 256), (3000, 96), (3001, 130), (4100, 256)])
+def test_tiles_of_batched_calls(backend, rows, E, ne):
+    # every tile that prompts take (16 to 64 rows by 32 or 64 experts), ragged in rows and experts, four and twelve copies along k
+    rng = np.random.default_rng(rows + E)
+    x = rng.standard_normal((rows, ne)).astype(np.float32)
+    router = (rng.standard_normal((E, ne)) * 0.1).astype(np.float32)
+    ids, wts = route(backend, x, router, 8)
+    at = np.unique(np.r_[0:16, rows // 2 : rows // 2 + 16, rows - 24 : rows])
+    ref = reference(np.ascontiguousarray(x[at]), router, 8)
+    same = (ids[at] == ref.ids).all(axis=1)
+    assert set(np.where(~same)[0]) <= set(near_tie_rows(ref, 8))
+    np.testing.assert_allclose(wts[at][same], ref.wts[same], rtol=1e-6)
