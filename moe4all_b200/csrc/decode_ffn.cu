@@ -488,15 +488,47 @@ size_t down_smem(int TI, int nff, int sh_ff, int n_used, size_t dbb) {
 }
 
 // TI rows per CTA: bulk copies need TI * row_bytes to be a multiple of 16 for both banks.
-int pick_down_tile(int ne, int nff, int sh_ff, int n_used, size_t dbb) {
+// `limit`: bytes of shared memory.  Which shapes these kernels take is decided at 200 KB; a shape that they take has the largest tile
+// that an SM holds (16 rows of nine 1536-wide Q6_K slots in 217 KB, one row of 2560: 54.8 -> 43.7 us the layer).
+constexpr size_t DN_SMEM_TAKEN = 200 * 1024, DN_SMEM_MOST = 225 * 1024;
+int pick_down_tile(int ne, int nff, int sh_ff, int n_used, size_t dbb, size_t limit = DN_SMEM_TAKEN) {
   const int cands[] = {16, 8, 4};
   for (int TI : cands) {
     if (ne % TI) continue;
     if (((size_t)TI * (nff / 256) * dbb) % 16) continue;
     if (sh_ff && ((size_t)TI * (sh_ff / 256) * dbb) % 16) continue;
-    if (down_smem(TI, nff, sh_ff, n_used, dbb) <= 200 * 1024) return TI;
+    if (down_smem(TI, nff, sh_ff, n_used, dbb) <= limit) return TI;
   }
   return 0;
+}
+
+// Warps of a down CTA.  Its time is a chain of latencies (activations read and rounded by all warps, a task of up to eight rows of a
+// slot per warp), so a CTA takes the warps that its SM's registers leave it: an SM holds 36 warps of these registers.
+//   grid of one wave: 20, which fit beside a gate/up CTA of 16 (128 experts of 768, one row: 16 warps 20.0 us the layer, 20 18.6);
+//   shared memory holds one CTA only: all 24 (7168 wide, 2048, one row: 9 warps 165 us, 24 143);
+//   past four waves: a divisor of the tasks under the cap (infr_cuda_config::dn_warps; 32 rows: 83 us with three CTAs of 12 to an SM,
+//   98 with two of 16), or the cap itself where that leaves fewer than nine (16 tasks, six rows: 8 warps 65.2 us, 12 63.5);
+//   else as many CTAs share an SM as the grid has for it and shared memory and a task per warp allow.  Q6_K: fewer where that takes no
+//   wave more and a round of tasks less.  Q4_K, whose tasks are lighter: whole rounds of tasks where there are several waves (256 experts
+//   of 512: three rows 18 warps 32.2 us, 12 30.0; Q4_K down, three rows 30.8 / 28.1, four rows 18 warps 35.2, 12 35.5, 9 32.3; two
+//   768-wide slots and a shared one, two rows 6 warps 19.9, 18 16.6).
+int pick_down_warps(int ctas, int n_tasks, size_t smem, bool q4k, int sms, int cap) {
+  const int fit = (int)((size_t)227 * 1024 / (smem + 2048));
+  if (ctas <= sms) return 20;
+  if (fit <= 1) return DN_MAX_WARPS;
+  if (ctas > 4 * sms && cap > 0) {
+    int c = std::min(cap, n_tasks);
+    while (n_tasks % c) --c;
+    return c < 9 && n_tasks > cap ? cap : c;
+  }
+  int k = std::min(std::min((ctas + sms - 1) / sms, fit), 36 / std::min(std::max(n_tasks, 6), 9));
+  auto waves = [&](int n) { return (ctas + n * sms - 1) / (n * sms); };
+  auto rounds = [&](int n) { return (n_tasks + 36 / n - 1) / (36 / n); };
+  while (!q4k && k > 2 && waves(k - 1) == waves(k) && rounds(k - 1) < rounds(k)) --k;
+  if (q4k && k > 2 && waves(k) > 1) return (n_tasks + rounds(k) - 1) / rounds(k);
+  const int nw = 36 / k;
+  if (k >= 4) return std::min(nw, std::max(n_tasks, 6));
+  return k == 2 && n_tasks >= 14 ? std::min(nw, n_tasks) : nw;
 }
 
 }  // namespace
@@ -532,7 +564,8 @@ int32_t launch_decode_ffn(infr_cuda_ctx* ctx, const DecodeParams& p, bool pdl, u
   // the generic pair.
   const bool five = p.gate_dt == INFR_CUDA_DT_Q5K;
   const size_t gbb = five ? Q5K_BLOCK_BYTES : Q4K_BLOCK_BYTES, dbb = p.down_q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
-  const int n_chunks = pick_chunks(p.ne, p.nff, sh_ff, gbb), TI = pick_down_tile(p.ne, p.nff, sh_ff, p.n_used, dbb);
+  const int n_chunks = pick_chunks(p.ne, p.nff, sh_ff, gbb);
+  const int TI = pick_down_tile(p.ne, p.nff, sh_ff, p.n_used, dbb) ? pick_down_tile(p.ne, p.nff, sh_ff, p.n_used, dbb, DN_SMEM_MOST) : 0;
   const bool wide_ok = bt.tuned() || p.ne / 64 <= 32 * 4;
   const bool gu_own = p.gate_dt == p.up_dt && (five || p.gate_dt == INFR_CUDA_DT_Q4K) && n_chunks && wide_ok;
   const bool dn_own = (p.down_q4k || p.down_dt == INFR_CUDA_DT_Q6K) && TI;
@@ -543,21 +576,31 @@ int32_t launch_decode_ffn(infr_cuda_ctx* ctx, const DecodeParams& p, bool pdl, u
     stages &= ~2u;
   }
   if (!dn_own && !(stages & 2u)) return (stages & 4u) ? launch_anyfmt_decode(ctx, p, pdl, 4u) : INFR_CUDA_OK;
-  int gw = GU_WARPS;
-  int TR = gw * std::max(n_chunks, 1);
-  int jobs = p.rows * p.n_used * (p.nff / TR) + (has_sh ? p.rows * (sh_ff / TR) : 0);
-  int n_chunks_gu = n_chunks;
+  int gw = GU_WARPS, n_chunks_gu = std::max(n_chunks, 1), jobs = 0;
+  auto jobs_of = [&](int tr) { return p.rows * p.n_used * (p.nff / tr) + (has_sh ? p.rows * (sh_ff / tr) : 0); };
+  auto take = [&](int w, int c) {  // w warps, c chunks: enough threads for the limbs of a row, whole tiles
+    if (p.ne / 16 > w * 32 || p.nff % (w * c) || (has_sh && sh_ff % (w * c)) || gateup_smem(p.ne, c, gbb, w) > 200 * 1024) return false;
+    gw = w;
+    n_chunks_gu = c;
+    jobs = jobs_of(w * c);
+    return true;
+  };
   {
-    // Grids of more than four waves: four warps taking four chunks of four rows each (same tile per role
-    // as 16 x 1, half the default tile).  The smaller CTAs put more independent chains of
-    // (ids -> copies -> unpack) on an SM: 69 us against 78 us for 32 tokens.
-    const int ew = (int)ctx->cfg.gu_warps, ec = (int)ctx->cfg.gu_chunks;
-    if (ew > 0 && ec > 0 && ec <= GU_MAX_CHUNKS && jobs > 4 * ctx->sm_count && p.ne / 16 <= ew * 32 && p.nff % (ew * ec) == 0 &&
-        (!has_sh || sh_ff % (ew * ec) == 0)) {
-      gw = ew;
-      n_chunks_gu = ec;
-      TR = gw * n_chunks_gu;
-      jobs = p.rows * p.n_used * (p.nff / TR) + (has_sh ? p.rows * (sh_ff / TR) : 0);
+    // One wave (a CTA to an SM): 16 warps x 2 chunks, x 1 while even half as many would do with Q4_K (1024 wide, 32 experts of 256, one
+    // row: 12.4 -> 11.2 us the layer).
+    // More: smaller CTAs put more independent chains of (ids -> copies -> unpack) on an SM.  Up to two waves 8 x 2, then 4 x 2 where
+    // four warps stage a row's limbs (2048 wide), else 8 x 2; past four waves 4 x 4 (the config's).  us the layer, 16 x 2 / 8 x 2 / 4 x 2:
+    // 2048 wide, 256 of 512, Q4_K: two rows 22.5 / 22.6 / 23.2, four 37.7 / 37.2 / 36.9; Q5_K: two 26.3 / 25.3 / 24.9, four 45.4 / 41.4 / 40.7;
+    // 4096 wide, 1024: one row 28.0 / 25.3, four 73.3 / 70.1; 3072 wide, 512: two rows 26.7 / 23.0, eight 73.8 / 64.8.
+    const int sms = ctx->sm_count, ew = (int)ctx->cfg.gu_warps, ec = (int)ctx->cfg.gu_chunks;
+    jobs = jobs_of(gw * n_chunks_gu);
+    const int full = jobs;
+    if (full <= sms) {
+      if (!five && n_chunks_gu == 2 && 2 * full <= sms) take(GU_WARPS, 1);
+    } else if (full > 4 * sms && ew > 0 && ec > 0 && ec <= GU_MAX_CHUNKS && take(ew, ec)) {
+      // (69 us against 78 us for 32 tokens)
+    } else if (!(full > 2 * sms && take(4, 2))) {
+      take(8, 2);
     }
   }
   size_t smem_gu = gateup_smem(p.ne, n_chunks_gu, gbb, gw);
@@ -589,24 +632,8 @@ int32_t launch_decode_ffn(infr_cuda_ctx* ctx, const DecodeParams& p, bool pdl, u
   const size_t smem_dn = down_smem(TI, p.nff, sh_ff, p.n_used, dbb);
   e = ensure_smem(reinterpret_cast<const void*>(k_decode_down), smem_dn);
   if (e != cudaSuccess) return check_cuda(ctx, e, "k_decode_down smem attribute");
-  // one warp per (slot, group of up to 8 rows) when that fits, else the largest divisor
-  const int n_tasks = (p.n_used + (has_sh ? 1 : 0)) * (TI > 8 ? TI / 8 : 1);
-  int nw = 16;
-  for (int c = DN_MAX_WARPS; c >= 8; --c)
-    if (n_tasks % c == 0) { nw = c; break; }
-  if (n_tasks < 8) nw = n_tasks < 4 ? 4 : n_tasks;
-  // One CTA per SM when the grid fits the device that way: with a whole number of warps per SM
-  // sub-partition, one of these CTAs shares the register file with a gate/up CTA but not with a
-  // second CTA of its own kind (which would only get going once the first has finished).
-  if (p.rows * (p.ne / TI) <= ctx->sm_count && nw > 16 && nw % 4) nw = std::min((int)DN_MAX_WARPS, (nw + 3) & ~3);
-  {
-    // Grids of more than four waves: at most 12 warps, so that three CTAs share an SM's registers and
-    // their latency chains overlap (83 us against 98 us for 32 tokens).
-    const int cap = (int)ctx->cfg.dn_warps;
-    if (cap > 0 && p.rows * (p.ne / TI) > 4 * ctx->sm_count)
-      for (int c = cap; c >= 1; --c)
-        if (n_tasks % c == 0) { nw = c; break; }
-  }
+  const int ctas_dn = p.rows * (p.ne / TI), n_tasks = (p.n_used + (has_sh ? 1 : 0)) * (TI > 8 ? TI / 8 : 1);
+  const int nw = pick_down_warps(ctas_dn, n_tasks, smem_dn, p.down_q4k != 0, ctx->sm_count, (int)ctx->cfg.dn_warps);
   e = launch_ex(k_decode_down, dim3(p.rows * (p.ne / TI)), dim3(nw * 32), smem_dn, ctx->stream, pdl, p, TI);
   ctx->launches += 1;
   return check_cuda(ctx, e, "k_decode_down launch");

@@ -214,3 +214,26 @@ def test_forms_in_turn_on_the_same_rows(backend, recorded):
             assert np.array_equal(be.download(hidden, np.float32), want)
     finally:
         be.set_config(expert_major=0)
+
+
+@pytest.mark.parametrize("ne,nff,used,shared,rows,mix", [
+    (1024, 256, 4, False, 1, (Q4K, Q4K, Q6K)), (1024, 256, 4, False, 2, (Q4K, Q4K, Q6K)),       # gate/up 16 rows a role; 20 and 18 warps down
+    (1024, 256, 4, False, 8, (Q4K, Q4K, Q6K)),                                                    # one task a warp, four CTAs to an SM
+    (2048, 768, 8, False, 1, (Q4K, Q4K, Q6K)), (2048, 768, 8, False, 6, (Q4K, Q4K, Q6K)),        # 20 warps; past four waves, 12 of 16 tasks
+    (2048, 512, 8, True, 3, (Q4K, Q4K, Q6K)), (2048, 512, 8, True, 4, (Q4K, Q4K, Q4K)),          # 12 warps, two rounds; nine
+    (2560, 1536, 8, True, 1, (Q4K, Q4K, Q6K)),                                                    # 16 output rows in 217 KB, 24 warps
+    (3072, 512, 6, False, 2, (Q4K, Q4K, Q4K)), (4096, 1024, 4, True, 1, (Q4K, Q4K, Q6K)),        # gate/up 8 x 2, two groups of x per lane
+    (1536, 768, 2, True, 2, (Q5K, Q5K, Q6K)), (1536, 768, 2, True, 8, (Q5K, Q5K, Q6K)), (2048, 512, 8, True, 2, (Q5K, Q5K, Q6K))])
+def test_per_pair_tiles_by_grid(backend, ne, nff, used, shared, rows, mix):
+    # what a CTA takes follows from how many the grid has and an SM holds
+    L = synth.make_layer(59, ne, 8, nff, sh_ff=nff if shared else 0, router_std=0.05, dtypes=mix)
+    x = synth.activations(88, rows, ne)
+    backend.set_config(expert_major=1)
+    try:
+        out, ids, _ = GpuLayer(backend, L).run(x, used, path=1)
+    finally:
+        backend.set_config(expert_major=0)
+    ref = oracle_layer(L, x, used)
+    keep = [i for i in range(rows) if i not in set(near_tie_rows(ref, used).tolist())]
+    assert np.array_equal(ids[keep], ref.ids[keep])
+    assert_close(out[keep], ref.dst[keep])
