@@ -310,16 +310,16 @@ int32_t infr_cuda_wrap(infr_cuda_ctx* ctx, void* device_ptr, size_t bytes, infr_
 void infr_cuda_free(infr_cuda_ctx* ctx, infr_cuda_buf* buf) {
   if (!buf) return;
   if (buf->owned && buf->ptr) {
+    CaptureRelaxed relaxed;
     if (ctx) {
       DeviceGuard g(ctx->device);
       std::lock_guard<std::mutex> lock(ctx->free_mu);
       if (!put_off(ctx, ctx->late_bufs, buf->ptr)) {
-        CaptureRelaxed relaxed;
         cudaStreamSynchronize(ctx->stream);
         cudaFree(buf->ptr);
       }
     } else {
-      cudaFree(buf->ptr);
+      cudaFree(buf->ptr);  // a buffer that has outlived its context
     }
   }
   delete buf;
@@ -568,11 +568,11 @@ int32_t infr_cuda_graph_launch(infr_cuda_ctx* ctx, infr_cuda_graph* graph) {
 
 void infr_cuda_graph_free(infr_cuda_ctx* ctx, infr_cuda_graph* graph) {
   if (!graph) return;
+  CaptureRelaxed relaxed;
   if (!ctx) return destroy_graph(graph);
   DeviceGuard g(ctx->device);
   std::lock_guard<std::mutex> lock(ctx->free_mu);
   if (put_off(ctx, ctx->late_graphs, graph)) return;
-  CaptureRelaxed relaxed;
   cudaStreamSynchronize(ctx->stream);
   destroy_graph(graph);
 }

@@ -187,3 +187,26 @@ def test_buffers_plans_and_contexts_may_go_while_recording(backend):
     be.sync()
     assert np.array_equal(be.download(dst).reshape(2, 512), eager)
     plan.free()
+
+
+def test_what_outlived_its_context_may_go_while_recording(backend):
+    # a collector may close a context before it frees the context's buffers and plans
+    from moe4all_b200 import CudaBackend
+    be = backend
+    src, dst = be.from_host(np.arange(256, dtype=np.float32)), be.alloc(1024)
+    other = CudaBackend(0)
+    a, b = other.alloc(1 << 20), other.alloc(1 << 20)
+    other.graph_begin()
+    other.add(a, a, b, 256)
+    plan_of_other = other.graph_end()
+    other.close()
+    be.graph_begin()
+    be.add(src, src, dst, 256)
+    a.free()
+    b.free()
+    plan_of_other.free()
+    plan = be.graph_end()
+    be.execute(plan)
+    be.sync()
+    assert np.array_equal(be.download(dst), 2.0 * np.arange(256, dtype=np.float32))
+    plan.free()
