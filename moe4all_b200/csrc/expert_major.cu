@@ -45,6 +45,48 @@ __device__ __forceinline__ void mma_u8s8_k16(int (&c)[4], uint32_t a0, uint32_t 
                : "r"(a0), "r"(a1), "r"(b0));
 }
 
+// The part of a block's result that the offsets of its codes make, sum over the scale groups of (min or scale) x (sum of the
+// group's fixed-point elements), is a small contraction of its own.  The sums, below 2^20, are split into three bytes, the upper one
+// signed, and take one MMA of K 16 each: in integers, exact.  (As multiply-adds of every thread, with the sums and the mins fetched and
+// taken apart per group, they were a fifth of the instructions, which are what these kernels are bound by.  Gate/up and down, us with the
+// wait for the router: 32 rows of 256 experts of 512 67 / 53 -> 65 / 46, 64 rows of 28 MB experts 607 / 580 -> 558 / 554.)
+#define EM_OFFSET_MMA(NAME, A, B)                                                                                          \
+  __device__ __forceinline__ void NAME(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {                               \
+    c[0] = c[1] = c[2] = c[3] = 0;                                                                                         \
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.s32." A "." B ".s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"      \
+                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(b0));                            \
+  }
+EM_OFFSET_MMA(mma_u8u8, "u8", "u8")
+EM_OFFSET_MMA(mma_u8s8, "u8", "s8")
+EM_OFFSET_MMA(mma_s8u8, "s8", "u8")
+EM_OFFSET_MMA(mma_s8s8, "s8", "s8")
+#undef EM_OFFSET_MMA
+
+// Rows g and g + 8 (a0, a1; SGN: signed bytes) against the sums of the tokens of this thread's accumulator columns, added to mv[row][token].
+// b0, b1, b2: the bytes of the sums of column g's token; NARROW: b0 is byte g & 1 of token g / 2's, b1 is not used.
+template <bool NARROW, bool SGN, int NT>
+__device__ __forceinline__ void offset_sums(uint32_t a0, uint32_t a1, uint32_t b0, uint32_t b1, uint32_t b2, int (&mv0)[NT], int (&mv1)[NT]) {
+  int lo[4], mid[4], hi[4];
+  SGN ? mma_s8u8(lo, a0, a1, b0) : mma_u8u8(lo, a0, a1, b0);
+  if (!NARROW) SGN ? mma_s8u8(mid, a0, a1, b1) : mma_u8u8(mid, a0, a1, b1);
+  SGN ? mma_s8s8(hi, a0, a1, b2) : mma_u8s8(hi, a0, a1, b2);
+#pragma unroll
+  for (int k = 0; k < NT; ++k) {
+    mv0[k] = lo[k] + (NARROW ? lo[1] : mid[k]) * 256 + hi[k] * 65536;
+    mv1[k] = lo[2 + k] + (NARROW ? lo[3] : mid[2 + k]) * 256 + hi[2 + k] * 65536;
+  }
+}
+
+// The eight scales, or mins, of a Q4_K block from its header, four to a word (s0, s1, s2: header words 1 to 3).
+__device__ __forceinline__ void q4k_scales(uint32_t s0, uint32_t s2, uint32_t (&sc)[2]) {
+  sc[0] = s0 & 0x3F3F3F3Fu;
+  sc[1] = (s2 & 0x0F0F0F0Fu) | ((s0 >> 2) & 0x30303030u);
+}
+__device__ __forceinline__ uint32_t q4k_mins(uint32_t s1, uint32_t s2, int upper) {
+  return upper ? ((s2 >> 4) & 0x0F0F0F0Fu) | ((s1 >> 2) & 0x30303030u) : s1 & 0x3F3F3F3Fu;
+}
+__device__ __forceinline__ int byte_of(uint32_t w, int i) { return (int)__byte_perm(w, 0, 0x4440 | i); }
+
 // ---------------------------------------------------------------------------------------------
 // bucket: pairs by expert, in segments of at most `seg_cap` pairs; the shared expert's rows are
 // appended as segments of "expert" n_expert over pair ids P + r.  One CTA.
@@ -176,8 +218,8 @@ __global__ void __launch_bounds__(1024) k_em_bucket(EmParams p, int seg_cap) {
 //   tokens side by side, so a sub-block takes one MMA per role and a thread ends with the low and high sums of rows g,
 //   g + 8 of token t: half the MMAs, fragment loads and scale multiplies.
 template <bool NARROW>
-__device__ __forceinline__ void gateup_block(const unsigned char* w, uint32_t box, const unsigned char* x, uint32_t xh, const int* sum0, int sum_step,
-                                             int b, float (&fg)[4], float (&fu)[4]) {
+__device__ __forceinline__ void gateup_block(const unsigned char* w, uint32_t box, const unsigned char* x, uint32_t xh, const int* sums, int b,
+                                             float (&fg)[4], float (&fu)[4]) {
   constexpr int NT = NARROW ? 1 : 2;  // tokens of a thread
   const int t = threadIdx.x & 3;
   const unsigned char* rows4[4] = {w, w + 8 * Q4K_BLOCK_BYTES, w + box, w + box + 8 * Q4K_BLOCK_BYTES};
@@ -185,43 +227,42 @@ __device__ __forceinline__ void gateup_block(const unsigned char* w, uint32_t bo
 #pragma unroll
   for (int r = 0; r < 4; ++r) hdr[r] = *reinterpret_cast<const uint4*>(rows4[r]);
   int svl[4][NT], svh[4][NT], mv[4][NT];  // [row][token]
+  uint32_t scales[4][2];
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
+  for (int r = 0; r < 4; ++r) {
+    q4k_scales(hdr[r].y, hdr[r].w, scales[r]);
 #pragma unroll
-    for (int k = 0; k < NT; ++k) svl[r][k] = svh[r][k] = mv[r][k] = 0;
+    for (int k = 0; k < NT; ++k) svl[r][k] = svh[r][k] = 0;
+  }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    uint32_t wA[4], wB[4], scp[4], mp[4];
+    uint32_t wA[4], wB[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const unsigned char* q = rows4[r] + 16 + 32 * j + 4 * t;
       wA[r] = *reinterpret_cast<const uint32_t*>(q);
       wB[r] = *reinterpret_cast<const uint32_t*>(q + 16);
-      q4k_scale_min_pair(hdr[r].y, hdr[r].z, hdr[r].w, j, scp[r], mp[r]);
     }
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const int lsb = b * 8 + 2 * j + half;  // sub-block index inside the stage
       const uint32_t b0 = *reinterpret_cast<const uint32_t*>(x + lsb * 32), b1 = *reinterpret_cast<const uint32_t*>(x + lsb * 32 + 16);
       uint32_t a[4][2];
-      int sc[4], mn[4];
+      int sc[4];
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         a[r][0] = (wA[r] >> (4 * half)) & 0x0F0F0F0Fu;
         a[r][1] = (wB[r] >> (4 * half)) & 0x0F0F0F0Fu;
-        sc[r] = (int)((scp[r] >> (8 * half)) & 0xFFu);
-        mn[r] = (int)((mp[r] >> (8 * half)) & 0xFFu);
+        sc[r] = byte_of(scales[r][j >> 1], 2 * (j & 1) + half);
       }
       int c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0};
       mma_u8s8_k32(c0, a[0][0], a[1][0], a[0][1], a[1][1], b0, b1);
       mma_u8s8_k32(c1, a[2][0], a[3][0], a[2][1], a[3][1], b0, b1);
       if (NARROW) {
-        const int sx = sum0[lsb];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           svl[r][0] += sc[r] * (r < 2 ? c0[2 * (r & 1)] : c1[2 * (r & 1)]);
           svh[r][0] += sc[r] * (r < 2 ? c0[2 * (r & 1) + 1] : c1[2 * (r & 1) + 1]);
-          mv[r][0] += mn[r] * sx;
         }
       } else {
         const uint32_t b0h = *reinterpret_cast<const uint32_t*>(x + xh + lsb * 32), b1h = *reinterpret_cast<const uint32_t*>(x + xh + lsb * 32 + 16);
@@ -235,10 +276,21 @@ __device__ __forceinline__ void gateup_block(const unsigned char* w, uint32_t bo
             const int i = 2 * (r & 1) + k;
             svl[r][k] += sc[r] * (r < 2 ? c0[i] : c1[i]);
             svh[r][k] += sc[r] * (r < 2 ? h0[i] : h1[i]);
-            mv[r][k] += mn[r] * sum0[lsb + k * sum_step];
           }
       }
     }
+  }
+  {
+    // K positions 4 t .. 4 t + 3 are sub-blocks; eight of the sixteen are padding, with no min
+    uint32_t mins[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) mins[r] = t < 2 ? q4k_mins(hdr[r].z, hdr[r].w, t) : 0u;
+    const int4 sx = *reinterpret_cast<const int4*>(sums + b * 8 + 4 * (t & 1));
+    const uint32_t p01 = __byte_perm(sx.x, sx.y, 0x5140), p23 = __byte_perm(sx.z, sx.w, 0x5140);
+    const uint32_t b2 = __byte_perm(__byte_perm(sx.x, sx.y, 0x0062), __byte_perm(sx.z, sx.w, 0x0062), 0x5410);
+    const uint32_t b0 = __byte_perm(p01, p23, NARROW && (threadIdx.x & 4) ? 0x7632 : 0x5410), b1 = NARROW ? 0u : __byte_perm(p01, p23, 0x7632);
+    offset_sums<NARROW, false>(mins[0], mins[1], b0, b1, b2, mv[0], mv[1]);
+    offset_sums<NARROW, false>(mins[2], mins[3], b0, b1, b2, mv[2], mv[3]);
   }
   // once per block: value = d * sum(sc * sum(q X)) - dmin * sum(m * sum(X)), X = 256 hi + lo
 #pragma unroll
@@ -301,7 +353,7 @@ __global__ void __launch_bounds__((2 * KS + 1) * 32, 2) k_em_gateup(EmParams p, 
   const int n_jobs = __ldcg(p.n_seg) * tiles_max;
   const int P = p.rows * p.n_used;
   const int n_kc = (p.ne / 256) / KB, nsb = p.ne / 32;
-  const int spitch = KB * 8 + 4;  // ints per token of the sub-block sums: tokens 2t land in different banks
+  const int spitch = KB * 8 + 4;  // ints per token of the sub-block sums: a block's are on a 16-byte boundary
   // stage layout: weights [KB blocks][2 roles][EM_FEAT rows][144] | x limbs [2][8 tokens][xpitch] | sub-block sums [8][spitch] ints
   constexpr uint32_t BOX = EM_FEAT * Q4K_BLOCK_BYTES;  // one block of one role's rows
   const uint32_t w_bytes = (uint32_t)KB * 2 * BOX, x_bytes = (uint32_t)16 * xpitch, s_bytes = (uint32_t)8 * spitch * 4;
@@ -415,9 +467,9 @@ __global__ void __launch_bounds__((2 * KS + 1) * 32, 2) k_em_gateup(EmParams p, 
       const int* sums = reinterpret_cast<const int*>(st + w_bytes + x_bytes);
       for (int b = ks; b < KB; b += KS) {
         if (narrow)
-          gateup_block<true>(wst + (size_t)b * 2 * BOX, BOX, x0 + (size_t)((g & 1) * EM_NARROW + (g >> 1)) * xpitch + 4 * t, 0, sums + t * spitch, 0, b, fg, fu);
+          gateup_block<true>(wst + (size_t)b * 2 * BOX, BOX, x0 + (size_t)((g & 1) * EM_NARROW + (g >> 1)) * xpitch + 4 * t, 0, sums + (g >> 1) * spitch, b, fg, fu);
         else
-          gateup_block<false>(wst + (size_t)b * 2 * BOX, BOX, x0 + (size_t)g * xpitch + 4 * t, (uint32_t)8 * xpitch, sums + 2 * t * spitch, spitch, b, fg, fu);
+          gateup_block<false>(wst + (size_t)b * 2 * BOX, BOX, x0 + (size_t)g * xpitch + 4 * t, (uint32_t)8 * xpitch, sums + g * spitch, b, fg, fu);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_empty[s]);  // (arrivals after the producer's last wait complete phases nobody waits for)
@@ -476,6 +528,9 @@ __global__ void __launch_bounds__((2 * KS + 1) * 32, 2) k_em_gateup(EmParams p, 
 // ---------------------------------------------------------------------------------------------
 // down
 // ---------------------------------------------------------------------------------------------
+// Four bytes of the 16-element sums of block b, K positions 4 t .. 4 t + 3 (`sums` is at the thread's own row and word).
+__device__ __forceinline__ uint32_t sum_bytes(const unsigned char* sums, int b) { return *reinterpret_cast<const uint32_t*>(sums + 16 * b); }
+
 // One 256-weight block of a warp's 16 output rows (rows g and g + 8) against the segment's tokens, added to acc (rows
 // g: 0, 1; g + 8: 2, 3; wide: tokens 2t, 2t + 1; narrow: token t in 0 and 2).
 //
@@ -483,45 +538,52 @@ __global__ void __launch_bounds__((2 * KS + 1) * 32, 2) k_em_gateup(EmParams p, 
 // group and high nibbles the second.
 template <bool NARROW>
 __device__ __forceinline__ void down_block_q4(const unsigned char* blk0, const unsigned char* blk1, const unsigned char* alo, const unsigned char* ahi,
-                                              const int* sum0, const int* sum1, int b, float (&acc)[4]) {
+                                              const unsigned char* sums, uint32_t sum_step, int b, float (&acc)[4]) {
   constexpr int NT = NARROW ? 1 : 2;
   const int t = threadIdx.x & 3;
   const unsigned char* blk[2] = {blk0, blk1};
   const uint4 hdr[2] = {*reinterpret_cast<const uint4*>(blk[0]), *reinterpret_cast<const uint4*>(blk[1])};
   int svl[2][NT], svh[2][NT], mv[2][NT];
+  uint32_t scales[2][2];
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
+  for (int r = 0; r < 2; ++r) {
+    q4k_scales(hdr[r].y, hdr[r].w, scales[r]);
 #pragma unroll
-    for (int k = 0; k < NT; ++k) svl[r][k] = svh[r][k] = mv[r][k] = 0;
+    for (int k = 0; k < NT; ++k) svl[r][k] = svh[r][k] = 0;
+  }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    uint32_t scp[2], mp[2], w0[2], w1[2];
+    uint32_t w0[2], w1[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      q4k_scale_min_pair(hdr[r].y, hdr[r].z, hdr[r].w, j, scp[r], mp[r]);
       w0[r] = *reinterpret_cast<const uint32_t*>(blk[r] + 16 + 32 * j + 4 * t);       // k = 4 t .. 4 t + 3 of a group
       w1[r] = *reinterpret_cast<const uint32_t*>(blk[r] + 32 + 32 * j + 4 * t);       // k = 16 + 4 t ..
     }
 #pragma unroll
     for (int hn = 0; hn < 2; ++hn) {
-      const int k0 = b * 256 + j * 64 + hn * 32, grp = k0 >> 4;
+      const int k0 = b * 256 + j * 64 + hn * 32;
       const uint32_t a00 = (w0[0] >> (4 * hn)) & 0x0F0F0F0Fu, a10 = (w0[1] >> (4 * hn)) & 0x0F0F0F0Fu,
                      a01 = (w1[0] >> (4 * hn)) & 0x0F0F0F0Fu, a11 = (w1[1] >> (4 * hn)) & 0x0F0F0F0Fu;
       int cl[4] = {0, 0, 0, 0}, ch[4] = {0, 0, 0, 0};
       mma_u8s8_k32(cl, a00, a10, a01, a11, *reinterpret_cast<const uint32_t*>(alo + k0), *reinterpret_cast<const uint32_t*>(alo + k0 + 16));
       if (!NARROW) mma_u8s8_k32(ch, a00, a10, a01, a11, *reinterpret_cast<const uint32_t*>(ahi + k0), *reinterpret_cast<const uint32_t*>(ahi + k0 + 16));
-      const int m[2] = {sum0[grp] + sum0[grp + 1], NARROW ? 0 : sum1[grp] + sum1[grp + 1]};
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const int sc = (int)((scp[r] >> (8 * hn)) & 0xFFu), mn = (int)((mp[r] >> (8 * hn)) & 0xFFu);
+        const int sc = byte_of(scales[r][j >> 1], 2 * (j & 1) + hn);
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           svl[r][k] += sc * cl[2 * r + k];
           svh[r][k] += sc * (NARROW ? cl[2 * r + 1] : ch[2 * r + k]);
-          mv[r][k] += mn * m[k];
         }
       }
     }
+  }
+  {
+    // K positions 4 t .. 4 t + 3 are the sums of 16 elements: a group's min stands twice
+    uint32_t mins[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) mins[r] = __byte_perm(q4k_mins(hdr[r].z, hdr[r].w, t >> 1), 0, (t & 1) ? 0x3322 : 0x1100);
+    offset_sums<NARROW, false>(mins[0], mins[1], sum_bytes(sums, b), NARROW ? 0u : sum_bytes(sums + sum_step, b), sum_bytes(sums + 2 * sum_step, b), mv[0], mv[1]);
   }
   // sum over the block of d sc sum(q X) - dmin m sum(X), X = 256 hi + lo
 #pragma unroll
@@ -543,7 +605,7 @@ __device__ __forceinline__ int sext_byte(uint32_t w, int i) {
 // Q6_K: the slab starts on a 16-byte boundary, the rows' blocks at byte offsets ro0, ro1 on 2-byte ones.
 template <bool NARROW>
 __device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_t ro0, uint32_t ro1, const unsigned char* alo, const unsigned char* ahi,
-                                              const int* sum0, const int* sum1, int b, float (&acc)[4]) {
+                                              const unsigned char* sums, uint32_t sum_step, int b, float (&acc)[4]) {
   constexpr int NT = NARROW ? 1 : 2;
   const int t = threadIdx.x & 3;
   // per row: aligned view of the block, the shift that realigns it, d and the 16 scales
@@ -564,7 +626,7 @@ __device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_
 #pragma unroll
   for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int k = 0; k < NT; ++k) svl[r][k] = svh[r][k] = mv[r][k] = 0;
+    for (int k = 0; k < NT; ++k) svl[r][k] = svh[r][k] = 0;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
 #pragma unroll
@@ -590,21 +652,28 @@ __device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_
           const int si = 8 * h + 2 * qd + lh;  // scale index inside the block
           scv[r] = sext_byte(sc[r][si >> 2], si & 3);
         }
-        const int k0 = b * 256 + h * 128 + qd * 32 + lh * 16, grp = k0 >> 4;
+        const int k0 = b * 256 + h * 128 + qd * 32 + lh * 16;
         int cl[4] = {0, 0, 0, 0}, ch[4] = {0, 0, 0, 0};
         mma_u8s8_k16(cl, a[0], a[1], *reinterpret_cast<const uint32_t*>(alo + k0));
         if (!NARROW) mma_u8s8_k16(ch, a[0], a[1], *reinterpret_cast<const uint32_t*>(ahi + k0));
-        const int m[2] = {sum0[grp], NARROW ? 0 : sum1[grp]};
 #pragma unroll
         for (int r = 0; r < 2; ++r)
 #pragma unroll
           for (int k = 0; k < NT; ++k) {
             svl[r][k] += scv[r] * cl[2 * r + k];
             svh[r][k] += scv[r] * (NARROW ? cl[2 * r + 1] : ch[2 * r + k]);
-            mv[r][k] += scv[r] * m[k];
           }
       }
     }
+  }
+  {
+    uint32_t own[2];  // the scales of K positions 4 t .. 4 t + 3
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const uint32_t even = (t & 2) ? sc[r][2] : sc[r][0], odd = (t & 2) ? sc[r][3] : sc[r][1];
+      own[r] = (t & 1) ? odd : even;
+    }
+    offset_sums<NARROW, true>(own[0], own[1], sum_bytes(sums, b), NARROW ? 0u : sum_bytes(sums + sum_step, b), sum_bytes(sums + 2 * sum_step, b), mv[0], mv[1]);
   }
   // sum over the block of sc * (sum(q X) - 32 sum(X)), X = 256 hi + lo
 #pragma unroll
@@ -656,11 +725,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 && !Q4 ? 2 : 0) k_em_do
   const int n_jobs = __ldcg(p.n_seg) * tiles;
   const int job0 = (int)((long long)blockIdx.x * n_jobs / gridDim.x), job1 = (int)((long long)(blockIdx.x + 1) * n_jobs / gridDim.x);
   if (job0 >= job1) return;
-  const int ngrp = (p.nffmax >> 4) + 4;  // ints per token of the sums: tokens 2t land in different banks
-  // shared memory: activation limbs [2][8 tokens][apitch] | sums [8][ngrp] ints | NBUF slab buffers
+  const int sum_pitch = 16 * ((p.nffmax >> 8) | 1);  // bytes of a row of one byte of the sums: 4 (mod 8) words
+  // shared memory: activation limbs [2][8 tokens][apitch] | bytes of the 16-element sums [3][8 tokens][sum_pitch] | NBUF slab buffers
   unsigned char* s_act = smem;
-  int* s_sum = reinterpret_cast<int*>(smem + (size_t)16 * apitch);
-  unsigned char* slab_area = reinterpret_cast<unsigned char*>(s_sum + 8 * ngrp);
+  unsigned char* s_sum = smem + (size_t)16 * apitch;
+  unsigned char* slab_area = s_sum + 24 * sum_pitch;
   slab_area += (128u - (smem_u32(slab_area) & 127u)) & 127u;
 
   auto width_of = [&](int e) { return e >= p.n_expert ? p.sh_ff : p.nff; };
@@ -733,7 +802,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 && !Q4 ? 2 : 0) k_em_do
           int sx = (X[0] + X[1]) + (X[2] + X[3]);  // 16 elements = four neighbouring lanes
           sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 1);
           sx += __shfl_xor_sync(0xFFFFFFFFu, sx, 2);
-          if ((i & 3) == 0) s_sum[tk * ngrp + (i >> 2)] = sx;
+          if ((i & 3) < 3) s_sum[((i & 3) * (cnt <= EM_NARROW ? EM_NARROW : 8) + tk) * sum_pitch + (i >> 2)] = (unsigned char)(sx >> (8 * (i & 3)));
         };
         float m = 0.f;
         if (n4 <= 128) {  // up to 512 wide: the row stays in registers
@@ -768,16 +837,17 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 && !Q4 ? 2 : 0) k_em_do
     const bool narrow = cnt <= EM_NARROW;
     const unsigned char* alo = s_act + (size_t)(narrow ? (g & 1) * EM_NARROW + (g >> 1) : g) * apitch + 4 * t;
     const unsigned char* ahi = alo + (size_t)8 * apitch;
-    const int* sum0 = s_sum + (narrow ? t : 2 * t) * ngrp;
-    const int* sum1 = sum0 + ngrp;
+    // bytes of the sums: wide - of token g, byte k 8 k rows on; narrow - byte g & 1 of token g / 2, byte 2 eight rows on from byte 0's
+    const uint32_t sum_step = (narrow ? EM_NARROW : 8) * sum_pitch;
+    const unsigned char* sums = s_sum + (narrow ? (g & 1) * EM_NARROW + (g >> 1) : g) * sum_pitch + 4 * t;
     const int rt = warp % n_rt, ks = warp / n_rt;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     const uint32_t rofs[2] = {(uint32_t)(rt * 16 + g) * drb, (uint32_t)(rt * 16 + g + 8) * drb};
     for (int b = ks; b < nb; b += ksplit) {
-      if (Q4 && narrow) down_block_q4<true>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
-      if (Q4 && !narrow) down_block_q4<false>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
-      if (!Q4 && narrow) down_block_q6<true>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
-      if (!Q4 && !narrow) down_block_q6<false>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sum0, sum1, b, acc);
+      if (Q4 && narrow) down_block_q4<true>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sums, sum_step, b, acc);
+      if (Q4 && !narrow) down_block_q4<false>(slab + rofs[0] + (uint32_t)b * DBB, slab + rofs[1] + (uint32_t)b * DBB, alo, ahi, sums, sum_step, b, acc);
+      if (!Q4 && narrow) down_block_q6<true>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sums, sum_step, b, acc);
+      if (!Q4 && !narrow) down_block_q6<false>(slab, rofs[0] + (uint32_t)b * DBB, rofs[1] + (uint32_t)b * DBB, alo, ahi, sums, sum_step, b, acc);
     }
     if (ksplit > 1) {
       if (ks > 0) {
@@ -888,7 +958,7 @@ DownShape down_shape(int ne, int nffmax, bool q4k) {
   DownShape d = {};
   d.apitch = nffmax + 16;  // 4 (mod 32) words
   const size_t dbb = q4k ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
-  const size_t fixed = (size_t)16 * d.apitch + (size_t)8 * (nffmax / 16 + 4) * 4 + 256;
+  const size_t fixed = (size_t)16 * d.apitch + (size_t)8 * (nffmax / 16 + 4) * 4 + 256;  // limbs, sums (with room to spare)
   const size_t drb = (size_t)nffmax / 256 * dbb;
   const int nb = nffmax / 256;
   d.warps = down_warps(nffmax);

@@ -86,6 +86,25 @@ def test_expert_major_segments(backend, ne, nff, down_q4k):
     assert_close(out, oracle_layer(L, x, 1, expert_ids=ids).dst)
 
 
+@pytest.mark.parametrize("down_q4k", [False, True])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_expert_major_largest_sums(backend, sign, down_q4k):
+    # rows of one value: every fixed-point element is +-32639 and a sum of 32 is +-1044448, all three of its bytes in use; in the
+    # last rows 24 elements of every 32 cancel or vanish (sums of any size, zero too)
+    counts = [1, 4, 5, 8, 9]
+    L = synth.make_layer(60, 1024, len(counts), 512, sh_ff=512, router_std=0.05, down_q4k=down_q4k)
+    ids = ids_of(counts, 6)
+    x = np.full((len(ids), 1024), 0.5 * sign, np.float32)
+    x[-4:, 1::2] *= -1.0
+    x[-2:].reshape(2, -1, 32)[:, :, 8:] = 0.0
+    backend.set_config(expert_major=2)
+    try:
+        out, _, _ = GpuLayer(backend, L).run(x, 1, path=1, expert_ids=ids)
+    finally:
+        backend.set_config(expert_major=0)
+    assert_close(out, oracle_layer(L, x, 1, expert_ids=ids).dst)
+
+
 @pytest.mark.parametrize("ne,nff,sh_ff", [(256, 256, 0), (2048, 512, 512), (4096, 256, 768), (8192, 256, 0)])
 @pytest.mark.parametrize("mix", [(Q5K, Q5K, Q6K), (Q5K, Q5K, Q8_0), (Q4K, Q5K, Q6K), (Q8_0, Q8_0, Q4K)])
 def test_decode_stage_mixes(backend, mix, ne, nff, sh_ff):
