@@ -700,11 +700,12 @@ __device__ __forceinline__ void down_block_q6(const unsigned char* slab, uint32_
 // other's waits (24 rows, Q6_K, 512 wide: 113 -> 107 us a layer; a scheduler then has 4.4 warps and still nothing to issue in
 // 41 % of its cycles at 32 rows).  Eight warps have two (768 wide, 16 rows: 103 us against 115 with one) unless two leave room for 16 rows only:
 // one of 32 then halves the jobs and their barriers (2048 wide, 64 rows: 1372 -> 1312 us).
-// Two CTAs per SM asked of the compiler where eight warps read Q6_K: left alone it takes 97 registers, told of them 118, with more
-// loads ahead of their use (128 experts of 1024, 32 rows: the layer 154 -> 148 us; of 768 121 -> 117).  Not with Q4_K, of which three
-// fit at 74 registers, nor with four warps (80 registers and spills: 512 wide, 32 rows 86 -> 89).
+// CTAs per SM asked of the compiler, as many as shared memory holds: left alone it takes 80 registers for eight warps of Q6_K, told of
+// two CTAs 124, with more loads ahead of their use (128 experts of 1024, 32 rows: the layer 154 -> 148 us; of 768 121 -> 117), and of
+// four warps 80 or 72 with spills instead of 96 or 80 (512 wide, the layer at 32 / 64 rows 108.4 / 137.3 -> 106.9 / 135.2, Q4_K at 32
+// 74.7 -> 73.8).  Not for eight warps of Q4_K, of which three fit at 78 registers.
 template <bool Q4, int WARPS, int NBUF>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 && !Q4 ? 2 : 0) k_em_down(EmParams p, int rows_cta, int apitch, uint32_t slab_pitch) {
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? (Q4 ? 6 : 5) : Q4 ? 0 : 2) k_em_down(EmParams p, int rows_cta, int apitch, uint32_t slab_pitch) {
   constexpr uint32_t DBB = Q4 ? Q4K_BLOCK_BYTES : Q6K_BLOCK_BYTES;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t s_bar[2];
