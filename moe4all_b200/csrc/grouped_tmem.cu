@@ -9,9 +9,10 @@
 // of tokens behind them, and the operand then crosses shared memory twice (written by the producers, read by the
 // MMAs).  So the weights are the A operand and A lives in tensor memory: a producer thread owns one weight row, unpacks
 // 64 of its weights into 32 registers and stores them with one tcgen05.st into its lane - no swizzle, no shared-memory
-// traffic, no proxy fence.  The tokens are the B operand (N = the tile's tokens rounded up to 16, at most 160), so the
-// tensor-core time of a tile is proportional to its tokens.  Tensor memory: two accumulators of 160 columns (gate and
-// up rows, or the two halves of 256 output features) and three A stages of 64 columns (64 K elements of 256 rows).
+// traffic, no proxy fence.  The tokens are the B operand (N = the tile's tokens rounded up to 32, at most 160): the
+// eight MMAs of a step take 640 cycles at 160 tokens, but 510 - 540 from 128 down, the time of reading A.  Tensor memory:
+// two accumulators of 160 columns (gate and up rows, or the two halves of 256 output features) and three A stages of 64 columns
+// (64 K elements of 256 rows).
 //
 // One persistent pair of CTAs per two SMs walks the jobs (tile, 2 x 256 weight rows, 256 of them in each CTA), tiles listed
 // heaviest first and dealt out in a snake.  The MMAs are the pair's (cta_group::2, M 256): each CTA unpacks its own rows into its
@@ -29,7 +30,7 @@
 //          tiled copies, other formats word by word with cp.async (rows on an odd word pitch, free of bank conflicts)
 // All rings run on across jobs; every wait is bounded.
 //
-// Reading out a full tile of the down kernel takes 7000 beside the 11000 of its K loop at 512 inputs, with the tensor core
+// Reading out a full tile of the down kernel takes 4800 cycles beside the 8800 of its K loop at 512 inputs, with the tensor cores
 // idle: there is one set of accumulators.
 // Down with Q6_K, whose blocks are 210 bytes: as words by cp.async the copies were what everything waited for (without them 3704 ->
 // 2104 us, 8192 tokens of 28 MB experts).  Now a tiled copy brings the 240 bytes around a block, of one row in every 1, 2, 4 or 8
