@@ -668,27 +668,28 @@ int32_t validate_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d, ui
 
 // Which kernels serve a call of `rows` rows: pp = one CTA per pair, em = expert-major integer tensor-core tiles, gg = grouped
 // GEMM on tcgen05.  us per layer on B200, 256 experts top-8 and the shared one (2 MB: 2048 wide, 512; 28 MB: 7168 wide, 2048):
-//   em / gg   2 MB, Q6_K down:  64 rows 146 / 225, 192: 236 / 269, 256: 278 / 269, 352: 349 / 271
-//             2 MB, Q4_K down:  64 rows 133 / 178, 128: 187 / 211, 192: 214 / 212, 256: 251 / 214
-//             28 MB, Q6_K down: 64 rows 1618 / 2377, 192: 2404 / 2840, 256: 3061 / 2848
-//             28 MB, Q4_K down: 8 rows 435 / 505, 64: 1569 / 1681, 128: 2017 / 1938, 256: 2984 / 1970
-//   pp / gg   2 MB, Q5_K / Q6_K: 16 rows 111 / 146, 32: 193 / 212, 64: 357 / 260
-//             2 MB, Q8_0: 2 rows 51 / 52, 8: 135 / 96, 64: 815 / 205;  MXFP4: 16 rows 310 / 390, 32: 581 / 585, 64: 1121 / 754
-//             28 MB: 4 rows of Q8_0 1240 / 361, of Q5_K / Q6_K 581 / 492, of MXFP4 1674 / 1523
+//   em / gg   2 MB, Q6_K down:  64 rows 137 / 191, 192: 197 / 201, 256: 237 / 204, 352: 301 / 209
+//             2 MB, Q4_K down:  64 rows 121 / 178, 128: 150 / 193, 192: 173 / 194, 256: 208 / 196
+//             28 MB, Q6_K down: 64 rows 1448 / 1745, 128: 1862 / 2012, 192: 2309 / 2085, 256: 2874 / 2053
+//             28 MB, Q4_K down: 8 rows 397 / 496, 64: 1392 / 1537, 128: 1781 / 1828, 192: 2166 / 1872, 256: 2674 / 1930
+//   pp / gg   2 MB, Q5_K / Q6_K: 16 rows 109 / 133, 32: 192 / 185, 64: 354 / 241
+//             2 MB, Q8_0: 2 rows 49 / 48, 8: 131 / 94, 64: 813 / 192;  MXFP4: 16 rows 309 / 372, 32: 579 / 578, 64: 1119 / 736
+//             28 MB: 4 rows of Q8_0 1229 / 340, of Q5_K / Q6_K 473 / 372, of MXFP4 1661 / 1458
 // The lines below were drawn on earlier kernels: eleven pairs per expert between em and gg, 2.75 rows per expert (8 rows of
-// large ones) between pp and gg.  On today's, em and gg cross at six to seven pairs per expert (three and a half for
-// large experts with Q4_K down), pp and gg between 0.1 rows per expert (Q8_0) and one (Q5_K, MXFP4).
+// large ones) between pp and gg.  On today's, em and gg cross at six pairs per expert (four to five for
+// large experts), pp and gg between 0.1 rows per expert (Q8_0) and one (Q5_K, MXFP4).
 // Per-pair against expert-major: the second reads an expert's blocks once for all its rows (about pairs^2 / (2 experts) fewer
 // reads of an expert) but takes two more launches and a pass over f32 rows, so what it saves has to reach some size, 25600 x 1024
 // weights; for experts so small that it never does, two pairs per expert.  The expert-major kernels round activations per row and
 // not per 128 as the per-pair ones (up to 1.2 times the error with Q6_K down banks, 1.05 with Q4_K), so the line is not drawn
 // where the times cross but behind it.  pp / em around the line, us per layer, Q6_K down and (Q4_K down):
-//   2048 wide, 256 of 512, top-8, shared: 8 rows 58.6 / 66.0 (55.7 / 59.8), 9 rows 65.1 / 63.2 (59.5 / 59.8), 13 rows 83.4 / 74.3 (76.7 / 68.9),
-//     15 rows 93.0 / 82.8 (86.3 / 75.2): the line is at 15
-//   2048 wide, 128 of 768, top-8: 7 rows 68.7 / 65.0 (58.6 / 59.6), 8 rows 74.8 / 68.9 (64.2 / 65.4), 9 rows 82.7 / 72.8 (71.8 / 67.5): at 9
+//   2048 wide, 256 of 512, top-8, shared: 8 rows 58 / 62 (53 / 56), 9 rows 64 / 60 (59 / 56), 13 rows 83 / 71 (76 / 65),
+//     15 rows 92 / 75 (86 / 68): the line is at 15
+//   2048 wide, 128 of 768, top-8: 7 rows 65 / 62 (55 / 54), 8 rows 71 / 67 (61 / 59), 9 rows 80 / 68 (69 / 64): at 9
+//   (the next three before the two forms' latest gains)
 //   2048 wide, 64 of 1024, top-8: 4 rows 56.8 / 51.0 (44.0 / 47.0), 5 rows 76.5 / 61.3 (60.4 / 59.0): at 5
 //   4096 wide, 96 of 1536, top-4: 5 rows 98.3 / 92.3 (86.5 / 80.9), 6 rows 113 / 97 (101 / 87), 8 rows 142 / 115 (128 / 105): at 8
-//   1024 wide, 32 of 256, top-4: 12 rows 26.1 / 25.6 (24.5 / 25.4), 16 rows 28.5 / 26.4 (27.6 / 25.8): at 16;  28 MB experts: 1 row 167 / 95, 2 rows 298 / 147
+//   1024 wide, 32 of 256, top-4: 12 rows 26.1 / 25.6 (24.5 / 25.4), 16 rows 28.5 / 26.4 (27.6 / 25.8): at 16;  28 MB experts: 2 rows 236 / 135
 bool em_preferred(uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff) {
   const uint64_t size = (uint64_t)ne * nff, pairs = (uint64_t)rows * n_used;
   if (size >= (1ull << 23)) return rows >= 2;  // experts of tens of megabytes
