@@ -930,6 +930,7 @@ int32_t launch_grouped_ffn(infr_cuda_ctx* ctx, const GroupedCall& c) {
     t.seg_off = seg_off;
     t.n_seg_routed = c.ids ? n_seg_routed : 0;
     t.n_used = c.n_used;
+    t.rows_bound = rows_total;
     const int32_t rc = launch_wt_grouped(ctx, p, t, max_tiles);
     if (rc) return rc;
   } else if (!tuned) {

@@ -23,11 +23,13 @@
 // and the MMAs, which take 640 cycles of eight at 160 tokens in pairs and 740 - 790 in one CTA with a wait for a stage between them.
 // Warp roles (24 warps of each CTA):
 //   0-15   producers, two groups of eight on alternate K steps; afterwards they drain the accumulators
-//   16     first CTA: issues the MMAs (one elected lane); second: passes on that its tokens are there
+//   16     first CTA: issues the MMAs (one elected lane); second, gate/up: passes on that its tokens are there
 //   then   token loaders: gate/up - four warps bring rows of the f16 token matrix straight from where the tokens are
-//          (cp.async), two of them per K step; down - one warp, one bulk copy per K step of the tile's activations
+//          (cp.async), two of them per K step; down - one warp, tiled copies of the tile's activations, 16 rows each, which
+//          both CTAs count on the first one's barriers
 //   last   raw-block loaders: 256 weights of 256 rows at a time, into a ring: Q4_K, Q5_K, Q8_0 and the down banks' Q6_K by
-//          tiled copies, other formats word by word with cp.async (rows on an odd word pitch, free of bank conflicts)
+//          tiled copies, which one warp requests (gate/up: two more pass tokens on), other formats word by word with cp.async
+//          (rows on an odd word pitch, free of bank conflicts)
 // All rings run on across jobs; every wait is bounded.
 //
 // Reading out a full tile of the down kernel takes 4800 cycles beside the 8800 of its K loop at 512 inputs, with the tensor cores
@@ -55,6 +57,15 @@ constexpr int W_MMA_WARP = 16, W_TOK_WARP = 17;
 __host__ __device__ constexpr int wt_tok_warps(int mode) { return mode == 0 ? 4 : 1; }
 __host__ __device__ constexpr int wt_raw_warp(int mode) { return W_TOK_WARP + wt_tok_warps(mode); }
 __host__ __device__ constexpr int wt_raw_warps(int mode) { return mode == 0 ? 3 : 4; }
+// Q4_K, Q5_K, Q8_0 (both roles): tiled copies, rows of whole 16-byte pieces.  Q6_K (down): tiled copies of the 240 bytes around a
+// block of 210, over 2^row_shift rows at a time, whose bytes are whole 16-byte pieces.  Any: words, on an odd word pitch.
+enum WtFormat { WT_Q4K, WT_Q5K, WT_Q80, WT_Q6K, WT_ANY };
+__host__ __device__ constexpr bool wt_tiled(int fmt) { return fmt <= WT_Q6K; }
+constexpr uint32_t W_Q6K_BOX = 240;  // 15 pieces of 16 bytes: 14 bytes of offset and 210 of block, rounded up; odd, so that eight
+                                     // rows' pieces are in different banks
+
+// Warps of the second CTA that pass its gate/up tokens on (relay_tokens).
+__host__ __device__ constexpr int wt_relays(int mode, int fmt) { return mode == 0 ? (wt_tiled(fmt) ? 3 : 1) : 0; }
 constexpr uint32_t W_B_STAGE = WN / 2 * 128;   // 64 K elements of half of the tile's tokens
 constexpr uint32_t W_PATCH = 1280;             // per warp: 16 rows x 80 B (f16) or 8 rows x 144 B (f32)
 constexpr int W_B_STAGES = 6;                  // (four: the down kernel 2 - 3 % slower)
@@ -121,11 +132,28 @@ __device__ __forceinline__ uint32_t pair_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// One arrival on `bar` of the pair's first CTA.  What it tells of is in tensor memory, complete, or fenced for the tensor cores, so it
-// orders no other memory of the pair (released and acquired at cluster scope the gate/up kernel of 4096 tokens takes 243 us, not 150).
+// One arrival on `bar` of the pair's first CTA.  What it tells of is in tensor memory and complete, ordered by tcgen05's own fences, so it
+// orders no other memory of the pair.
 __device__ __forceinline__ void arrive_first(uint64_t* bar) {
   asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\tmbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}"
                ::"r"(smem_u32(bar)) : "memory");
+}
+// The same on the barriers of ring positions i .. i + PER - 1 for what threads wrote to this CTA's shared memory: released at the scope of
+// the pair, acquired there by pair_wait.
+template <int PER>
+__device__ __forceinline__ void release_first(uint64_t* ring, int i) {
+  asm volatile("fence.acq_rel.cluster;" ::: "memory");
+#pragma unroll
+  for (int k = 0; k < PER; ++k)
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\tmbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [ra];\n\t}"
+                 ::"r"(smem_u32(&ring[(i + k) % W_B_STAGES])) : "memory");
+}
+// One tiled copy into this CTA's shared memory, counted in bytes on `bar` of the pair's first CTA.
+__device__ __forceinline__ void tma_load_2d_first(void* smem_dst, const CUtensorMap* tm, int x, int y, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %2, 0;\n\t"
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [ra];\n\t}"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tm)), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ void pair_sync() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
@@ -156,18 +184,22 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uin
 
 // Bounded wait of these kernels: a look, then waits that the hardware suspends (spinning warps took a third of the issue
 // slots from the producers).  The limit is a few seconds.
-__device__ __forceinline__ bool wt_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-  if (ok) return true;
-  for (uint32_t i = 0; i < (1u << 21); ++i) {
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(1000u) : "memory");
-    if (ok) return true;
+#define WT_WAIT(NAME, SCOPE)                                                                                                                     \
+  __device__ __forceinline__ bool NAME(uint64_t* bar, uint32_t parity) {                                                                         \
+    uint32_t ok;                                                                                                                                 \
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire." SCOPE ".shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"    \
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");                                                                        \
+    if (ok) return true;                                                                                                                         \
+    for (uint32_t i = 0; i < (1u << 21); ++i) {                                                                                                  \
+      asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire." SCOPE ".shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}" \
+                   : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(1000u) : "memory");                                                          \
+      if (ok) return true;                                                                                                                       \
+    }                                                                                                                                            \
+    return false;                                                                                                                                \
   }
-  return false;
-}
+WT_WAIT(wt_wait, "cta")
+WT_WAIT(pair_wait, "cluster")  // acquires what release_first released
+#undef WT_WAIT
 
 // Meeting of the four warps behind `bar` (bounded, unlike the barriers of the CTA).
 __device__ __forceinline__ bool meet(uint64_t* bar, uint32_t& phase) {
@@ -437,13 +469,6 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr) {
 
 // ---- the kernel ---------------------------------------------------------------------------------------
 
-// Q4_K, Q5_K, Q8_0 (both roles): tiled copies, rows of whole 16-byte pieces.  Q6_K (down): tiled copies of the 240 bytes around a
-// block of 210, over 2^row_shift rows at a time, whose bytes are whole 16-byte pieces.  Any: words, on an odd word pitch.
-enum WtFormat { WT_Q4K, WT_Q5K, WT_Q80, WT_Q6K, WT_ANY };
-__host__ __device__ constexpr bool wt_tiled(int fmt) { return fmt <= WT_Q6K; }
-constexpr uint32_t W_Q6K_BOX = 240;  // 15 pieces of 16 bytes: 14 bytes of offset and 210 of block, rounded up; odd, so that eight
-                                     // rows' pieces are in different banks
-
 struct WtBars {
   uint64_t full_a[W_A_STAGES], empty_a[W_A_STAGES];      // A stages in tensor memory
   uint64_t full_b[W_B_STAGES], empty_b[W_B_STAGES];      // token stages
@@ -497,6 +522,28 @@ __device__ __forceinline__ JobBlock wt_block(int job, int n_pair, int n_blk, int
   return j;
 }
 
+// The second CTA, gate/up: passes on to the first that its tokens are there, PER steps at a time, from step PER `first` of all its jobs' on
+// PER `by` apart.  They are ordinary writes to shared memory (cp.async) that the MMAs of another CTA read, so they are released at the scope
+// of the pair.  Such a release takes longer than a step of 800 cycles: one warp, a release a step, is what everything waits for (777 tokens
+// 220 us the call, 1024 of Q8_0 251, 64 rows of 28 MB experts of Q8_0 2220).  Three warps 177, 208, 1440; and two steps a release 177, 208,
+// 1399.  Formats that come word by word leave one warp, and their steps are longer: a release a step (48 rows of 28 MB experts of MXFP4
+// 5640 us, two steps a release 5970).
+template <int PER>
+__device__ __forceinline__ bool relay_tokens(WtBars& bars, int n_jobs, int steps, int first, int by) {
+  int n = 0;
+  for (int it = 0; wt_job(it) < n_jobs; ++it) n += steps;  // a multiple of four
+  for (int i = PER * first; i < n; i += PER * by) {
+    for (int k = 0; k < PER; ++k)
+      if (!__all_sync(0xFFFFFFFFu, wt_wait(&bars.full_b[(i + k) % W_B_STAGES], ((i + k) / W_B_STAGES) & 1))) return false;
+    if (elect_one()) {
+      umma::fence_proxy_async();
+      release_first<PER>(bars.full_b, i);
+    }
+    __syncwarp();
+  }
+  return true;
+}
+
 // Lane of an operand tile -> weight row: gate/up rows go in the order 0,2,1,3 inside every four, so that the
 // activations come out in the K order of the down kernel's operands.
 __device__ __forceinline__ int wt_row_of_lane(int mode, int l) { return mode == 0 ? ((l & ~3) | ((l & 1) << 1) | ((l >> 1) & 1)) : l; }
@@ -509,11 +556,11 @@ __device__ __forceinline__ int wt_row_of_lane(int mode, int l) { return mode == 
 template <int MODE, int FMT, bool TRACED>
 __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant__ WtParams w, const __grid_constant__ CUtensorMap tm_w0,
                                                          const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__ CUtensorMap tm_s0,
-                                                         const __grid_constant__ CUtensorMap tm_s1) {
+                                                         const __grid_constant__ CUtensorMap tm_s1, const __grid_constant__ CUtensorMap tm_act) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) WtBars bars;
   __shared__ uint32_t s_tmem;
-  constexpr int RAW_WARP = wt_raw_warp(MODE), RAW_WARPS = wt_raw_warps(MODE);
+  constexpr int RAW_WARP = wt_raw_warp(MODE), RAW_WARPS = wt_raw_warps(MODE), RELAYS = wt_relays(MODE, FMT), PER = RELAYS > 1 ? 2 : 1;
   const GroupedParams& p = w.g;
   unsigned char* b_ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char* raw_ring = b_ring + W_B_STAGES * W_B_STAGE;
@@ -537,7 +584,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       mbar_init(&bars.empty_a[s], 1);
     }
     for (int s = 0; s < W_B_STAGES; ++s) {
-      mbar_init(&bars.full_b[s], (MODE == 0 ? 64 : 1) + (rank == 0 ? 1 : 0));
+      mbar_init(&bars.full_b[s], MODE == 1 ? 1 : rank == 0 ? 65 : 64);
       mbar_init(&bars.empty_b[s], 1);
     }
     for (int s = 0; s < W_MAX_RAW; ++s) {
@@ -763,18 +810,12 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     }
     if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
   } else if (warp == W_MMA_WARP) {
-    // ---- MMA issue: the first CTA's warp waits, one elected lane issues for both; the other's passes on that its tokens are there ----
+    // ---- MMA issue: the first CTA's warp waits, one elected lane issues for both; the second's passes on that its tokens are there ----
     RingPos bp, ap;
     if (rank != 0) {
+      if (MODE == 0) ok = ok && relay_tokens<PER>(bars, n_jobs, 4 * kb, 0, RELAYS);
       for (int it = 0; ok && wt_job(it) < n_jobs; ++it)
         for (int step = 0; step < 4 * kb; ++step) {
-          ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.full_b[bp.s], bp.phase));
-          if (!ok) break;
-          if (elect_one()) {
-            if (MODE == 0) umma::fence_proxy_async();  // the copies behind full_b were cp.async
-            arrive_first(&bars.full_b[bp.s]);
-          }
-          __syncwarp();
           bp.next(W_B_STAGES);
           ap.next(W_A_STAGES);
         }
@@ -789,7 +830,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
         if (!ok) break;
         r_phase ^= 1;
         for (int step = 0; step < 4 * kb; ++step) {
-          ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.full_b[bp.s], bp.phase) && wt_wait(&bars.full_a[ap.s], ap.phase));
+          ok = __all_sync(0xFFFFFFFFu, (MODE == 0 ? pair_wait(&bars.full_b[bp.s], bp.phase) : wt_wait(&bars.full_b[bp.s], bp.phase)) &&
+                                          wt_wait(&bars.full_a[ap.s], ap.phase));
           if (!ok) break;
           umma::fence_after_sync();
           if (elect_one()) {
@@ -822,21 +864,18 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     // ---- token operand ----
     RingPos bp;
     if (MODE == 1) {
-      // the tile's activations: [K step][rows of the tile][128 B], swizzled - one copy per step (past the tile's last row
-      // it reads on into the next step: columns of the accumulators that nothing looks at)
+      // the tile's activations: [K step][rows of the tile][128 B], swizzled - this CTA's half as copies of 16 rows, a lane each
+      // (past the tile's last row they read on into the next step: columns of the accumulators that nothing looks at)
       pdl_wait();
       for (int it = 0; ok; ++it) {
         const int job = wt_job(it);
         if (job >= n_jobs) break;
-        const int tile = job / w.n_pair, rows_valid = __ldcg(p.tile_rows + tile);
-        const uint32_t bytes = (uint32_t)((rows_valid + 31) & ~31) * 64u;
-        const unsigned char* src = reinterpret_cast<const unsigned char*>(p.act) + (size_t)__ldcg(p.tile_row0 + tile) * p.nff * 2 + rank * bytes;
+        const int tile = job / w.n_pair, rows_valid = __ldcg(p.tile_rows + tile), half = (rows_valid + 31) >> 5;  // copies of 16 rows
+        const int y0 = __ldcg(p.tile_row0 + tile) * (p.nff >> 6) + 16 * (rank * half + lane);
         for (int step = 0; step < 4 * kb; ++step) {
           if (!wt_wait(&bars.empty_b[bp.s], bp.phase ^ 1)) { ok = false; break; }
-          if (elect_one()) {
-            mbar_arrive_expect_tx(&bars.full_b[bp.s], bytes);
-            bulk_g2s(b_ring + (size_t)bp.s * W_B_STAGE, src + (size_t)step * rows_valid * 128, bytes, &bars.full_b[bp.s]);
-          }
+          if (rank == 0 && lane == 0) mbar_arrive_expect_tx(&bars.full_b[bp.s], (uint32_t)half * 2 * 16 * 128);
+          if (lane < half) tma_load_2d_first(b_ring + (size_t)bp.s * W_B_STAGE + lane * 2048, &tm_act, 0, y0 + step * rows_valid, &bars.full_b[bp.s]);
           __syncwarp();
           bp.next(W_B_STAGES);
         }
@@ -879,6 +918,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       asm volatile("cp.async.wait_all;" ::: "memory");
     }
     if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
+  } else if (RELAYS > 1 && warp > RAW_WARP) {
+    if (rank != 0 && ok && !relay_tokens<PER>(bars, n_jobs, 4 * kb, warp - RAW_WARP, RELAYS) && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
   } else if (warp < RAW_WARP + RAW_WARPS) {
     // ---- raw blocks ----
     RingPos rp;
@@ -994,7 +1035,7 @@ uint32_t raw_pitch_of(int fmt, int dt) {
 }
 
 template <int MODE, int FMT>
-int32_t launch_wt(infr_cuda_ctx* ctx, WtParams w, const CUtensorMap (&tm)[4], int max_tiles) {
+int32_t launch_wt(infr_cuda_ctx* ctx, WtParams w, const CUtensorMap (&tm)[5], int max_tiles) {
   // the token stages, and as many raw stages as fit beside them, two at least
   const size_t patches = (size_t)(W_PRODUCERS / 32) * W_PATCH;
   const size_t room = 227 * 1024 - 1024 - 1024 - patches - W_B_STAGES * W_B_STAGE;  // alignment slack, static shared memory
@@ -1017,7 +1058,7 @@ int32_t launch_wt(infr_cuda_ctx* ctx, WtParams w, const CUtensorMap (&tm)[4], in
   attr[1].val.clusterDim = {2, 1, 1};
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  e = cudaLaunchKernelEx(&cfg, kern, w, tm[0], tm[1], tm[2], tm[3]);
+  e = cudaLaunchKernelEx(&cfg, kern, w, tm[0], tm[1], tm[2], tm[3], tm[4]);
   if (e != cudaSuccess) return check_cuda(ctx, e, "grouped GEMM launch");
   ctx->launches += 1;
   return check_cuda(ctx, cudaGetLastError(), "grouped GEMM launch");
@@ -1042,7 +1083,7 @@ int32_t launch_wt_grouped(infr_cuda_ctx* ctx, const GroupedParams& p, const WtTo
   w.seg_off = t.seg_off;
   w.n_seg_routed = t.n_seg_routed;
   w.n_used = t.n_used;
-  CUtensorMap tm[4] = {};
+  CUtensorMap tm[5] = {};
   bool ok = true;
 
   // gate / up.  A bank's rows are one 2-D tensor; with gate and up in one bank an expert has 2 nff rows and the up map
@@ -1073,6 +1114,9 @@ int32_t launch_wt_grouped(infr_cuda_ctx* ctx, const GroupedParams& p, const WtTo
   w.raw_pitch = raw_pitch_of(fmt, p.down_dt);
   w.raw_stage = WR * w.raw_pitch;
   w.row_shift = p.y_shift;
+  // the activations as a tensor of 128-byte rows: 16 of them a copy
+  if (!raw_rows_map(&tm[4], reinterpret_cast<const uint8_t*>(p.act), ((size_t)t.rows_bound + 256) * (p.nff / 64), 128, 128, 16))
+    return fail(ctx, INFR_CUDA_ERR_CUDA, "grouped GEMM: the driver refused a tensor map for the activations");
   if (wt_tiled(fmt)) {
     const size_t rb = row_bytes(p.down_dt, p.nff) << w.row_shift;
     const uint32_t box_rows = fmt == WT_Q6K ? (uint32_t)WR >> w.row_shift : 128u;

@@ -150,6 +150,7 @@ struct WtTokens {
   const int* pair_of_pos;  // pair behind every grouped row, or null: `xg` is in grouped order itself
   const int* seg_off;      // [n_seg_routed] = grouped rows ahead of the shared expert's, which follow in token order
   int n_seg_routed, n_used;
+  int rows_bound;          // grouped rows, 256 fewer than `act` has room for
 };
 int wt_tile_rows();
 int wt_y_shift(int down_dt, int nff);

@@ -256,3 +256,28 @@ def test_per_pair_tiles_by_grid(backend, ne, nff, used, shared, rows, mix):
     keep = [i for i in range(rows) if i not in set(near_tie_rows(ref, used).tolist())]
     assert np.array_equal(ids[keep], ref.ids[keep])
     assert_close(out[keep], ref.dst[keep])
+
+
+@pytest.mark.parametrize("mix", [(Q4K, Q4K, Q6K), (Q8_0, Q8_0, Q8_0)])
+def test_both_halves_of_a_tiles_tokens_are_this_calls(backend, mix):
+    # each CTA of a pair brings half of a tile's tokens (the second has none of its own up to 16), 64 steps through six stages, and the
+    # MMAs of one read both: rows that change from call to call in the same buffers are those of the call, every time
+    from moe4all_b200 import DType, MoeFfn
+    be, counts = backend, [1, 16, 17, 32, 33, 100, 160, 161]
+    L = synth.make_layer(61, 4096, len(counts), 512, sh_ff=512, router_std=0.05, dtypes=mix)
+    g, ids = GpuLayer(be, L), ids_of(counts, 7)
+    xs = [synth.activations(96 + i, len(ids), 4096) for i in range(2)]
+    xb, dst = be.from_host(xs[0]), be.alloc(xs[0].nbytes)
+    op = MoeFfn(x=xb, router=g.router, gate_exps=g.gate, up_exps=g.up, down_exps=g.down, dst=dst, rows=len(ids), ne=4096, n_expert=len(counts),
+                n_used=1, n_ff_exp=512, sh_gate=g.sh_gate, sh_up=g.sh_up, sh_down=g.sh_down, sh_gate_inp=g.sh_gate_inp, sh_ff=512,
+                expert_ids=be.from_host(ids), path=2, gate_dtype=DType(mix[0]), up_dtype=DType(mix[1]), down_dtype=DType(mix[2]))
+    first = [None, None]
+    for rep in range(40):
+        i = rep & 1
+        be.upload(xb, xs[i])
+        be.moe_ffn(op)
+        out = be.download(dst, np.float32).reshape(-1, 4096)
+        if first[i] is None:
+            first[i] = out
+            assert_close(out, oracle_layer(L, xs[i], 1, expert_ids=ids).dst)
+        assert np.array_equal(out, first[i])
