@@ -92,7 +92,9 @@ int32_t infr_cuda_set_stream(infr_cuda_ctx* ctx, void* cuda_stream);
  * field has a working default and none changes results beyond the stated tolerances. */
 typedef struct infr_cuda_config {
   uint32_t gu_warps, gu_chunks;  /* per-pair gate/up kernel on grids of more than four waves: warps per CTA
-                                    and row chunks per CTA (default 4 x 4); 0 = keep the one-wave shape   */
+                                    and row chunks per CTA (default 4 x 4); either 0 = keep the one-wave
+                                    shape; a shape that does not fit the layer's dims is passed over for
+                                    the one that grids of two to four waves take                          */
   uint32_t dn_warps;             /* per-pair down kernel on grids of more than four waves whose CTAs share
                                     an SM: warp cap (default 12); 0 = no cap                              */
   uint32_t upload_by_copy;       /* 1: small pinned-memory copies of the *_async calls go through the copy

@@ -19,15 +19,12 @@
 //
 // The format decoders' header stays out of this file: with its constant-memory tables in the module every launch of these
 // kernels took 0.3 us longer (8 layers of one row 152.0 -> 154.9 us).
+#include "decode_shape.h"
 #include "kernels.cuh"
 
 namespace infr {
 
 namespace {
-
-constexpr int GU_WARPS = 16;  // rows per chunk and role: one per warp
-constexpr int GU_MAX_CHUNKS = 4;
-constexpr int GU_XQPITCH = 144;  // bytes per 64-element group of fixed-point x: 64 low limbs, 64 high limbs, pad
 
 constexpr int DN_MAX_WARPS = 24;
 constexpr int DN_XPITCH = 36;     // words per 128-activation chunk and limb: four neighbouring chunks start in four 16-byte bank groups
@@ -465,21 +462,6 @@ __global__ void __maxnreg__(56) k_decode_down(DecodeParams p, int TI) {
   }
 }
 
-size_t gateup_smem(int ne, int n_chunks, size_t gbb, int gw = GU_WARPS) {
-  return (size_t)n_chunks * 2 * gw * (ne / 256 * gbb) + (size_t)(ne / 64) * GU_XQPITCH;
-}
-
-// Chunks per CTA for gate/up banks of gbb bytes per block.
-int pick_chunks(int ne, int nff, int sh_ff, size_t gbb) {
-  for (int c = 2; c >= 1; c >>= 1) {
-    const int TR = GU_WARPS * c;
-    if (nff % TR) continue;
-    if (sh_ff && sh_ff % TR) continue;
-    if (gateup_smem(ne, c, gbb) <= 200 * 1024) return c;
-  }
-  return 0;
-}
-
 size_t down_smem(int TI, int nff, int sh_ff, int n_used, size_t dbb) {
   const size_t slab = align_up((size_t)TI * (nff / 256 * dbb) + 8, 128) + 128;
   const size_t sh_slab = sh_ff ? align_up((size_t)TI * (sh_ff / 256 * dbb) + 8, 128) + 128 : 0;
@@ -576,33 +558,8 @@ int32_t launch_decode_ffn(infr_cuda_ctx* ctx, const DecodeParams& p, bool pdl, u
     stages &= ~2u;
   }
   if (!dn_own && !(stages & 2u)) return (stages & 4u) ? launch_anyfmt_decode(ctx, p, pdl, 4u) : INFR_CUDA_OK;
-  int gw = GU_WARPS, n_chunks_gu = std::max(n_chunks, 1), jobs = 0;
-  auto jobs_of = [&](int tr) { return p.rows * p.n_used * (p.nff / tr) + (has_sh ? p.rows * (sh_ff / tr) : 0); };
-  auto take = [&](int w, int c) {  // w warps, c chunks: enough threads for the limbs of a row, whole tiles
-    if (p.ne / 16 > w * 32 || p.nff % (w * c) || (has_sh && sh_ff % (w * c)) || gateup_smem(p.ne, c, gbb, w) > 200 * 1024) return false;
-    gw = w;
-    n_chunks_gu = c;
-    jobs = jobs_of(w * c);
-    return true;
-  };
-  {
-    // One wave (a CTA to an SM): 16 warps x 2 chunks, x 1 while even half as many would do with Q4_K (1024 wide, 32 experts of 256, one
-    // row: 12.4 -> 11.2 us the layer).
-    // More: smaller CTAs put more independent chains of (ids -> copies -> unpack) on an SM.  Up to two waves 8 x 2, then 4 x 2 where
-    // four warps stage a row's limbs (2048 wide), else 8 x 2; past four waves 4 x 4 (the config's).  us the layer, 16 x 2 / 8 x 2 / 4 x 2:
-    // 2048 wide, 256 of 512, Q4_K: two rows 22.5 / 22.6 / 23.2, four 37.7 / 37.2 / 36.9; Q5_K: two 26.3 / 25.3 / 24.9, four 45.4 / 41.4 / 40.7;
-    // 4096 wide, 1024: one row 28.0 / 25.3, four 73.3 / 70.1; 3072 wide, 512: two rows 26.7 / 23.0, eight 73.8 / 64.8.
-    const int sms = ctx->sm_count, ew = (int)ctx->cfg.gu_warps, ec = (int)ctx->cfg.gu_chunks;
-    jobs = jobs_of(gw * n_chunks_gu);
-    const int full = jobs;
-    if (full <= sms) {
-      if (!five && n_chunks_gu == 2 && 2 * full <= sms) take(GU_WARPS, 1);
-    } else if (full > 4 * sms && ew > 0 && ec > 0 && ec <= GU_MAX_CHUNKS && take(ew, ec)) {
-      // (69 us against 78 us for 32 tokens)
-    } else if (!(full > 2 * sms && take(4, 2))) {
-      take(8, 2);
-    }
-  }
+  const GateUpShape gu = gateup_shape(p.ne, p.nff, sh_ff, p.rows, p.n_used, gbb, five, ctx->sm_count, (int)ctx->cfg.gu_warps, (int)ctx->cfg.gu_chunks);
+  const int gw = gu.warps, n_chunks_gu = gu.chunks, jobs = gu.ctas;
   size_t smem_gu = gateup_smem(p.ne, n_chunks_gu, gbb, gw);
   // A grid that fits the device one CTA per SM is spread that way: gate/up CTAs start while the
   // router's CTAs still hold some SMs and would otherwise pair up on the free ones, halving their

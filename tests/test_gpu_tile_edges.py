@@ -281,3 +281,19 @@ def test_both_halves_of_a_tiles_tokens_are_this_calls(backend, mix):
             first[i] = out
             assert_close(out, oracle_layer(L, xs[i], 1, expert_ids=ids).dst)
         assert np.array_equal(out, first[i])
+
+
+@pytest.mark.parametrize("warps,chunks", [(0, 0), (0, 4), (16, 1), (3, 4)])
+def test_gateup_shapes_by_config(backend, warps, chunks):
+    # past four waves: the one-wave shape, a named one, and one that does not fit
+    L = synth.make_layer(62, 2048, 8, 512, sh_ff=512, router_std=0.05)
+    x = synth.activations(98, 6, 2048)
+    backend.set_config(expert_major=1, gu_warps=warps, gu_chunks=chunks)
+    try:
+        out, ids, _ = GpuLayer(backend, L).run(x, 8, path=1)
+    finally:
+        backend.set_config(expert_major=0, gu_warps=4, gu_chunks=4)
+    ref = oracle_layer(L, x, 8)
+    keep = [i for i in range(6) if i not in set(near_tie_rows(ref, 8).tolist())]
+    assert np.array_equal(ids[keep], ref.ids[keep])
+    assert_close(out[keep], ref.dst[keep])
