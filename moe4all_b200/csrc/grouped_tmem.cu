@@ -508,17 +508,20 @@ __device__ __forceinline__ int wt_job(int i) {
   const int pairs = (int)gridDim.x >> 1, me = (int)blockIdx.x >> 1;
   return i * pairs + ((i & 1) ? pairs - 1 - me : me);
 }
-// Weight rows of a job that are this CTA's; where the blocks are odd in number the last one's pair does it twice and keeps one.
+// Weight rows of a job that are this CTA's: block blk0 of 256, or, where the blocks (of a down bank) are odd in number and the last one is
+// left to a pair by itself, half of it: 128 rows go through the first accumulator, the second and its producers rest.
+// (Both CTAs doing all of it, us a call of 4096 tokens of Q4_K / Q6_K: 256 wide 122 -> 116, 768 wide 191 -> 187, of 2048-wide experts 438 -> 426;
+// 512 tokens of Q4_K, 256 wide: 61 -> 59, one CTA by itself 55; 768 wide 91 -> 89, 88.)
 struct JobBlock {
   int tile, blk0;
-  bool keep;
+  bool lone;
 };
 __device__ __forceinline__ JobBlock wt_block(int job, int n_pair, int n_blk, int rank) {
   JobBlock j;
   j.tile = job / n_pair;
-  const int b = 2 * (job - j.tile * n_pair) + rank;
-  j.keep = b < n_blk;
-  j.blk0 = min(b, n_blk - 1);
+  const int b = 2 * (job - j.tile * n_pair);
+  j.lone = b + 1 == n_blk;
+  j.blk0 = j.lone ? b : b + rank;
   return j;
 }
 
@@ -552,8 +555,9 @@ __device__ __forceinline__ int wt_row_of_lane(int mode, int l) { return mode == 
 // (down: 4 slots on): 40 the job's start, 41 its first raw blocks there, 42 accumulators complete, 43 drained.  Of its first 16
 // K steps (down: 64 slots on): 64 + 4 i the first producer warp looks for the raw blocks of step 2 i, 65 + 4 i has them, 66 + 4 i
 // has unpacked its weights, 67 + 4 i has stored them; 96 + 2 i the operands of step i are there, 97 + 2 i its MMAs are issued.
-// A variant of its own: the plain one has neither the pointer's registers nor a branch per step.
-template <int MODE, int FMT, bool TRACED>
+// A variant of its own: the plain one has neither the pointer's registers nor a branch per step.  ODD: the 256-row blocks are odd in number
+// (down), a variant of its own too (in one kernel 4096 tokens of 2048 wide take 488 us a call, not 480).
+template <int MODE, int FMT, bool TRACED, bool ODD>
 __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant__ WtParams w, const __grid_constant__ CUtensorMap tm_w0,
                                                          const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__ CUtensorMap tm_s0,
                                                          const __grid_constant__ CUtensorMap tm_s1, const __grid_constant__ CUtensorMap tm_act) {
@@ -609,10 +613,6 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
   if (warp < W_PRODUCERS / 32) {
     // ---- producers: unpack, then drain ----
     const int g = warp >> 3, role = (warp >> 2) & 1, q = warp & 3;
-    const int w8 = warp & 7, sub = w8 & ((1 << w.row_shift) - 1);
-    // row of the raw stage (down: the rows of a warp have one offset from the 16-byte boundary)
-    const int slot = MODE == 0 ? role * 128 + wt_row_of_lane(MODE, q * 32 + lane)
-                               : (sub << (8 - w.row_shift)) + (w8 >> w.row_shift) * 32 + lane;
     const int dt = MODE == 1 ? p.down_dt : (role ? p.up_dt : p.gate_dt);
     const int half_word = (int)(row_bytes(dt, 256) & 2);  // blocks of an odd number of half-words: every other one is off a word boundary
     const uint32_t a_addr = tmem + ((uint32_t)(q * 32) << 16) + W_A_COL + 32u * role;
@@ -627,6 +627,11 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       if (job >= n_jobs) break;
       const JobBlock jb = wt_block(job, w.n_pair, w.n_blk, rank);
       const int tile = jb.tile, blk0 = jb.blk0;
+      const bool lone = ODD && jb.lone;
+      // row of the raw stage (down: the rows of a warp have one offset from the 16-byte boundary)
+      const int w8 = (lone ? 4 * rank : 4 * role) + q, sub = w8 & ((1 << w.row_shift) - 1);
+      const int slot = MODE == 0 ? role * 128 + wt_row_of_lane(MODE, q * 32 + lane)
+                                 : (sub << (8 - w.row_shift)) + (w8 >> w.row_shift) * 32 + lane;
       const int e = __ldcg(p.tile_expert + tile), row0 = __ldcg(p.tile_row0 + tile), rows_valid = __ldcg(p.tile_rows + tile);
       const int wrow = MODE == 0 ? blk0 * 128 + (slot & 127) : blk0 * WR + slot;
       unsigned long long* tr = TRACED && tile == p.trace_tile && blk0 == 0 && rank == 0 ? p.trace : nullptr;
@@ -636,6 +641,18 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
         if (!wt_wait(&bars.full_raw[rp.s], rp.phase)) { ok = false; break; }
         if (TRACED && blk == 0) trace_stamp(tr, 41 + 4 * MODE);
         if (TRACED && blk < 4) trace_stamp(tr, 65 + 64 * MODE + 8 * blk);
+        if (lone && role) {  // nothing to unpack: only the arrivals that the barriers count
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars.empty_raw[rp.s]);
+          for (int h = 0; h < 2 && ok; ++h) {
+            ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.empty_a[ap.s], ap.phase ^ 1));
+            if (ok && lane == 0) arrive_first(&bars.full_a[ap.s]);
+            for (int i = FMT != WT_Q6K ? 2 : h ? 3 : 1; i > 0; --i) ap.next(W_A_STAGES);
+          }
+          if (!ok) break;
+          rp.next(w.rb);
+          continue;
+        }
         const unsigned char* row = raw_ring + (size_t)rp.s * w.raw_stage + (size_t)slot * w.raw_pitch;
         const int mis = ((wrow * kb + blk) & 1) * half_word;  // bytes of the stage's first word ahead of the block
         Q6kHalf half;
@@ -709,7 +726,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       // the down kernel's operand: [K step][rows of the tile][128 B], swizzled like its image in shared memory
       unsigned char* act = reinterpret_cast<unsigned char*>(p.act) + (size_t)row0 * p.nff * 2 + (size_t)(2 * blk0 + (q >> 1)) * rows_valid * 128;
       // warps of one lane quarter share the tile's tokens, 16 at a time
-      for (int t0 = 16 * (warp >> 2); t0 < rows_valid && jb.keep; t0 += 64) {
+      for (int t0 = 16 * (warp >> 2); t0 < rows_valid; t0 += 64) {
         const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)t0;
         float v[2][2][8];  // [accumulator][16 lanes][fragment]
         tmem_ld_16x16_quad(tq, tq + (16u << 16), tq + WN, tq + WN + (16u << 16), v[0][0], v[0][1], v[1][0], v[1][1]);
@@ -743,7 +760,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
         } else {
 #pragma unroll
           for (int m = 0; m < 2; ++m) {
-            const int wq = m * 4 + q, f0 = blk0 * WR + wq * 32;  // first of the lane quarter's 32 places among the output features
+            if (m == 1 && lone) break;
+            const int mw = lone ? rank : m, f0 = blk0 * WR + (mw * 4 + q) * 32;  // first of the lane quarter's 32 places among the output features
             if (p.y_packed) {
               // the combine kernel is the only reader: this thread's four outputs of a token (8 places apart) as one item
 #pragma unroll
@@ -795,7 +813,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
                   const int t = q + 4 * i;
                   const float4 x = *reinterpret_cast<const float4*>(pf + t * 132 + lane * 4);
                   if (t0 + 8 * cg + t < rows_valid)
-                    *reinterpret_cast<float4*>(p.y + (size_t)(row0 + t0 + 8 * cg + t) * p.ne + blk0 * WR + (sh == 3 ? 8 * lane + 4 * m : m * 128 + 4 * lane)) = x;
+                    *reinterpret_cast<float4*>(p.y + (size_t)(row0 + t0 + 8 * cg + t) * p.ne + blk0 * WR + (sh == 3 ? 8 * lane + 4 * mw : mw * 128 + 4 * lane)) = x;
                 }
                 if (ok) ok = meet(&bars.patch[warp >> 2], m_phase);
               }
@@ -825,7 +843,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       for (int it = 0; ok; ++it) {
         const int job = wt_job(it);
         if (job >= n_jobs) break;
-        const uint32_t idesc = umma::idesc_f16_f32(256, (__shfl_sync(0xFFFFFFFFu, __ldcg(p.tile_rows + job / w.n_pair), 0) + 31) & ~31);
+        const JobBlock jb = wt_block(job, w.n_pair, w.n_blk, 0);
+        const uint32_t idesc = umma::idesc_f16_f32(256, (__shfl_sync(0xFFFFFFFFu, __ldcg(p.tile_rows + jb.tile), 0) + 31) & ~31);
         ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.drained, r_phase));
         if (!ok) break;
         r_phase ^= 1;
@@ -843,7 +862,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               mma_f16_ta(tmem, a + 8 * k, db + 2 * k, idesc, k > 0 ? 1u : acc);
-              mma_f16_ta(tmem + WN, a + 32 + 8 * k, db + 2 * k, idesc, k > 0 ? 1u : acc);
+              if (!ODD || !jb.lone) mma_f16_ta(tmem + WN, a + 32 + 8 * k, db + 2 * k, idesc, k > 0 ? 1u : acc);
             }
             commit_pair(&bars.empty_a[ap.s]);
             commit_pair(&bars.empty_b[bp.s]);
@@ -937,19 +956,22 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           if (!wt_wait(&bars.empty_raw[rp.s], rp.phase ^ 1)) { ok = false; break; }
           unsigned char* dst = raw_ring + (size_t)rp.s * w.raw_stage;
           if (FMT == WT_Q6K) {
+            const int n = 1 << w.row_shift, i0 = ODD && jb.lone && n == 8 ? 4 * rank : 0, i1 = ODD && jb.lone && n == 8 ? i0 + 4 : n;
             // the rows of one place among 2^row_shift rows per copy, from the 16-byte boundary at or ahead of the block (a box that
             // runs on past the last block's row is filled up with zeros)
-            mbar_arrive_expect_tx(&bars.full_raw[rp.s], w.raw_stage);
-            for (int i = 0; i < 1 << w.row_shift; ++i)
+            mbar_arrive_expect_tx(&bars.full_raw[rp.s], (w.raw_stage >> w.row_shift) * (i1 - i0));
+            for (int i = i0; i < i1; ++i)
               tma_load_2d(dst + i * (w.raw_stage >> w.row_shift), shared_seg ? &tm_s0 : &tm_w0, (((int)Q6K_BLOCK_BYTES * (i * kb + blk)) & ~15) >> 1,
                           r0 >> w.row_shift, &bars.full_raw[rp.s]);
             rp.next(w.rb);
             continue;
           }
           const int x = blk * (int)(w.raw_pitch >> 1);  // in half-words
-          mbar_arrive_expect_tx(&bars.full_raw[rp.s], w.raw_stage);
-          tma_load_2d(dst, shared_seg ? &tm_s0 : &tm_w0, x, r0, &bars.full_raw[rp.s]);
-          tma_load_2d(dst + 128 * w.raw_pitch, shared_seg ? &tm_s1 : &tm_w1, x, r0 + (MODE == 0 ? 0 : 128), &bars.full_raw[rp.s]);
+          const bool lone = ODD && jb.lone;
+          mbar_arrive_expect_tx(&bars.full_raw[rp.s], lone ? w.raw_stage / 2 : w.raw_stage);
+          if (!lone || rank == 0) tma_load_2d(dst, shared_seg ? &tm_s0 : &tm_w0, x, r0, &bars.full_raw[rp.s]);
+          if (!lone || rank != 0)
+            tma_load_2d(dst + 128 * w.raw_pitch, shared_seg ? &tm_s1 : &tm_w1, x, r0 + (MODE == 0 ? 0 : 128), &bars.full_raw[rp.s]);
           rp.next(w.rb);
         }
       } else {
@@ -1042,7 +1064,10 @@ int32_t launch_wt(infr_cuda_ctx* ctx, WtParams w, const CUtensorMap (&tm)[5], in
   w.rb = (int)std::min<size_t>(W_MAX_RAW, room / w.raw_stage);
   if (w.rb < 2) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "grouped GEMM: blocks too large for the raw ring");
   const size_t smem = 1024 + W_B_STAGES * W_B_STAGE + (size_t)w.rb * w.raw_stage + patches;
-  auto kern = w.g.trace != nullptr ? k_wt_gemm<MODE, FMT, true> : k_wt_gemm<MODE, FMT, false>;
+  constexpr bool MAY_BE_ODD = MODE == 1;  // gate/up: blocks of 128 features, of 256 k
+  const bool odd = w.n_blk & 1;
+  auto kern = w.g.trace != nullptr ? (odd ? k_wt_gemm<MODE, FMT, true, MAY_BE_ODD> : k_wt_gemm<MODE, FMT, true, false>)
+                                   : (odd ? k_wt_gemm<MODE, FMT, false, MAY_BE_ODD> : k_wt_gemm<MODE, FMT, false, false>);
   cudaError_t e = ensure_smem(reinterpret_cast<const void*>(kern), smem);
   if (e != cudaSuccess) return check_cuda(ctx, e, "grouped GEMM: shared-memory attribute");
   const long long jobs = (long long)max_tiles * w.n_pair;

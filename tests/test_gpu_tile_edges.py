@@ -297,3 +297,22 @@ def test_gateup_shapes_by_config(backend, warps, chunks):
     keep = [i for i in range(6) if i not in set(near_tie_rows(ref, 8).tolist())]
     assert np.array_equal(ids[keep], ref.ids[keep])
     assert_close(out[keep], ref.dst[keep])
+
+
+@pytest.mark.parametrize("mix,nff", [((Q4K, Q4K, Q6K), 256), ((Q4K, Q4K, Q6K), 512), ((Q4K, Q4K, Q6K), 1024), ((Q4K, Q4K, Q6K), 2048), ((Q4K, Q4K, Q4K), 512),
+                                     ((Q5K, Q5K, Q5K), 512), ((Q8_0, Q8_0, Q8_0), 512), ((39, 39, 39), 512)])
+@pytest.mark.parametrize("ne", [256, 1280])
+@pytest.mark.parametrize("raw_f32", [0, 1])
+def test_odd_widths(backend, mix, nff, ne, raw_f32):
+    # 256-row blocks of an odd number: the last one of a tile goes half to each CTA of a pair, between jobs of whole blocks (1280) or alone
+    # (256); Q6_K rows 8, 4, 2 and 1 apart, packed and f32 outputs
+    counts = [1, 16, 17, 0, 33, 160, 161, 48]
+    L = synth.make_layer(63, ne, len(counts), nff, sh_ff=nff, router_std=0.05, dtypes=mix)
+    ids = ids_of(counts, 8)
+    x = synth.activations(99, len(ids), ne)
+    backend.set_config(raw_rows_f32=raw_f32)
+    try:
+        out, _, _ = GpuLayer(backend, L).run(x, 1, path=2, expert_ids=ids)
+    finally:
+        backend.set_config(raw_rows_f32=0)
+    assert_close(out, oracle_layer(L, x, 1, expert_ids=ids).dst)
