@@ -128,3 +128,18 @@ def test_tiles_of_batched_calls(backend, rows, E, ne):
     same = (ids[at] == ref.ids).all(axis=1)
     assert set(np.where(~same)[0]) <= set(near_tie_rows(ref, 8))
     np.testing.assert_allclose(wts[at][same], ref.wts[same], rtol=1e-6)
+
+
+@pytest.mark.parametrize("rows,E", [(4705, 160), (4705, 131)])
+@pytest.mark.parametrize("ne", [256, 768])
+def test_tile_of_32_rows_by_64_experts(backend, rows, E, ne):
+    # the smallest of the wide tiles, which the counts above do not reach: whole and ragged in experts
+    rng = np.random.default_rng(rows + E)
+    x = rng.standard_normal((rows, ne)).astype(np.float32)
+    router = (rng.standard_normal((E, ne)) * 0.1).astype(np.float32)
+    ids, wts = route(backend, x, router, 8)
+    at = np.unique(np.r_[0:16, rows // 2 : rows // 2 + 16, rows - 24 : rows])
+    ref = reference(np.ascontiguousarray(x[at]), router, 8)
+    same = (ids[at] == ref.ids).all(axis=1)
+    assert set(np.where(~same)[0]) <= set(near_tie_rows(ref, 8))
+    np.testing.assert_allclose(wts[at][same], ref.wts[same], rtol=1e-6)
