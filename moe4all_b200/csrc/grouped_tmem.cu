@@ -49,6 +49,8 @@
 namespace infr {
 namespace {
 
+using namespace umma;
+
 constexpr int WN = 160;              // most tokens of a tile
 constexpr int WR = 256;              // weight rows of a job
 constexpr int W_PRODUCERS = 512;
@@ -79,67 +81,10 @@ __device__ __forceinline__ uint32_t h2_as_u32(__half2 h) { return *reinterpret_c
 __device__ __forceinline__ __half2 u32_as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ __half2 h2_const(uint32_t bits) { return u32_as_h2(bits | (bits << 16)); }
 
-// ---- tensor-memory and copy forms only this file uses ------------------------------------------------
+// ---- copy forms only this file uses -------------------------------------------------------------------
 
-// 32 registers of every lane -> 32 consecutive columns of the lane's row (warp w: lanes 32 (w % 4) ..).
-__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n\t"
-      "tcgen05.wait::st.sync.aligned;"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
-        "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
-        "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-
-// 16 accumulator rows (lanes) x 16 columns at each of four addresses as 8x8 fragments: thread T holds of row T / 4 (v[0],
-// v[1]) and row T / 4 + 8 (v[2], v[3]) the columns 2 (T % 4), + 1; v[4..7] the same of the columns 8 further on.
-__device__ __forceinline__ void tmem_ld_16x16_quad(uint32_t ta, uint32_t tb, uint32_t tc, uint32_t td, float (&a)[8], float (&b)[8], float (&c)[8],
-                                                   float (&d)[8]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%32];\n\t"
-      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%33];\n\t"
-      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%34];\n\t"
-      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%24,%25,%26,%27,%28,%29,%30,%31}, [%35];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]), "=f"(a[7]), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]),
-        "=f"(b[3]), "=f"(b[4]), "=f"(b[5]), "=f"(b[6]), "=f"(b[7]), "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]), "=f"(c[4]), "=f"(c[5]),
-        "=f"(c[6]), "=f"(c[7]), "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]), "=f"(d[4]), "=f"(d[5]), "=f"(d[6]), "=f"(d[7])
-      : "r"(ta), "r"(tb), "r"(tc), "r"(td)
-      : "memory");
-}
-
-// D[tmem] (+)= A[tmem] * B[smem]^T for one K = 16 slice; A: lane = row, a 32-bit column = two K elements.  A and D: 128 rows in
-// each CTA of the pair, at the same columns; B: half of the rows (tokens) in each, at the same place of shared memory.
-__device__ __forceinline__ void mma_f16_ta(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(acc)
-      : "memory");
-}
-// All MMAs issued so far by this thread arrive on `bar` of both CTAs when they have completed.
-__device__ __forceinline__ void commit_pair(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
-}
-
-__device__ __forceinline__ uint32_t pair_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// One arrival on `bar` of the pair's first CTA.  What it tells of is in tensor memory and complete, ordered by tcgen05's own fences, so it
-// orders no other memory of the pair.
-__device__ __forceinline__ void arrive_first(uint64_t* bar) {
-  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\tmbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}"
-               ::"r"(smem_u32(bar)) : "memory");
-}
-// The same on the barriers of ring positions i .. i + PER - 1 for what threads wrote to this CTA's shared memory: released at the scope of
-// the pair, acquired there by pair_wait.
+// One arrival on the first CTA's barriers of ring positions i .. i + PER - 1, for what threads wrote to this CTA's shared memory: released at
+// the scope of the pair, acquired there by pair_wait.
 template <int PER>
 __device__ __forceinline__ void release_first(uint64_t* ring, int i) {
   asm volatile("fence.acq_rel.cluster;" ::: "memory");
@@ -155,18 +100,6 @@ __device__ __forceinline__ void tma_load_2d_first(void* smem_dst, const CUtensor
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [ra];\n\t}"
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tm)), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ void pair_sync() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-
-// One lane of a converged warp.  Branching on this (and not on a lane number), in a branch the compiler knows to be
-// warp-uniform, keeps the MMA operands in uniform registers: 9 cycles per tcgen05.mma against 55 from `if (lane == 0)`.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
-  return p != 0;
-}
-
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -458,15 +391,6 @@ __device__ __forceinline__ void pack_y4(float a, float b, float c, float d, uint
   lo = __byte_perm(__byte_perm(q[0], q[1], 0x0051), __byte_perm(q[2], q[3], 0x0051), 0x5410);
 }
 
-// All 512 columns of both CTAs' tensor memory; one warp of each takes part.
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(slot)) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(taddr) : "memory");
-}
-
 // ---- the kernel ---------------------------------------------------------------------------------------
 
 struct WtBars {
@@ -539,7 +463,7 @@ __device__ __forceinline__ bool relay_tokens(WtBars& bars, int n_jobs, int steps
     for (int k = 0; k < PER; ++k)
       if (!__all_sync(0xFFFFFFFFu, wt_wait(&bars.full_b[(i + k) % W_B_STAGES], ((i + k) / W_B_STAGES) & 1))) return false;
     if (elect_one()) {
-      umma::fence_proxy_async();
+      fence_proxy_async();
       release_first<PER>(bars.full_b, i);
     }
     __syncwarp();
@@ -601,9 +525,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     mbar_fence_init();
   }
   if (warp == W_MMA_WARP) tmem_alloc_pair(&s_tmem);
-  umma::fence_before_sync();
+  fence_before_sync();
   pair_sync();  // the other CTA's barriers are there, and both have their tensor memory
-  umma::fence_after_sync();
+  fence_after_sync();
   // All 512 columns are this CTA's, so they start at column 0 of lane 0, and addresses below are constants.  Were it ever
   // otherwise, every role would leave at once and the call report it.
   constexpr uint32_t tmem = 0;
@@ -700,9 +624,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           }
           if (TRACED && blk < 4) trace_stamp(tr, 66 + 64 * MODE + 8 * blk + 4 * h);
           if (!wt_wait(&bars.empty_a[ap.s], ap.phase ^ 1)) { ok = false; break; }
-          umma::fence_after_sync();
+          fence_after_sync();
           tmem_st_32x32(a_addr + 64u * ap.s, o);
-          umma::fence_before_sync();
+          fence_before_sync();
           __syncwarp();
           if (lane == 0) arrive_first(&bars.full_a[ap.s]);
           if (TRACED && blk < 4) trace_stamp(tr, 67 + 64 * MODE + 8 * blk + 4 * h);
@@ -720,7 +644,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       if (!ok) break;
       if (!wt_wait(&bars.done, d_phase)) { ok = false; break; }
       d_phase ^= 1;
-      umma::fence_after_sync();
+      fence_after_sync();
       if (TRACED) trace_stamp(tr, 42 + 4 * MODE);
       const float clamp = e < p.n_expert ? p.clamp : 0.f;  // the shared expert's segment is not clamped
       // the down kernel's operand: [K step][rows of the tile][128 B], swizzled like its image in shared memory
@@ -821,7 +745,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           }
         }
       }
-      umma::fence_before_sync();
+      fence_before_sync();
       __syncwarp();
       if (lane == 0) arrive_first(&bars.drained);
       if (TRACED) trace_stamp(tr, 43 + 4 * MODE);
@@ -838,13 +762,13 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           ap.next(W_A_STAGES);
         }
     } else {
-      const uint64_t db0 = umma::smem_desc_k_major_swz128(b_ring, 0);
+      const uint64_t db0 = smem_desc_k_major_swz128(b_ring, 0);
       uint32_t r_phase = 1;
       for (int it = 0; ok; ++it) {
         const int job = wt_job(it);
         if (job >= n_jobs) break;
         const JobBlock jb = wt_block(job, w.n_pair, w.n_blk, 0);
-        const uint32_t idesc = umma::idesc_f16_f32(256, (__shfl_sync(0xFFFFFFFFu, __ldcg(p.tile_rows + jb.tile), 0) + 31) & ~31);
+        const uint32_t idesc = idesc_f16_f32(256, (__shfl_sync(0xFFFFFFFFu, __ldcg(p.tile_rows + jb.tile), 0) + 31) & ~31);
         ok = __all_sync(0xFFFFFFFFu, wt_wait(&bars.drained, r_phase));
         if (!ok) break;
         r_phase ^= 1;
@@ -852,13 +776,13 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           ok = __all_sync(0xFFFFFFFFu, (MODE == 0 ? pair_wait(&bars.full_b[bp.s], bp.phase) : wt_wait(&bars.full_b[bp.s], bp.phase)) &&
                                           wt_wait(&bars.full_a[ap.s], ap.phase));
           if (!ok) break;
-          umma::fence_after_sync();
+          fence_after_sync();
           if (elect_one()) {
             const uint64_t db = db0 + (uint64_t)(bp.s * (W_B_STAGE >> 4));
             const uint32_t a = W_A_COL + 64u * ap.s, acc = step > 0;
             unsigned long long* tr = TRACED && job == p.trace_tile * w.n_pair && step < 16 ? p.trace : nullptr;
             if (TRACED) trace_write(tr, 96 + 64 * MODE + 2 * step);
-            if (MODE == 0) umma::fence_proxy_async();
+            if (MODE == 0) fence_proxy_async();
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               mma_f16_ta(tmem, a + 8 * k, db + 2 * k, idesc, k > 0 ? 1u : acc);
@@ -1019,7 +943,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     if (!wt_tiled(FMT)) asm volatile("cp.async.wait_all;" ::: "memory");
     if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
   }
-  umma::fence_before_sync();
+  fence_before_sync();
   __syncwarp();
   pair_sync();
   __syncwarp();
