@@ -26,7 +26,6 @@ namespace infr {
 
 namespace {
 
-constexpr int DN_MAX_WARPS = 24;
 constexpr int DN_XPITCH = 36;     // words per 128-activation chunk and limb: four neighbouring chunks start in four 16-byte bank groups
 constexpr int DN_MAX_SLOTS = 33;  // n_used ≤ 32 plus the shared expert
 
@@ -484,35 +483,6 @@ int pick_down_tile(int ne, int nff, int sh_ff, int n_used, size_t dbb, size_t li
   return 0;
 }
 
-// Warps of a down CTA.  Its time is a chain of latencies (activations read and rounded by all warps, a task of up to eight rows of a
-// slot per warp), so a CTA takes the warps that its SM's registers leave it: an SM holds 36 warps of these registers.
-//   grid of one wave: 20, which fit beside a gate/up CTA of 16 (128 experts of 768, one row: 16 warps 20.0 us the layer, 20 18.6);
-//   shared memory holds one CTA only: all 24 (7168 wide, 2048, one row: 9 warps 165 us, 24 143);
-//   past four waves: a divisor of the tasks under the cap (infr_cuda_config::dn_warps; 32 rows: 83 us with three CTAs of 12 to an SM,
-//   98 with two of 16), or the cap itself where that leaves fewer than nine (16 tasks, six rows: 8 warps 65.2 us, 12 63.5);
-//   else as many CTAs share an SM as the grid has for it and shared memory and a task per warp allow.  Q6_K: fewer where that takes no
-//   wave more and a round of tasks less.  Q4_K, whose tasks are lighter: whole rounds of tasks where there are several waves (256 experts
-//   of 512: three rows 18 warps 32.2 us, 12 30.0; Q4_K down, three rows 30.8 / 28.1, four rows 18 warps 35.2, 12 35.5, 9 32.3; two
-//   768-wide slots and a shared one, two rows 6 warps 19.9, 18 16.6).
-int pick_down_warps(int ctas, int n_tasks, size_t smem, bool q4k, int sms, int cap) {
-  const int fit = (int)((size_t)227 * 1024 / (smem + 2048));
-  if (ctas <= sms) return 20;
-  if (fit <= 1) return DN_MAX_WARPS;
-  if (ctas > 4 * sms && cap > 0) {
-    int c = std::min(cap, n_tasks);
-    while (n_tasks % c) --c;
-    return c < 9 && n_tasks > cap ? cap : c;
-  }
-  int k = std::min(std::min((ctas + sms - 1) / sms, fit), 36 / std::min(std::max(n_tasks, 6), 9));
-  auto waves = [&](int n) { return (ctas + n * sms - 1) / (n * sms); };
-  auto rounds = [&](int n) { return (n_tasks + 36 / n - 1) / (36 / n); };
-  while (!q4k && k > 2 && waves(k - 1) == waves(k) && rounds(k - 1) < rounds(k)) --k;
-  if (q4k && k > 2 && waves(k) > 1) return (n_tasks + rounds(k) - 1) / rounds(k);
-  const int nw = 36 / k;
-  if (k >= 4) return std::min(nw, std::max(n_tasks, 6));
-  return k == 2 && n_tasks >= 14 ? std::min(nw, n_tasks) : nw;
-}
-
 }  // namespace
 
 bool decode_ffn_supported(const infr_cuda_ctx*, int ne, int nff, int sh_ff, int n_used, BankTypes bt, std::string* why) {
@@ -587,10 +557,11 @@ int32_t launch_decode_ffn(infr_cuda_ctx* ctx, const DecodeParams& p, bool pdl, u
   if (!dn_own) return launch_anyfmt_decode(ctx, p, pdl, 4u);
 
   const size_t smem_dn = down_smem(TI, p.nff, sh_ff, p.n_used, dbb);
-  e = ensure_smem(reinterpret_cast<const void*>(k_decode_down), smem_dn);
-  if (e != cudaSuccess) return check_cuda(ctx, e, "k_decode_down smem attribute");
   const int ctas_dn = p.rows * (p.ne / TI), n_tasks = (p.n_used + (has_sh ? 1 : 0)) * (TI > 8 ? TI / 8 : 1);
-  const int nw = pick_down_warps(ctas_dn, n_tasks, smem_dn, p.down_q4k != 0, ctx->sm_count, (int)ctx->cfg.dn_warps);
+  int fit = 1;  // CTAs that an SM's shared memory holds
+  e = resident_ctas(reinterpret_cast<const void*>(k_decode_down), 128, smem_dn, &fit);
+  if (e != cudaSuccess) return check_cuda(ctx, e, "k_decode_down occupancy");
+  const int nw = down_warps(ctas_dn, n_tasks, fit, p.down_q4k != 0, ctx->sm_count, (int)ctx->cfg.dn_warps);
   e = launch_ex(k_decode_down, dim3(p.rows * (p.ne / TI)), dim3(nw * 32), smem_dn, ctx->stream, pdl, p, TI);
   ctx->launches += 1;
   return check_cuda(ctx, e, "k_decode_down launch");

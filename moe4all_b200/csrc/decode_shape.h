@@ -1,4 +1,4 @@
-// CTAs of the per-pair gate/up kernel (decode_ffn.cu): plain host arithmetic.
+// Shapes of the per-pair kernels' launches (decode_ffn.cu): plain host arithmetic.
 #pragma once
 #include <algorithm>
 #include <cstddef>
@@ -57,6 +57,40 @@ inline GateUpShape gateup_shape(int ne, int nff, int sh_ff, int rows, int n_used
   }
   if (!(full > 2 * sms && take(4, 2))) take(8, 2);
   return s;
+}
+
+constexpr int DN_MAX_WARPS = 24;
+
+// Warps of a down CTA.  Its time is a chain of latencies (activations read and rounded by all warps, a task of up to eight rows of a
+// slot per warp), so a CTA takes the warps that its SM's registers leave it: an SM holds 36 warps of these registers.
+// fit: CTAs that an SM's shared memory holds, as the driver has it (two of 114 KB: 2560 wide, six 1024-wide slots and a shared one, Q6_K, one /
+// three rows 33.8 / 58.4 us the layer, 38 / 66.6 where a bound with room to spare said one).
+//   grid of one wave: 20, which fit beside a gate/up CTA of 16 (128 experts of 768, one row: 16 warps 20.0 us the layer, 20 18.6);
+//   shared memory holds one CTA only: all 24 (7168 wide, 2048, one row: 9 warps 165 us, 24 143);
+//   past four waves: a divisor of the tasks under the cap (infr_cuda_config::dn_warps; 32 rows: 83 us with three CTAs of 12 to an SM,
+//   98 with two of 16), or the cap itself where that leaves fewer than nine and tasks are heavy or two CTAs fit (16 tasks of Q6_K, six rows:
+//   8 warps 65.2 us, 12 63.5; 14 tasks, two fit, eight rows 124 / 120, Q4_K 120 / 115; but of Q4_K with more to an SM 7 warps 52.3, 12 56.3);
+//   else as many CTAs share an SM as the grid has for it and shared memory and a task per warp allow, fewer where that takes no
+//   wave more and a round of tasks less (16 tasks of Q4_K, 512 CTAs: three of 8 warps 48.7, two of 16 46.9).  Q4_K, whose tasks are lighter:
+//   whole rounds of tasks where there are several waves.  256 experts of 512: three rows 18 warps 32.2 us, 12 30.0; Q4_K down, three rows
+//   30.8 / 28.1, four rows 18 warps 35.2, 12 35.5, 9 32.3; two 768-wide slots and a shared one, two rows 6 warps 19.9, 18 16.6.
+// Over 280 launches (18 layers, one to twelve rows, both formats) this is 1.4 % over the best count of warps for each, and 9 % at most.
+inline int down_warps(int ctas, int n_tasks, int fit, bool q4k, int sms, int cap) {
+  if (ctas <= sms) return 20;
+  if (fit <= 1) return DN_MAX_WARPS;
+  if (ctas > 4 * sms && cap > 0) {
+    int c = std::min(cap, n_tasks);
+    while (n_tasks % c) --c;
+    return c < 9 && n_tasks > cap && (!q4k || fit == 2) ? cap : c;
+  }
+  int k = std::min(std::min((ctas + sms - 1) / sms, fit), 36 / std::min(std::max(n_tasks, 6), 9));
+  auto waves = [&](int n) { return (ctas + n * sms - 1) / (n * sms); };
+  auto rounds = [&](int n) { return (n_tasks + 36 / n - 1) / (36 / n); };
+  while (k > 2 && waves(k - 1) == waves(k) && rounds(k - 1) < rounds(k)) --k;
+  if (q4k && k > 2 && waves(k) > 1) return (n_tasks + rounds(k) - 1) / rounds(k);
+  const int nw = 36 / k;
+  if (k >= 4) return std::min(nw, std::max(n_tasks, 6));
+  return k == 2 && n_tasks >= 14 ? std::min(nw, n_tasks) : nw;
 }
 
 }  // namespace infr
