@@ -59,6 +59,7 @@ constexpr int W_MMA_WARP = 16, W_TOK_WARP = 17;
 __host__ __device__ constexpr int wt_tok_warps(int mode) { return mode == 0 ? 4 : 1; }
 __host__ __device__ constexpr int wt_raw_warp(int mode) { return W_TOK_WARP + wt_tok_warps(mode); }
 __host__ __device__ constexpr int wt_raw_warps(int mode) { return mode == 0 ? 3 : 4; }
+
 // Q4_K, Q5_K, Q8_0 (both roles): tiled copies, rows of whole 16-byte pieces.  Q6_K (down): tiled copies of the 240 bytes around a
 // block of 210, over 2^row_shift rows at a time, whose bytes are whole 16-byte pieces.  Any: words, on an odd word pitch.
 enum WtFormat { WT_Q4K, WT_Q5K, WT_Q80, WT_Q6K, WT_ANY };
@@ -68,9 +69,13 @@ constexpr uint32_t W_Q6K_BOX = 240;  // 15 pieces of 16 bytes: 14 bytes of offse
 
 // Warps of the second CTA that pass its gate/up tokens on (relay_tokens).
 __host__ __device__ constexpr int wt_relays(int mode, int fmt) { return mode == 0 ? (wt_tiled(fmt) ? 3 : 1) : 0; }
+// Stages of the token ring.  Gate/up of Q4_K and Q5_K: as many as leave room for two raw stages, over which the hand-over's time (relay_tokens)
+// is spread (six and four of Q4_K -> ten and two: 777 tokens 176 -> 170 us the call, 4096 482 -> 474; Q5_K level); Q8_0's raw stages leave
+// room for six, and words need no more (MXFP4 840 either way).  Down: six (four 2 - 3 % slower, eight level).
+__host__ __device__ constexpr int wt_b_stages(int mode, int fmt) { return mode == 0 && (fmt == WT_Q4K || fmt == WT_Q5K) ? 10 : 6; }
+constexpr int W_MAX_B_STAGES = 10;
 constexpr uint32_t W_B_STAGE = WN / 2 * 128;   // 64 K elements of half of the tile's tokens
 constexpr uint32_t W_PATCH = 1280;             // per warp: 16 rows x 80 B (f16) or 8 rows x 144 B (f32)
-constexpr int W_B_STAGES = 6;                  // (four: the down kernel 2 - 3 % slower)
 constexpr int W_MAX_RAW = 4;
 constexpr int W_A_STAGES = 3;
 constexpr uint32_t W_A_COL = 2 * WN;           // first A column of tensor memory
@@ -85,13 +90,13 @@ __device__ __forceinline__ __half2 h2_const(uint32_t bits) { return u32_as_h2(bi
 
 // One arrival on the first CTA's barriers of ring positions i .. i + PER - 1, for what threads wrote to this CTA's shared memory: released at
 // the scope of the pair, acquired there by pair_wait.
-template <int PER>
+template <int PER, int STAGES>
 __device__ __forceinline__ void release_first(uint64_t* ring, int i) {
   asm volatile("fence.acq_rel.cluster;" ::: "memory");
 #pragma unroll
   for (int k = 0; k < PER; ++k)
     asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\tmbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [ra];\n\t}"
-                 ::"r"(smem_u32(&ring[(i + k) % W_B_STAGES])) : "memory");
+                 ::"r"(smem_u32(&ring[(i + k) % STAGES])) : "memory");
 }
 // One tiled copy into this CTA's shared memory, counted in bytes on `bar` of the pair's first CTA.
 __device__ __forceinline__ void tma_load_2d_first(void* smem_dst, const CUtensorMap* tm, int x, int y, uint64_t* bar) {
@@ -395,7 +400,7 @@ __device__ __forceinline__ void pack_y4(float a, float b, float c, float d, uint
 
 struct WtBars {
   uint64_t full_a[W_A_STAGES], empty_a[W_A_STAGES];      // A stages in tensor memory
-  uint64_t full_b[W_B_STAGES], empty_b[W_B_STAGES];      // token stages
+  uint64_t full_b[W_MAX_B_STAGES], empty_b[W_MAX_B_STAGES];  // token stages
   uint64_t full_raw[W_MAX_RAW], empty_raw[W_MAX_RAW];    // raw-block stages
   uint64_t done, drained;                                // accumulators complete / read
   uint64_t patch[4];                                     // down: the four warps of a set of tokens have their outputs in order
@@ -455,16 +460,16 @@ __device__ __forceinline__ JobBlock wt_block(int job, int n_pair, int n_blk, int
 // 220 us the call, 1024 of Q8_0 251, 64 rows of 28 MB experts of Q8_0 2220).  Three warps 177, 208, 1440; and two steps a release 177, 208,
 // 1399.  Formats that come word by word leave one warp, and their steps are longer: a release a step (48 rows of 28 MB experts of MXFP4
 // 5640 us, two steps a release 5970).
-template <int PER>
+template <int PER, int STAGES>
 __device__ __forceinline__ bool relay_tokens(WtBars& bars, int n_jobs, int steps, int first, int by) {
   int n = 0;
   for (int it = 0; wt_job(it) < n_jobs; ++it) n += steps;  // a multiple of four
   for (int i = PER * first; i < n; i += PER * by) {
     for (int k = 0; k < PER; ++k)
-      if (!__all_sync(0xFFFFFFFFu, wt_wait(&bars.full_b[(i + k) % W_B_STAGES], ((i + k) / W_B_STAGES) & 1))) return false;
+      if (!__all_sync(0xFFFFFFFFu, wt_wait(&bars.full_b[(i + k) % STAGES], ((i + k) / STAGES) & 1))) return false;
     if (elect_one()) {
       fence_proxy_async();
-      release_first<PER>(bars.full_b, i);
+      release_first<PER, STAGES>(bars.full_b, i);
     }
     __syncwarp();
   }
@@ -488,10 +493,10 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) WtBars bars;
   __shared__ uint32_t s_tmem;
-  constexpr int RAW_WARP = wt_raw_warp(MODE), RAW_WARPS = wt_raw_warps(MODE), RELAYS = wt_relays(MODE, FMT), PER = RELAYS > 1 ? 2 : 1;
+  constexpr int RAW_WARP = wt_raw_warp(MODE), RAW_WARPS = wt_raw_warps(MODE), RELAYS = wt_relays(MODE, FMT), PER = RELAYS > 1 ? 2 : 1, B_STAGES = wt_b_stages(MODE, FMT);
   const GroupedParams& p = w.g;
   unsigned char* b_ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  unsigned char* raw_ring = b_ring + W_B_STAGES * W_B_STAGE;
+  unsigned char* raw_ring = b_ring + B_STAGES * W_B_STAGE;
   unsigned char* patches = raw_ring + (size_t)w.rb * w.raw_stage;
   // (shuffles and votes mark what is the same in the whole warp: the MMA operands then stay in uniform registers)
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
@@ -511,7 +516,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       mbar_init(&bars.full_a[s], 16);
       mbar_init(&bars.empty_a[s], 1);
     }
-    for (int s = 0; s < W_B_STAGES; ++s) {
+    for (int s = 0; s < B_STAGES; ++s) {
       mbar_init(&bars.full_b[s], MODE == 1 ? 1 : rank == 0 ? 65 : 64);
       mbar_init(&bars.empty_b[s], 1);
     }
@@ -755,10 +760,10 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
     // ---- MMA issue: the first CTA's warp waits, one elected lane issues for both; the second's passes on that its tokens are there ----
     RingPos bp, ap;
     if (rank != 0) {
-      if (MODE == 0) ok = ok && relay_tokens<PER>(bars, n_jobs, 4 * kb, 0, RELAYS);
+      if (MODE == 0) ok = ok && relay_tokens<PER, B_STAGES>(bars, n_jobs, 4 * kb, 0, RELAYS);
       for (int it = 0; ok && wt_job(it) < n_jobs; ++it)
         for (int step = 0; step < 4 * kb; ++step) {
-          bp.next(W_B_STAGES);
+          bp.next(B_STAGES);
           ap.next(W_A_STAGES);
         }
     } else {
@@ -794,13 +799,13 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
             if (TRACED) trace_write(tr, 97 + 64 * MODE + 2 * step);
           }
           __syncwarp();
-          bp.next(W_B_STAGES);
+          bp.next(B_STAGES);
           ap.next(W_A_STAGES);
         }
       }
     }
     // every commit that this CTA was promised has arrived before either leaves
-    for (int i = 0; i < W_B_STAGES && ok; ++i, bp.next(W_B_STAGES)) ok = wt_wait(&bars.empty_b[bp.s], bp.phase ^ 1);
+    for (int i = 0; i < B_STAGES && ok; ++i, bp.next(B_STAGES)) ok = wt_wait(&bars.empty_b[bp.s], bp.phase ^ 1);
     for (int i = 0; i < W_A_STAGES && ok; ++i, ap.next(W_A_STAGES)) ok = wt_wait(&bars.empty_a[ap.s], ap.phase ^ 1);
     if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
   } else if (warp < RAW_WARP) {
@@ -820,7 +825,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           if (rank == 0 && lane == 0) mbar_arrive_expect_tx(&bars.full_b[bp.s], (uint32_t)half * 2 * 16 * 128);
           if (lane < half) tma_load_2d_first(b_ring + (size_t)bp.s * W_B_STAGE + lane * 2048, &tm_act, 0, y0 + step * rows_valid, &bars.full_b[bp.s]);
           __syncwarp();
-          bp.next(W_B_STAGES);
+          bp.next(B_STAGES);
         }
       }
     } else {
@@ -831,7 +836,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
       const uint32_t dst0 = smem_u32(b_ring) + (uint32_t)r8 * 128u + (uint32_t)((c ^ r8) << 4);
       const uint4* tok = reinterpret_cast<const uint4*>(p.xg) + c;
       const int n_sorted = __ldcg(w.seg_off + w.n_seg_routed);
-      if (tw & 2) bp.next(W_B_STAGES);
+      if (tw & 2) bp.next(B_STAGES);
       for (int it = 0; ok; ++it) {
         const int job = wt_job(it);
         if (job >= n_jobs) break;
@@ -854,15 +859,15 @@ __global__ void __launch_bounds__(W_THREADS, 1) k_wt_gemm(const __grid_constant_
           for (int i = 0; i < WN / 16; ++i)
             if (i < ni) cp_async16(dst + i * 1024, ts + src[i]);
           cp_async_arrive(&bars.full_b[bp.s]);
-          bp.next(W_B_STAGES);
-          bp.next(W_B_STAGES);
+          bp.next(B_STAGES);
+          bp.next(B_STAGES);
         }
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
     }
     if (!ok && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
   } else if (RELAYS > 1 && warp > RAW_WARP) {
-    if (rank != 0 && ok && !relay_tokens<PER>(bars, n_jobs, 4 * kb, warp - RAW_WARP, RELAYS) && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
+    if (rank != 0 && ok && !relay_tokens<PER, B_STAGES>(bars, n_jobs, 4 * kb, warp - RAW_WARP, RELAYS) && lane == 0) atomicExch(&p.status->timeout, 5 + MODE);
   } else if (warp < RAW_WARP + RAW_WARPS) {
     // ---- raw blocks ----
     RingPos rp;
@@ -984,10 +989,11 @@ template <int MODE, int FMT>
 int32_t launch_wt(infr_cuda_ctx* ctx, WtParams w, const CUtensorMap (&tm)[5], int max_tiles) {
   // the token stages, and as many raw stages as fit beside them, two at least
   const size_t patches = (size_t)(W_PRODUCERS / 32) * W_PATCH;
-  const size_t room = 227 * 1024 - 1024 - 1024 - patches - W_B_STAGES * W_B_STAGE;  // alignment slack, static shared memory
+  constexpr uint32_t b_ring = wt_b_stages(MODE, FMT) * W_B_STAGE;
+  const size_t room = 227 * 1024 - 1024 - 1024 - patches - b_ring;  // alignment slack, static shared memory
   w.rb = (int)std::min<size_t>(W_MAX_RAW, room / w.raw_stage);
   if (w.rb < 2) return fail(ctx, INFR_CUDA_ERR_UNSUPPORTED, "grouped GEMM: blocks too large for the raw ring");
-  const size_t smem = 1024 + W_B_STAGES * W_B_STAGE + (size_t)w.rb * w.raw_stage + patches;
+  const size_t smem = 1024 + b_ring + (size_t)w.rb * w.raw_stage + patches;
   constexpr bool MAY_BE_ODD = MODE == 1;  // gate/up: blocks of 128 features, of 256 k
   const bool odd = w.n_blk & 1;
   auto kern = w.g.trace != nullptr ? (odd ? k_wt_gemm<MODE, FMT, true, MAY_BE_ODD> : k_wt_gemm<MODE, FMT, true, false>)
