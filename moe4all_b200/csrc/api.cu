@@ -668,13 +668,13 @@ int32_t validate_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d, ui
 
 // Which kernels serve a call of `rows` rows: pp = one CTA per pair, em = expert-major integer tensor-core tiles, gg = grouped
 // GEMM on tcgen05.  us per layer on B200, 256 experts top-8 and the shared one (2 MB: 2048 wide, 512; 28 MB: 7168 wide, 2048):
-//   em / gg   2 MB, Q6_K down:  64 rows 137 / 191, 192: 197 / 201, 256: 237 / 204, 352: 301 / 209
-//             2 MB, Q4_K down:  64 rows 121 / 178, 128: 150 / 193, 192: 173 / 194, 256: 208 / 196
-//             28 MB, Q6_K down: 64 rows 1448 / 1745, 128: 1862 / 2012, 192: 2309 / 2085, 256: 2874 / 2053
-//             28 MB, Q4_K down: 8 rows 397 / 496, 64: 1392 / 1537, 128: 1781 / 1828, 192: 2166 / 1872, 256: 2674 / 1930
-//   pp / gg   2 MB, Q5_K / Q6_K: 16 rows 109 / 133, 32: 192 / 185, 64: 354 / 241
-//             2 MB, Q8_0: 2 rows 49 / 48, 8: 131 / 94, 64: 813 / 192;  MXFP4: 16 rows 309 / 372, 32: 579 / 578, 64: 1119 / 736
-//             28 MB: 4 rows of Q8_0 1229 / 340, of Q5_K / Q6_K 473 / 372, of MXFP4 1661 / 1458
+//   em / gg   2 MB, Q6_K down:  64 rows 135 / 188, 192: 198 / 203, 256: 236 / 205, 352: 302 / 212
+//             2 MB, Q4_K down:  64 rows 120 / 181, 128: 150 / 194, 192: 176 / 195, 256: 208 / 197
+//             28 MB, Q6_K down: 64 rows 1443 / 1798, 128: 1867 / 2088, 192: 2350 / 2145, 256: 2857 / 2219
+//             28 MB, Q4_K down: 8 rows 397 / 498, 64: 1420 / 1646, 128: 1808 / 1944, 192: 2170 / 1992, 256: 2697 / 2152
+//   pp / gg   2 MB, Q5_K / Q6_K: 16 rows 109 / 135, 32: 192 / 187, 64: 354 / 237
+//             2 MB, Q8_0: 2 rows 49 / 48, 8: 130 / 95, 64: 813 / 200;  MXFP4: 16 rows 308 / 387, 32: 580 / 584, 64: 1119 / 750
+//             28 MB: 4 rows of Q8_0 1226 / 335, of Q5_K / Q6_K 471 / 371, of MXFP4 1661 / 1411
 // The lines below were drawn on earlier kernels: eleven pairs per expert between em and gg, 2.75 rows per expert (8 rows of
 // large ones) between pp and gg.  On today's, em and gg cross at six pairs per expert (four to five for
 // large experts), pp and gg between 0.1 rows per expert (Q8_0) and one (Q5_K, MXFP4).
@@ -683,13 +683,12 @@ int32_t validate_moe_ffn(infr_cuda_ctx* ctx, const infr_cuda_moe_ffn_desc* d, ui
 // weights; for experts so small that it never does, two pairs per expert.  The expert-major kernels round activations per row and
 // not per 128 as the per-pair ones (up to 1.2 times the error with Q6_K down banks, 1.05 with Q4_K), so the line is not drawn
 // where the times cross but behind it.  pp / em around the line, us per layer, Q6_K down and (Q4_K down):
-//   2048 wide, 256 of 512, top-8, shared: 8 rows 58 / 62 (53 / 56), 9 rows 64 / 60 (59 / 56), 13 rows 83 / 71 (76 / 65),
-//     15 rows 92 / 75 (86 / 68): the line is at 15
-//   2048 wide, 128 of 768, top-8: 7 rows 65 / 62 (55 / 54), 8 rows 71 / 67 (61 / 59), 9 rows 80 / 68 (69 / 64): at 9
-//   (the next three before the two forms' latest gains)
-//   2048 wide, 64 of 1024, top-8: 4 rows 56.8 / 51.0 (44.0 / 47.0), 5 rows 76.5 / 61.3 (60.4 / 59.0): at 5
-//   4096 wide, 96 of 1536, top-4: 5 rows 98.3 / 92.3 (86.5 / 80.9), 6 rows 113 / 97 (101 / 87), 8 rows 142 / 115 (128 / 105): at 8
-//   1024 wide, 32 of 256, top-4: 12 rows 26.1 / 25.6 (24.5 / 25.4), 16 rows 28.5 / 26.4 (27.6 / 25.8): at 16;  28 MB experts: 2 rows 236 / 135
+//   2048 wide, 256 of 512, top-8, shared: 8 rows 59 / 62 (55 / 57), 9 rows 65 / 61 (59 / 57), 13 rows 83 / 72 (77 / 66),
+//     15 rows 93 / 79 (86 / 71): the line is at 15
+//   2048 wide, 128 of 768, top-8: 7 rows 65 / 62 (58 / 56), 8 rows 72 / 66 (63 / 59), 9 rows 81 / 70 (71 / 64): at 9
+//   2048 wide, 64 of 1024, top-8: 4 rows 55 / 51 (45 / 46), 5 rows 66 / 59 (58 / 52): at 5
+//   4096 wide, 96 of 1536, top-4: 5 rows 93 / 82 (81 / 74), 6 rows 106 / 88 (93 / 80), 8 rows 132 / 106 (119 / 96): at 8
+//   1024 wide, 32 of 256, top-4: 12 rows 25.5 / 25.4 (24.3 / 25.2), 16 rows 27.7 / 26.4 (26.8 / 25.8): at 16;  28 MB experts: 2 rows 237 / 134 (190 / 134)
 bool em_preferred(uint32_t rows, uint32_t n_used, uint32_t n_expert, uint32_t ne, uint32_t nff) {
   const uint64_t size = (uint64_t)ne * nff, pairs = (uint64_t)rows * n_used;
   if (size >= (1ull << 23)) return rows >= 2;  // experts of tens of megabytes

@@ -470,7 +470,7 @@ size_t down_smem(int TI, int nff, int sh_ff, int n_used, size_t dbb) {
 
 // TI rows per CTA: bulk copies need TI * row_bytes to be a multiple of 16 for both banks.
 // `limit`: bytes of shared memory.  Which shapes these kernels take is decided at 200 KB; a shape that they take has the largest tile
-// that an SM holds (16 rows of nine 1536-wide Q6_K slots in 217 KB, one row of 2560: 54.8 -> 43.7 us the layer).
+// that an SM holds (16 rows of nine 1536-wide Q6_K slots in 217 KB, one row of 2560: 52.6 -> 41.0 us the layer).
 constexpr size_t DN_SMEM_TAKEN = 200 * 1024, DN_SMEM_MOST = 225 * 1024;
 int pick_down_tile(int ne, int nff, int sh_ff, int n_used, size_t dbb, size_t limit = DN_SMEM_TAKEN) {
   const int cands[] = {16, 8, 4};

@@ -64,9 +64,9 @@ constexpr int DN_MAX_WARPS = 24;
 // Warps of a down CTA.  Its time is a chain of latencies (activations read and rounded by all warps, a task of up to eight rows of a
 // slot per warp), so a CTA takes the warps that its SM's registers leave it: an SM holds 36 warps of these registers.
 // fit: CTAs that an SM's shared memory holds, as the driver has it (two of 114 KB: 2560 wide, six 1024-wide slots and a shared one, Q6_K, one /
-// three rows 33.8 / 58.4 us the layer, 38 / 66.6 where a bound with room to spare said one).
+// three rows 24.8 / 47.5 us the layer, 29.0 / 56.1 where a bound with room to spare said one).
 //   grid of one wave: 20, which fit beside a gate/up CTA of 16 (128 experts of 768, one row: 16 warps 20.0 us the layer, 20 18.6);
-//   shared memory holds one CTA only: all 24 (7168 wide, 2048, one row: 9 warps 165 us, 24 143);
+//   shared memory holds one CTA only: all 24 (7168 wide, 2048, one row: 9 warps 158 us, 24 132);
 //   past four waves: a divisor of the tasks under the cap (infr_cuda_config::dn_warps; 32 rows: 83 us with three CTAs of 12 to an SM,
 //   98 with two of 16), or the cap itself where that leaves fewer than nine and tasks are heavy or two CTAs fit (16 tasks of Q6_K, six rows:
 //   8 warps 65.2 us, 12 63.5; 14 tasks, two fit, eight rows 124 / 120, Q4_K 120 / 115; but of Q4_K with more to an SM 7 warps 52.3, 12 56.3);

@@ -16,11 +16,13 @@
 //
 // One persistent pair of CTAs per two SMs walks the jobs (tile, 2 x 256 weight rows, 256 of them in each CTA), tiles listed
 // heaviest first and dealt out in a snake.  The MMAs are the pair's (cta_group::2, M 256): each CTA unpacks its own rows into its
-// own tensor memory and brings half of the tile's tokens, and the tensor cores read both halves.  What it gives (us, gate/up /
-// down, one CTA by itself -> pairs): 777 tokens 58 / 56 -> 54 / 52, 4096 177 / 141 -> 150 / 133, 1024 of Q8_0 82 / 76 -> 74 / 69,
-// 8192 of 28 MB experts 4150 / 2470 -> 3610 / 2320.  Two things were in the way: the 16-byte asynchronous copies of the gathered
+// own tensor memory and brings half of the tile's tokens, and the tensor cores read both halves.  What it gives, with the Q6_K copies below
+// (us cold and serialised, gate/up / down, one CTA by itself -> now): 777 tokens 60.5 / 58.8 -> 55.2 / 43.6, 4096 191 / 181 -> 164 / 139,
+// 8192 of 28 MB experts 4058 / 3406 -> 3870 / 2346.  Two things were in the way: the 16-byte asynchronous copies of the gathered
 // tokens (all their writes, not their latency: 20 KB a step, one copy instead of twenty a lane 177 -> 151; in a pair it is 10),
 // and the MMAs, which take 640 cycles of eight at 160 tokens in pairs and 740 - 790 in one CTA with a wait for a stage between them.
+// What it costs: 0.8 us a kernel (the cluster's two barriers, the paired allocation) and 500 - 1500 cycles a job, so calls of light tiles
+// alone whose banks have no other gain are slower (4 - 64 rows of Q8_0 or Q4_K down banks 2 - 4 %, 256-wide experts 3 us of 53).
 // Warp roles (24 warps of each CTA):
 //   0-15   producers, two groups of eight on alternate K steps; afterwards they drain the accumulators
 //   16     first CTA: issues the MMAs (one elected lane); second, gate/up: passes on that its tokens are there
@@ -30,9 +32,10 @@
 //   last   raw-block loaders: 256 weights of 256 rows at a time, into a ring: Q4_K, Q5_K, Q8_0 and the down banks' Q6_K by
 //          tiled copies, which one warp requests (gate/up: two more pass tokens on), other formats word by word with cp.async
 //          (rows on an odd word pitch, free of bank conflicts)
-// All rings run on across jobs; every wait is bounded.
+// All rings run on across jobs; every wait on a barrier of shared memory is bounded (the cluster's two barriers and the paired allocation
+// have no limit of their own: nothing that either CTA does ahead of them waits for long).
 //
-// Reading out a full tile of the down kernel takes 4800 cycles beside the 8800 of its K loop at 512 inputs, with the tensor cores
+// Reading out a full tile of the down kernel takes 5100 cycles beside the 7700 of its K loop at 512 inputs, with the tensor cores
 // idle: there is one set of accumulators.
 // Down with Q6_K, whose blocks are 210 bytes: as words by cp.async the copies were what everything waited for (without them 3704 ->
 // 2104 us, 8192 tokens of 28 MB experts).  Now a tiled copy brings the 240 bytes around a block, of one row in every 1, 2, 4 or 8

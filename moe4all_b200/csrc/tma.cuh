@@ -1,5 +1,5 @@
-// Tiled TMA copies (cp.async.bulk.tensor, never multicast) over the Q4_K expert banks: a bank is a 2-D byte
-// tensor [rows][row bytes]; a box is one 144-byte block of a run of consecutive rows, which lands in shared
+// Tiled TMA copies (cp.async.bulk.tensor, never multicast): the copy itself, the driver's tensor-map encoder, and the map of a Q4_K expert
+// bank as a 2-D byte tensor [rows][row bytes], whose box is one 144-byte block of a run of consecutive rows, which lands in shared
 // memory at a 144-byte pitch (36 words: eight rows x four consecutive words hit 32 different banks).
 #pragma once
 #include <cuda.h>
@@ -17,7 +17,6 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* t
       "l"(reinterpret_cast<uint64_t>(tm)), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
-
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
